@@ -542,56 +542,18 @@ int nwg_score_pairs(nwg_ctx* ctx, const int8_t* codes, const int64_t* offsets, i
   c->recs.clear();
   for (int64_t k = 0; k < npairs; ++k)
     if (pi[k] < 0 || pi[k] >= n || pj[k] < 0 || pj[k] >= n) return c->fail(NWG_ERR_INVALID, "pair index");
-  int maxlen = 0;
-  for (int s = 0; s < n; ++s) {
-    const int64_t L = offsets[s + 1] - offsets[s];
-    if (L <= 0) return c->fail(NWG_ERR_EMPTY_SEQ, "zero-length sequence");
-    maxlen = std::max<int>(maxlen, (int)L);
-  }
+  for (int s = 0; s < n; ++s)
+    if (offsets[s + 1] <= offsets[s]) return c->fail(NWG_ERR_EMPTY_SEQ, "zero-length sequence");
   if (npairs == 0) return NWG_OK;
-  const int64_t total = offsets[n];
-  std::vector<int32_t> len(n);
-  for (int s = 0; s < n; ++s) len[s] = (int32_t)(offsets[s + 1] - offsets[s]);
-  int rc;
-  const int64_t kMax = (int64_t)c->sms * 512;
-  if ((rc = c->b_codes.ensure((size_t)total)) || (rc = c->b_start.ensure(sizeof(int64_t) * n)) ||
-      (rc = c->b_len.ensure(sizeof(int32_t) * n)) || (rc = c->b_pi.ensure(sizeof(int32_t) * npairs)) ||
-      (rc = c->b_pj.ensure(sizeof(int32_t) * npairs)) || (rc = c->b_out.ensure(sizeof(int32_t) * npairs)) ||
-      (rc = c->b_pscratch.ensure(sizeof(int2) * (size_t)kMax * maxlen)))
-    return c->fail(rc, "pair-list allocation");
-  cudaStream_t s = c->stream;
-  if ((rc = c->cuda(cudaMemcpyAsync(c->b_codes.p, codes, (size_t)total, cudaMemcpyHostToDevice, s), "upload")) ||
-      (rc = c->cuda(cudaMemcpyAsync(c->b_start.p, offsets, sizeof(int64_t) * n, cudaMemcpyHostToDevice, s), "upload")) ||
-      (rc = c->cuda(cudaMemcpyAsync(c->b_len.p, len.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, s), "upload")) ||
-      (rc = c->cuda(cudaMemcpyAsync(c->b_pi.p, pi, sizeof(int32_t) * npairs, cudaMemcpyHostToDevice, s), "upload")) ||
-      (rc = c->cuda(cudaMemcpyAsync(c->b_pj.p, pj, sizeof(int32_t) * npairs, cudaMemcpyHostToDevice, s), "upload")))
-    return rc;
-  // validate codes on the host side of the copy
-  for (int64_t k = 0; k < total; ++k)
+  for (int64_t k = 0; k < offsets[n]; ++k)
     if ((unsigned)codes[k] >= (unsigned)nwg::kLetters) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
-  nwg::PairListArgs a{};
-  a.codes = (const int8_t*)c->b_codes.p;
-  a.start = (const int64_t*)c->b_start.p;
-  a.len = (const int32_t*)c->b_len.p;
-  a.pi = (const int32_t*)c->b_pi.p;
-  a.pj = (const int32_t*)c->b_pj.p;
-  a.out = (int32_t*)c->b_out.p;
-  a.scratch = (int2*)c->b_pscratch.p;
-  a.npairs = npairs;
-  a.go = c->go;
-  a.ge = c->ge;
-  a.sub = (const int8_t*)c->b_sub.p;
-  for (int64_t b = 0; b < npairs; b += kMax) {
-    a.base = b;
-    if ((rc = c->cuda(nwg::launch_pairlist(a, std::min(kMax, npairs - b), s), "pair-list launch"))) return rc;
-    ++c->launches;
-  }
-  if ((rc = c->cuda(cudaMemcpyAsync(out, c->b_out.p, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, s), "download")) ||
-      (rc = c->cuda(cudaStreamSynchronize(s), "pair-list sync")))
-    return rc;
+  int64_t pairs16 = 0;
+  const int rc = c->score_pairs(codes, offsets, n, pi, pj, npairs, out, &pairs16);
+  if (rc) return rc;
   if (stats) {
     stats->pairs = npairs;
-    stats->pairs_int32 = npairs;
+    stats->pairs_int16 = pairs16;
+    stats->pairs_int32 = npairs - pairs16;
     stats->launches = c->launches;
     stats->total_ms = nwg::now_ms() - t0;
   }

@@ -126,20 +126,6 @@ struct PlainArgs {
   const int8_t* sub;
 };
 
-struct PairListArgs {
-  const int8_t* codes;
-  const int64_t* start;
-  const int32_t* len;
-  const int32_t* pi;
-  const int32_t* pj;
-  int32_t* out;
-  int2* scratch;              // [column][thread]
-  int64_t npairs;
-  int64_t base;               // first pair of this launch
-  int go, ge;
-  const int8_t* sub;
-};
-
 // Launchers (score_kernels.cu, wave_r*.cu).  R is the rows per lane; P = 2
 // for int16x2 lanes (two pairs per warp), 1 for int32 lanes.
 // V: register layout of the wave kernel (0: H, H-go, E per row; 1: H, E per
@@ -174,6 +160,5 @@ int nj_cluster_size();
 constexpr int kServeMaxN = 8192;   // largest job of the serving loop (neighbor joining on the device)
 cudaError_t launch_dpx_peak(int P, int form, int cols, int grid, uint32_t* sink, int go, int ge, cudaStream_t s);
 int dpx_peak_ctas_per_sm(int P, int form);
-cudaError_t launch_pairlist(const PairListArgs& a, int64_t count, cudaStream_t s);
 
 }  // namespace nwg

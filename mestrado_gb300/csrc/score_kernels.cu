@@ -16,7 +16,6 @@
 //    global scratch, one launch per length group.  It is the baseline the
 //    batched form is measured against.
 //  * rerun_kernel: int32 re-run of the pairs the int16 overflow guard queued.
-//  * pairlist_kernel: explicit pair lists.
 //  * dpx_peak_kernel: the roofline denominator (cell update only).
 #include "wave_impl.cuh"
 
@@ -70,18 +69,6 @@ __global__ void __launch_bounds__(kPlainThreads) rerun_kernel(const WaveArgs a, 
                                a.go, a.ge, s_sub, scratch + t, nthreads);
     put_score(a, a.xorig[q.x], a.yorig[q.y], v);
   }
-}
-
-__global__ void __launch_bounds__(kPlainThreads) pairlist_kernel(const PairListArgs a, int64_t count) {
-  __shared__ int8_t s_sub[kLetters * kLetters];
-  for (int e = threadIdx.x; e < kLetters * kLetters; e += blockDim.x) s_sub[e] = a.sub[e];
-  __syncthreads();
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const int64_t k = a.base + t;
-  const int i = a.pi[k], j = a.pj[k];
-  a.out[k] = score_thread(a.codes + a.start[i], a.len[i], a.codes + a.start[j], a.len[j], a.go,
-                          a.ge, s_sub, a.scratch + t, count);
 }
 
 // Peak of the cell update alone (roofline denominator): the inner loop of
@@ -268,12 +255,6 @@ cudaError_t launch_rerun(const WaveArgs& a, int2* scratch, int64_t nthreads, cud
 cudaError_t launch_plain(const PlainArgs& a, cudaStream_t s) {
   const int64_t blocks = (a.nthreads + kPlainThreads - 1) / kPlainThreads;
   plain_kernel<<<(unsigned)blocks, kPlainThreads, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_pairlist(const PairListArgs& a, int64_t count, cudaStream_t s) {
-  const int64_t blocks = (count + kPlainThreads - 1) / kPlainThreads;
-  pairlist_kernel<<<(unsigned)blocks, kPlainThreads, 0, s>>>(a, count);
   return cudaGetLastError();
 }
 

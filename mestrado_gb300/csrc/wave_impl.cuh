@@ -117,8 +117,8 @@ __device__ __forceinline__ unsigned clamp_code(int c) {
 
 // One pair per thread, int32, 16-row register strip; the (H, F) row between
 // strips lives in global scratch, one int2 per X column at stride `stride`
-// (consecutive threads adjacent: coalesced).  Used by the plain, re-run and
-// pair-list kernels and by the allocation-free entry point.  Same loop structure as
+// (consecutive threads adjacent: coalesced).  Used by the plain and re-run
+// kernels and by the allocation-free entry point.  Same loop structure as
 // NeedlemanWunschGlobalScoreKernel with its 12-row strips widened to 16.
 __device__ __forceinline__ int score_thread(const int8_t* __restrict__ X, int Lx,
                                             const int8_t* __restrict__ Y, int Ly, int go, int ge,
