@@ -28,7 +28,7 @@
 #include <vector>
 
 #include "nwg_ctx.h"
-#include "walk.cuh"
+#include "pipe.cuh"
 
 namespace nwg {
 namespace {
@@ -41,13 +41,11 @@ struct MergeDesc {
   int64_t nib;                // first flag byte
   int64_t src;                // first entry of the alignment's columns (capacity lx + ly)
   int64_t scratch;            // 64-bit form: first (H, F) pair of the strip-boundary scratch (lx entries)
-  int64_t score;              // wave form: first int4 of the cell scores
+  int64_t score;              // wave form: first int of the cell scores
   int64_t bnd;                // wave form: first entry of the band-boundary row (lx entries)
   int32_t lx, ly, kx, ky;
-  int32_t nsup;               // wave form: supersteps of a band
   int32_t tile0;              // wave form: first CTA of the score kernel
   int32_t mac32;              // kx * ky * max|S| < 2^31: a cell's score sum fits int32
-  int32_t pad;
 };
 
 __device__ __forceinline__ int64_t mx64(int64_t a, int64_t b) { return a > b ? a : b; }
@@ -221,52 +219,36 @@ __global__ void __launch_bounds__(kMR) msa_dp_kernel(const MergeDesc* md, const 
 }
 
 // ---- the wave form ------------------------------------------------------------
-// Every value of the recurrence is held relative to a neighbouring cell, in 32
-// bits: with u(r,c) = H(r,c) - H(r-1,c), v(r,c) = H(r,c) - H(r,c-1),
-// a = F - H and b = E - H of a cell, and H(r-1,c-1) as the zero,
-//   F = v(r-1,c) + max(a(r-1,c) - GE, -GO),   E = u(r,c-1) + max(b(r,c-1) - GE, -GO),
-//   H = max(E, F, S),  u = H - v(r-1,c),  v = H - u(r,c-1)
-// -- the same comparisons, so the same flags.  With GO >= GE every one of
-// these lies within k * (max S + |min S| + 4 go), k = kX * kY: u, v >= -GO from
-// H >= F >= Hup - GO (and likewise E); u <= max S + GO, since a diagonal step
-// gives u = S - v(r-1,c), an F step u <= 0, and an E step no more than the cell
-// where its gap opened; the others follow.  The host takes this form while that
-// bound stays below 2^30 (a set of 8,000 sequences under the usual penalties).
-//
-// A band is 128 rows, four per lane of a warp, lane l a column behind lane
-// l - 1; v and a of a lane's bottom row go to the next lane by shuffle, of a
-// band's bottom row to the next warp through a ring in shared memory (to the
-// first warp, for more bands than warps, through a row in global memory).  The
-// CTA's warps work on consecutive bands kLag supersteps of kStep columns
-// apart, one CTA barrier per superstep.  A tree's deep levels hold one or two
-// merges, so a level costs one merge's chain of steps: 0.21 ms for 560 columns
-// x 560 rows of 8,000 sequences (0.43 ms at 339 columns with 64-bit cells, one
-// row per thread and a barrier per anti-diagonal).  The whole alignment of
-// 8,000 sequences of 100-300 residues: 22.1 to 10.2 ms.
-constexpr int kWRows = 4;                  // rows per lane
-constexpr int kWBand = 32 * kWRows;        // rows per band
-constexpr int kStep = 8;                   // columns per superstep
-constexpr int kLag = 5;                    // supersteps between the bands of consecutive warps: the
-                                           // last lane is 31 columns behind the first
-constexpr int kWMax = 8;                   // warps per CTA, at most
-constexpr int kRing = 64;                  // ring columns: the 8 being read to the 8 being written span 40
+// The pipeline of pipe.cuh in 32 bits: its values lie within
+// kX kY (2 max|S| + 4 go), and the host takes this form while that stays
+// below 2^31 (a set of 8,000 sequences under the usual penalties).  A tree's
+// deep levels hold one or two merges, so such a level costs one merge's chain
+// of steps.  Four rows per lane: two give a shorter step but more hops between
+// bands and more instructions a cell, and measured the same on a deep level.
+// A level of one merge of 560 columns x 560 rows takes 82 us, of which the walk
+// 10 (207 us with one CTA barrier per eight steps on a single SM and the scores
+// in registers; 0.43 ms at 339 columns with 64-bit cells, one row per thread
+// and a barrier per anti-diagonal).
 constexpr int kScoreSteps = 16;            // steps per warp of the score kernel
 constexpr int kScoreWarps = 8;
-constexpr int kWinSteps = 16;              // supersteps of flags in the walk's window
-constexpr int kDiffSent = -(1 << 30);      // a and b of the cells above row 0 and left of column 0
+constexpr int kMsaWindow = 8192;           // bytes of flags in the walk's window
 
-// Scores of the cells of a level's merges in the wave kernel's order: int4
-// (g * nsup * 8 + t) * 32 + l of a merge holds rows 128 g + 4 l .. + 3 at
-// column t - l (0 outside).  One CTA per 128 rows x 128 steps: the rows' scores
+constexpr int kRows = 4;                   // rows per lane of the pipeline
+
+// Scores of the cells of a level's merges in the wave kernel's order: entry
+// (g * nsup * 8 + t) * 32 + l of a merge holds rows 128 g + 4 l .. + 3 at column
+// t - l (2 GE outside).  One CTA per 128 rows x 128 steps: the rows' scores
 // against each letter, W[x] = sum_y cY[y] S[y][x], go to shared memory once,
 // then each warp runs 16 steps with its lanes' 4 x 24 of them in registers:
 // 96 multiply-adds for three 16-byte loads of column counts.
 __global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const MergeDesc* __restrict__ md, int nm,
                                                                     const int16_t* __restrict__ cnt,
-                                                                    const int8_t* __restrict__ sub,
-                                                                    int4* __restrict__ score) {
+                                                                    const int8_t* __restrict__ sub, int ge,
+                                                                    int* __restrict__ score) {
+  constexpr int R = kRows, kBand = 32 * R;
+  constexpr int kPer = kLetters * R / 8;   // letters per thread of the row scores: two threads a row
   __shared__ int8_t s_sub[kLetters * kLetters];
-  __shared__ int s_w[kLetters][kWBand];
+  __shared__ __align__(16) int s_w[kLetters][kBand];
   int lo = 0, hi = nm - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -274,40 +256,44 @@ __global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const Merge
     else hi = mid - 1;
   }
   const MergeDesc m = md[lo];
-  const int nchunk = (m.nsup * kStep + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps);
+  const int steps = pipe::supersteps_of(m.lx) * pipe::kStep;
+  const int nchunk = (steps + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps);
   const int tile = (int)blockIdx.x - m.tile0;
   const int g = tile / nchunk, chunk = tile - g * nchunk;
   for (int e = threadIdx.x; e < kLetters * kLetters; e += blockDim.x) s_sub[e] = sub[e];
   __syncthreads();
   {
-    // two threads per row, twelve letters each
-    const int row = threadIdx.x % kWBand, x0 = (threadIdx.x / kWBand) * 12;
-    int w[12];
+    const int row = threadIdx.x % kBand, x0 = (threadIdx.x / kBand) * kPer;
+    int w[kPer];
 #pragma unroll
-    for (int x = 0; x < 12; ++x) w[x] = 0;
-    const int r = g * kWBand + row;
+    for (int x = 0; x < kPer; ++x) w[x] = 0;
+    const int r = g * kBand + row;
     if (r < m.ly) {
       const int16_t* cy = cnt + (m.yoff + r) * kLetters;
       for (int b = 0; b < kLetters; ++b) {
         const int c = cy[b];
         if (c == 0) continue;
 #pragma unroll
-        for (int x = 0; x < 12; ++x) w[x] += c * (int)s_sub[b * kLetters + x0 + x];
+        for (int x = 0; x < kPer; ++x) w[x] += c * (int)s_sub[b * kLetters + x0 + x];
       }
     }
 #pragma unroll
-    for (int x = 0; x < 12; ++x) s_w[x0 + x][row] = w[x];
+    for (int x = 0; x < kPer; ++x) s_w[x0 + x][row] = w[x];
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = (chunk * kScoreWarps + warp) * kScoreSteps;
-  const int t1 = min(t0 + kScoreSteps, m.nsup * kStep);
+  const int t1 = min(t0 + kScoreSteps, steps);
   if (t0 >= t1) return;
-  int4 W[kLetters];
+  int W[kLetters][R];
 #pragma unroll
-  for (int x = 0; x < kLetters; ++x) W[x] = *reinterpret_cast<const int4*>(&s_w[x][kWRows * lane]);
+  for (int x = 0; x < kLetters; ++x) {
+    const int4 w = *reinterpret_cast<const int4*>(&s_w[x][R * lane]);
+    W[x][0] = w.x, W[x][1] = w.y, W[x][2] = w.z, W[x][3] = w.w;
+  }
   const uint4* X = reinterpret_cast<const uint4*>(cnt + m.xoff * kLetters);   // 48 bytes a column
-  int4* out = score + m.score + ((int64_t)g * m.nsup * kStep + t0) * 32 + lane;
+  int4* out = reinterpret_cast<int4*>(score + m.score) + ((int64_t)g * steps + t0) * 32 + lane;
+  const int base = 2 * ge * m.kx * m.ky;   // the pipeline's S' = S + 2 GE
   uint4 nxt[3] = {};
   auto load = [&](int t) {
     const int c = t - lane;
@@ -319,175 +305,104 @@ __global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const Merge
   for (int t = t0; t < t1; ++t) {
     const uint4 cur[3] = {nxt[0], nxt[1], nxt[2]};
     if (t + 1 < t1) load(t + 1);
-    int4 s = make_int4(0, 0, 0, 0);
+    int s[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) s[r] = base;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       const uint32_t w[4] = {cur[q].x, cur[q].y, cur[q].z, cur[q].w};
 #pragma unroll
       for (int h = 0; h < 8; ++h) {
         const int n = (h & 1) ? (int)w[h >> 1] >> 16 : (int)(int16_t)(w[h >> 1] & 0xFFFFu);
-        const int4 k = W[q * 8 + h];
-        s.x += n * k.x;
-        s.y += n * k.y;
-        s.z += n * k.z;
-        s.w += n * k.w;
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[r] += n * W[q * 8 + h][r];
       }
     }
-    *out = s;
+    *out = make_int4(s[0], s[1], s[2], s[3]);
     out += 32;
   }
 }
 
-// The walk's window over a merge's flags: up to kWinSteps supersteps of one band.
-struct MsaWindow {
-  const uint4* flags;    // the merge's flags
-  uint4* win;            // shared: [kWinSteps][32]
+// The pipeline's scores: a superstep's are one block of 4 KB, copied to shared
+// memory kSlots supersteps ahead by one bulk copy (a superstep takes about as
+// long as a read from the far L2, so registers loaded one ahead left the warp
+// waiting, and two ahead cost 64 of them).
+struct MsaScore {
+  static constexpr int kSlots = 3;
+  static constexpr int kBytes = pipe::kStep * 32 * (int)sizeof(int4);
+  struct Ring {
+    int4 v[kSlots][pipe::kStep * 32];
+    unsigned long long bar[kSlots];
+  };
+  Ring* ring;           // this warp's, in shared memory
+  const int4* base;     // the merge's scores
   int nsup;
-  int g = -1, j0 = 0;    // band, first superstep held
-  static __device__ __forceinline__ int superstep(int x, int y) { return (x + ((y & (kWBand - 1)) >> 2)) >> 3; }
-  __device__ __forceinline__ bool covers(int x, int y) const {
-    const int j = superstep(x, y) - j0;
-    return (y >> 7) == g && j >= 0 && j < kWinSteps;
+  const int4* band = nullptr;
+  const int4* cur = nullptr;
+  unsigned used = 0;    // supersteps begun
+  __device__ __forceinline__ void ask(int j, unsigned use) {
+    pipe::bar_expect(&ring->bar[use % kSlots], kBytes);
+    pipe::copy_bulk(ring->v[use % kSlots], band + (int64_t)j * pipe::kStep * 32, kBytes, &ring->bar[use % kSlots]);
   }
-  __device__ __forceinline__ unsigned cell(int x, int y) const {
-    const int l = (y & (kWBand - 1)) >> 2, t = x + l, i = t & 7;
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(win + ((t >> 3) - j0) * 32 + l);
-    return (w[i >> 1] >> (4 * (7 - ((i & 1) * 4 + (y & 3))))) & 15u;
+  __device__ __forceinline__ void load(int g) {
+    band = base + (int64_t)g * nsup * pipe::kStep * 32;
+    if ((threadIdx.x & 31) == 0)
+      for (int j = 0; j < kSlots && j < nsup; ++j) ask(j, used + j);
   }
-  __device__ __forceinline__ void load(int x, int y) {
-    const int lane = threadIdx.x & 31;
-    g = y >> 7;
-    j0 = superstep(x, y) - (kWinSteps - 1);
+  __device__ __forceinline__ void begin(int, pipe::Link& ln) {
+    ln.wait(&ring->bar[used % kSlots], (used / kSlots) & 1);
+    cur = ring->v[used % kSlots] + (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ void get(int i, int, int (&s)[kRows]) const {
+    const int4 v = cur[i * 32];
+    s[0] = v.x, s[1] = v.y, s[2] = v.z, s[3] = v.w;
+  }
+  __device__ __forceinline__ void end(int j) {
     __syncwarp();
-    uint4 v[kWinSteps];
-#pragma unroll
-    for (int k = 0; k < kWinSteps; ++k)
-      if (j0 + k >= 0) v[k] = flags[((int64_t)g * nsup + j0 + k) * 32 + lane];
-#pragma unroll
-    for (int k = 0; k < kWinSteps; ++k)
-      if (j0 + k >= 0) win[k * 32 + lane] = v[k];
-    __syncwarp();
+    if ((threadIdx.x & 31) == 0 && j + kSlots < nsup) ask(j + kSlots, used + kSlots);
+    ++used;
   }
+  __device__ __forceinline__ void column_done(int, const int (&)[kRows]) const {}
+  __device__ __forceinline__ void band_done() const {}
 };
 
-__global__ void __launch_bounds__(32 * kWMax) msa_wave_kernel(const MergeDesc* __restrict__ md,
-                                                             const int4* __restrict__ score, uint4* flags,
-                                                             int2* bnd, int2* __restrict__ src,
-                                                             int32_t* __restrict__ nops, int go, int ge) {
-  __shared__ int2 s_ring[kWMax][kRing];
-  __shared__ uint4 s_win[kWinSteps * 32];
-  const MergeDesc m = md[blockIdx.x];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int kk = m.kx * m.ky;
-  const int GO = go * kk, GE = ge * kk;
-  const int nb = (m.ly + kWBand - 1) / kWBand, nsup = m.nsup;
-  // warp w runs bands w, w + nwarp, ..: band p * nwarp + w from superstep p * period + kLag * w on
-  const int period = max(nsup, kLag * nwarp);
-  const int last = (nb - 1) / nwarp * period + (nb - 1) % nwarp * kLag + nsup;
-  uint4* fl = flags + m.nib / 16;
-  const int4* sc = score + m.score + lane;
-  int2* bd = bnd + m.bnd;
-  const int2* in_ring = s_ring[warp == 0 ? nwarp - 1 : warp - 1];
-  int uL[kWRows], bL[kWRows];
-  int vbot = 0, abot = 0;
-  int4 cur[kStep];
-  int g = warp, j = -kLag * warp;
-  for (int q = 0; q < last; ++q) {
-    if (j >= 0 && j < nsup && g < nb) {
-      const int4* band = sc + (int64_t)g * nsup * kStep * 32;
-      if (j == 0) {
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) cur[i] = band[i * 32];
-#pragma unroll
-        for (int r = 0; r < kWRows; ++r) {
-          uL[r] = -GE;
-          bL[r] = kDiffSent;
-        }
-      }
-      int4 nxt[kStep];
-      if (j + 1 < nsup) {
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) nxt[i] = band[((j + 1) * kStep + i) * 32];
-      }
-      if (warp == 0 && g > 0) {   // the row above, left in global memory by the last warp
-        const int c = j * kStep + lane;
-        if (lane < kStep && c < m.lx) s_ring[nwarp - 1][c & (kRing - 1)] = bd[c];
-        __syncwarp();
-      }
-      uint32_t word[kStep / 2] = {};
-      auto steps = [&](auto checked) {
-#pragma unroll
-        for (int i = 0; i < kStep; ++i) {
-          const int t = j * kStep + i;
-          int vU = __shfl_up_sync(0xffffffffu, vbot, 1);
-          int aU = __shfl_up_sync(0xffffffffu, abot, 1);
-          if (g == 0) {
-            if (lane == 0) {
-              vU = -GE;
-              aU = kDiffSent;
-            }
-          } else {
-            const int2 in = in_ring[t & (kRing - 1)];
-            if (lane == 0) {
-              vU = in.x;
-              aU = in.y;
-            }
-          }
-          if (decltype(checked)::value && t == lane) {   // the lane's column 0: what came before was no cell
-#pragma unroll
-            for (int r = 0; r < kWRows; ++r) {
-              uL[r] = -GE;
-              bL[r] = kDiffSent;
-            }
-          }
-          const int sv[kWRows] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
-          uint32_t w = word[i >> 1];
-#pragma unroll
-          for (int r = 0; r < kWRows; ++r) {
-            // flags as sign bits, appended by funnel shifts: cU = a(up) - GE >= -GO,
-            // cL likewise, F >= E, H == S; then U = ps || pf, L = ps || !pf
-            const uint32_t xcu = (uint32_t)(GE - GO - 1 - aU);
-            const int F = vU + __viaddmax_s32(aU, -GE, -GO);
-            const uint32_t xcl = (uint32_t)(GE - GO - 1 - bL[r]);
-            const int E = uL[r] + __viaddmax_s32(bL[r], -GE, -GO);
-            const uint32_t xpf = (uint32_t)(E - F - 1);
-            const int h = __vimax3_s32(E, F, sv[r]);
-            const uint32_t xps = (uint32_t)(h - sv[r] - 1);
-            w = __funnelshift_l(xps | ~xpf, w, 1);   // L
-            w = __funnelshift_l(xps | xpf, w, 1);    // U
-            w = __funnelshift_l(xcu, w, 1);          // cU
-            w = __funnelshift_l(xcl, w, 1);          // cL
-            const int v = h - uL[r];
-            uL[r] = h - vU;
-            aU = F - h;
-            bL[r] = E - h;
-            vU = v;
-          }
-          word[i >> 1] = w;
-          vbot = vU;
-          abot = aU;
-          const int c = t - 31;
-          if (lane == 31 && c >= 0 && c < m.lx) {
-            if (warp + 1 < nwarp) s_ring[warp][c & (kRing - 1)] = make_int2(vbot, abot);
-            else if (g + 1 < nb) bd[c] = make_int2(vbot, abot);
-          }
-        }
-      };
-      if (j < 32 / kStep) steps(std::true_type{});
-      else steps(std::false_type{});
-      fl[((int64_t)g * nsup + j) * 32 + lane] = make_uint4(word[0], word[1], word[2], word[3]);
-#pragma unroll
-      for (int i = 0; i < kStep; ++i) cur[i] = nxt[i];
-    }
-    if (++j == period) {
-      j = 0;
-      g += nwarp;
-    }
-    __syncthreads();
-  }
-  if (warp != 0) return;
+// C CTAs (one cluster) per merge; dynamic shared memory: a score ring per warp,
+// then the walk's window in its place.
+__global__ void __launch_bounds__(32 * pipe::kWarps, 4) msa_wave_kernel(const MergeDesc* __restrict__ md, int C,
+                                                                       const int* __restrict__ score,
+                                                                       uint32_t* flags, int2* bnd, unsigned* done,
+                                                                       int2* __restrict__ src,
+                                                                       int32_t* __restrict__ nops, int* err, int go,
+                                                                       int ge) {
+  using Ring = MsaScore::Ring;
+  static_assert(sizeof(Ring) >= kMsaWindow, "the window takes a ring's place");
+  __shared__ pipe::Inbox s_box[pipe::kWarps];
+  extern __shared__ __align__(128) unsigned char s_dyn[];
+  Ring* s_ring = reinterpret_cast<Ring*>(s_dyn);
+  const int q = blockIdx.x / C, rank = blockIdx.x - q * C;
+  const MergeDesc m = md[q];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
+  const int gw = rank * wpc + warp, nwarp = C * wpc;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < wpc; ++w)
+      for (int k = 0; k < MsaScore::kSlots; ++k) pipe::bar_init(&s_ring[w].bar[k]);
+  pipe::init_inboxes(s_box, wpc);
+  pipe::Link ln;
+  ln.in = &s_box[warp];
+  ln.out = pipe::cluster_addr(pipe::smem_addr(&s_box[(gw + 1) % wpc]), (gw + 1) % nwarp / wpc);
+  ln.back = pipe::cluster_addr(pipe::smem_addr(&s_box[(gw + nwarp - 1) % wpc]), (gw + nwarp - 1) % nwarp / wpc);
+  ln.err = err;
+  const int nsup = pipe::supersteps_of(m.lx);
+  uint32_t* fl = flags + m.nib / 4;
+  MsaScore sc;
+  sc.ring = s_ring + warp;
+  sc.base = reinterpret_cast<const int4*>(score + m.score);
+  sc.nsup = nsup;
+  pipe::run_bands<kRows>(ln, pipe::Wrap{bnd + m.bnd, done + q}, sc, fl, m.lx, m.ly, (go - ge) * m.kx * m.ky, gw, nwarp);
+  pipe::cluster_barrier();   // every band's flags are written, every copy has arrived
+  if (rank != 0 || warp != 0) return;
   // the walk: the alignment's columns in forward order (X column, Y column; -1 a gap)
-  MsaWindow win{fl, s_win, nsup};
+  pipe::Window<kRows, kMsaWindow> win{fl, reinterpret_cast<uint32_t*>(s_dyn), nsup};
   int2* out = src + m.src;
   WalkPos p = run_walk(win, m.lx, m.ly, m.lx + m.ly, [&](int k, int n, int x, int y, int sx, int sy) {
     if (lane < n) out[k + lane] = make_int2(sx ? x - lane : -1, sy ? y - lane : -1);
@@ -497,7 +412,28 @@ __global__ void __launch_bounds__(32 * kWMax) msa_wave_kernel(const MergeDesc* _
   p.k += p.x + 1;
   for (int i = lane; i <= p.y; i += 32) out[p.k + i] = make_int2(-1, p.y - i);
   p.k += p.y + 1;
-  if (lane == 0) nops[blockIdx.x] = p.k;
+  if (lane == 0) nops[q] = p.k;
+}
+
+cudaError_t launch_msa_wave(const MergeDesc* md, int count, int warps, const int* score, uint32_t* flags, int2* bnd,
+                            unsigned* done, int2* src, int32_t* nops, int* err, int go, int ge, cudaStream_t s) {
+  const int C = (warps + pipe::kWarps - 1) / pipe::kWarps;
+  const int wpc = (warps + C - 1) / C;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(count * C));
+  cfg.blockDim = dim3((unsigned)(32 * wpc));
+  cfg.dynamicSmemBytes = sizeof(MsaScore::Ring) * wpc;
+  cfg.stream = s;
+  const cudaError_t e = cudaFuncSetAttribute(msa_wave_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(MsaScore::Ring) * pipe::kWarps);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, msa_wave_kernel, md, C, score, flags, bnd, done, src, nops, err, go, ge);
 }
 
 // Merged profile and child maps: three threads per column, eight letters each
@@ -643,31 +579,28 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
   int64_t cells = 0;
   int64_t smax = 1;   // largest |S| of the context's matrix
   for (int k = 0; k < kLetters * kLetters; ++k) smax = std::max<int64_t>(smax, sub[k] < 0 ? -sub[k] : sub[k]);
-  const int64_t diff_bound = 2 * smax + 4 * (int64_t)go;   // the wave form's differences, per kX * kY
-  constexpr int64_t kScoreBatch = (int64_t)1 << 25;        // int4 scores of one batch of merges (512 MiB)
-  constexpr int64_t kScoreMax = (int64_t)1 << 29;          // of one merge (8 GiB; beyond, the 64-bit form)
+  const int64_t diff_bound = 2 * smax + 4 * (int64_t)go;   // the wave form's values, per kX * kY
+  constexpr int64_t kScoreBatch = (int64_t)1 << 27;        // cell scores of one batch of merges (512 MiB)
+  constexpr int64_t kScoreMax = (int64_t)1 << 31;          // of one merge (8 GiB; beyond, the 64-bit form)
   std::vector<MergeDesc> md;
   std::vector<int32_t> nops;
   for (int l = 1; l <= levels; ++l) {
     // wave-form merges first, most supersteps first; then the 64-bit ones
     std::vector<int>& nodes = bylevel[l];
     const int nm = (int)nodes.size();
-    auto shape = [&](int v, int64_t& bands, int64_t& nsup) {
-      bands = (len[right[v - n]] + kWBand - 1) / kWBand;
-      nsup = (len[left[v - n]] + 31 + kStep - 1) / kStep;
+    constexpr int kBand = 32 * kRows;
+    auto padded = [&](int v) {   // cell scores of a merge
+      return (int64_t)((len[right[v - n]] + kBand - 1) / kBand) * kBand * pipe::supersteps_of((int)len[left[v - n]]) *
+             pipe::kStep;
     };
     auto is_wave = [&](int v) {
-      int64_t bands, nsup;
-      shape(v, bands, nsup);
-      return go >= ge && (int64_t)kseq[left[v - n]] * kseq[right[v - n]] * diff_bound < ((int64_t)1 << 30) &&
-             bands * nsup * kStep * 32 <= kScoreMax;
+      return go >= ge && (int64_t)kseq[left[v - n]] * kseq[right[v - n]] * diff_bound < ((int64_t)1 << 31) &&
+             padded(v) <= kScoreMax;
     };
     const int nwave = (int)(std::stable_partition(nodes.begin(), nodes.end(), is_wave) - nodes.begin());
     std::stable_sort(nodes.begin(), nodes.begin() + nwave, [&](int u, int v) {
-      int64_t bu, su, bv, sv;
-      shape(u, bu, su);
-      shape(v, bv, sv);
-      return bu != bv ? bu > bv : su > sv;
+      const int64_t bu = (len[right[u - n]] + kBand - 1) / kBand, bv = (len[right[v - n]] + kBand - 1) / kBand;
+      return bu != bv ? bu > bv : len[left[u - n]] > len[left[v - n]];
     });
     md.assign(nm, MergeDesc{});
     int64_t nib_total = 0, src_total = 0, scr_total = 0, score_cap = 0, bnd_total = 0;
@@ -699,10 +632,8 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
       maxcols = std::max(maxcols, d.lx + d.ly);
       cells += (int64_t)d.lx * d.ly;
       if (q < nwave) {
-        int64_t bands, nsup;
-        shape(v, bands, nsup);
-        d.nsup = (int)nsup;
-        const int64_t words = bands * nsup * kStep * 32;
+        const int64_t bands = (d.ly + kBand - 1) / kBand, nsup = pipe::supersteps_of(d.lx);
+        const int64_t words = padded(v);
         if (batches.empty() || score_used + words > kScoreBatch) {
           batches.push_back({q, 0, 0, 1});
           score_used = 0;
@@ -712,12 +643,12 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
         score_used += words;
         score_cap = std::max(score_cap, score_used);
         d.tile0 = bt.tiles;
-        bt.tiles += (int)(bands * ((nsup * kStep + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps)));
+        bt.tiles += (int)(bands * ((nsup * pipe::kStep + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps)));
         bt.count += 1;
-        bt.warps = std::max(bt.warps, (int)std::min<int64_t>(bands, kWMax));
+        bt.warps = std::max(bt.warps, (int)std::min<int64_t>(bands, pipe::kWarps * pipe::kCluster));
         d.bnd = bnd_total;
-        if (bands > kWMax) bnd_total += d.lx;
-        nib_total += bands * nsup * 512;
+        if (bands > pipe::kWarps * pipe::kCluster) bnd_total += d.lx;
+        nib_total += bands * nsup * 128 * kRows;
       } else {
         const int nstr = (d.ly + kMR - 1) / kMR;
         nib_total += ((int64_t)nstr * (d.lx + kMR - 1) * kMR + 15) / 16 * 16;
@@ -728,19 +659,26 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
     if ((rc = M.nib.ensure((size_t)std::max<int64_t>(nib_total, 1))) ||
         (rc = M.src.ensure(sizeof(int2) * (size_t)std::max<int64_t>(src_total, 1))) ||
         (rc = M.scratch.ensure(sizeof(longlong2) * (size_t)std::max<int64_t>(scr_total, 1))) ||
-        (rc = M.score.ensure(sizeof(int4) * (size_t)std::max<int64_t>(score_cap, 1))) ||
+        (rc = M.score.ensure(sizeof(int) * (size_t)std::max<int64_t>(score_cap, 1))) ||
         (rc = M.bnd.ensure(sizeof(int2) * (size_t)std::max<int64_t>(bnd_total, 1))) ||
-        (rc = M.nops.ensure(sizeof(int32_t) * nm)) || (rc = M.md.ensure(sizeof(MergeDesc) * nm)))
+        (rc = M.nops.ensure(sizeof(int32_t) * (2 * (size_t)nm + 1))) || (rc = M.md.ensure(sizeof(MergeDesc) * nm)))
       return fail(rc, "msa allocation");
     if ((rc = cuda(cudaMemcpyAsync(M.md.p, md.data(), sizeof(MergeDesc) * nm, cudaMemcpyHostToDevice, s), "msa upload")))
       return rc;
     const MergeDesc* dmd = (const MergeDesc*)M.md.p;
+    // nops: the merges' lengths, an error flag, the wave form's wrap counters
+    int32_t* dnops = (int32_t*)M.nops.p;
+    int* derr = (int*)dnops + nm;
+    unsigned* ddone = (unsigned*)dnops + nm + 1;
+    if ((rc = cuda(cudaMemsetAsync(derr, 0, sizeof(int) * ((size_t)nm + 1), s), "msa"))) return rc;
     for (const Batch& b : batches) {
-      msa_score_kernel<<<b.tiles, 32 * kScoreWarps, 0, s>>>(dmd + b.first, b.count, (const int16_t*)M.cnt.p,
-                                                            (const int8_t*)b_sub.p, (int4*)M.score.p);
-      msa_wave_kernel<<<b.count, 32 * b.warps, 0, s>>>(dmd + b.first, (const int4*)M.score.p, (uint4*)M.nib.p,
-                                                       (int2*)M.bnd.p, (int2*)M.src.p, (int32_t*)M.nops.p + b.first,
-                                                       go, ge);
+      const MergeDesc* bmd = dmd + b.first;
+      msa_score_kernel<<<b.tiles, 32 * kScoreWarps, 0, s>>>(bmd, b.count, (const int16_t*)M.cnt.p,
+                                                            (const int8_t*)b_sub.p, ge, (int*)M.score.p);
+      if ((rc = cuda(launch_msa_wave(bmd, b.count, b.warps, (const int*)M.score.p, (uint32_t*)M.nib.p, (int2*)M.bnd.p,
+                                     ddone + b.first, (int2*)M.src.p, dnops + b.first, derr, go, ge, s),
+                     "msa launch")))
+        return rc;
       launches += 2;
     }
     if (nwave < nm) {
@@ -754,10 +692,12 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
     ++launches;
     if ((rc = cuda(cudaGetLastError(), "msa launch"))) return rc;
     // the new profiles' lengths (the next level sizes its work with them)
-    nops.resize(nm);
-    if ((rc = cuda(cudaMemcpyAsync(nops.data(), M.nops.p, sizeof(int32_t) * nm, cudaMemcpyDeviceToHost, s), "msa")) ||
+    nops.resize((size_t)nm + 1);
+    if ((rc = cuda(cudaMemcpyAsync(nops.data(), M.nops.p, sizeof(int32_t) * ((size_t)nm + 1), cudaMemcpyDeviceToHost, s),
+                   "msa")) ||
         (rc = cuda(cudaStreamSynchronize(s), "msa sync")))
       return rc;
+    if (nops[nm]) return fail(NWG_ERR_TIMEOUT, "progressive alignment: a bounded device wait ran out");
     for (int q = 0; q < nm; ++q) len[nodes[q]] = nops[q];
   }
   // final positions, parents first, then the rows
