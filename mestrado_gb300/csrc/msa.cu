@@ -29,6 +29,7 @@
 
 #include "nwg_ctx.h"
 #include "pipe.cuh"
+#include "profile8.cuh"
 
 namespace nwg {
 namespace {
@@ -46,6 +47,8 @@ struct MergeDesc {
   int32_t lx, ly, kx, ky;
   int32_t tile0;              // wave form: first CTA of the score kernel
   int32_t mac32;              // kx * ky * max|S| < 2^31: a cell's score sum fits int32
+  int32_t bytes;              // wave form: X's counts fit a byte and Y's row scores this many (0: they don't)
+  int32_t pad;
 };
 
 __device__ __forceinline__ int64_t mx64(int64_t a, int64_t b) { return a > b ? a : b; }
@@ -229,71 +232,61 @@ __global__ void __launch_bounds__(kMR) msa_dp_kernel(const MergeDesc* md, const 
 // 10 (207 us with one CTA barrier per eight steps on a single SM and the scores
 // in registers; 0.43 ms at 339 columns with 64-bit cells, one row per thread
 // and a barrier per anti-diagonal).
-constexpr int kScoreSteps = 16;            // steps per warp of the score kernel
-constexpr int kScoreWarps = 8;
+constexpr int kScoreSteps = 32;            // steps per warp of the score kernel
+constexpr int kScoreWarps = 4;
 constexpr int kMsaWindow = 8192;           // bytes of flags in the walk's window
 
 constexpr int kRows = 4;                   // rows per lane of the pipeline
 
-// Scores of the cells of a level's merges in the wave kernel's order: entry
-// (g * nsup * 8 + t) * 32 + l of a merge holds rows 128 g + 4 l .. + 3 at column
-// t - l (2 GE outside).  One CTA per 128 rows x 128 steps: the rows' scores
-// against each letter, W[x] = sum_y cY[y] S[y][x], go to shared memory once,
-// then each warp runs 16 steps with its lanes' 4 x 24 of them in registers:
-// 96 multiply-adds for three 16-byte loads of column counts.
-__global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const MergeDesc* __restrict__ md, int nm,
-                                                                    const int16_t* __restrict__ cnt,
-                                                                    const int8_t* __restrict__ sub, int ge,
-                                                                    int* __restrict__ score) {
-  constexpr int R = kRows, kBand = 32 * R;
-  constexpr int kPer = kLetters * R / 8;   // letters per thread of the row scores: two threads a row
-  __shared__ int8_t s_sub[kLetters * kLetters];
-  __shared__ __align__(16) int s_w[kLetters][kBand];
-  int lo = 0, hi = nm - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (md[mid].tile0 <= (int)blockIdx.x) lo = mid;
-    else hi = mid - 1;
-  }
-  const MergeDesc m = md[lo];
-  const int steps = pipe::supersteps_of(m.lx) * pipe::kStep;
-  const int nchunk = (steps + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps);
-  const int tile = (int)blockIdx.x - m.tile0;
-  const int g = tile / nchunk, chunk = tile - g * nchunk;
-  for (int e = threadIdx.x; e < kLetters * kLetters; e += blockDim.x) s_sub[e] = sub[e];
-  __syncthreads();
-  {
-    const int row = threadIdx.x % kBand, x0 = (threadIdx.x / kBand) * kPer;
-    int w[kPer];
+// Sum of four products of unsigned bytes of a with signed (unsigned) bytes of b.
+__device__ __forceinline__ int dot4_us(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ int dot4_uu(uint32_t a, uint32_t b, int c) {
+  int d;
+  asm("dp4a.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// The steps [t0, t1) of one warp of the score kernel.  Bytes: 0 for any counts
+// and row scores (24 multiply-adds a cell); 1 when X's counts fit a byte and
+// the row scores a signed one (6 four-byte dot products); 2 when the row scores
+// need two (6 with the high bytes, 6 with the low).
+template <int Bytes>
+__device__ __forceinline__ void score_steps(const MergeDesc& m, const int (*s_w)[32 * kRows],
+                                            const int16_t* __restrict__ cnt, int4* __restrict__ out, int base, int t0,
+                                            int t1) {
+  constexpr int R = kRows;
+  const int lane = threadIdx.x & 31;
+  constexpr int kW = Bytes == 0 ? kLetters : kLetters / 4;
+  int W[kW][R], V[Bytes == 2 ? kW : 1][R];   // row scores (their high and low bytes)
 #pragma unroll
-    for (int x = 0; x < kPer; ++x) w[x] = 0;
-    const int r = g * kBand + row;
-    if (r < m.ly) {
-      const int16_t* cy = cnt + (m.yoff + r) * kLetters;
-      for (int b = 0; b < kLetters; ++b) {
-        const int c = cy[b];
-        if (c == 0) continue;
+  for (int q = 0; q < kLetters / 4; ++q) {
+    int w[4][R];
 #pragma unroll
-        for (int x = 0; x < kPer; ++x) w[x] += c * (int)s_sub[b * kLetters + x0 + x];
-      }
+    for (int x = 0; x < 4; ++x) {
+      const int4 v = *reinterpret_cast<const int4*>(&s_w[4 * q + x][R * lane]);
+      w[x][0] = v.x, w[x][1] = v.y, w[x][2] = v.z, w[x][3] = v.w;
     }
 #pragma unroll
-    for (int x = 0; x < kPer; ++x) s_w[x0 + x][row] = w[x];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t0 = (chunk * kScoreWarps + warp) * kScoreSteps;
-  const int t1 = min(t0 + kScoreSteps, steps);
-  if (t0 >= t1) return;
-  int W[kLetters][R];
+    for (int r = 0; r < R; ++r) {
+      if constexpr (Bytes == 0) {
 #pragma unroll
-  for (int x = 0; x < kLetters; ++x) {
-    const int4 w = *reinterpret_cast<const int4*>(&s_w[x][R * lane]);
-    W[x][0] = w.x, W[x][1] = w.y, W[x][2] = w.z, W[x][3] = w.w;
+        for (int x = 0; x < 4; ++x) W[4 * q + x][r] = w[x][r];
+      } else {
+        const uint32_t lo = perm(perm(w[0][r], w[1][r], 0x0040), perm(w[2][r], w[3][r], 0x0040), 0x5410);
+        if constexpr (Bytes == 2) {
+          W[q][r] = (int)perm(perm(w[0][r], w[1][r], 0x0051), perm(w[2][r], w[3][r], 0x0051), 0x5410);
+          V[q][r] = (int)lo;
+        } else {
+          W[q][r] = (int)lo;
+        }
+      }
+    }
   }
   const uint4* X = reinterpret_cast<const uint4*>(cnt + m.xoff * kLetters);   // 48 bytes a column
-  int4* out = reinterpret_cast<int4*>(score + m.score) + ((int64_t)g * steps + t0) * 32 + lane;
-  const int base = 2 * ge * m.kx * m.ky;   // the pipeline's S' = S + 2 GE
   uint4 nxt[3] = {};
   auto load = [&](int t) {
     const int c = t - lane;
@@ -307,20 +300,110 @@ __global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const Merge
     if (t + 1 < t1) load(t + 1);
     int s[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) s[r] = base;
+    for (int r = 0; r < R; ++r) s[r] = Bytes == 2 ? 0 : base;
+    if constexpr (Bytes == 0) {
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const uint32_t w[4] = {cur[q].x, cur[q].y, cur[q].z, cur[q].w};
+      for (int q = 0; q < 3; ++q) {
+        const uint32_t w[4] = {cur[q].x, cur[q].y, cur[q].z, cur[q].w};
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
-        const int n = (h & 1) ? (int)w[h >> 1] >> 16 : (int)(int16_t)(w[h >> 1] & 0xFFFFu);
+        for (int h = 0; h < 8; ++h) {
+          const int n = (h & 1) ? (int)w[h >> 1] >> 16 : (int)(int16_t)(w[h >> 1] & 0xFFFFu);
 #pragma unroll
-        for (int r = 0; r < R; ++r) s[r] += n * W[q * 8 + h][r];
+          for (int r = 0; r < R; ++r) s[r] += n * W[q * 8 + h][r];
+        }
+      }
+    } else {
+      uint32_t n[kW];   // the column's counts, a byte each
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        n[2 * q] = perm(cur[q].x, cur[q].y, 0x6420);
+        n[2 * q + 1] = perm(cur[q].z, cur[q].w, 0x6420);
+      }
+#pragma unroll
+      for (int q = 0; q < kW; ++q)
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[r] = dot4_us(n[q], (uint32_t)W[q][r], s[r]);
+      if constexpr (Bytes == 2) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[r] = s[r] * 256 + base;
+#pragma unroll
+        for (int q = 0; q < kW; ++q)
+#pragma unroll
+          for (int r = 0; r < R; ++r) s[r] = dot4_uu(n[q], (uint32_t)V[q][r], s[r]);
       }
     }
-    *out = make_int4(s[0], s[1], s[2], s[3]);
-    out += 32;
+    out[(int64_t)t * 32] = make_int4(s[0], s[1], s[2], s[3]);
   }
+}
+
+// Scores of the cells of a level's merges in the wave kernel's order: entry
+// (g * nsup * 8 + t) * 32 + l of a merge holds rows 128 g + 4 l .. + 3 at column
+// t - l (2 GE outside).  One CTA per 128 rows x 128 steps: the rows' scores
+// against each letter, W[x] = sum_y cY[y] S[y][x], go to shared memory once,
+// then each warp runs 32 steps with its lanes' in registers, for three 16-byte
+// loads of column counts a step.  Where counts and row scores fit bytes (a
+// tree's lower levels, most of the cells) four products are one instruction.
+// The lowest level of 8,000 sequences (2.7e8 padded cells, 1.1 GB of scores):
+// 0.64 to 0.35 ms, 3.1 TB/s of stores; the whole tree 2.3 to 1.4 ms.
+__global__ void __launch_bounds__(32 * kScoreWarps) msa_score_kernel(const MergeDesc* __restrict__ md, int nm,
+                                                                    const int16_t* __restrict__ cnt,
+                                                                    const int8_t* __restrict__ sub, int ge,
+                                                                    int* __restrict__ score) {
+  constexpr int kBand = 32 * kRows;
+  static_assert(kBand == 32 * kScoreWarps, "one thread per row");
+  __shared__ __align__(16) int8_t s_sub[kLetters * kLetters];
+  __shared__ __align__(16) int s_w[kLetters][kBand];
+  int lo = 0, hi = nm - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (md[mid].tile0 <= (int)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  const MergeDesc m = md[lo];
+  const int steps = pipe::supersteps_of(m.lx) * pipe::kStep;
+  const int nchunk = (steps + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps);
+  const int tile = (int)blockIdx.x - m.tile0;
+  const int g = tile / nchunk, chunk = tile - g * nchunk;
+  for (int e = threadIdx.x; e < kLetters * kLetters / 4; e += blockDim.x)
+    reinterpret_cast<int*>(s_sub)[e] = reinterpret_cast<const int*>(sub)[e];
+  __syncthreads();
+  {
+    int w[kLetters];
+#pragma unroll
+    for (int x = 0; x < kLetters; ++x) w[x] = 0;
+    const int r = g * kBand + threadIdx.x;
+    if (r < m.ly) {
+      const uint4* cy = reinterpret_cast<const uint4*>(cnt + (m.yoff + r) * kLetters);
+      const uint4 v[3] = {cy[0], cy[1], cy[2]};
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const uint32_t h[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const int c = (b & 1) ? (int)h[b >> 1] >> 16 : (int)(int16_t)(h[b >> 1] & 0xFFFFu);
+          if (c == 0) continue;
+          const int* row = reinterpret_cast<const int*>(s_sub + (q * 8 + b) * kLetters);
+#pragma unroll
+          for (int x4 = 0; x4 < kLetters / 4; ++x4) {
+            const int p = row[x4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) w[4 * x4 + x] += c * (int)(int8_t)(p >> (8 * x));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kLetters; ++x) s_w[x][threadIdx.x] = w[x];
+  }
+  __syncthreads();
+  const int t0 = (chunk * kScoreWarps + (int)(threadIdx.x >> 5)) * kScoreSteps;
+  const int t1 = min(t0 + kScoreSteps, steps);
+  if (t0 >= t1) return;
+  int4* out = reinterpret_cast<int4*>(score + m.score) + (int64_t)g * steps * 32 + (threadIdx.x & 31);
+  const int base = 2 * ge * m.kx * m.ky;   // the pipeline's S' = S + 2 GE
+  if (m.bytes == 1) score_steps<1>(m, s_w, cnt, out, base, t0, t1);
+  else if (m.bytes == 2) score_steps<2>(m, s_w, cnt, out, base, t0, t1);
+  else score_steps<0>(m, s_w, cnt, out, base, t0, t1);
 }
 
 // The pipeline's scores: a superstep's are one block of 4 KB, copied to shared
@@ -463,15 +546,18 @@ __global__ void __launch_bounds__(3 * kBuildCols) msa_build_kernel(const MergeDe
   }
 }
 
-// Leaf profiles: one column per residue (reversed codes), count 1.
-__global__ void msa_leaf_kernel(const int8_t* __restrict__ codes, int64_t total, int16_t* cnt) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= total) return;
-  int16_t* o = cnt + c * kLetters;
+// Leaf profiles: one column per residue (reversed codes), count 1; three
+// threads per column, so a warp's stores are whole lines (1.6 million residues:
+// 210 to 18 us).
+__global__ void msa_leaf_kernel(const int8_t* __restrict__ codes, int64_t total, uint4* __restrict__ cnt) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 3 * total) return;
+  const int64_t c = e / 3;
   int x = codes[c];
   if (x < 0 || x >= kLetters) x = kLetters - 1;
-#pragma unroll
-  for (int k = 0; k < kLetters; ++k) o[k] = (int16_t)(k == x);
+  x -= 8 * (int)(e - 3 * c);   // the letter's place among this thread's eight
+  const uint32_t one = (x & 1) ? 0x10000u : 1u;
+  cnt[e] = make_uint4(x >> 1 == 0 ? one : 0u, x >> 1 == 1 ? one : 0u, x >> 1 == 2 ? one : 0u, x >> 1 == 3 ? one : 0u);
 }
 
 struct PosJob {
@@ -572,7 +658,8 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
       (rc = M.pos.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(cap, 1))))
     return fail(rc, "msa allocation");
   if (st) cudaEventRecord(ev0, s);
-  msa_leaf_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>((const int8_t*)M.codes.p, total, (int16_t*)M.cnt.p);
+  msa_leaf_kernel<<<(unsigned)((3 * total + 255) / 256), 256, 0, s>>>((const int8_t*)M.codes.p, total,
+                                                                     (uint4*)M.cnt.p);
   ++launches;
   std::vector<std::vector<int>> bylevel(levels + 1);
   for (int k = 0; k < n - 1; ++k) bylevel[height[n + k]].push_back(n + k);
@@ -621,6 +708,7 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
       d.kx = kseq[a];
       d.ky = kseq[b];
       d.mac32 = (int64_t)d.kx * d.ky * smax < ((int64_t)1 << 31) ? 1 : 0;
+      d.bytes = d.kx > 255 ? 0 : d.ky * smax <= 127 ? 1 : d.ky * smax <= 32767 ? 2 : 0;
       d.xmap = col[a];
       d.ymap = col[b];
       d.ooff = pool;

@@ -69,3 +69,38 @@ def test_counts_beyond_32_bit_differences():
         level = sorted(nxt)
     with Context(1000, 1) as c:
         assert c.msa(seqs, left, right) == O.msa(seqs, left, right, go=1000, ge=1)
+
+
+def _balanced(n):
+    left, right, level, node = [], [], list(range(n)), n
+    while len(level) > 1:
+        nxt = []
+        for k in range(0, len(level) - 1, 2):
+            left.append(level[k])
+            right.append(level[k + 1])
+            nxt.append(node)
+            node += 1
+        if len(level) % 2:
+            nxt.append(level[-1])
+        level = sorted(nxt)
+    return left, right
+
+
+@pytest.mark.parametrize("n", [26, 600])
+def test_column_counts_past_a_byte(ctx, n):
+    # 'W' scores 11: row scores pass 127 from 12 sequences on, X's counts pass 255 at the root of 600
+    rng = np.random.default_rng(n)
+    seqs = [b"W" * int(k) + s for k, s in zip(rng.integers(1, 4, n), _rand(rng, rng.integers(1, 7, n)))]
+    left, right = _balanced(n)
+    assert ctx.msa(seqs, left, right) == O.msa(seqs, left, right)
+
+
+def test_row_scores_past_two_bytes(ctx):
+    # one sequence against a growing profile: 2,978 'W's in a column still score within 16 bits, 2,979 do not
+    n = 2985
+    seqs = [b"W" if k % 7 else b"WA" for k in range(n)]
+    left, right = [0], [1]
+    for k in range(1, n - 1):
+        left.append(k + 1)
+        right.append(n + k - 1)
+    assert ctx.msa(seqs, left, right) == O.msa(seqs, left, right)
