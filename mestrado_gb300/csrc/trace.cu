@@ -18,23 +18,23 @@
 //   from the sign bits of four differences, appended by funnel shifts.
 //   A lane's 8 rows of one column make one 32-bit word; the W lanes of a
 //   front store W consecutive words per step: word (b*(Lx+W-1) + t)*W + k
-//   holds rows b*8W + 8k .. +7 at column t-k, row r in bits 4(7-r)..4(7-r)+3.
-// The walk runs in the same warp right after the pairs' last bands, while
-//   their flags are still in L2, from (Lx-1, Ly-1) with the reference's rule
-//   set (continue flags of the previous move first, then up, then left, else
-//   diagonal); row -1 reads as left+continue, column -1 as up+continue, and
-//   an up move out of row 0 ends the walk (the reference's word reload at
-//   :456-457 never fires for row -1).  Each front stages the flags of a
-//   window of 32 columns x 40 rows ending at its walk's cell in shared memory
-//   (one load round trip), with the window's residue codes, and its lane 0
-//   walks inside it; a walk leaves a window after 32 to 72 steps.
-//   Characters come out in forward order, so the reorder/byte-swap pass is
-//   not needed.
+//   holds rows b*8W + 8k .. +7 at column t-k, a byte per flag (L highest),
+//   row r in bit 7-r.
+// trace_pipe_kernel: one pair as a pipeline of warps over a cluster (pipe.cuh),
+//   four rows per lane, for launches whose pairs do not fill the chip.
+// The walk runs in the warp right after the pair's last band, while its flags
+//   are still in L2, from (Lx-1, Ly-1), in runs (walk.cuh), over a window of
+//   4 or 8 KB of flags staged in shared memory.  The moves go through a small
+//   queue in shared memory, so that the residues' loads and the characters'
+//   stores are 128 at a time.  Characters come out in forward order, so the
+//   reorder/byte-swap pass is not needed.
 #include <algorithm>
 #include <cstring>
 #include <vector>
 
 #include "nwg_ctx.h"
+#include "pipe.cuh"
+#include "profile8.cuh"
 
 namespace nwg {
 
@@ -63,6 +63,9 @@ struct TraceArgs {
   int scratch_cols;
   int go, ge;
   const int8_t* sub;
+  // pipeline form
+  unsigned* done;           // per pair: columns handed on through the scratch row
+  int* err;                 // set when a wait runs out
 };
 
 __device__ __forceinline__ unsigned tclamp(int c) {
@@ -70,135 +73,107 @@ __device__ __forceinline__ unsigned tclamp(int c) {
   return u < (unsigned)kLetters ? u : (unsigned)(kLetters - 1);
 }
 
-__constant__ char c_dec[kLetters + 1] = "ARNDCQEGHILKMFPSTWYVBZX*";   // code -> letter
-
 static_assert(kTR == 8, "a lane's scores of one column are one 8-byte load");
 
-// Shared memory of one front's walk: the flag words of the window (row group
-// g0+gi of column x0-j at gi*32 + j) and its residue codes.
-struct WalkWindow {
-  uint32_t flags[5 * 32];
-  int8_t xs[32];   // X[x0 - j]
-  int8_t ys[40];   // Y[8*g0 + i]
+// The gapped strings of one walk: its moves queue in shared memory and leave
+// 128 at a time (a load and a store per move on the walk itself would make
+// every run wait for memory).
+constexpr int kQueue = 256;
+__device__ const char d_dec[kLetters + 1] = "ARNDCQEGHILKMFPSTWYVBZX*";   // code -> letter
+struct TextOut {
+  const int8_t* X;
+  const int8_t* Y;
+  char* ox;
+  char* oy;
+  int2* queue;      // shared, kQueue entries: the move's column and row, -1 for a gap
+  int done = 0;     // moves written out
+  static __device__ __forceinline__ char letter(int c) { return d_dec[tclamp(c)]; }
+  __device__ __forceinline__ void flush(int count) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    int cx[4], cy[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = q * 32 + lane;
+      cx[q] = cy[q] = -1;
+      if (e < count) {
+        const int2 p = queue[(done + e) % kQueue];
+        if (p.x >= 0) cx[q] = tclamp(X[p.x]);
+        if (p.y >= 0) cy[q] = tclamp(Y[p.y]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = q * 32 + lane;
+      if (e < count) {
+        ox[done + e] = cx[q] >= 0 ? letter(cx[q]) : '-';
+        oy[done + e] = cy[q] >= 0 ? letter(cy[q]) : '-';
+      }
+    }
+    done += count;
+    __syncwarp();
+  }
+  __device__ __forceinline__ void operator()(int k, int m, int x, int y, int sx, int sy) {
+    const int lane = threadIdx.x & 31;
+    if (lane < m) queue[(k + lane) % kQueue] = make_int2(sx ? x - lane : -1, sy ? y - lane : -1);
+    if (k + m - done >= 128) flush(128);
+  }
+  // the last moves, the terminators
+  __device__ __forceinline__ void finish(int k) {
+    flush(k - done);
+    if ((threadIdx.x & 31) == 0) ox[k] = oy[k] = 0;
+  }
 };
 
-// The backtraces of the warp's fronts (every lane calls it; p < 0: the
-// front has no pair).  Lane 0 of each front walks; all lanes of a front load
-// its windows.
+// Window over a pair's flags in the match kernel's layout: 1,024 words, the
+// steps of one band that end at the walk's cell.
 template <int W>
-__device__ void walk_pairs(const TraceArgs& a, int p, int lane, WalkWindow& w) {
-  const int sl = lane % W, lead = lane - sl;
-  const int8_t* X = nullptr;
-  const int8_t* Y = nullptr;
-  const uint32_t* nib = nullptr;
-  char* ox = nullptr;
-  char* oy = nullptr;
-  int Lx = 0, Ly = 0;
-  if (p >= 0) {
-    const int ix = a.px[p], iy = a.py[p];
-    X = a.codes + a.start[ix];
-    Y = a.codes + a.start[iy];
-    Lx = a.len[ix];
-    Ly = a.len[iy];
-    nib = a.nib + a.nib_off[p];
-    ox = a.outx + (size_t)p * a.stride;
-    oy = a.outy + (size_t)p * a.stride;
+struct MatchWindow {
+  static constexpr int kSteps = 1024 / W;
+  const uint32_t* nib;
+  uint32_t* win;           // shared, 1,024 words
+  int Lx;
+  int b = -1, t0 = 0;      // band, first step held
+  __device__ __forceinline__ bool covers(int x, int y) const {
+    const int t = x + y % (8 * W) / 8 - t0;
+    return y / (8 * W) == b && t >= 0 && t < kSteps;
   }
-  const int cap = Lx + Ly;
-  // walk state (meaningful in the front's lane 0): 1 = needs a window, 2 = done
-  int state = p >= 0 ? 1 : 2;
-  int x = Lx - 1, y = Ly - 1, k = 0;
-  unsigned prev = 12u, cell = 0u;
-  bool have_cell = false, stop = false;
-  for (;;) {
-    const int st = __shfl_sync(0xffffffffu, state, lead);
-    if (__all_sync(0xffffffffu, st == 2)) break;
-    // (re)load the window ending at (x, y) of the fronts that need one; x, y >= 0 there
-    const int x0 = __shfl_sync(0xffffffffu, x, lead);
-    const int g0 = (__shfl_sync(0xffffffffu, y, lead) >> 3) - 4;
-    if (st == 1) {
+  __device__ __forceinline__ unsigned cell(int x, int y) const {
+    const int k = y % (8 * W) / 8;
+    const uint32_t w = win[(x + k - t0) * W + k] >> (7 - (y & 7));
+    return (w >> 24 & 1u) << 3 | (w >> 16 & 1u) << 2 | (w >> 8 & 1u) << 1 | (w & 1u);
+  }
+  __device__ __forceinline__ void load(int x, int y) {
+    const int lane = threadIdx.x & 31;
+    b = y / (8 * W);
+    t0 = x + y % (8 * W) / 8 - (kSteps - 1);
+    __syncwarp();
+    const uint32_t* src = nib + ((int64_t)b * (Lx + W - 1) + t0) * W;
+    uint4 v[8];
 #pragma unroll
-      for (int j = 0; j < 32 / W; ++j) {
-        const int col = sl + j * W, c = x0 - col;
+    for (int q = 0; q < 8; ++q) {
+      const int e = (q * 32 + lane) * 4;
+      if (t0 + e / W >= 0) v[q] = *reinterpret_cast<const uint4*>(src + e);
+    }
 #pragma unroll
-        for (int gi = 0; gi < 5; ++gi) {
-          const int g = g0 + gi;
-          uint32_t v = 0u;
-          if (g >= 0 && c >= 0) v = nib[((size_t)(g / W) * (Lx + W - 1) + (c + g % W)) * W + g % W];
-          w.flags[gi * 32 + col] = v;
-        }
-        w.xs[col] = c >= 0 ? X[c] : (int8_t)0;
-      }
-      for (int i = sl; i < 40; i += W) {
-        const int r = 8 * g0 + i;
-        w.ys[i] = (r >= 0 && r < Ly) ? Y[r] : (int8_t)0;
-      }
+    for (int q = 0; q < 8; ++q) {
+      const int e = (q * 32 + lane) * 4;
+      if (t0 + e / W >= 0) *reinterpret_cast<uint4*>(win + e) = v[q];
     }
     __syncwarp();
-    if (sl == 0 && st == 1) {
-      for (;;) {
-        if (!have_cell) {
-          if (stop) {
-            cell = 0u;   // no word reload for row -1 after an up move
-          } else if (y < 0) {
-            cell = x < 0 ? 0u : 9u;   // row -1: left + continue-left; corner: stop
-          } else if (x < 0) {
-            cell = 6u;                // column -1: up + continue-up
-          } else if (x0 - x < 32 && (y >> 3) >= g0) {
-            cell = (w.flags[((y >> 3) - g0) * 32 + (x0 - x)] >> (4 * (7 - (y & 7)))) & 15u;
-          } else {
-            state = 1;
-            break;
-          }
-          have_cell = true;
-        }
-        if (!((cell & 12u) && k < cap)) {
-          state = 2;
-          break;
-        }
-        unsigned todo;
-        if (((prev & 12u) == 4u) && (prev & 2u)) todo = 4u;
-        else if (((prev & 12u) == 8u) && (prev & 1u)) todo = 8u;
-        else if ((cell & 12u) == 4u) todo = 4u;
-        else if ((cell & 12u) == 8u) todo = 8u;
-        else todo = 12u;
-        // a well-formed matrix never asks for a move off the -1 row/column
-        // other than the ones handled here; stop rather than read outside
-        if ((todo != 4u && x < 0) || (todo != 8u && y < 0)) {
-          state = 2;
-          break;
-        }
-        // residue codes: from the window inside it, else (the runs along row
-        // -1 and column -1) from the sequences
-        const bool xin = x >= 0 && x0 - x < 32;
-        const bool yin = y >= 8 * g0 && y - 8 * g0 < 40;
-        if (todo == 8u) {
-          ox[k] = c_dec[tclamp(xin ? w.xs[x0 - x] : X[x])];
-          oy[k] = '-';
-          --x;
-        } else if (todo == 4u) {
-          ox[k] = '-';
-          oy[k] = c_dec[tclamp(yin ? w.ys[y - 8 * g0] : Y[y])];
-          --y;
-          stop = y < 0;
-        } else {
-          ox[k] = c_dec[tclamp(xin ? w.xs[x0 - x] : X[x])];
-          oy[k] = c_dec[tclamp(yin ? w.ys[y - 8 * g0] : Y[y])];
-          --x;
-          --y;
-        }
-        prev = todo | (cell & 3u);
-        ++k;
-        have_cell = false;
-      }
-      if (state == 2) {
-        ox[k] = 0;
-        oy[k] = 0;
-        a.outlen[p] = k;
-      }
-    }
-    __syncwarp();   // the walkers are done with the windows before they are overwritten
   }
+};
+
+// One pair's walk by one warp.
+template <class Window>
+__device__ void walk_pair(const TraceArgs& a, int p, Window& win, int2* queue) {
+  const int ix = a.px[p], iy = a.py[p];
+  TextOut out{a.codes + a.start[ix], a.codes + a.start[iy], a.outx + (size_t)p * a.stride,
+              a.outy + (size_t)p * a.stride, queue};
+  const int Lx = a.len[ix], Ly = a.len[iy];
+  const WalkPos w = run_walk(win, Lx, Ly, Lx + Ly, out);
+  out.finish(w.k);
+  if ((threadIdx.x & 31) == 0) a.outlen[p] = w.k;
 }
 
 template <int W>
@@ -274,7 +249,7 @@ __global__ void __launch_bounds__(32 * kTWarps) match_kernel(const TraceArgs a) 
         int diag = hprev;
         hprev = hin;
         int f = fin, hup = hin;
-        uint32_t word = 0;
+        uint32_t aL = 0, aU = 0, aCu = 0, aCl = 0;
 #pragma unroll
         for (int r = 0; r < kTR; ++r) {
           // Each flag is the sign bit of one difference (a - b - 1 < 0 <=> a <= b):
@@ -282,8 +257,9 @@ __global__ void __launch_bounds__(32 * kTWarps) match_kernel(const TraceArgs a) 
           // pf = (F >= E), ps = (diag + S >= max(F, E)), i.e. H == diag + S;
           // then U = ps || pf and L = ps || !pf, since otherwise H = max(F, E)
           // and H == F <=> pf, (H == E && H != F) <=> !pf.  The bits are
-          // appended to the word by funnel shifts: L, U, cU, cL of row r land
-          // in bits 4(7-r)+3 .. 4(7-r).
+          // appended by funnel shifts to a word per flag (one word for all
+          // would chain 32 shifts a step), the words' low bytes then joined:
+          // L, U, cU, cL of row r land in bits 31-r, 23-r, 15-r and 7-r.
           const int fo = f - ge, hgo = hup - go;
           const uint32_t xcu = (uint32_t)(hgo - fo - 1);
           f = max(fo, hgo);
@@ -296,16 +272,16 @@ __global__ void __launch_bounds__(32 * kTWarps) match_kernel(const TraceArgs a) 
           const int t2 = max(f, e);
           const uint32_t xps = (uint32_t)(t2 - sim - 1);
           const int h = max(sim, t2);
-          word = __funnelshift_l(xps | ~xpf, word, 1);   // L
-          word = __funnelshift_l(xps | xpf, word, 1);    // U
-          word = __funnelshift_l(xcu, word, 1);          // cU
-          word = __funnelshift_l(xcl, word, 1);          // cL
+          aL = __funnelshift_l(xps | ~xpf, aL, 1);
+          aU = __funnelshift_l(xps | xpf, aU, 1);
+          aCu = __funnelshift_l(xcu, aCu, 1);
+          aCl = __funnelshift_l(xcl, aCl, 1);
           diag = H[r];
           H[r] = h;
           E[r] = e;
           hup = h;
         }
-        nb_base[(size_t)t * W + sl] = word;
+        nb_base[(size_t)t * W + sl] = perm(perm(aCl, aCu, 0x0040), perm(aU, aL, 0x0040), 0x5410);
         hbot = H[kTR - 1];
         fbot = f;
         if (sl == W - 1 && b + 1 < nb) {
@@ -325,49 +301,156 @@ __global__ void __launch_bounds__(32 * kTWarps) match_kernel(const TraceArgs a) 
       }
     }
   }
-  // the walks, while the pairs' flags are still in L2 (the warp's stores are
-  // visible to the warp after the warp barrier); their windows take the
-  // place of the fronts' profiles
+  // the walks, one after another, while the pairs' flags are still in L2 (the
+  // warp's stores are visible to the warp after the warp barrier); window and
+  // queue take the place of the fronts' profiles
   __syncwarp();
-  static_assert(S * sizeof(WalkWindow) <= kTProfBytes, "walk windows fit the profile's space");
-  walk_pairs<W>(a, p, lane, reinterpret_cast<WalkWindow*>(s_prof[warp])[front]);
+  static_assert(4096 + kQueue * sizeof(int2) <= kTProfBytes, "window and queue fit the profile's space");
+  for (int f = 0; f < S; ++f) {
+    const int q = __shfl_sync(0xffffffffu, p, f * W);
+    if (q < 0) break;   // pairs fill the fronts from the first on
+    MatchWindow<W> win{a.nib + a.nib_off[q], reinterpret_cast<uint32_t*>(s_prof[warp]), a.len[a.px[q]]};
+    walk_pair(a, q, win, reinterpret_cast<int2*>(s_prof[warp] + 4096));
+  }
+}
+
+// ---- the pipeline form ------------------------------------------------------------
+
+// The pipeline's scores: a byte profile of the warp's band (S' = S + 2 ge, as a
+// signed byte) and the CTA's copy of X's codes, both in shared memory.
+struct TraceScore {
+  uint32_t* prof;        // this warp's, [letter][lane] words of four rows
+  const int8_t* xs;      // X's codes from column -32 on
+  const int8_t* s_sub;   // the matrix plus 2 ge
+  const int8_t* Y;
+  int lx, ly;
+  uint32_t zero;         // 2 ge in every byte: rows past Y
+  int row0 = 0, sum = 0; // first row of the lane; sum of u(r, lx - 1) over its rows
+  __device__ __forceinline__ void load(int g) {
+    const int lane = threadIdx.x & 31;
+    row0 = g * 128 + 4 * lane;
+    __syncwarp();
+    build_profile<4>(prof, s_sub, Y, row0, ly, zero, lane);
+    __syncwarp();
+  }
+  __device__ __forceinline__ void begin(int, pipe::Link&) const {}
+  __device__ __forceinline__ void end(int) const {}
+  __device__ __forceinline__ void get(int, int t, int (&s)[4]) const {
+    const int lane = threadIdx.x & 31;
+    const uint32_t w = prof[(int)xs[32 + t - lane] * 32 + lane];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) s[r] = (int)perm(w, 0u, r | (r | 8) << 4 | (r | 8) << 8 | (r | 8) << 12);
+  }
+  __device__ __forceinline__ void column_done(int t, const int (&n)[4]) {
+    if (t >= lx - 1 && t - (int)(threadIdx.x & 31) == lx - 1) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (row0 + r < ly) sum -= n[r];
+    }
+  }
+  __device__ __forceinline__ void band_done() const {}
+};
+
+constexpr int kTraceWindow = 8192;   // bytes of flags in the walk's window
+
+// Dynamic shared memory of a pipeline CTA: profiles, then X's codes; the walk's
+// window and queue take their place.
+inline size_t trace_pipe_smem(int wpc, int lx_max) {
+  const size_t score = (size_t)wpc * kLetters * 128 + (size_t)(lx_max + 128);
+  const size_t walk = kTraceWindow + kQueue * sizeof(int2);
+  return (std::max(score, walk) + 127) / 128 * 128;
+}
+
+// C CTAs (one cluster) per pair.
+__global__ void __launch_bounds__(32 * pipe::kWarps, 4) trace_pipe_kernel(const TraceArgs a, int C) {
+  __shared__ pipe::Inbox s_box[pipe::kWarps];
+  __shared__ __align__(16) int8_t s_sub[kLetters * kLetters];
+  extern __shared__ __align__(128) unsigned char s_dyn[];
+  const int p = a.order[blockIdx.x / C], rank = blockIdx.x % C;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
+  const int gw = rank * wpc + warp, nwarp = C * wpc;
+  const int ix = a.px[p], iy = a.py[p];
+  const int8_t* X = a.codes + a.start[ix];
+  const int Lx = a.len[ix], Ly = a.len[iy];
+  int8_t* xs = reinterpret_cast<int8_t*>(s_dyn) + wpc * kLetters * 128;
+  for (int e = threadIdx.x; e < kLetters * kLetters; e += blockDim.x) s_sub[e] = (int8_t)(a.sub[e] + 2 * a.ge);
+  for (int e = threadIdx.x; e < Lx + 80; e += blockDim.x)   // 32 before column 0, past the last superstep
+    xs[e] = e >= 32 && e - 32 < Lx ? (int8_t)tclamp(X[e - 32]) : (int8_t)0;
+  pipe::init_inboxes(s_box, wpc);
+  pipe::Link ln;
+  ln.in = &s_box[warp];
+  ln.out = pipe::cluster_addr(pipe::smem_addr(&s_box[(gw + 1) % wpc]), (gw + 1) % nwarp / wpc);
+  ln.back = pipe::cluster_addr(pipe::smem_addr(&s_box[(gw + nwarp - 1) % wpc]), (gw + nwarp - 1) % nwarp / wpc);
+  ln.err = a.err;
+  TraceScore sc{reinterpret_cast<uint32_t*>(s_dyn) + warp * kLetters * 32, xs, s_sub, a.codes + a.start[iy], Lx, Ly,
+                0x01010101u * (uint32_t)(2 * a.ge & 255)};
+  uint32_t* fl = a.nib + a.nib_off[p];
+  pipe::run_bands<4>(ln, pipe::Wrap{reinterpret_cast<int2*>(a.scratch + (size_t)p * 4 * a.scratch_cols), a.done + p},
+                     sc, fl, Lx, Ly, a.go - a.ge, gw, nwarp);
+  // H(Ly-1, Lx-1): the last column's sum of u, less the free extension's ge a cell
+  const int sum = __reduce_add_sync(0xffffffffu, sc.sum) - (gw == 0 ? a.ge * (Lx + Ly) : 0);
+  if (lane == 0 && sum != 0) atomicAdd(&a.score[p], sum);
+  pipe::cluster_barrier();   // every band's flags are written
+  if (rank != 0 || warp != 0) return;
+  pipe::Window<4, kTraceWindow> win{fl, reinterpret_cast<uint32_t*>(s_dyn), pipe::supersteps_of(Lx)};
+  walk_pair(a, p, win, reinterpret_cast<int2*>(s_dyn + kTraceWindow));
 }
 
 }  // namespace
 
 struct TraceState {
-  DevBuf codes, start, len, px, py, order, off, nib, scratch, score, outx, outy, outlen;
+  DevBuf codes, start, len, px, py, order, off, nib, scratch, score, outx, outy, outlen, done;
   ~TraceState() {
-    for (DevBuf* b : {&codes, &start, &len, &px, &py, &order, &off, &nib, &scratch, &score, &outx, &outy, &outlen})
+    for (DevBuf* b : {&codes, &start, &len, &px, &py, &order, &off, &nib, &scratch, &score, &outx, &outy, &outlen, &done})
       b->release();
   }
 };
 
 namespace {
 
-// Front width of the match kernel for a set of pairs: the least estimated
-// cost, in cells, of the rows x columns computed (whole bands of 8W rows,
-// ramps of W-1 columns) plus the walks, which run one after another for the
-// 32/W fronts of a warp (a walk step costs about as much as kWalkStep cells:
-// fitted to the kernel's times at W = 32, 16 and 8 on 3,640 pairs of 100-300
-// residues on a GB300: 0.436, 0.422 and 0.652 ms).
-constexpr double kWalkStep = 38.0;
-int trace_lanes(const std::vector<int32_t>& len, const int32_t* px, const int32_t* py, int npairs) {
-  int best = 32;
-  double best_cost = 0.0;
-  for (int W : {32, 16, 8}) {
-    const int band = 8 * W;
-    double cost = 0.0;
-    for (int k = 0; k < npairs; ++k) {
-      const int Lx = len[px[k]], Ly = len[py[k]];
-      cost += (double)((Ly + band - 1) / band) * band * (Lx + W - 1) + kWalkStep * (32 / W) * (Lx + Ly);
-    }
-    if (W == 32 || cost < best_cost) {
-      best = W;
-      best_cost = cost;
-    }
+// Front width of the match kernel: 16 lanes (two pairs a warp, bands of 128
+// rows, ramps of 15 columns) for short Y, else 32.  Kernel times on a GB300 at
+// W = 32 / 16 / 8, ms: 4,000 pairs of 60 residues 0.143 / 0.092 / 0.151, 1,000
+// of 100 0.086 / 0.156 / 0.252, 4,000 of 190 0.44 / 0.66 / 1.25 (a second band
+// of a narrow front waits for the first one's row).
+constexpr int kShortRows = 80;
+int trace_lanes(double mean_rows) { return mean_rows <= kShortRows ? 16 : 32; }
+
+// Whether the pipeline form gives this context's alignments of sequences up to
+// maxlen: it needs open >= extension, scores that fit a signed byte with the
+// extension folded in, X's codes in shared memory, and lengths at which the
+// recurrence's finite sentinel (-32768 + ge before row 0 and column 0) never
+// beats a gap opened at the border.
+bool pipe_ok(const Ctx& c, int maxlen) {
+  int smin = 127, smax = -128;
+  for (int k = 0; k < kLetters * kLetters; ++k) {
+    smin = std::min<int>(smin, c.sub[k]);
+    smax = std::max<int>(smax, c.sub[k]);
   }
-  return best;
+  return c.go >= c.ge && smin + 2 * c.ge >= -128 && smax + 2 * c.ge <= 127 && 2 * c.ge <= 127 && maxlen <= 100000 &&
+         (int64_t)c.ge * (maxlen + 1) + c.go < 32768;
+}
+
+cudaError_t launch_pipe(const TraceArgs& a, int first, int count, int warps, int lx_max, cudaStream_t s) {
+  const int C = (warps + pipe::kWarps - 1) / pipe::kWarps;
+  const int wpc = (warps + C - 1) / C;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(count * C));
+  cfg.blockDim = dim3((unsigned)(32 * wpc));
+  cfg.dynamicSmemBytes = trace_pipe_smem(wpc, lx_max);
+  cfg.stream = s;
+  const cudaError_t e = cudaFuncSetAttribute(trace_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)trace_pipe_smem(pipe::kWarps, lx_max));
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  TraceArgs b = a;
+  b.order += first;
+  return cudaLaunchKernelEx(&cfg, trace_pipe_kernel, b, C);
 }
 
 cudaError_t launch_match(int W, const TraceArgs& a, cudaStream_t s) {
@@ -380,6 +463,53 @@ cudaError_t launch_match(int W, const TraceArgs& a, cudaStream_t s) {
 }
 
 }  // namespace
+
+// The pipeline launches of one batch (pairs in order: most bands first).  A
+// pair takes one warp per band over as many CTAs (of four warps) as that needs,
+// at most so many that all pairs' CTAs come to about five an SM; a deeper pair
+// runs its bands in passes.  With one CTA a pair, pairs of one or two bands go
+// to CTAs of as many warps, in launches of their own side by side (a launch's
+// shape is its first pair's).  Kernel times on a GB300 against one warp per
+// pair: 4,000 pairs of 210 residues 0.71 to 0.38 ms, 200 of 867 4.0 to 0.40 ms,
+// 200 of 2,000 21.1 to 1.6 ms (one CTA each 3.3), 1,500 of 867 4.45 to 1.43 ms
+// (two CTAs each 2.0), one of 2,000 5.3 to 0.40 ms.
+static int launch_pipes(Ctx* c, const TraceArgs& a, const std::vector<int32_t>& order,
+                        const std::vector<int32_t>& len, const int32_t* px, const int32_t* py, cudaStream_t s) {
+  const int m = (int)order.size();
+  auto bands = [&](int k) { return (len[py[order[(size_t)k]]] + 127) / 128; };
+  int lx = 1;
+  for (int k = 0; k < m; ++k) lx = std::max(lx, len[px[k]]);
+  const int ctas = std::min(std::max((5 * c->sms + m / 2) / m, 1), pipe::kCluster);
+  int rc;
+  if (ctas > 1) return c->cuda(launch_pipe(a, 0, m, std::min(bands(0), ctas * pipe::kWarps), lx, s), "traceback launch");
+  int first[4] = {0, 0, 0, m};   // pairs of three bands or more, of two, of one
+  while (first[1] < m && bands(first[1]) > 2) ++first[1];
+  first[2] = first[1];
+  while (first[2] < m && bands(first[2]) > 1) ++first[2];
+  for (int g = 2; g > 0; --g)   // a group that would not fill the SMs joins the wider one
+    if (first[g + 1] - first[g] < c->sms) first[g] = first[g + 1];
+  // the first non-empty group stays on the stream, the others fork from it
+  if ((rc = c->cuda(cudaEventRecord(c->fork_ev, s), "fork"))) return rc;
+  int used = 0, b = -1;
+  for (int g = 0; g < 3; ++g) {
+    const int count = first[g + 1] - first[g];
+    if (count == 0) continue;
+    cudaStream_t bs = s;
+    if (b >= 0) {
+      bs = c->branch[(size_t)b];
+      if ((rc = c->cuda(cudaStreamWaitEvent(bs, c->fork_ev, 0), "fork"))) return rc;
+    }
+    if ((rc = c->cuda(launch_pipe(a, first[g], count, std::min(bands(first[g]), pipe::kWarps), lx, bs),
+                      "traceback launch")))
+      return rc;
+    if (b >= 0 && (rc = c->cuda(cudaEventRecord(c->join_ev[(size_t)b], bs), "join"))) return rc;
+    if (used++) ++c->launches;   // the caller counts the first
+    ++b;
+  }
+  for (int k = 0; k < b; ++k)
+    if ((rc = c->cuda(cudaStreamWaitEvent(s, c->join_ev[(size_t)k], 0), "join"))) return rc;
+  return NWG_OK;
+}
 
 void Ctx::extra_release() {
   delete reinterpret_cast<TraceState*>(trace_state);
@@ -433,8 +563,15 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
       if (e) cudaEventDestroy(e);
     }
   } guard{ev_copied};
-  const int W = trace_lanes_forced ? trace_lanes_forced : trace_lanes(len, px, py, npairs);
-  const int band = 8 * W;
+  double mean_rows = 0.0;
+  for (int k = 0; k < npairs; ++k) mean_rows += len[py[k]];
+  mean_rows /= npairs;
+  const int W = trace_lanes_forced ? trace_lanes_forced : trace_lanes(mean_rows);
+  // the pipeline form, except for many short pairs (4,000 of 60 residues: 0.111
+  // against 0.092 ms with two pairs a warp; 2,000: 0.054 against 0.067)
+  const bool piped = !trace_lanes_forced && pipe_ok(*this, maxlen) &&
+                     !(mean_rows <= kShortRows && npairs > 4 * pipe::kWarps * sms);
+  const int band = piped ? 128 : 8 * W;
   int k0 = 0;
   while (k0 < npairs) {
     std::vector<int64_t> off;
@@ -442,7 +579,8 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
     int k1 = k0;
     while (k1 < npairs) {
       const int Lx = len[px[k1]], Ly = len[py[k1]];
-      const int64_t w = (int64_t)((Ly + band - 1) / band) * (Lx + W - 1) * W;
+      const int64_t w = piped ? (int64_t)((Ly + band - 1) / band) * pipe::supersteps_of(Lx) * 128
+                              : (int64_t)((Ly + band - 1) / band) * (Lx + W - 1) * W;
       if (k1 > k0 && words + w > kBudgetWords) break;
       off.push_back(words);
       words += w;
@@ -462,7 +600,8 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
         (rc = T.off.ensure(sizeof(int64_t) * m)) || (rc = T.nib.ensure(sizeof(uint32_t) * (size_t)words)) ||
         (rc = T.scratch.ensure(sizeof(int32_t) * 4 * (size_t)m * maxlen)) ||
         (rc = T.score.ensure(sizeof(int32_t) * m)) || (rc = T.outx.ensure((size_t)m * stride)) ||
-        (rc = T.outy.ensure((size_t)m * stride)) || (rc = T.outlen.ensure(sizeof(int32_t) * m)))
+        (rc = T.outy.ensure((size_t)m * stride)) || (rc = T.outlen.ensure(sizeof(int32_t) * m)) ||
+        (rc = T.done.ensure(sizeof(int32_t) * ((size_t)m + 1))))
       return fail(rc, "traceback allocation");
     if ((rc = cuda(cudaMemcpyAsync(T.px.p, px + k0, sizeof(int32_t) * m, cudaMemcpyHostToDevice, s), "upload")) ||
         (rc = cuda(cudaMemcpyAsync(T.py.p, py + k0, sizeof(int32_t) * m, cudaMemcpyHostToDevice, s), "upload")) ||
@@ -490,9 +629,18 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
     a.go = go;
     a.ge = ge;
     a.sub = (const int8_t*)b_sub.p;
+    a.done = (unsigned*)T.done.p;
+    a.err = (int*)T.done.p + m;
+    if (piped && ((rc = cuda(cudaMemsetAsync(T.done.p, 0, sizeof(int32_t) * ((size_t)m + 1), s), "traceback")) ||
+                  (rc = cuda(cudaMemsetAsync(T.score.p, 0, sizeof(int32_t) * m, s), "traceback"))))
+      return rc;
     if (st) cudaEventRecord(ev0, s);
     ++launches;
-    if ((rc = cuda(launch_match(W, a, s), "traceback launch"))) return rc;
+    if (piped) {
+      if ((rc = launch_pipes(this, a, order, len, px + k0, py + k0, s))) return rc;
+    } else if ((rc = cuda(launch_match(W, a, s), "traceback launch"))) {
+      return rc;
+    }
     if (st) cudaEventRecord(ev1, s);
     if ((rc = cuda(cudaMemcpyAsync(outx + (size_t)k0 * stride, T.outx.p, (size_t)m * stride, cudaMemcpyDeviceToHost, s),
                    "download")) ||
@@ -504,8 +652,11 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
     if (score &&
         (rc = cuda(cudaMemcpyAsync(score + k0, T.score.p, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, s), "download")))
       return rc;
+    int err = 0;
+    if (piped && (rc = cuda(cudaMemcpyAsync(&err, a.err, sizeof(err), cudaMemcpyDeviceToHost, s), "download"))) return rc;
     if (st) cudaEventRecord(ev_copied, s);
     if ((rc = cuda(cudaStreamSynchronize(s), "traceback sync"))) return rc;
+    if (err) return fail(NWG_ERR_TIMEOUT, "traceback: a bounded device wait ran out");
     if (st) {
       for (int k = k0; k < k1; ++k) st->cells += (int64_t)len[px[k]] * len[py[k]];
       float ms = 0.f, ms2 = 0.f;
