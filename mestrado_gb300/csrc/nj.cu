@@ -29,31 +29,24 @@
 // since the last build; that bound is tracked and any check it cannot exclude
 // is counted.
 //
-// Search per join:
-//  1. one streaming pass over the live triangle of D (4 B per live pair):
-//     q in float, fl(fl(fl(d*(n-2)) - Tf_r) - Tf_c) with Tf the float copy of
-//     T; per row its two smallest q (and the column of the smallest), overall
-//     the minimum and the largest magnitude M = |d|(n-2) + |T_r| + |T_c|.
-//     Every float q is within E = 8 * 2^-24 * M of the exact q.
-//  2. the candidates are the pairs whose float q is at most min + 3E: when
-//     each row within that threshold has one such pair (its second smallest q
-//     is beyond), they are those rows' minima; otherwise the rows are scanned
-//     again into a list (up to 2048 candidates; beyond that, as in the
-//     one-CTA form always, the CTAs reduce their first candidates and a
-//     second scan counts the ties).  Each candidate gets its exact double q in
-//     both roundings.
+// Search per join: q in float, fl(fl(fl(d*(n-2)) - Tf_r) - Tf_c) with Tf the
+// float copy of T, is within E = 8 * 2^-24 * M of the exact q, M the largest
+// |d|(n-2) + |T_r| + |T_c|.  The candidates are the pairs whose float q is at most
+// the smallest + 3E; each gets its exact double q in both roundings.  One CTA
+// looks at every pair for every join; a team of CTAs keeps a lower bound per row
+// and looks only at the rows whose bound reaches the best known pair (the section
+// on the lazy search).
 // The winner follows the tie-break; the ambiguity check runs over the
 // candidates: any pair left out has q > winner + E, beyond reach of either
 // rounding.  All floating-point operations use the _rn intrinsics in the
 // reference's evaluation order (no contraction).
 //
-// Four launch forms run a job's whole join loop (several jobs per launch in
+// Three launch forms run a job's whole join loop (several jobs per launch in
 // the serving loop):
-//  * one CTA with the job in its shared memory (up to 160 taxa);
-//  * one thread-block cluster with the matrix in its distributed shared
-//    memory (up to 768 taxa);
-//  * one cluster with the matrix in global memory (up to 2048 taxa);
-//  * the whole GPU, one cooperative launch per segment between compactions
+//  * one CTA with the job in its shared memory (up to 136 taxa);
+//  * one thread-block cluster, the matrix in L2 (up to 600 taxa, and every larger
+//    job of the serving loop);
+//  * the whole GPU, one cooperative launch per segment between rebuilds
 //    (compacted to the live slots, in slot order), above that.
 #include <algorithm>
 #include <cfloat>
@@ -85,11 +78,19 @@ struct NJDev {
   unsigned long long* stats;  // [0] ambiguous steps, [1] tie steps, [2] internal errors,
                               // [3] open heap-size checks, [4] rebuilds (cluster form)
   nwg_join* joins;
+  int* prow;           // slot -> its row's place in D (n0: xrow); [n0] the free place
+  float* xrow;         // one more row (ld floats)
+  double* tx;          // [2 * n0]: every slot's T for the exchanges of even and of odd number
   int n0;              // slots
   int ld;              // row stride of D (floats), a multiple of 4
   int cand_cap;        // candidate list capacity
   int pad;
 };
+
+// Row at place q of the matrix.
+__device__ __forceinline__ float* row_at(const NJDev& s, int q) {
+  return q < s.n0 ? s.D + (size_t)q * s.ld : s.xrow;
+}
 
 __device__ __forceinline__ int ford(float f) {
   // order-preserving map float -> int (for atomicMin / atomicMax)
@@ -148,7 +149,7 @@ __global__ void rowsum_kernel(NJDev s, const int* abort) {
   const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (k >= na) return;
   const int sk = s.slot[s.act[k]];
-  const float* row = s.D + (size_t)sk * s.ld;
+  const float* row = row_at(s, s.prow[sk]);
   double part = 0.0, ab = 0.0;
   int lowexp = INT_MAX;
   for (int j = lane; j < na; j += 32) {
@@ -189,32 +190,7 @@ __device__ __forceinline__ void record_pick(const NJDev& s, const PickOut& r) {
   else if (r.ties > 1) atomicAdd(&s.stats[1], 1ull);
 }
 
-// ---- large n: one cooperative launch over the whole GPU per segment ---------
-// Every CTA takes part in every phase of every join, with two grid barriers
-// per join in the usual case:
-//  P  the live triangle, one row pair (p, n0-1-p) per warp, warps numbered
-//     across CTAs first; 16-byte loads (rows are padded to a multiple of 4
-//     floats and the padding's float row sums are NaN).  Per row its two
-//     smallest float q and the column of the smallest (grmin, grec); per CTA
-//     the smallest q and the largest magnitude (part).
-//  -- barrier --
-//  K  every CTA reduces the CTA partials to the candidate threshold and finds
-//     the rows whose minimum is within it.  When each such row's second
-//     smallest q is beyond the threshold, the candidates are exactly those
-//     rows' minima: every CTA evaluates them (exact q in both roundings) and
-//     takes the same winner.  Otherwise (ties, close pairs) every CTA scans
-//     its slice of the selected rows into a global list and, after one more
-//     barrier, picks from it.
-//  J  every CTA applies the join to its own share of the slots (T, the new
-//     row and column, the new row's values with their exponent range and
-//     integer sum) and of the active list (shifted into the other list).
-//  -- barrier --
-// At the start of the next join (or at the end of the segment) every CTA
-// combines the shares into the new node's row sum and writes it, with the
-// dead slot's NaN and the slot -> node map, itself -- the same values in
-// every CTA, so each CTA reads its own writes; CTA 0 keeps the join record
-// (branch lengths are filled in after the loop) and the id -> slot map.
-// Rebuilds (row sums) and compactions run between segments.
+// ---- candidates, the grid barrier ------------------------------------------
 
 struct GCand {
   long long k1, k2;   // order-preserving integer keys of q1 and q2
@@ -234,23 +210,17 @@ struct KCand {
 };
 
 struct GridNJ {
-  unsigned* bar;        // [0] barrier arrivals (counts up from 0 per launch)
+  unsigned* bar;        // [0] barrier arrivals, [1] publications (both count up from 0 per launch)
   int* abort;           // set when a barrier wait gave up; every CTA then leaves
-  int* act2;            // the other active list (the join writes the shifted list there)
-  int* grmin;           // per slot: smallest float q of the row's pairs (ordered int)
-  int4* grec;           // per slot: second smallest q (ordered int), column and distance of the smallest
-  double* tsnap;        // per slot: T as the pass saw it (the pick reads these, never T itself)
-  float* tv;            // per slot: the new row's value
-  float* part;          // [2 * grid]: per CTA smallest q and largest magnitude
-  long long* jsum;      // [2 * grid]: per CTA integer sum and sum of magnitudes (units of 2^jexp)
-  int* jexp;            // [2 * grid]: per CTA lowest and highest exponent of its values
+  float4* gather;       // [2 * CTAs]: the grid's exchanges
   KCand* cand;          // the candidate list of the fallback scan
-  KCand* cbest;         // [grid]: per CTA its first candidate of the fallback scan
+  KCand* cbest;         // [CTAs]: per CTA its first candidate of the fallback scan
+  int stall;            // failure injection: the first CTA never publishes
+  int pad;
 };
 
 constexpr long long kBarrierSpinCycles = 4000000000ll;   // about two seconds: no phase takes a millisecond
 constexpr int kFastRows = 32;                             // candidate rows the direct pick evaluates
-constexpr int kGridMax = 256;                             // CTAs of the cooperative launch, at most
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
@@ -339,92 +309,6 @@ __device__ __forceinline__ void pass_elem(float d, float tc, int c, float tr, fl
   c1 = lt ? c : c1;
   m1 = lt ? q : m1;
   mag = fmaxf(mag, __fadd_rn(fabsf(x), fabsf(tc)));
-}
-
-// Odd joins scan every row backwards: the lines the previous pass read last
-// are still in L2 when the triangle is a little larger than L2.
-__device__ void grid_pass(const NJDev& s, const GridNJ& g, Team tm, float nm2f, bool rev) {
-  __shared__ float sq[32], sm[32];
-  const int lane = threadIdx.x & 31;
-  const int n0 = s.n0, nv = s.ld >> 2;
-  const int nw = tm.size * (int)(blockDim.x >> 5);
-  const int npairs = (n0 + 1) >> 1;
-  const float4* Tf4 = reinterpret_cast<const float4*>(s.Tf);
-  float qmin = FLT_MAX, mmax = 0.f;
-  for (int p = (int)(threadIdx.x >> 5) * tm.size + tm.rank; p < npairs; p += nw) {
-    for (int h = 0; h < 2; ++h) {
-      if (n0 - 1 - p == p && h) break;
-      const int r = (h != (int)rev) ? n0 - 1 - p : p;
-      const float tr = s.Tf[r];
-      if (tr != tr) {   // dead slot
-        if (lane == 0) g.grmin[r] = 0x7F7FFFFF;
-        continue;
-      }
-      const double Tr = s.T[r];
-      const float* row = s.D + (size_t)r * s.ld;
-      float m1 = FLT_MAX, m2 = FLT_MAX, mag = 0.f;
-      int c1 = -1;
-      const int c0 = r + 1, v0 = (c0 + 3) >> 2;
-      // columns c0 .. 4*v0-1 (at most three) one by one
-      if (lane < 4 * v0 - c0 && c0 + lane < n0)
-        pass_elem(row[c0 + lane], s.Tf[c0 + lane], c0 + lane, tr, nm2f, m1, m2, c1, mag);
-      const float4* row4 = reinterpret_cast<const float4*>(row);
-      auto vec = [&](int v) {
-        const float4 d = row4[v];
-        const float4 tc = Tf4[v];
-        pass_elem(d.x, tc.x, 4 * v, tr, nm2f, m1, m2, c1, mag);
-        pass_elem(d.y, tc.y, 4 * v + 1, tr, nm2f, m1, m2, c1, mag);
-        pass_elem(d.z, tc.z, 4 * v + 2, tr, nm2f, m1, m2, c1, mag);
-        pass_elem(d.w, tc.w, 4 * v + 3, tr, nm2f, m1, m2, c1, mag);
-      };
-      if (!rev) {
-#pragma unroll 4
-        for (int v = v0 + lane; v < nv; v += 32) vec(v);
-      } else {
-#pragma unroll 4
-        for (int v = nv - 1 - lane; v >= v0; v -= 32) vec(v);
-      }
-      // the row's two smallest over the warp (an equal pair makes m2 = m1)
-      for (int o = 16; o > 0; o >>= 1) {
-        const float om1 = __shfl_xor_sync(0xffffffffu, m1, o);
-        const float om2 = __shfl_xor_sync(0xffffffffu, m2, o);
-        const int oc1 = __shfl_xor_sync(0xffffffffu, c1, o);
-        const bool take = om1 < m1 || (om1 == m1 && oc1 < c1);
-        const float lo = take ? om1 : m1, hi = take ? m1 : om1;
-        m2 = fminf(hi, fminf(m2, om2));
-        m1 = lo;
-        c1 = take ? oc1 : c1;
-        mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, o));
-      }
-      if (lane == 0) {
-        // the pick reads only what the pass wrote: a fast CTA's join share may
-        // already be changing T and D while a slow one still picks
-        g.grmin[r] = ford(m1);
-        g.grec[r] = make_int4(ford(m2), c1, __float_as_int(c1 >= 0 ? row[c1] : 0.f), 0);
-        g.tsnap[r] = Tr;
-      }
-      qmin = fminf(qmin, m1);
-      mmax = fmaxf(mmax, __fadd_rn(mag, fabsf(tr)));
-    }
-  }
-  if (lane == 0) {
-    sq[threadIdx.x >> 5] = qmin;
-    sm[threadIdx.x >> 5] = mmax;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int nwb = (int)(blockDim.x >> 5);
-    qmin = lane < nwb ? sq[lane] : FLT_MAX;
-    mmax = lane < nwb ? sm[lane] : 0.f;
-    for (int o = 16; o > 0; o >>= 1) {
-      qmin = fminf(qmin, __shfl_xor_sync(0xffffffffu, qmin, o));
-      mmax = fmaxf(mmax, __shfl_xor_sync(0xffffffffu, mmax, o));
-    }
-    if (lane == 0) {
-      g.part[2 * tm.rank] = qmin;
-      g.part[2 * tm.rank + 1] = mmax;
-    }
-  }
 }
 
 // A candidate from its pair: slots r, c with their node ids, T and d.
@@ -568,160 +452,6 @@ __device__ __forceinline__ void add_counts(unsigned ties, unsigned amb, int* cnt
   }
 }
 
-// K.  Returns 1 when the winner is in *win, 0 when the fallback scan is
-// needed (the same in every CTA).
-__device__ int grid_pick_direct(const NJDev& s, const GridNJ& g, Team tm, double nm2, float nm2f, int watermark, GCand* win,
-                                PickOut* pk, float* sthr) {
-  __shared__ int rows[kFastRows];
-  __shared__ GCand fc[kFastRows];
-  __shared__ int nrows, s_ok;
-  const int n0 = s.n0;
-  // the row minima load together with the CTA partials (n0 <= 8 * blockDim)
-  constexpr int kPerThread = 8;
-  int rm[kPerThread];
-#pragma unroll
-  for (int t = 0; t < kPerThread; ++t) {
-    const int p = (int)threadIdx.x + t * (int)blockDim.x;
-    rm[t] = p < n0 ? g.grmin[p] : 0x7F7FFFFF;
-  }
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    float q = FLT_MAX, m = 0.f;
-    // every partial in flight at once (at most kGridMax CTAs)
-#pragma unroll
-    for (int t = 0; t < kGridMax / 32; ++t) {
-      const int b = l + 32 * t;
-      if (b < tm.size) {
-        const float2 pm = reinterpret_cast<const float2*>(g.part)[b];
-        q = fminf(q, pm.x);
-        m = fmaxf(m, pm.y);
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      q = fminf(q, __shfl_xor_sync(0xffffffffu, q, o));
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    }
-    if (l == 0) {
-      *sthr = q + 3.f * (8.f * 5.9604645e-8f * m) + 1e-30f;
-      nrows = 0;
-    }
-  }
-  __syncthreads();
-  const float thr = *sthr;
-  const int othr = ford(thr);
-#pragma unroll
-  for (int t = 0; t < kPerThread; ++t) {
-    if (rm[t] <= othr) {
-      const int k = atomicAdd(&nrows, 1);
-      if (k < kFastRows) rows[k] = (int)threadIdx.x + t * (int)blockDim.x;
-    }
-  }
-  __syncthreads();
-  const int nr = nrows;
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    int ok = nr >= 1 && nr <= kFastRows;
-    if (ok && l < nr) {
-      const int r = rows[l];
-      const int4 rec = g.grec[r];
-      const int c = rec.y;
-      if (rec.x <= othr || c < 0) {
-        ok = 0;   // a second pair of the row within the threshold
-      } else {
-        const int ur = s.node[r], uc = s.node[c];
-        const double Tr = g.tsnap[r], Tc = g.tsnap[c];
-        const float d = __int_as_float(rec.z);
-        fc[l] = make_cand(r, c, ur, uc, Tr, Tc, d, nm2, watermark);
-        if (ur < 0 || uc < 0) ok = 0;
-      }
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    PickOut r{};
-    if (ok && nr == 1) {
-      r.idx = 0;     // one candidate: the winner, a tie with itself only
-      r.ties = 1;
-      r.amb = 0;
-      r.error = false;
-    } else if (ok) {
-      r = pick_keys(nr, [&](int k) { return fc[k]; });
-    }
-    if (l == 0) {
-      s_ok = ok;
-      if (ok) {
-        *pk = r;
-        *win = fc[r.idx];
-      }
-    }
-  }
-  __syncthreads();
-  return s_ok;
-}
-
-// K, fallback: visit(pred, candidate) for this CTA's share of the pairs of
-// every row within the threshold, called by whole warps together (pred is
-// false on lanes without a candidate in that step); the same pairs on every
-// call of one join.  Up to kSplitRows rows, the team's warps split each row's
-// columns; more rows (wide ties), one warp per row, warps numbered across the
-// team, lanes over the columns.
-constexpr int kSplitRows = 16;
-
-template <class Visit>
-__device__ void grid_cand_scan(const NJDev& s, const GridNJ& g, Team tm, float nm2f, double nm2, int watermark,
-                               float thr, Visit&& visit) {
-  constexpr int kRows = 512;
-  __shared__ int rows[kRows];
-  __shared__ int nrows;
-  const int n0 = s.n0;
-  const int othr = ford(thr);
-  if (threadIdx.x == 0) nrows = 0;
-  __syncthreads();
-  for (int p = threadIdx.x; p < n0; p += blockDim.x) {
-    if (g.grmin[p] <= othr) {
-      const int t = atomicAdd(&nrows, 1);
-      if (t < kRows) rows[t] = p;
-    }
-  }
-  __syncthreads();
-  const bool all = nrows > kRows;   // more near-minimal rows than the list holds: every row
-  const int nr = all ? n0 : nrows;
-  const int lane = threadIdx.x & 31;
-  const int wpc = (int)blockDim.x >> 5;
-  const int gw = tm.rank * wpc + ((int)threadIdx.x >> 5), nw = tm.size * wpc;
-  // columns c0 + lane, c0 + cstep + lane, ... of row r (c0 and cstep the same in the warp)
-  auto scan_row = [&](int r, int c0, int cstep) {
-    const int ur = s.node[r];
-    if (ur < 0 || g.grmin[r] > othr) return;
-    const float tr = s.Tf[r];
-    const double Tr = s.T[r];
-    const float* row = s.D + (size_t)r * s.ld;
-    for (int cb = c0; cb < n0; cb += cstep) {
-      const int c = cb + lane;
-      bool pred = false;
-      KCand kc = kc_none();
-      if (c < n0) {
-        const int uc = s.node[c];
-        const float d = row[c];
-        const float q = __fsub_rn(__fsub_rn(__fmul_rn(d, nm2f), tr), s.Tf[c]);
-        if (uc >= 0 && q <= thr) {
-          const GCand cd = make_cand(r, c, ur, uc, Tr, s.T[c], d, nm2, watermark);
-          kc = KCand{cd.k1, cd.k2, cd.a, cd.b};
-          pred = true;
-        }
-      }
-      visit(pred, kc);
-    }
-  };
-  if (nr <= kSplitRows) {
-    for (int t = 0; t < nr; ++t) {   // every CTA's list holds the same rows, in its own order
-      const int r = all ? t : rows[t];
-      scan_row(r, r + 1 + 32 * gw, 32 * nw);
-    }
-  } else {
-    // rows by slot (an order the same in every CTA); scan_row skips the others
-    for (int r = gw; r < n0; r += nw) scan_row(r, r + 1, 32);
-  }
-}
-
 // A warp's candidates of one scan step into the list, one atomic per warp.
 // s.g32[2] ends at the number of candidates when that is at most
 // kListPickMax, else above kListPickMax: a warp that saw the count pass it
@@ -738,35 +468,6 @@ __device__ __forceinline__ void list_push(const NJDev& s, const GridNJ& g, bool 
   full = base + __popc(bal) > kListPickMax;
 }
 
-// The scan into the candidate list; returns this thread's first candidate
-// (reduced over the CTA only when the list is not used).
-__device__ KCand grid_cand(const NJDev& s, const GridNJ& g, Team tm, float nm2f, double nm2, int watermark, float thr) {
-  KCand first = kc_none();
-  bool full = false;
-  grid_cand_scan(s, g, tm, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
-    list_push(s, g, pred, c, full);
-    if (pred && kc_first(c, first)) first = c;
-  });
-  return first;
-}
-
-// The second scan of a long list: ties and ambiguous pairs against the winner
-// w into s.g32[0] and s.g32[1].
-__device__ void grid_cand_count(const NJDev& s, const GridNJ& g, Team tm, float nm2f, double nm2, int watermark,
-                                float thr, const KCand& w) {
-  unsigned ties = 0, amb = 0;
-  grid_cand_scan(s, g, tm, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
-    if (pred) count_vs(c, w, ties, amb);
-  });
-  add_counts(ties, amb, s.g32);
-}
-
-// J: this CTA's share of the slots (SpeciesBlock.cpp:787-841: tmp = ((Dik +
-// Djk) - d) / 2 in float, T[k] += (float)(tmp - (Dik + Djk)), the new row and
-// column of slot si, whose diagonal keeps i's old value) and of the active
-// list; the share's exponent range and integer sum go to jexp / jsum.  The
-// shares hold at most one slot and one list position per thread (the launch
-// has at least n0 / blockDim CTAs).
 // An exact sum of floats as u * 2^e (|u| < 2^62), with a = sum of |values| in
 // the same units and t the highest exponent; e = INT_MAX for no values.  A
 // sum whose values span 48 bits or more is not kept (the row's range then
@@ -805,261 +506,877 @@ __device__ __forceinline__ void usum_warp(USum& x) {
   }
 }
 
-__device__ void grid_join_share(const NJDev& s, const GridNJ& g, Team tm, const GCand& w, int na, const int* act, int* act2) {
-  __shared__ USum swarp[32];
-  const int i = w.a, j = w.b, si = w.sa, sj = w.sb;
-  const float dmin = w.d;
-  const int n0 = s.n0;
-  const size_t ld = (size_t)s.ld;
-  const int per = (n0 + tm.size - 1) / tm.size;
-  const int p = tm.rank * per + (int)threadIdx.x;
-  USum x;
-  x.u = x.a = 0;
-  x.e = INT_MAX;
-  x.t = INT_MIN;
-  if ((int)threadIdx.x < per && p < n0) {
-    const int v = s.node[p];
-    const float Dik = s.D[(size_t)si * ld + p];
-    const float Djk = s.D[(size_t)sj * ld + p];
-    const double Tk = s.T[p];
-    if (v >= 0 && p != si && p != sj) {
-      const float sumf = __fadd_rn(Dik, Djk);
-      const float tmp = __fmul_rn(__fsub_rn(sumf, dmin), 0.5f);
-      const double t = __dadd_rn(Tk, (double)__fsub_rn(tmp, sumf));
-      s.T[p] = t;
-      s.Tf[p] = (float)t;
-      s.D[(size_t)p * ld + si] = tmp;
-      s.D[(size_t)si * ld + p] = tmp;
-      g.tv[p] = tmp;
-      if (tmp != 0.f) {
-        x.e = low_bit_exp(tmp);
-        x.t = top_bit_exp(tmp);
-        x.u = float_units(tmp, x.e);
-        x.a = x.u < 0 ? -x.u : x.u;
-      }
+// ---- lazy search: one job per team of CTAs, one exchange per join --------------
+// The team is the whole cooperative grid or one thread-block cluster.  Two
+// things keep a join short.
+//
+// Replicated state.  Every CTA holds the slot -> node map and T of the whole job
+// in its shared memory, T as the sum of two floats, and applies every join to
+// its own copy: it reads the two joined rows, updates every T, and forms the new
+// node's row sum itself (in integers).  The copies are the same in every CTA, so
+// a join needs no exchange but the search's: one all-gather of each CTA's best
+// pair.  The exact double T of row r is kept by the row's owner (CTA r modulo the
+// team's size) and read from global memory where a pick needs it; only the owner
+// writes row r of the matrix.  A new node's row goes to a free place (the one
+// that the last join's row left), since the other CTAs may still be reading the
+// joined rows.  (With the double T in every copy a join of 8,000 taxa spent 8 us
+// in the FP64 pipe.)
+//
+// Lower bounds.  A join changes q(r,c) = d (n-2) - T_r - T_c by
+// -(d(r,c) + dT_r + dT_c), so a lower bound L_r of row r's smallest q moves by
+// at most dmax_r + dT_r + max dT (dmax_r: the row's largest d), rounded down.
+// The pair of r and the new node is looked at itself.  A row is scanned again
+// only when L_r reaches the best pair known: the smallest current q among the
+// CTA's own rows' last best pairs and the pairs that the CTAs published for the
+// last join.  8,000 sequences scan 1.2 % of the live rows a join, 1,000 about a
+// tenth.
+//
+// What bounds it: a chain of a few dependent steps per join (pick, the two rows
+// through L2, the update and its reduction, the scan, the exchange), each a CTA
+// barrier or an L2 round trip; 5.5-10 us.  Against one streaming pass over the
+// whole live triangle per join with three to four barriers, which it replaced
+// (bounded by L2 and HBM bandwidth at 8,000 taxa, by its barriers below 2,000),
+// whole job, matrix on the device: 15.1 -> 7.8 ms at 1,200 taxa, 131 -> 78.6 ms
+// at 8,000.
+//
+// The pick is exact as with a full pass: every float q is within E of the exact
+// q; every pair whose float q is at most the smallest + 3E lies in a row whose
+// bound reaches the best known pair + 5E, so it was scanned for this join.  A CTA
+// publishes its smallest q and its second smallest (of the same row or another
+// row); when no second is within the threshold, the published pairs within it
+// are all the candidates.  Otherwise the CTAs scan their rows within the
+// threshold into the candidate list.
+constexpr int kLazyThreads = 1024;
+constexpr int kLazyMaxCtas = 160;         // team size, at most
+
+struct LazyLayout {
+  size_t tf, tl, tv, node, prow, ord, made, row, town, parts, bytes;
+  int rows;                                // own rows per CTA
+};
+
+__host__ __device__ inline LazyLayout lazy_layout(int n0, int ld, int size) {
+  auto al = [](size_t x) { return (x + 15) / 16 * 16; };
+  LazyLayout L;
+  L.rows = (n0 + size - 1) / size;
+  size_t o = 0;
+  L.tf = o; o += al(sizeof(float) * ld);
+  L.tl = o; o += al(sizeof(float) * ld);
+  L.tv = o; o += al(sizeof(float) * ld);
+  L.node = o; o += al(sizeof(int16_t) * ld);
+  L.prow = o; o += al(sizeof(int16_t) * n0);
+  L.ord = o; o += al(sizeof(int16_t) * n0);
+  L.made = o; o += al(sizeof(int16_t) * n0);
+  L.row = o; o += al((sizeof(float) * 5 + sizeof(int)) * L.rows);
+  L.town = o; o += al(sizeof(double) * L.rows);
+  L.parts = o; o += al(sizeof(float4) * 2 * size);
+  L.bytes = o;
+  return L;
+}
+
+// Threads per CTA: one per four slots between 256 and 512 (more make every CTA
+// barrier dearer than their loads in flight save), at least one per own row and
+// per CTA of the team (a multiple of 32).
+inline int lazy_threads(int ld, int rows, int size) {
+  const int t = std::max(std::max(std::min(std::max(ld / 4, 256), 512), rows), size);
+  return std::min((t + 31) / 32 * 32, kLazyThreads);
+}
+
+// The job's state in the CTA's shared memory.
+struct LazyMem {
+  float* Tf;        // T = Tf + Tl; NaN at dead and padding slots
+  float* Tl;
+  float* tv;        // the join's new values
+  int16_t* node;    // slot -> node id, -1 dead or padding
+  int16_t* prow;    // slot -> its row's place
+  int16_t* ord;     // slots by ascending node id at the segment's start
+  int16_t* made;    // slots of the nodes made since, in order
+  // own rows (row l * size + rank)
+  double* To;       // exact T
+  float* L;         // lower bound of the row's smallest exact q
+  float* U;         // float q of its last best pair (FLT_MAX: none)
+  float* d1;        // that pair's d and column
+  int* c1;
+  float* dmax;      // the row's largest d
+  float* m2;        // its second smallest q if scanned for this join, else FLT_MAX
+  float4* parts;    // [2][size]: per CTA smallest q, second, pair (r | c << 16), d
+};
+
+// What every CTA knows alike.
+struct LazyRep {
+  float dabs;       // largest |d| of any pair so far
+  float tabs;       // largest |T| of a live slot
+  int elow;         // every d is a multiple of 2^elow (INT_MAX: all zero)
+};
+
+__device__ __forceinline__ float lazy_err(const LazyRep& k, float nm2f) {   // E for this join's float q
+  const float m = __fadd_ru(__fmul_ru(k.dabs, fabsf(nm2f)), __fmul_ru(2.f, k.tabs));
+  return __fadd_ru(__fmul_ru(8.f * 5.9604645e-8f, m), 1e-30f);
+}
+
+__device__ __forceinline__ float lazy_q(float d, float tr, float tc, float nm2f) {
+  return __fsub_rn(__fsub_rn(__fmul_rn(d, nm2f), tr), tc);
+}
+
+__device__ __forceinline__ float unford(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7FFFFFFF); }
+
+// One row's two smallest q and largest d (and, at a segment's start, largest
+// |d| and lowest exponent).
+struct RowScan {
+  float m1, m2, d1, mx, ma;   // d1: d of the smallest (in column c1)
+  int c1, el;
+};
+
+__device__ __forceinline__ RowScan scan_none() { return RowScan{FLT_MAX, FLT_MAX, 0.f, -FLT_MAX, 0.f, -1, INT_MAX}; }
+
+template <bool First>
+__device__ __forceinline__ void scan_elem(RowScan& x, float d, float tc, int c, float tr, float nm2f) {
+  const float q = lazy_q(d, tr, tc, nm2f);   // NaN at dead and padding slots: drops out below
+  const bool lt = q < x.m1;
+  x.m2 = lt ? x.m1 : fminf(x.m2, q);
+  x.c1 = lt ? c : x.c1;
+  x.d1 = lt ? d : x.d1;
+  x.m1 = lt ? q : x.m1;
+  if (tc == tc) {
+    x.mx = fmaxf(x.mx, d);
+    if (First) {
+      x.ma = fmaxf(x.ma, fabsf(d));
+      x.el = min(x.el, low_bit_exp(d));
     }
-  }
-  // the active list without i and j (ascending ids), shifted into act2
-  const int kper = (na + tm.size - 1) / tm.size;
-  const int k = tm.rank * kper + (int)threadIdx.x;
-  if ((int)threadIdx.x < kper && k < na) {
-    const int v = act[k];
-    if (v != i && v != j) act2[k - (v > i) - (v > j)] = v;
-  }
-  // the share's slots sit in its first warps (per <= blockDim)
-  const int nwv = (per + 31) >> 5;
-  if ((int)(threadIdx.x >> 5) < nwv) usum_warp(x);
-  if (nwv > 1) {
-    if ((threadIdx.x & 31) == 0 && (int)(threadIdx.x >> 5) < nwv) swarp[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w2 = 1; w2 < nwv; ++w2) usum_add(x, swarp[w2]);
-  }
-  if (threadIdx.x == 0) {
-    g.jsum[2 * tm.rank] = x.u;
-    g.jsum[2 * tm.rank + 1] = x.a;
-    g.jexp[2 * tm.rank] = x.e;
-    g.jexp[2 * tm.rank + 1] = x.t;
   }
 }
 
-// After the barrier that ends join `step`: the new node's row sum
-// (SpeciesBlock.cpp:799, :818 -- the sequential double sum in ascending id
-// order, taken as the exact integer sum of the shares when that provably
-// equals it), written by every CTA for itself; CTA 0 also writes the join
-// record (TreeNode::join's inputs; the lengths follow after the loop) and the
-// id -> slot map.  When the integer sum cannot be used, CTA 0 runs the
-// sequential loop and one more grid barrier follows.
-template <bool CL>
-__device__ bool grid_join_apply(const NJDev& s, const GridNJ& g, Team tm, const GCand& w, const PickOut& pk, int step,
-                                int n, const int* act_old, int* act_new, unsigned& target) {
-  __shared__ double s_sum;
-  __shared__ int s_exact;
-  const int i = w.a, j = w.b, si = w.sa, sj = w.sb;
-  const int m_n = n - step, next = n + step;
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    // at most kGridMax CTAs: kGridMax / 32 shares per lane, held in registers
-    constexpr int kPer = kGridMax / 32;
-    int je[kPer];
-    long long jsv[kPer], jav[kPer];
-    int lowexp = INT_MAX, topexp = INT_MIN;
-#pragma unroll
-    for (int t = 0; t < kPer; ++t) {
-      const int b = l + 32 * t;
-      je[t] = INT_MAX;
-      jsv[t] = jav[t] = 0;
-      if (b < tm.size) {
-        je[t] = g.jexp[2 * b];
-        jsv[t] = g.jsum[2 * b];
-        jav[t] = g.jsum[2 * b + 1];
-        topexp = max(topexp, g.jexp[2 * b + 1]);
-      }
-      lowexp = min(lowexp, je[t]);
+// Warp `sub` of the `wpr` that scan row r.
+template <bool First>
+__device__ RowScan scan_row_part(const NJDev& s, const LazyMem& m, int r, int sub, int wpr, float nm2f) {
+  const int lane = threadIdx.x & 31;
+  RowScan x = scan_none();
+  const float tr = m.Tf[r];
+  if (tr != tr) return x;   // dead
+  const float* row = row_at(s, m.prow[r]);
+  const int c0 = r + 1, v0 = (c0 + 3) >> 2, nv = s.ld >> 2;
+  if (sub == 0 && lane < 4 * v0 - c0 && c0 + lane < s.n0)
+    scan_elem<First>(x, __ldcg(row + c0 + lane), m.Tf[c0 + lane], c0 + lane, tr, nm2f);
+  const float4* row4 = reinterpret_cast<const float4*>(row);
+  const float4* Tf4 = reinterpret_cast<const float4*>(m.Tf);
+#pragma unroll 4
+  for (int v = v0 + sub * 32 + lane; v < nv; v += 32 * wpr) {
+    const float4 d = __ldcg(row4 + v);
+    const float4 tc = Tf4[v];
+    scan_elem<First>(x, d.x, tc.x, 4 * v, tr, nm2f);
+    scan_elem<First>(x, d.y, tc.y, 4 * v + 1, tr, nm2f);
+    scan_elem<First>(x, d.z, tc.z, 4 * v + 2, tr, nm2f);
+    scan_elem<First>(x, d.w, tc.w, 4 * v + 3, tr, nm2f);
+  }
+  return x;
+}
+
+// Two smallest (an equal pair makes m2 = m1; of equal ones the lowest lane's
+// first), the largest and the lowest over the lanes.
+template <bool First>
+__device__ __forceinline__ void scan_warp(RowScan& x) {
+  const int lane = threadIdx.x & 31;
+  const int key = ford(x.m1);
+  const int k1 = __reduce_min_sync(0xffffffffu, key);
+  const int first = __ffs(__ballot_sync(0xffffffffu, key == k1)) - 1;
+  // the second: the first lane's own second, or another lane's smallest
+  const int k2 = __reduce_min_sync(0xffffffffu, lane == first ? ford(x.m2) : key);
+  x.m1 = unford(k1);
+  x.m2 = unford(k2);
+  x.c1 = __shfl_sync(0xffffffffu, x.c1, first);
+  x.d1 = __shfl_sync(0xffffffffu, x.d1, first);
+  x.mx = unford(__reduce_max_sync(0xffffffffu, ford(x.mx)));
+  if (First) {
+    x.ma = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x.ma)));
+    x.el = __reduce_min_sync(0xffffffffu, x.el);
+  }
+}
+
+// Scans the own rows row_of(0) .. row_of(cnt - 1) (the same in every warp): U,
+// d1, c1, dmax, m2, and L = m1 - E.  Few rows are split over the CTA's warps (a
+// power of two per row).  First: the largest |d| and lowest exponent go to ma /
+// el.  Every thread calls it; the results are visible after the caller's next
+// CTA barrier.
+template <bool First, class Rows>
+__device__ void scan_rows(const NJDev& s, const LazyMem& m, Team tm, Rows&& row_of, int cnt, float nm2f, float E,
+                          int* ma, int* el) {
+  __shared__ RowScan part[32];
+  const int lane = threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  if (cnt == 0) return;   // the same in the CTA
+  int wpr = 1;
+  while (2 * wpr * cnt <= nw) wpr *= 2;
+  const int per = nw / wpr;   // rows at a time
+  for (int k0 = 0; k0 < cnt; k0 += per) {
+    const int k = k0 + warp / wpr, sub = warp % wpr;
+    const bool mine = k < cnt && warp / wpr < per;
+    const int l = mine ? row_of(k) : 0;
+    RowScan x = scan_none();
+    if (mine) {
+      x = scan_row_part<First>(s, m, l * tm.size + tm.rank, sub, wpr, nm2f);
+      scan_warp<First>(x);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      lowexp = min(lowexp, __shfl_xor_sync(0xffffffffu, lowexp, o));
-      topexp = max(topexp, __shfl_xor_sync(0xffffffffu, topexp, o));
-    }
-    // every value below 2^49 units of 2^lowexp: a share's sum (at most 8192
-    // values) moved to those units stays below 2^62
-    const bool fits = lowexp == INT_MAX || topexp - lowexp < 48;
-    long long isum = 0, iabs = 0;
-    if (fits && lowexp != INT_MAX) {
-#pragma unroll
-      for (int t = 0; t < kPer; ++t) {
-        if (je[t] == INT_MAX) continue;   // a share without values
-        const long long m = 1ll << (je[t] - lowexp);
-        isum += jsv[t] * m;
-        iabs += jav[t] * m;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        isum += __shfl_xor_sync(0xffffffffu, isum, o);
-        iabs += __shfl_xor_sync(0xffffffffu, iabs, o);
+    if (wpr > 1) {
+      if (lane == 0) part[warp] = x;
+      __syncthreads();
+      if (mine && sub == 0) {
+        x = lane < wpr ? part[warp + lane] : scan_none();
+        scan_warp<First>(x);
       }
     }
-    if (l == 0) {
-      if (lowexp == INT_MAX) {
-        s_sum = 0.0;                                 // every value is zero
-        s_exact = 1;
-      } else if (fits && iabs < (1ll << 53)) {
-        s_sum = units_to_double(isum, lowexp);       // exact: |isum| < 2^53
-        s_exact = 1;
-      } else {
-        s_exact = 0;
+    if (mine && sub == 0 && lane == 0) {
+      m.U[l] = x.m1;
+      m.m2[l] = x.m2;
+      m.c1[l] = x.c1;
+      m.d1[l] = x.d1;
+      m.dmax[l] = x.c1 >= 0 ? x.mx : 0.f;
+      m.L[l] = x.c1 >= 0 ? __fsub_rd(x.m1, E) : FLT_MAX;
+      if (First) {
+        atomicMax(ma, __float_as_int(x.ma));
+        atomicMin(el, x.el);
       }
+    }
+    if (wpr > 1 && k0 + per < cnt) __syncthreads();   // part is free again
+  }
+}
+
+// Exchange of the CTAs' published float4 through global memory (the grid): the
+// value, then an arrival count that one thread of each CTA polls, then all the
+// values at once.  (Polling the values themselves, 152 readers of 152 lines,
+// kept the L2 slices that hold them busy: 12,000 cycles an exchange.)
+// Publishing: one thread, after a CTA barrier that follows the CTA's writes to
+// global memory.
+__device__ __forceinline__ void grid_publish(const GridNJ& g, Team tm, unsigned seq, float4 v) {
+  g.gather[(size_t)(seq & 1) * tm.size + tm.rank] = v;
+  red_release_add(&g.bar[1], 1u);
+}
+
+// Every CTA's published value into parts' half seq & 1; every thread calls it.
+// False when a wait ran out or another CTA gave up.
+__device__ bool grid_gather(const GridNJ& g, Team tm, unsigned seq, float4* parts) {
+  int bad = 0;
+  if (threadIdx.x == 0) {
+    const unsigned target = seq * (unsigned)tm.size;
+    const long long t0 = clock64();
+    while ((int)(ld_acquire_u32(&g.bar[1]) - target) < 0) {
+      if (*(volatile int*)g.abort) bad = 1;
+      else if (clock64() - t0 > kBarrierSpinCycles) {
+        atomicExch(g.abort, 1);
+        bad = 1;
+      }
+      if (bad) break;
     }
   }
+  if (__syncthreads_or(bad)) return false;
+  const size_t at = (size_t)(seq & 1) * tm.size + threadIdx.x;
+  if ((int)threadIdx.x < tm.size) parts[at] = __ldcg(g.gather + at);
   __syncthreads();
-  const bool exact = s_exact != 0;
-  if (threadIdx.x == 0) {
-    if (exact) {
-      s.T[si] = s_sum;
-      s.Tf[si] = __double2float_rn(s_sum);
-    } else if (tm.rank == 0) {
-      double sum = 0.0;   // the reference's loop: active ids ascending, i and j skipped
-      for (int k = 0; k < m_n; ++k) {
-        const int v = act_old[k];
-        if (v != i && v != j) sum = __dadd_rn(sum, (double)g.tv[s.slot[v]]);
+  return true;
+}
+
+// Publishes this CTA's value (v, in warp 0's lanes) and gathers every CTA's into
+// m.parts' half seq & 1; every thread calls it, after a CTA barrier that follows
+// the CTA's writes to global memory.
+template <bool CL>
+__device__ bool team_exchange(const GridNJ& g, const LazyMem& m, Team tm, unsigned seq, float4 v) {
+  if constexpr (CL) {
+    if ((int)threadIdx.x < tm.size)
+      cooperative_groups::this_cluster().map_shared_rank(m.parts, threadIdx.x)[(seq & 1) * tm.size + tm.rank] = v;
+    cooperative_groups::this_cluster().sync();
+    return true;
+  } else {
+    if (threadIdx.x == 0 && !(g.stall && tm.rank == 0)) grid_publish(g, tm, seq, v);
+    return grid_gather(g, tm, seq, m.parts);
+  }
+}
+
+// The CTA's smallest and second smallest q over its own rows, by one warp (the
+// result in every lane).
+__device__ __forceinline__ float4 cta_best(const LazyMem& m, Team tm, int rows) {
+  const int lane = threadIdx.x & 31;
+  float b1 = FLT_MAX, b2 = FLT_MAX;
+  int bl = 0;
+  for (int l = lane; l < rows; l += 32) {
+    const float u = m.U[l], v = m.m2[l];
+    const bool lt = u < b1;
+    b2 = lt ? fminf(b1, v) : fminf(b2, u);
+    bl = lt ? l : bl;
+    b1 = lt ? u : b1;
+  }
+  const int key = ford(b1);
+  const int k1 = __reduce_min_sync(0xffffffffu, key);
+  const int first = __ffs(__ballot_sync(0xffffffffu, key == k1)) - 1;
+  const int k2 = __reduce_min_sync(0xffffffffu, lane == first ? ford(b2) : key);
+  bl = __shfl_sync(0xffffffffu, bl, first);
+  return make_float4(unford(k1), unford(k2), __uint_as_float((unsigned)(bl * tm.size + tm.rank) | (unsigned)m.c1[bl] << 16),
+                     m.d1[bl]);
+}
+
+// Candidate scan of the fallback: this CTA's own rows within the threshold,
+// visit(pred, candidate) by whole warps.  tx: every slot's exact T.
+template <class Visit>
+__device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int rows, const double* tx, float nm2f,
+                               double nm2, int watermark, float thr, Visit&& visit) {
+  const int lane = threadIdx.x & 31;
+  for (int l = (int)threadIdx.x >> 5; l < rows; l += (int)blockDim.x >> 5) {
+    const int r = l * tm.size + tm.rank;
+    if (m.U[l] > thr) continue;
+    const int ur = m.node[r];
+    const float tr = m.Tf[r];
+    const double Tr = m.To[l];
+    const float* row = row_at(s, m.prow[r]);
+    for (int cb = r + 1; cb < s.n0; cb += 32) {
+      const int c = cb + lane;
+      bool pred = false;
+      KCand kc = kc_none();
+      if (c < s.n0 && m.node[c] >= 0) {
+        const float d = __ldcg(row + c);
+        if (lazy_q(d, tr, m.Tf[c], nm2f) <= thr) {
+          const GCand cd = make_cand(r, c, ur, m.node[c], Tr, __ldcg(tx + c), d, nm2, watermark);
+          kc = KCand{cd.k1, cd.k2, cd.a, cd.b};
+          pred = true;
+        }
       }
-      s.T[si] = sum;
-      s.Tf[si] = __double2float_rn(sum);
+      visit(pred, kc);
     }
-    s.Tf[sj] = __int_as_float(0x7FC00000);   // dead: NaN
-    s.node[sj] = -1;
-    s.node[si] = next;
-    if (tm.rank == 0) {
+  }
+}
+
+// The pick when the published pairs do not decide it alone (several within the
+// threshold, or a CTA's second): the winner in *win and *pk, the same in every
+// CTA.  False when a wait ran out.
+template <bool CL>
+__device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m, Team tm, int rows,
+                               const float4* parts, const double* tx, float thr, bool listed, float nm2f, double nm2,
+                               int watermark, GCand* win, PickOut* pk, unsigned& target) {
+  __shared__ GCand fc[32];
+  const int lane = threadIdx.x & 31;
+  if (listed) {   // at most 32 published pairs are all the candidates
+    if (threadIdx.x < 32) {
+      int base = 0;
+      for (int b0 = 0; b0 < tm.size; b0 += 32) {
+        const float4 v = b0 + lane < tm.size ? parts[b0 + lane] : make_float4(FLT_MAX, FLT_MAX, 0.f, 0.f);
+        const bool in = v.x <= thr;
+        const unsigned bal = __ballot_sync(0xffffffffu, in);
+        if (in) {
+          const unsigned rc = __float_as_uint(v.z);
+          const int r = rc & 0xFFFFu, c = rc >> 16;
+          fc[base + __popc(bal & ((1u << lane) - 1u))] =
+              make_cand(r, c, m.node[r], m.node[c], __ldcg(tx + r), __ldcg(tx + c), v.w, nm2, watermark);
+        }
+        base += __popc(bal);
+      }
+      __syncwarp();
+      const PickOut r = pick_keys(base, [&](int k) { return fc[k]; });
+      if (lane == 0) {
+        *pk = r;
+        *win = fc[r.idx];
+      }
+    }
+    __syncthreads();
+    return true;
+  }
+  KCand first = kc_none();
+  bool full = false;
+  lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
+    list_push(s, g, pred, c, full);
+    if (pred && kc_first(c, first)) first = c;
+  });
+  if (!team_sync<CL>(g, target)) return false;
+  // the winner's pair again, as the scan read it (row = the smaller slot)
+  auto rederive = [&](const KCand& w) {
+    const int sa = __ldcg(s.slot + w.a), sb = __ldcg(s.slot + w.b);
+    const int r0 = min(sa, sb), c0 = max(sa, sb);
+    *win = make_cand(r0, c0, m.node[r0], m.node[c0], __ldcg(tx + r0), __ldcg(tx + c0),
+                     __ldcg(row_at(s, m.prow[r0]) + c0), nm2, watermark);
+  };
+  const int ncount = __ldcg(&s.g32[2]);   // the same in every CTA
+  if (ncount <= min(s.cand_cap, kListPickMax)) {
+    if (threadIdx.x < 32) {
+      const PickOut r = pick_keys(ncount, [&](int k) { return ld_kcand(&g.cand[k]); });
+      if (lane == 0) {
+        *pk = r;
+        if (!r.error) rederive(ld_kcand(&g.cand[r.idx]));
+      }
+    }
+  } else {
+    __shared__ KCand sw[32];
+    __shared__ KCand sfirst;
+    const KCand cf = cta_first(first, sw);
+    if (threadIdx.x == 0) g.cbest[tm.rank] = cf;
+    if (!team_sync<CL>(g, target)) return false;
+    if (threadIdx.x < 32) {
+      const PickOut r = pick_keys(tm.size, [&](int k) { return ld_kcand(&g.cbest[k]); });
+      if (lane == 0) sfirst = r.error ? kc_none() : ld_kcand(&g.cbest[r.idx]);
+    }
+    __syncthreads();
+    const KCand w = sfirst;
+    unsigned ties = 0, amb = 0;
+    lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
+      if (pred) count_vs(c, w, ties, amb);
+    });
+    add_counts(ties, amb, s.g32);
+    if (!team_sync<CL>(g, target)) return false;
+    if (threadIdx.x == 0) {
+      pk->idx = 0;
+      pk->ties = (unsigned)__ldcg(&s.g32[0]);
+      pk->amb = (unsigned)__ldcg(&s.g32[1]);
+      pk->error = w.b < 0;
+      if (!pk->error) rederive(w);
+    }
+  }
+  // every CTA has read the counts before they are reset for the next scan
+  if (!team_sync<CL>(g, target)) return false;
+  if (tm.rank == 0 && threadIdx.x == 0) s.g32[0] = s.g32[1] = s.g32[2] = 0;
+  return true;
+}
+
+// The sequential double sum of the join's values over the active nodes in
+// ascending id order (SpeciesBlock.cpp:799, :818), by one thread.
+__device__ double lazy_seq_sum(const LazyMem& m, int n_ord, int id0, int n_made, int si, int sj) {
+  double sum = 0.0;
+  for (int k = 0; k < n_ord; ++k) {
+    const int p = m.ord[k], v = m.node[p];
+    if (v >= 0 && v < id0 && p != si && p != sj) sum = __dadd_rn(sum, (double)m.tv[p]);
+  }
+  for (int k = 0; k < n_made; ++k) {
+    const int p = m.made[k];
+    if (m.node[p] == id0 + k && p != si && p != sj) sum = __dadd_rn(sum, (double)m.tv[p]);
+  }
+  return sum;
+}
+
+// Joins step0 .. step1 - 1 of an n-taxon job by one team (the active count
+// before join t is n - t); T, Tf, node, prow, slot and the active list come from
+// and go back to global memory.  seq: exchanges so far.  False when the team
+// stops (a wait ran out, the pick failed) -- the same in every CTA.
+template <bool CL>
+__device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned char* smem, int step0, int step1, int n,
+                             int watermark, unsigned& seq, unsigned& target) {
+  const int tid = (int)threadIdx.x, nth = (int)blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
+  const int n0 = s.n0, ld = s.ld, nv = ld >> 2;
+  LazyMem m;
+  int rows;
+  {
+    const LazyLayout Y = lazy_layout(n0, ld, tm.size);
+    rows = Y.rows;
+    m.Tf = reinterpret_cast<float*>(smem + Y.tf);
+    m.Tl = reinterpret_cast<float*>(smem + Y.tl);
+    m.tv = reinterpret_cast<float*>(smem + Y.tv);
+    m.node = reinterpret_cast<int16_t*>(smem + Y.node);
+    m.prow = reinterpret_cast<int16_t*>(smem + Y.prow);
+    m.ord = reinterpret_cast<int16_t*>(smem + Y.ord);
+    m.made = reinterpret_cast<int16_t*>(smem + Y.made);
+    m.To = reinterpret_cast<double*>(smem + Y.town);
+    m.L = reinterpret_cast<float*>(smem + Y.row);
+    m.U = m.L + rows;
+    m.d1 = m.U + rows;
+    m.dmax = m.d1 + rows;
+    m.m2 = m.dmax + rows;
+    m.c1 = reinterpret_cast<int*>(m.m2 + rows);
+    m.parts = reinterpret_cast<float4*>(smem + Y.parts);
+  }
+  __shared__ int s_ma, s_el, s_hint;
+  __shared__ int16_t s_list[1024];         // own rows to scan
+  __shared__ GCand swin;
+  __shared__ PickOut spick;
+  __shared__ double s_seq;
+  __shared__ float s_thr;
+  __shared__ int s_cands;
+  __shared__ float4 s_pair;
+  __shared__ LazyRep s_rep;
+  __shared__ long long w_u[32];            // per warp: the join's integer sum,
+  __shared__ int4 w_x[32];                 // largest dT (ordered), |T|, |tmp|, lowest exponent
+  const int id0 = n + step0;               // ids from here on are made in this segment
+  const int n_ord = __ldcg(s.na);
+  int spare = __ldcg(s.prow + n0);         // the free place
+  float ta = 0.f;
+  for (int p = tid; p < ld; p += nth) {
+    const int v = p < n0 ? __ldcg(s.node + p) : -1;
+    m.node[p] = (int16_t)v;
+    if (p < n0) m.prow[p] = (int16_t)__ldcg(s.prow + p);
+    const double t = v >= 0 ? __ldcg(s.T + p) : 0.0;
+    const float hi = __double2float_rn(t);
+    m.Tf[p] = v >= 0 ? hi : __int_as_float(0x7FC00000);
+    m.Tl[p] = __double2float_rn(__dsub_rn(t, (double)hi));
+    m.tv[p] = 0.f;
+    ta = fmaxf(ta, fabsf(hi));
+  }
+  for (int k = tid; k < n_ord; k += nth) m.ord[k] = (int16_t)__ldcg(s.slot + __ldcg(s.act + k));
+  for (int l = tid; l < rows; l += nth) {
+    m.L[l] = m.U[l] = m.m2[l] = FLT_MAX;
+    m.d1[l] = m.dmax[l] = 0.f;
+    m.c1[l] = 0;
+    const int r = l * tm.size + tm.rank;
+    const bool live = r < n0 && __ldcg(s.node + r) >= 0;
+    m.To[l] = live ? __ldcg(s.T + r) : 0.0;
+    // the exact T that go with the first exchange of pairs (seq + 2)
+    if (live) s.tx[(size_t)(seq & 1) * n0 + r] = m.To[l];
+  }
+  if (tid == 0) {
+    s_ma = 0;
+    s_el = INT_MAX;
+  }
+  ta = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(ta)));
+  if (lane == 0) w_x[warp].x = __float_as_int(ta);
+  __syncthreads();
+  // ---- every own row once: best pairs, bounds; the largest |d|, |T| and the
+  // lowest exponent of the whole job
+  LazyRep rep{0.f, 0.f, INT_MAX};
+  float nm2f = (float)(n - step0 - 2);
+  {
+    const int own = n0 > tm.rank ? (n0 - tm.rank + tm.size - 1) / tm.size : 0;   // dead rows scan to nothing
+    scan_rows<true>(s, m, tm, [](int k) { return k; }, own, nm2f, 0.f, &s_ma, &s_el);
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) rep.tabs = fmaxf(rep.tabs, __int_as_float(w_x[w].x));
+    rep.tabs = __fmul_ru(rep.tabs, 1.000001f);
+    if (!team_exchange<CL>(g, m, tm, ++seq, make_float4(__int_as_float(s_ma), 0.f, __int_as_float(s_el), 0.f)))
+      return false;
+    const float4* pp = m.parts + (seq & 1) * tm.size;
+    for (int b = 0; b < tm.size; ++b) {
+      rep.dabs = fmaxf(rep.dabs, pp[b].x);
+      rep.elow = min(rep.elow, __float_as_int(pp[b].z));
+    }
+    const float E = lazy_err(rep, nm2f);
+    for (int l = tid; l < rows; l += nth)
+      if (m.U[l] < FLT_MAX) m.L[l] = __fsub_rd(m.U[l], E);
+    __syncthreads();
+  }
+  float4 pub = make_float4(FLT_MAX, FLT_MAX, 0.f, 0.f);
+  if (warp == 0) pub = cta_best(m, tm, rows);
+  if (!team_exchange<CL>(g, m, tm, ++seq, pub)) return false;
+  for (int step = step0; step < step1; ++step) {
+    const int m_n = n - step, next = n + step;
+    const double nm2 = (double)(m_n - 2);
+    const float4* const parts = m.parts + (seq & 1) * tm.size;
+    const double* const tx = s.tx + (size_t)(seq & 1) * n0;
+    // ---- pick: the published pairs within the threshold
+    if (warp == 0) {
+      const float E = lazy_err(rep, nm2f);
+      constexpr int kPer = kLazyMaxCtas / 32;
+      float x[kPer], own = FLT_MAX;
+      int at = 0, cands = 0;
+#pragma unroll
+      for (int t = 0; t < kPer; ++t) {
+        const int b = lane + 32 * t;
+        x[t] = b < tm.size ? parts[b].x : FLT_MAX;
+        if (x[t] < own) {
+          own = x[t];
+          at = b;
+        }
+      }
+      const float q = unford(__reduce_min_sync(0xffffffffu, ford(own)));
+      const float thr = q < FLT_MAX ? __fadd_ru(q, __fmul_ru(3.f, E)) : -FLT_MAX;
+      bool second = false;
+#pragma unroll
+      for (int t = 0; t < kPer; ++t) {
+        const bool in = x[t] <= thr;
+        if (in) second |= parts[lane + 32 * t].y <= thr;
+        cands += __popc(__ballot_sync(0xffffffffu, in));
+      }
+      if (__any_sync(0xffffffffu, second)) cands = -1;
+      const unsigned has = __ballot_sync(0xffffffffu, own <= thr);
+      if (lane == (has ? __ffs(has) - 1 : 0)) {
+        s_thr = thr;
+        s_cands = cands;
+        s_pair = parts[at];
+      }
+    }
+    __syncthreads();
+    const float thr = s_thr;
+    const int cands = s_cands;
+    const unsigned rc = __float_as_uint(s_pair.z);
+    float dmin = s_pair.w;
+    int i, j, si, sj;
+    const bool fast = cands == 1;
+    if (fast) {
+      const int r = rc & 0xFFFFu, c = rc >> 16;
+      const int ur = m.node[r], uc = m.node[c];
+      i = min(ur, uc);
+      j = max(ur, uc);
+      si = ur < uc ? r : c;
+      sj = ur < uc ? c : r;
+    } else {
+      if (!lazy_pick_slow<CL>(s, g, m, tm, rows, parts, tx, thr, cands >= 1 && cands <= 32, nm2f, nm2, watermark, &swin,
+                              &spick, target))
+        return false;
+      __syncthreads();
+      if (spick.error) {
+        if (tm.rank == 0 && tid == 0) record_pick(s, spick);
+        return false;
+      }
+      i = swin.a;
+      j = swin.b;
+      si = swin.sa;
+      sj = swin.sb;
+      dmin = swin.d;
+    }
+    // ---- the join, in every CTA: modifyMatrix (SpeciesBlock.cpp:787-841) on its
+    // copy of T; the owners write the new row and their rows' new column
+    const bool own_si = si % tm.size == tm.rank;
+    const int place = m.prow[si];
+    const float* const rowi = row_at(s, place);
+    float* const newrow = row_at(s, spare);
+    // every new value is a multiple of 2^eu, and at most 1.5 dabs (rounding aside)
+    const int eu = rep.elow == INT_MAX ? 0 : rep.elow - 1;
+    const int span_max = rep.dabs > 0.f ? top_bit_exp(rep.dabs) + 3 - eu : 0;
+    const bool u32 = span_max <= 30 && eu >= -100 && eu <= 100;
+    const bool u64 = span_max < 47;
+    const float scale = u32 ? __int_as_float((127 - eu) << 23) : 0.f;
+    long long u = 0;
+    int x_el = INT_MAX, x_or = 0;
+    float x_t = 0.f, x_d = 0.f, x_dt = -FLT_MAX;
+    const float* const rowj = row_at(s, m.prow[sj]);
+    // this thread's own row: the new column's value and the change of T
+    const int r_own = tid * tm.size + tm.rank;
+    const bool has_own = tid < rows && r_own < n0;
+    const float a_own = has_own ? __ldcg(rowi + r_own) : 0.f, b_own = has_own ? __ldcg(rowj + r_own) : 0.f;
+    for (int v = tid; v < nv; v += nth) {
+      const float4 a4 = __ldcg(reinterpret_cast<const float4*>(rowi) + v);
+      const float4 b4 = __ldcg(reinterpret_cast<const float4*>(rowj) + v);
+      const float4 h4 = reinterpret_cast<const float4*>(m.Tf)[v], l4 = reinterpret_cast<const float4*>(m.Tl)[v];
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+      const float hi[4] = {h4.x, h4.y, h4.z, h4.w}, lo[4] = {l4.x, l4.y, l4.z, l4.w};
+      float nh[4], nl[4], nt[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float sumf = __fadd_rn(a[k], b[k]);
+        const float tmp = __fmul_rn(__fsub_rn(sumf, dmin), 0.5f);
+        const float dt = __fsub_rn(tmp, sumf);
+        // T as two floats: two-sum, then the carry (NaN stays NaN at dead
+        // slots; si's and sj's are set below)
+        const float sm = __fadd_rn(hi[k], dt), bb = __fsub_rn(sm, hi[k]);
+        const float c = __fadd_rn(lo[k], __fadd_rn(__fsub_rn(hi[k], __fsub_rn(sm, bb)), __fsub_rn(dt, bb)));
+        nh[k] = __fadd_rn(sm, c);
+        nl[k] = __fsub_rn(c, __fsub_rn(nh[k], sm));
+        nt[k] = tmp;
+        const int p = 4 * v + k;
+        if (hi[k] == hi[k] && p != si && p != sj) {
+          x_dt = fmaxf(x_dt, dt);
+          x_t = fmaxf(x_t, fabsf(nh[k]));
+          x_d = fmaxf(x_d, fabsf(tmp));
+          if (u32) {
+            const int y = __float2int_rn(__fmul_rn(tmp, scale));   // exact
+            u += y;
+            x_or |= y;
+          } else {
+            x_el = min(x_el, low_bit_exp(tmp));
+            if (u64) u += float_units(tmp, eu);
+          }
+        }
+      }
+      reinterpret_cast<float4*>(m.Tf)[v] = make_float4(nh[0], nh[1], nh[2], nh[3]);
+      reinterpret_cast<float4*>(m.Tl)[v] = make_float4(nl[0], nl[1], nl[2], nl[3]);
+      reinterpret_cast<float4*>(m.tv)[v] = make_float4(nt[0], nt[1], nt[2], nt[3]);
+      if (own_si) reinterpret_cast<float4*>(newrow)[v] = make_float4(nt[0], nt[1], nt[2], nt[3]);
+    }
+    const float sum_own = __fadd_rn(a_own, b_own);
+    const float nd = __fmul_rn(__fsub_rn(sum_own, dmin), 0.5f), dt = __fsub_rn(nd, sum_own);
+    const bool upd = has_own && m.node[r_own] >= 0 && r_own != si && r_own != sj;
+    if (upd) row_at(s, m.prow[r_own])[si] = nd;
+    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+    if (x_or) x_el = eu + __ffs(x_or) - 1;
+    x_el = __reduce_min_sync(0xffffffffu, x_el);
+    int k_dt = __reduce_max_sync(0xffffffffu, ford(x_dt));
+    x_t = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x_t)));
+    x_d = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x_d)));
+    if (lane == 0) {
+      w_u[warp] = u;
+      w_x[warp] = make_int4(k_dt, __float_as_int(x_t), __float_as_int(x_d), x_el);
+    }
+    if (tid == 0) s_hint = 0x7F7FFFFF;
+    __syncthreads();
+    // the whole CTA's, in the warps that go on with it
+    const bool lead = warp * 32 < max(rows, tm.size) || warp == nw - 1;
+    double tsum = 0.0;
+    float tsf = 0.f, drift = 0.f;
+    if (lead) {
+      const int4 y = lane < nw ? w_x[lane] : make_int4(ford(-FLT_MAX), 0, 0, INT_MAX);
+      u = lane < nw ? w_u[lane] : 0;
+      for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+      k_dt = __reduce_max_sync(0xffffffffu, y.x);
+      x_t = __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)y.y));
+      x_d = __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)y.z));
+      x_el = __reduce_min_sync(0xffffffffu, y.w);
+    } else {
+      // whether the sequential sum is needed is the same in every warp
+      const int4 y = lane < nw ? w_x[lane] : make_int4(0, 0, 0, INT_MAX);
+      x_d = __uint_as_float(__reduce_max_sync(0xffffffffu, (unsigned)y.z));
+      x_el = __reduce_min_sync(0xffffffffu, y.w);
+    }
+    // the new node's row sum: the integer sum when every partial sum of the
+    // sequential double sum is exact (all terms multiples of 2^eu, together
+    // below 2^53 of them), else the sequential sum itself
+    const int span = x_el == INT_MAX ? 0 : top_bit_exp(x_d) + 1 - eu;
+    if (x_el == INT_MAX) {
+      // every value is zero
+    } else if (u64 && x_el >= eu && span <= span_max && span + 32 - __clz(m_n) <= 53) {
+      tsum = units_to_double(u, eu);
+    } else {
+      if (tid == 0) s_seq = lazy_seq_sum(m, n_ord, id0, step - step0, si, sj);
+      __syncthreads();
+      tsum = s_seq;
+    }
+    if (lead) {
+      rep.dabs = fmaxf(rep.dabs, x_d);
+      rep.elow = min(rep.elow, x_el);
+      tsf = __double2float_rn(tsum);
+      rep.tabs = __fmul_ru(fmaxf(x_t, fabsf(tsf)), 1.000001f);
+      drift = k_dt == ford(-FLT_MAX) ? 0.f : unford(k_dt);
+    }
+    if (warp == nw - 1 && lane == 0 && tm.rank == 0) {   // the join record
       nwg_join& J = s.joins[step];
       J.i = i;
       J.j = j;
       J.node = next;
       J.n = m_n;
-      J.d = w.d;
+      J.d = dmin;
       J.pad = 0.f;
-      J.q = w.q1;
-      J.ti = w.ta;
-      J.tj = w.tb;
-      act_new[m_n - 2] = next;
-      *s.na = m_n - 1;
+      if (fast) {
+        const int r = min(si, sj), c = max(si, sj);
+        const GCand cd = make_cand(r, c, r == si ? i : j, r == si ? j : i, __ldcg(tx + r), __ldcg(tx + c), dmin, nm2,
+                                   watermark);
+        J.q = cd.q1;
+        J.ti = cd.ta;
+        J.tj = cd.tb;
+      } else {
+        J.q = swin.q1;
+        J.ti = swin.ta;
+        J.tj = swin.tb;
+        record_pick(s, spick);
+      }
       s.slot[j] = -1;
       s.slot[i] = -1;
       s.slot[next] = si;
-      s.g32[0] = s.g32[1] = s.g32[2] = 0;   // every CTA took its pick before the barrier
-      record_pick(s, pk);
     }
+    if (tid == 0) {   // read again only after the next barrier
+      s_rep = rep;
+      if (own_si) newrow[si] = __ldcg(rowi + si);   // the diagonal keeps i's value
+      m.Tf[si] = tsf;
+      m.Tl[si] = __double2float_rn(__dsub_rn(tsum, (double)tsf));
+      m.Tf[sj] = __int_as_float(0x7FC00000);   // dead: NaN
+      m.node[si] = (int16_t)next;
+      m.node[sj] = -1;
+      m.prow[si] = (int16_t)spare;
+      m.made[step - step0] = (int16_t)si;
+    }
+    spare = place;
+    nm2f = (float)(m_n - 3);
+    // ---- the rows' bounds and best pairs under the new T; the best pair known
+    int hint = 0x7F7FFFFF;
+    if (tid < rows) {
+      const int l = tid;
+      m.m2[l] = FLT_MAX;
+      float L = FLT_MAX, U = FLT_MAX;
+      if (r_own == si) {
+        L = -FLT_MAX;   // the new row: scanned below
+        m.To[l] = tsum;
+        s.tx[(size_t)((seq + 1) & 1) * n0 + r_own] = tsum;
+      } else if (upd) {
+        const float tr = m.Tf[r_own];
+        const double t = __dadd_rn(m.To[l], (double)dt);
+        m.To[l] = t;
+        s.tx[(size_t)((seq + 1) & 1) * n0 + r_own] = t;
+        const int c1 = m.c1[l];
+        L = m.L[l];
+        if (L < FLT_MAX) L = __fsub_rd(L, __fadd_ru(m.dmax[l], __fadd_ru(dt, drift)));
+        if (m.U[l] < FLT_MAX && c1 != si && c1 != sj) U = lazy_q(m.d1[l], tr, m.Tf[c1], nm2f);
+        if (r_own < si) {
+          const float q = lazy_q(nd, tr, tsf, nm2f);
+          L = fminf(L, __fsub_rd(q, lazy_err(rep, nm2f)));
+          m.dmax[l] = fmaxf(m.dmax[l], nd);
+          if (q < U) {
+            U = q;
+            m.c1[l] = si;
+            m.d1[l] = nd;
+          }
+        }
+        hint = ford(U);
+      }
+      m.L[l] = L;
+      m.U[l] = U;
+    }
+    if (tid < tm.size) {   // the pairs published for this join that still stand
+      const float4 v = parts[tid];
+      const unsigned e = __float_as_uint(v.z);
+      const int r = e & 0xFFFFu, c = e >> 16;
+      if (v.x < FLT_MAX && r != si && r != sj && c != si && c != sj)
+        hint = min(hint, ford(lazy_q(v.w, m.Tf[r], m.Tf[c], nm2f)));
+    }
+    if (warp * 32 < max(rows, tm.size)) {
+      hint = __reduce_min_sync(0xffffffffu, hint);
+      if (lane == 0) atomicMin(&s_hint, hint);
+    }
+    __syncthreads();
+    if (step + 1 == step1) break;
+    // ---- the rows whose bound reaches it, counted by every warp for itself
+    rep = s_rep;
+    const float E = lazy_err(rep, nm2f);
+    const float best = unford(s_hint);
+    const float reach = best < FLT_MAX ? __fadd_ru(best, __fmul_ru(5.f, E)) : FLT_MAX;
+    int cnt = 0;
+    for (int l0 = 0; l0 < rows; l0 += 32) {
+      const float L = l0 + lane < rows ? m.L[l0 + lane] : FLT_MAX;
+      cnt += __popc(__ballot_sync(0xffffffffu, L <= reach && L < FLT_MAX));
+    }
+    if (cnt) {   // the same in every warp
+      if (warp == 0) {
+        int base = 0;
+        for (int l0 = 0; l0 < rows; l0 += 32) {
+          const float L = l0 + lane < rows ? m.L[l0 + lane] : FLT_MAX;
+          const bool in = L <= reach && L < FLT_MAX;
+          const unsigned bal = __ballot_sync(0xffffffffu, in);
+          if (in) s_list[base + __popc(bal & ((1u << lane) - 1u))] = (int16_t)(l0 + lane);
+          base += __popc(bal);
+        }
+      }
+      __syncthreads();   // also: the bounds are read before the scan changes them
+      scan_rows<false>(s, m, tm, [&](int k) { return (int)s_list[k]; }, cnt, nm2f, E, nullptr, nullptr);
+      __syncthreads();
+    }
+    if (warp == 0) pub = cta_best(m, tm, rows);
+    if (!team_exchange<CL>(g, m, tm, ++seq, pub)) return false;
   }
-  if (!exact) return team_sync<CL>(g, target);   // T[si] from CTA 0
-  __syncthreads();
+  // ---- back to global memory: T, maps and the active list (ascending ids)
+  for (int l = tid; l < rows; l += nth) {
+    const int r = l * tm.size + tm.rank;
+    if (r < n0 && m.node[r] >= 0) s.T[r] = m.To[l];
+  }
+  if (tm.rank == 0) {
+    for (int p = tid; p < n0; p += nth) {
+      s.Tf[p] = m.Tf[p];
+      s.node[p] = m.node[p];
+      s.prow[p] = m.prow[p];
+    }
+    if (tid == 0) s.prow[n0] = spare;
+    __shared__ int w_cnt[33];
+    const int ids = n + step1, per = (ids + nth - 1) / nth;
+    const int a0 = min(tid * per, ids), a1 = min(a0 + per, ids);
+    int keep = 0;
+    for (int v = a0; v < a1; ++v) keep += __ldcg(s.slot + v) >= 0;
+    int incl = keep;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) w_cnt[warp] = incl;
+    __syncthreads();
+    int off = incl - keep;
+    for (int w = 0; w < warp; ++w) off += w_cnt[w];
+    for (int v = a0; v < a1; ++v)
+      if (__ldcg(s.slot + v) >= 0) s.act[off++] = v;
+    if (tid == 0) *s.na = n - step1;
+  }
   return true;
 }
 
-// One join of the team: pass, pick, share.  False when the team stops (a
-// barrier gave up or the pick failed -- the same in every CTA).
-template <bool CL>
-__device__ bool team_join(const NJDev& s, const GridNJ& g, Team tm, int step, int n, int watermark, int*& act,
-                          int*& act2, PickOut& spick, GCand& swin, float& sthr, unsigned& target) {
-  const int m_n = n - step;
-  const float nm2f = (float)(m_n - 2);
-  const double nm2 = (double)(m_n - 2);
-  grid_pass(s, g, tm, nm2f, (step & 1) != 0);
-  if (!team_sync<CL>(g, target)) return false;
-  if (!grid_pick_direct(s, g, tm, nm2, nm2f, watermark, &swin, &spick, &sthr)) {
-    const KCand tfirst = grid_cand(s, g, tm, nm2f, nm2, watermark, sthr);
-    if (!team_sync<CL>(g, target)) return false;
-    // the winner's pair again, as the scan read it (row = the smaller slot)
-    auto rederive = [&](const KCand& w) {
-      const int sa = s.slot[w.a], sb = s.slot[w.b];
-      const int r0 = min(sa, sb), c0 = max(sa, sb);
-      swin = make_cand(r0, c0, s.node[r0], s.node[c0], s.T[r0], s.T[c0], s.D[(size_t)r0 * s.ld + c0], nm2,
-                       watermark);
-    };
-    const int ncount = *(volatile int*)&s.g32[2];   // the same in every CTA
-    if (ncount <= min(s.cand_cap, kListPickMax)) {
-      if (threadIdx.x < 32) {
-        const PickOut r = pick_keys(ncount, [&](int k) { return g.cand[k]; });
-        if (threadIdx.x == 0) {
-          spick = r;
-          if (!r.error) rederive(g.cand[r.idx]);
-        }
-      }
-      __syncthreads();
-    } else {
-      __shared__ KCand sw[32];
-      __shared__ KCand sfirst;
-      const KCand cf = cta_first(tfirst, sw);
-      if (threadIdx.x == 0) g.cbest[tm.rank] = cf;
-      if (!team_sync<CL>(g, target)) return false;
-      if (threadIdx.x < 32) {
-        const PickOut r = pick_keys(tm.size, [&](int k) { return ld_kcand(&g.cbest[k]); });
-        if (threadIdx.x == 0) sfirst = r.error ? kc_none() : ld_kcand(&g.cbest[r.idx]);
-      }
-      __syncthreads();
-      const KCand w = sfirst;
-      grid_cand_count(s, g, tm, nm2f, nm2, watermark, sthr, w);
-      if (!team_sync<CL>(g, target)) return false;
-      if (threadIdx.x == 0) {
-        spick.idx = 0;
-        spick.ties = (unsigned)__ldcg(&s.g32[0]);
-        spick.amb = (unsigned)__ldcg(&s.g32[1]);
-        spick.error = w.b < 0;
-        if (!spick.error) rederive(w);
-      }
-      __syncthreads();
-    }
-  }
-  if (spick.error) {
-    if (tm.rank == 0 && threadIdx.x == 0) record_pick(s, spick);
-    return false;
-  }
-  grid_join_share(s, g, tm, swin, m_n, act, act2);
-  int* t = act;
-  act = act2;
-  act2 = t;
-  return team_sync<CL>(g, target);
-}
-
-// Joins step0 .. step1-1 of an n-taxon job over the whole GPU (the active
-// count before join t is n - t).
-__global__ void __launch_bounds__(1024, 1) nj_grid_kernel(NJDev s, GridNJ g, int step0, int step1, int n,
-                                                         int watermark) {
-  __shared__ PickOut spick;
-  __shared__ GCand swin;
-  __shared__ float sthr;
-  const Team tm{(int)blockIdx.x, (int)gridDim.x};
-  unsigned target = 0;
+// Joins step0 .. step1-1 of an n-taxon job over the whole GPU (one cooperative
+// launch between two rebuilds).
+__global__ void __launch_bounds__(kLazyThreads, 1) nj_lazy_grid_kernel(NJDev s, GridNJ g, int step0, int step1, int n,
+                                                                       int watermark) {
+  extern __shared__ __align__(16) unsigned char smem[];
   if (*(volatile int*)g.abort) return;   // an earlier segment gave up: every CTA leaves
-  for (int p = (int)(blockIdx.x * blockDim.x + threadIdx.x); p < s.n0; p += (int)(gridDim.x * blockDim.x))
-    g.grmin[p] = 0x7F7FFFFF;   // ordered int of FLT_MAX
-  if (blockIdx.x == 0 && threadIdx.x == 0) s.g32[0] = s.g32[1] = s.g32[2] = 0;
-  if (!grid_barrier(g, target)) return;
-  int* act = s.act;
-  int* act2 = g.act2;
-  for (int step = step0; step < step1; ++step) {
-    // the previous join's new list is act, its old one act2
-    if (step > step0 && !grid_join_apply<false>(s, g, tm, swin, spick, step - 1, n, act2, act, target)) return;
-    if (!team_join<false>(s, g, tm, step, n, watermark, act, act2, spick, swin, sthr, target)) return;
-  }
-  if (step1 > step0) grid_join_apply<false>(s, g, tm, swin, spick, step1 - 1, n, act2, act, target);
+  const Team tm{(int)blockIdx.x, (int)gridDim.x};
+  unsigned seq = 0, target = 0;
+  lazy_segment<false>(s, g, tm, smem, step0, step1, n, watermark, seq, target);
 }
 
 // TreeNode::join (TreeNode.cpp:31-58) for a recorded join: L_i = (d + (T_i -
@@ -1146,7 +1463,7 @@ __global__ void __launch_bounds__(256) compact_copy_kernel(NJDev s, const int* m
   const int p = blockIdx.x;
   const int np = map[p];
   if (np < 0) return;
-  const float* row = s.D + (size_t)p * s.ld;
+  const float* row = row_at(s, s.prow[p]);
   float* out = D2 + (size_t)np * ld2;
   for (int c = threadIdx.x; c < s.n0; c += blockDim.x) {
     const int nc = map[c];
@@ -1154,11 +1471,21 @@ __global__ void __launch_bounds__(256) compact_copy_kernel(NJDev s, const int* m
   }
 }
 
-// ---- one job per thread-block cluster (serving and up to 2048 taxa) --------
-// The same phases as the large-n form, with the C CTAs of a cluster as the
-// team and hardware cluster barriers between the phases; the reference's
-// rebuild schedule runs inside the kernel (row sums over the cluster, no
-// compaction: the matrix stays in L2).
+// Every row of the compacted matrix at its slot's place.
+__global__ void compact_rows_kernel(int* prow, int n0, const int* abort) {
+  if (*(volatile const int*)abort) return;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p <= n0) prow[p] = p;
+}
+
+// ---- one job per thread-block cluster ------------------------------------------
+// The lazy search with the C CTAs of a cluster as the team; the exchange goes
+// through distributed shared memory, and the reference's rebuild schedule runs
+// inside the kernel (row sums over the cluster, no compaction: the matrix stays
+// in L2).  Against holding the matrix in the cluster's shared memory and passing
+// over all of it for every join (the form this replaced, up to 768 taxa): 2.31 ms
+// instead of 2.81 for 400 taxa, 3.70 / 4.72 for 600; against a full pass over L2
+// for every join, see the thresholds at cluster_nj_max_n.
 
 struct NJJob {
   NJDev s;
@@ -1175,7 +1502,7 @@ __device__ void team_rowsums(const NJDev& s, const int* act, int w0, int wstride
   const int lane = threadIdx.x & 31;
   for (int k = w0; k < na; k += wstride) {
     const int sk = s.slot[act[k]];
-    const float* row = s.D + (size_t)sk * s.ld;
+    const float* row = row_at(s, s.prow[sk]);
     double part = 0.0, ab = 0.0;
     int lowexp = INT_MAX;
     for (int j = lane; j < na; j += 32) {
@@ -1202,10 +1529,9 @@ __device__ void team_rowsums(const NJDev& s, const int* act, int w0, int wstride
 }
 
 template <int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(1024, 1) nj_cluster_kernel(const NJJob* jobs, int njobs) {
-  __shared__ PickOut spick;
-  __shared__ GCand swin;
-  __shared__ float sthr;
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kLazyThreads, 1) nj_cluster_kernel(const NJJob* jobs,
+                                                                                              int njobs) {
+  extern __shared__ __align__(16) unsigned char smem[];
   __shared__ NJJob sjob;   // the job's descriptor (shared memory keeps registers free)
   const int job = (int)blockIdx.x / C;   // the same for every CTA of the cluster
   if (job >= njobs) return;
@@ -1218,14 +1544,13 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(1024, 1) nj_cluster_
   const int w0 = tm.rank * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
   const int wstride = C * (int)(blockDim.x >> 5);
   const int t0 = tm.rank * (int)blockDim.x + (int)threadIdx.x, tstride = C * (int)blockDim.x;
-  unsigned target = 0;   // (grid barriers only)
+  unsigned seq = 0, target = 0;
   for (int k = t0; k < 2 * n - 1; k += tstride) s.slot[k] = k < n ? k : -1;
   for (int k = t0; k < n; k += tstride) {
     s.node[k] = k;
     s.act[k] = k;
-    g.grmin[k] = 0x7F7FFFFF;
   }
-  for (int k = n + t0; k < s.ld; k += tstride) s.Tf[k] = __int_as_float(0x7FC00000);   // padding: NaN
+  for (int k = t0; k <= n; k += tstride) s.prow[k] = k;
   if (tm.rank == 0 && threadIdx.x == 0) {
     *s.na = n;
     s.g32[0] = s.g32[1] = s.g32[2] = 0;
@@ -1242,36 +1567,36 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(1024, 1) nj_cluster_
   long long ave0 = (((long long)(n - 1) * n) / 2) / kBinT;
   long long ub = ((long long)n * (n - 1)) / 2;
   int watermark = n;
-  int* act = s.act;
-  int* act2 = g.act2;
-  bool pending = false;   // a join whose row sum and maps are still to be written
-  for (int step = 0; step < n - 1; ++step) {
-    if (pending) grid_join_apply<true>(s, g, tm, swin, spick, step - 1, n, act2, act, target);
-    if (!team_join<true>(s, g, tm, step, n, watermark, act, act2, spick, swin, sthr, target)) return;
-    pending = true;
-    if (--pq_ck == 0) {
-      pq_ck = 500;
-      if (steps > 0 && (double)(ub / kBinT) / (double)ave0 > 2.0 && tm.rank == 0 && threadIdx.x == 0) s.stats[3] += 1;
+  for (int step = 0; step < n - 1;) {
+    const int seg_end = steps == INT_MAX ? n - 1 : min(n - 1, step + steps + 1);
+    const bool ok = lazy_segment<true>(s, g, tm, smem, step, seg_end, n, watermark, seq, target);
+    cooperative_groups::this_cluster().sync();   // the state is back in global memory; no CTA writes another's memory
+    if (!ok) return;
+    bool rebuild = false;
+    for (; step < seg_end; ++step) {
+      if (--pq_ck == 0) {
+        pq_ck = 500;
+        if (steps > 0 && (double)(ub / kBinT) / (double)ave0 > 2.0 && tm.rank == 0 && threadIdx.x == 0) s.stats[3] += 1;
+      }
+      const int m_after = n - step - 1;
+      if (steps == 0) {
+        rebuild = true;
+      } else {
+        if (steps != INT_MAX) --steps;
+        ub += m_after - 1;
+      }
     }
-    const int m_after = n - step - 1;
-    if (steps == 0) {
-      grid_join_apply<true>(s, g, tm, swin, spick, step, n, act2, act, target);
-      pending = false;
-      cooperative_groups::this_cluster().sync();
-      team_rowsums(s, act, w0, wstride);
+    if (rebuild) {
+      const int m_after = n - step;
+      team_rowsums(s, s.act, w0, wstride);
       if (tm.rank == 0 && threadIdx.x == 0) s.stats[4] += 1;
-      watermark = n + step + 1;
+      watermark = n + step;
       steps = (m_after < 200) ? INT_MAX : (int)((float)m_after * 0.5f);
       ave0 = (((long long)(m_after - 1) * m_after) / 2) / kBinT;
       ub = ((long long)m_after * (m_after - 1)) / 2;
       cooperative_groups::this_cluster().sync();
-    } else {
-      --steps;
-      ub += m_after - 1;
     }
   }
-  if (pending) grid_join_apply<true>(s, g, tm, swin, spick, n - 2, n, act2, act, target);
-  cooperative_groups::this_cluster().sync();
   for (int k = t0; k < n - 1; k += tstride) join_lengths(s.joins[k]);
 }
 
@@ -1282,7 +1607,11 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(1024, 1) nj_cluster_
 // phase boundary is a CTA barrier; the new node's row sum is complete when the
 // join share's block reduction is.  The arithmetic is that of the other forms.
 
-constexpr int kCtaNJMax = 160;   // above it a cluster's shared memory is faster (measured crossover near 170)
+constexpr int kCtaNJMax = 160;       // at most: shared memory
+// Up to here the CTA is faster than a cluster, whose join costs the same at any
+// small size: 4.94 / 5.63 us a join (CTA / cluster) at 100 taxa, 5.43 / 5.62 at
+// 130, 6.21 / 5.54 at 160.
+constexpr int kCtaNJDefault = 136;
 constexpr int kCtaThreads = 256;
 
 struct CtaLayout {
@@ -1334,7 +1663,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
   if (threadIdx.x == 0) sjob = jobs[blockIdx.x];
   __syncthreads();
   const NJDev& s = sjob.s;
-  const GridNJ& g = sjob.g;
   const int n = sjob.n;
   const CtaLayout L = cta_layout(n);
   const int ldl = L.ldl;
@@ -1645,664 +1973,30 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
   for (int k = tid; k < n - 1; k += nth) join_lengths(s.joins[k]);
 }
 
-// ---- small jobs: the whole join loop in the cluster's shared memory --------
-// Up to kSmemNJMax taxa the matrix fits the distributed shared memory of one
-// cluster.  CTA q holds the rows of the folded slot pairs p = q, q + C, ...
-// (rows p and n-1-p; local row 2*(p/C) + (row != p)); every CTA keeps its own
-// copy of the float row sums, the slot -> node and id -> slot maps and the
-// active list, updated identically, and reads the other CTAs' row minima,
-// partials, row sums and rows through distributed shared memory.  The phases
-// and the arithmetic are those of the global forms (pass with the two
-// smallest q per row, direct pick or fallback scan, join share, apply, the
-// reference's rebuild schedule); only the join records and a fallback
-// candidate list use global memory.
-
-constexpr int kSmemNJMax = 768;
-
-struct SmemLayout {
-  int ldl;   // local row stride (floats, a multiple of 4)
-  int lr;    // local rows per CTA (two per local pair)
-  size_t rows, tf, tloc, tsn, node, slot, act_a, act_b, grm, grc, tvl, bytes;   // grm: every slot
-};
-
-__host__ __device__ inline SmemLayout smem_layout(int n, int C) {
-  auto al = [](size_t x) { return (x + 15) / 16 * 16; };
-  SmemLayout L;
-  L.ldl = (n + 3) & ~3;
-  const int npairs = (n + 1) / 2;
-  L.lr = 2 * ((npairs + C - 1) / C);
-  size_t o = 0;
-  L.rows = o; o += al(sizeof(float) * (size_t)L.lr * L.ldl);
-  L.tf = o; o += al(sizeof(float) * L.ldl);
-  L.tloc = o; o += al(sizeof(double) * L.lr);
-  L.tsn = o; o += al(sizeof(double) * L.lr);
-  L.node = o; o += al(sizeof(int) * n);
-  L.slot = o; o += al(sizeof(int) * 2 * n);
-  L.act_a = o; o += al(sizeof(int) * (n + 1));
-  L.act_b = o; o += al(sizeof(int) * (n + 1));
-  L.grm = o; o += al(sizeof(int) * n);
-  L.grc = o; o += al(sizeof(int4) * L.lr);
-  L.tvl = o; o += al(sizeof(float) * L.lr);
-  L.bytes = o;
-  return L;
-}
-
-template <int C>
-struct SmemNJ {
-  int n, npairs, ldl, lr, rank;
-  float* rows;     // local rows, ldl floats each
-  float* Tf;       // float row sums of every slot (NaN dead / padding)
-  double* Tloc;    // T of the local rows
-  double* Tsn;     // T of the local rows as the pass saw it (the pick reads these)
-  int* node;       // slot -> node id
-  int* slot;       // node id -> slot
-  int* grm;        // every slot: smallest float q of its row (ordered int), pushed by the row's owner
-  int4* grc;       // local rows: second smallest q (ordered int), column and distance of the smallest
-  float* tvl;      // local rows: the new row's value in this join
-  // slot -> owner CTA and local row
-  __device__ __forceinline__ int owner(int r) const {
-    const int p = min(r, n - 1 - r);
-    return p % C;
-  }
-  __device__ __forceinline__ int local_row(int r) const {
-    const int p = min(r, n - 1 - r);
-    return 2 * (p / C) + (r != p ? 1 : 0);
-  }
-  // local row lr of CTA q -> slot, or -1
-  __device__ __forceinline__ int slot_of(int q, int l) const {
-    const int p = (l >> 1) * C + q;
-    if (p >= npairs) return -1;
-    if (l & 1) return n - 1 - p == p ? -1 : n - 1 - p;
-    return p;
-  }
-  template <class T>
-  __device__ __forceinline__ T* at(T* local, int q) const {
-    return cooperative_groups::this_cluster().map_shared_rank(local, q);
-  }
-};
-
-// Row sums of this CTA's live rows over the active list (the reference's
-// ascending-id order; any-order lanes when provably exact), with the float
-// copies written into every CTA's row-sum array.
-template <int C>
-__device__ void smem_rowsums(const SmemNJ<C>& m, const int* act, int na) {
-  const int lane = threadIdx.x & 31;
-  for (int l = (int)(threadIdx.x >> 5); l < m.lr; l += (int)(blockDim.x >> 5)) {
-    const int r = m.slot_of(m.rank, l);
-    if (r < 0 || m.node[r] < 0) continue;
-    const float* row = m.rows + (size_t)l * m.ldl;
-    double part = 0.0, ab = 0.0;
-    int lowexp = INT_MAX;
-    for (int j = lane; j < na; j += 32) {
-      const float x = row[m.slot[act[j]]];
-      part = __dadd_rn(part, (double)x);
-      ab = __dadd_rn(ab, (double)fabsf(x));
-      lowexp = min(lowexp, low_bit_exp(x));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      part = __dadd_rn(part, __shfl_down_sync(0xffffffffu, part, o));
-      ab = __dadd_rn(ab, __shfl_down_sync(0xffffffffu, ab, o));
-      lowexp = min(lowexp, __shfl_down_sync(0xffffffffu, lowexp, o));
-    }
-    double sum = __shfl_sync(0xffffffffu, part, 0);
-    if (lane == 0 && !sum_is_exact(ab, lowexp)) {
-      sum = 0.0;
-      for (int j = 0; j < na; ++j) sum = __dadd_rn(sum, (double)row[m.slot[act[j]]]);
-    }
-    sum = __shfl_sync(0xffffffffu, sum, 0);
-    if (lane == 0) m.Tloc[l] = sum;
-    const float tf = __double2float_rn(sum);
-    if (lane < C) m.at(m.Tf, lane)[r] = tf;
-  }
-}
-
-template <int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(1024, 1) nj_smem_kernel(const NJJob* jobs, int njobs) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ NJJob sjob;
-  __shared__ float sparts[2 * 16];   // every CTA's pass partial (pushed by each CTA)
-  __shared__ USum susums[16];        // every CTA's share sum (pushed by each CTA)
-  __shared__ int rows_sel[kFastRows];
-  __shared__ GCand fc[kFastRows];
-  __shared__ int nsel, s_ok;
-  __shared__ PickOut spick;
-  __shared__ GCand swin;
-  __shared__ float sthr;
-  __shared__ double s_sum;
-  __shared__ int s_exact;
-  namespace cg = cooperative_groups;
-  const int crank = (int)cg::this_cluster().block_rank();
-  const int job = (int)blockIdx.x / C;   // the same for every CTA of the cluster
-  if (job >= njobs) return;
-  if (threadIdx.x == 0) sjob = jobs[job];
-  __syncthreads();
-  const NJDev& s = sjob.s;
-  const GridNJ& g = sjob.g;
-  const int n = sjob.n;
-  __shared__ SmemNJ<C> sm;   // the layout's pointers (shared memory keeps registers free)
-  const SmemLayout L = smem_layout(n, C);
-  if (threadIdx.x == 0) {
-    sm.n = n;
-    sm.npairs = (n + 1) / 2;
-    sm.ldl = L.ldl;
-    sm.lr = L.lr;
-    sm.rank = crank;
-    sm.rows = reinterpret_cast<float*>(smem + L.rows);
-    sm.Tf = reinterpret_cast<float*>(smem + L.tf);
-    sm.Tloc = reinterpret_cast<double*>(smem + L.tloc);
-    sm.node = reinterpret_cast<int*>(smem + L.node);
-    sm.slot = reinterpret_cast<int*>(smem + L.slot);
-    sm.grm = reinterpret_cast<int*>(smem + L.grm);
-    sm.grc = reinterpret_cast<int4*>(smem + L.grc);
-    sm.Tsn = reinterpret_cast<double*>(smem + L.tsn);
-    sm.tvl = reinterpret_cast<float*>(smem + L.tvl);
-  }
-  __syncthreads();
-  const SmemNJ<C>& m = sm;
-  int* act = reinterpret_cast<int*>(smem + L.act_a);
-  int* act2 = reinterpret_cast<int*>(smem + L.act_b);
-  const int rank = m.rank;
-  const int tid = (int)threadIdx.x, nth = (int)blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  // this CTA's rows from the matrix (padding columns 0); maps and lists
-  for (int l = 0; l < m.lr; ++l) {
-    const int r = m.slot_of(rank, l);
-    float* row = m.rows + (size_t)l * m.ldl;
-    for (int c = tid; c < m.ldl; c += nth) row[c] = (r >= 0 && c < n) ? s.D[(size_t)r * s.ld + c] : 0.f;
-  }
-  for (int k = tid; k < m.ldl; k += nth) m.Tf[k] = __int_as_float(0x7FC00000);
-  for (int k = tid; k < 2 * n; k += nth) m.slot[k] = k < n ? k : -1;
-  for (int k = tid; k < n; k += nth) {
-    m.node[k] = k;
-    act[k] = k;
-  }
-  for (int k = tid; k < n; k += nth) m.grm[k] = 0x7F7FFFFF;
-  if (rank == 0 && tid == 0) {
-    s.g32[0] = s.g32[1] = s.g32[2] = 0;
-    s.stats[0] = s.stats[1] = s.stats[2] = s.stats[3] = s.stats[4] = 0;
-  }
-  cg::this_cluster().sync();   // every CTA's row-sum array is NaN before any broadcast lands
-  if (n >= 2) {
-    __syncthreads();
-    smem_rowsums(m, act, n);
-  }
-  cg::this_cluster().sync();
-  const int kBinT = 30 * 31 / 2;
-  int steps = max((int)((float)n * 0.5f), 200);
-  int pq_ck = 500;
-  long long ave0 = (((long long)(n - 1) * n) / 2) / kBinT;
-  long long ub = ((long long)n * (n - 1)) / 2;
-  int watermark = n;
-  bool failed = false;
-  for (int step = 0; step < n - 1 && !failed; ++step) {
-    const int m_n = n - step, next = n + step;
-    const float nm2f = (float)(m_n - 2);
-    const double nm2 = (double)(m_n - 2);
-    // ---- pass: each warp one local pair, 16-byte loads from shared memory
-    {
-      float qmin = FLT_MAX, mmax = 0.f;
-      // the layout's fields in registers (shared-memory stores below would
-      // otherwise make the compiler reload them)
-      const float* const Tfp = m.Tf;
-      const float* const rowsp = m.rows;
-      const int ldl = m.ldl;
-      int* const grmp = m.grm;
-      int4* const grcp = m.grc;
-      double* const tsnp = m.Tsn;
-      const double* const tlocp = m.Tloc;
-      const float4* Tf4 = reinterpret_cast<const float4*>(Tfp);
-      const int nv = ldl >> 2;
-      auto row_pass = [&](int l) {
-        const int r = m.slot_of(rank, l);
-        if (r < 0) return;
-        const float tr = Tfp[r];
-        if (tr != tr) {   // dead
-          if (lane < C) m.at(grmp, lane)[r] = 0x7F7FFFFF;
-          return;
-        }
-        const float* row = rowsp + (size_t)l * ldl;
-        float m1 = FLT_MAX, m2 = FLT_MAX, mag = 0.f;
-        int c1 = -1;
-        const int c0 = r + 1, v0 = (c0 + 3) >> 2;
-        if (lane < 4 * v0 - c0 && c0 + lane < n) pass_elem(row[c0 + lane], Tfp[c0 + lane], c0 + lane, tr, nm2f, m1, m2, c1, mag);
-        const float4* row4 = reinterpret_cast<const float4*>(row);
-        for (int v = v0 + lane; v < nv; v += 32) {
-          const float4 d = row4[v];
-          const float4 tc = Tf4[v];
-          pass_elem(d.x, tc.x, 4 * v, tr, nm2f, m1, m2, c1, mag);
-          pass_elem(d.y, tc.y, 4 * v + 1, tr, nm2f, m1, m2, c1, mag);
-          pass_elem(d.z, tc.z, 4 * v + 2, tr, nm2f, m1, m2, c1, mag);
-          pass_elem(d.w, tc.w, 4 * v + 3, tr, nm2f, m1, m2, c1, mag);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-          const float om1 = __shfl_xor_sync(0xffffffffu, m1, o);
-          const float om2 = __shfl_xor_sync(0xffffffffu, m2, o);
-          const int oc1 = __shfl_xor_sync(0xffffffffu, c1, o);
-          const bool take = om1 < m1 || (om1 == m1 && oc1 < c1);
-          const float lo = take ? om1 : m1, hi = take ? m1 : om1;
-          m2 = fminf(hi, fminf(m2, om2));
-          m1 = lo;
-          c1 = take ? oc1 : c1;
-          mag = fmaxf(mag, __shfl_xor_sync(0xffffffffu, mag, o));
-        }
-        // the pick reads only what the pass wrote (a fast CTA's join share
-        // may already be changing rows and row sums); the row minimum goes to
-        // every CTA
-        if (lane < C) m.at(grmp, lane)[r] = ford(m1);
-        if (lane == 0) {
-          grcp[l] = make_int4(ford(m2), c1, __float_as_int(c1 >= 0 ? row[c1] : 0.f), 0);
-          tsnp[l] = tlocp[l];
-        }
-        qmin = fminf(qmin, m1);
-        mmax = fmaxf(mmax, __fadd_rn(mag, fabsf(tr)));
-      };
-      // a row pair per warp, the two rows' warp reductions in the same
-      // shuffle rounds
-      auto pair_pass = [&](int lp) {
-        float m1[2], m2[2], mag[2], trs[2];
-        int c1[2], rs[2];
-        bool live[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int l = 2 * lp + h;
-          rs[h] = m.slot_of(rank, l);
-          trs[h] = rs[h] >= 0 ? Tfp[rs[h]] : 0.f;
-          live[h] = rs[h] >= 0 && trs[h] == trs[h];
-          if (rs[h] >= 0 && !live[h] && lane < C) m.at(grmp, lane)[rs[h]] = 0x7F7FFFFF;   // dead
-          m1[h] = m2[h] = FLT_MAX;
-          mag[h] = 0.f;
-          c1[h] = -1;
-          if (!live[h]) continue;
-          const int r = rs[h];
-          const float tr = trs[h];
-          const float* row = rowsp + (size_t)l * ldl;
-          const int c0 = r + 1, v0 = (c0 + 3) >> 2;
-          if (lane < 4 * v0 - c0 && c0 + lane < n)
-            pass_elem(row[c0 + lane], Tfp[c0 + lane], c0 + lane, tr, nm2f, m1[h], m2[h], c1[h], mag[h]);
-          const float4* row4 = reinterpret_cast<const float4*>(row);
-          for (int v = v0 + lane; v < nv; v += 32) {
-            const float4 d = row4[v];
-            const float4 tc = Tf4[v];
-            pass_elem(d.x, tc.x, 4 * v, tr, nm2f, m1[h], m2[h], c1[h], mag[h]);
-            pass_elem(d.y, tc.y, 4 * v + 1, tr, nm2f, m1[h], m2[h], c1[h], mag[h]);
-            pass_elem(d.z, tc.z, 4 * v + 2, tr, nm2f, m1[h], m2[h], c1[h], mag[h]);
-            pass_elem(d.w, tc.w, 4 * v + 3, tr, nm2f, m1[h], m2[h], c1[h], mag[h]);
-          }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float om1 = __shfl_xor_sync(0xffffffffu, m1[h], o);
-            const float om2 = __shfl_xor_sync(0xffffffffu, m2[h], o);
-            const int oc1 = __shfl_xor_sync(0xffffffffu, c1[h], o);
-            const bool take = om1 < m1[h] || (om1 == m1[h] && oc1 < c1[h]);
-            const float lo = take ? om1 : m1[h], hi = take ? m1[h] : om1;
-            m2[h] = fminf(hi, fminf(m2[h], om2));
-            m1[h] = lo;
-            c1[h] = take ? oc1 : c1[h];
-            mag[h] = fmaxf(mag[h], __shfl_xor_sync(0xffffffffu, mag[h], o));
-          }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (!live[h]) continue;
-          const int l = 2 * lp + h, r = rs[h];
-          if (lane < C) m.at(grmp, lane)[r] = ford(m1[h]);
-          if (lane == 0) {
-            const float* row = rowsp + (size_t)l * ldl;
-            grcp[l] = make_int4(ford(m2[h]), c1[h], __float_as_int(c1[h] >= 0 ? row[c1[h]] : 0.f), 0);
-            tsnp[l] = tlocp[l];
-          }
-          qmin = fminf(qmin, m1[h]);
-          mmax = fmaxf(mmax, __fadd_rn(mag[h], fabsf(trs[h])));
-        }
-      };
-      // one row per warp when the CTA's rows fit its warps, else one row pair
-      // per warp
-      const int nw = nth >> 5;
-      if (m.lr <= nw) {
-        if (warp < m.lr) row_pass(warp);
-      } else {
-        for (int lp = warp; 2 * lp < m.lr; lp += nw) pair_pass(lp);
-      }
-      __shared__ float wq[32], wm[32];
-      if (lane == 0) {
-        wq[warp] = qmin;
-        wm[warp] = mmax;
-      }
-      __syncthreads();
-      if (warp == 0) {
-        qmin = lane < (nth >> 5) ? wq[lane] : FLT_MAX;
-        mmax = lane < (nth >> 5) ? wm[lane] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) {
-          qmin = fminf(qmin, __shfl_xor_sync(0xffffffffu, qmin, o));
-          mmax = fmaxf(mmax, __shfl_xor_sync(0xffffffffu, mmax, o));
-        }
-        if (lane < C) {
-          float* dst = m.at(sparts, lane);
-          dst[2 * rank] = qmin;
-          dst[2 * rank + 1] = mmax;
-        }
-      }
-    }
-    cg::this_cluster().sync();
-    // ---- pick: threshold from the CTA partials, rows within it, candidates
-    if (warp == 0) {
-      float q = lane < C ? sparts[2 * lane] : FLT_MAX, mm = lane < C ? sparts[2 * lane + 1] : 0.f;
-      for (int o = 16; o > 0; o >>= 1) {
-        q = fminf(q, __shfl_xor_sync(0xffffffffu, q, o));
-        mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-      }
-      if (lane == 0) {
-        sthr = q + 3.f * (8.f * 5.9604645e-8f * mm) + 1e-30f;
-        nsel = 0;
-      }
-    }
-    __syncthreads();
-    const float thr = sthr;
-    const int othr = ford(thr);
-    for (int r = tid; r < n; r += nth) {
-      if (m.grm[r] <= othr) {
-        const int k = atomicAdd(&nsel, 1);
-        if (k < kFastRows) rows_sel[k] = r;
-      }
-    }
-    __syncthreads();
-    const int nr = nsel;
-    if (warp == 0) {
-      int ok = nr >= 1 && nr <= kFastRows;
-      if (ok && lane < nr) {
-        const int r = rows_sel[lane];
-        const int q = m.owner(r), l = m.local_row(r);
-        const int4 rec = m.at(m.grc, q)[l];
-        const int c = rec.y;
-        if (rec.x <= othr || c < 0) {
-          ok = 0;   // a second pair of the row within the threshold
-        } else {
-          const int qc = m.owner(c), lc = m.local_row(c);
-          const double Tr = m.at(m.Tsn, q)[l], Tc = m.at(m.Tsn, qc)[lc];
-          const float d = __int_as_float(rec.z);
-          const int ur = m.node[r], uc = m.node[c];
-          fc[lane] = make_cand(r, c, ur, uc, Tr, Tc, d, nm2, watermark);
-          if (ur < 0 || uc < 0) ok = 0;
-        }
-      }
-      ok = __all_sync(0xffffffffu, ok);
-      PickOut pr{};
-      if (ok && nr == 1) {
-        pr.idx = 0;
-        pr.ties = 1;
-        pr.amb = 0;
-        pr.error = false;
-      } else if (ok) {
-        pr = pick_keys(nr, [&](int k) { return fc[k]; });
-      }
-      if (lane == 0) {
-        s_ok = ok;
-        if (ok) {
-          spick = pr;
-          swin = fc[pr.idx];
-        }
-      }
-    }
-    __syncthreads();
-    if (!s_ok) {
-      // fallback: each CTA scans its own rows within the threshold into the
-      // list (as grid_cand does; beyond the list's capacity the winner comes
-      // from the CTAs' first candidates and a second scan counts against it)
-      // (one warp per local row, lanes over the columns; visit(pred, candidate)
-      // by whole warps as in grid_cand_scan)
-      auto scan = [&](auto&& visit) {
-        for (int l = warp; l < m.lr; l += nth >> 5) {
-          const int r = m.slot_of(rank, l);
-          if (r < 0 || m.grm[r] > othr) continue;
-          const int ur = m.node[r];
-          const float tr = m.Tf[r];
-          const double Tr = m.Tloc[l];
-          const float* row = m.rows + (size_t)l * m.ldl;
-          for (int cb = r + 1; cb < n; cb += 32) {
-            const int c = cb + lane;
-            bool pred = false;
-            KCand kc = kc_none();
-            if (c < n) {
-              const int uc = m.node[c];
-              const float d = row[c];
-              const float q = __fsub_rn(__fsub_rn(__fmul_rn(d, nm2f), tr), m.Tf[c]);
-              if (uc >= 0 && q <= thr) {
-                const double Tc = m.at(m.Tloc, m.owner(c))[m.local_row(c)];
-                const GCand cd = make_cand(r, c, ur, uc, Tr, Tc, d, nm2, watermark);
-                kc = KCand{cd.k1, cd.k2, cd.a, cd.b};
-                pred = true;
-              }
-            }
-            visit(pred, kc);
-          }
-        }
-      };
-      // the winner's pair again, as the scan read it (row = the smaller slot)
-      auto rederive = [&](const KCand& w) {
-        const int sa = m.slot[w.a], sb = m.slot[w.b];
-        const int r0 = min(sa, sb), c0 = max(sa, sb);
-        const int q = m.owner(r0), l = m.local_row(r0);
-        const double Tr = m.at(m.Tloc, q)[l], Tc = m.at(m.Tloc, m.owner(c0))[m.local_row(c0)];
-        const float d = m.at(m.rows, q)[(size_t)l * m.ldl + c0];
-        swin = make_cand(r0, c0, m.node[r0], m.node[c0], Tr, Tc, d, nm2, watermark);
-      };
-      __shared__ KCand skw[32];
-      __shared__ KCand sfirst;
-      KCand first = kc_none();
-      bool full = false;
-      scan([&](bool pred, const KCand& c) {
-        list_push(s, g, pred, c, full);
-        if (pred && kc_first(c, first)) first = c;
-      });
-      cg::this_cluster().sync();
-      const int ncount = *(volatile int*)&s.g32[2];   // the same in every CTA
-      if (ncount <= min(s.cand_cap, kListPickMax)) {
-        if (warp == 0) {
-          const PickOut pr = pick_keys(ncount, [&](int k) { return g.cand[k]; });
-          if (lane == 0) {
-            spick = pr;
-            if (!pr.error) rederive(g.cand[pr.idx]);
-          }
-        }
-        __syncthreads();
-      } else {
-        first = cta_first(first, skw);
-        if (tid == 0) g.cbest[rank] = first;
-        cg::this_cluster().sync();
-        if (warp == 0) {
-          const PickOut pr = pick_keys(C, [&](int k) { return ld_kcand(&g.cbest[k]); });
-          if (lane == 0) sfirst = pr.error ? kc_none() : ld_kcand(&g.cbest[pr.idx]);
-        }
-        __syncthreads();
-        const KCand w = sfirst;
-        unsigned ties = 0, amb = 0;
-        scan([&](bool pred, const KCand& c) {
-          if (pred) count_vs(c, w, ties, amb);
-        });
-        add_counts(ties, amb, s.g32);
-        cg::this_cluster().sync();
-        if (tid == 0) {
-          spick.idx = 0;
-          spick.ties = (unsigned)__ldcg(&s.g32[0]);
-          spick.amb = (unsigned)__ldcg(&s.g32[1]);
-          spick.error = w.b < 0;
-          if (!spick.error) rederive(w);
-        }
-        __syncthreads();
-      }
-      if (spick.error) {   // the same in every CTA
-        if (rank == 0 && tid == 0) record_pick(s, spick);
-        failed = true;
-        break;
-      }
-    }
-    // ---- join share: this CTA's rows
-    const GCand w = swin;
-    const int i = w.a, j = w.b, si = w.sa, sj = w.sb;
-    {
-      USum x;
-      x.u = x.a = 0;
-      x.e = INT_MAX;
-      x.t = INT_MIN;
-      if (tid < m.lr) {
-        const int l = tid;
-        const int r = m.slot_of(rank, l);
-        if (r >= 0 && m.node[r] >= 0 && r != si && r != sj) {
-          float* row = m.rows + (size_t)l * m.ldl;
-          const float Dik = row[si], Djk = row[sj];
-          const float sumf = __fadd_rn(Dik, Djk);
-          const float tmp = __fmul_rn(__fsub_rn(sumf, w.d), 0.5f);
-          const double t = __dadd_rn(m.Tloc[l], (double)__fsub_rn(tmp, sumf));
-          m.Tloc[l] = t;
-          const float tf = __double2float_rn(t);
-          row[si] = tmp;
-          m.at(m.rows, m.owner(si))[(size_t)m.local_row(si) * m.ldl + r] = tmp;   // the new row
-#pragma unroll
-          for (int q = 0; q < C; ++q) m.at(m.Tf, q)[r] = tf;
-          m.tvl[l] = tmp;
-          if (tmp != 0.f) {
-            x.e = low_bit_exp(tmp);
-            x.t = top_bit_exp(tmp);
-            x.u = float_units(tmp, x.e);
-            x.a = x.u < 0 ? -x.u : x.u;
-          }
-        }
-      }
-      const int nwv = (m.lr + 31) >> 5;
-      if (warp < nwv) usum_warp(x);
-      __shared__ USum swp[32];
-      if (lane == 0 && warp < nwv) swp[warp] = x;
-      __syncthreads();   // also: every read of this join's maps is done
-      if (tid == 0) {
-        for (int w2 = 1; w2 < nwv; ++w2) usum_add(x, swp[w2]);
-        for (int q = 0; q < C; ++q) m.at(susums, q)[rank] = x;   // to every CTA
-      }
-      // the maps and the active list, identically in every CTA
-      for (int k = tid; k < m_n; k += nth) {
-        const int v = act[k];
-        if (v != i && v != j) act2[k - (v > i) - (v > j)] = v;
-      }
-      if (tid == 0) {
-        act2[m_n - 2] = next;
-        m.node[sj] = -1;
-        m.node[si] = next;
-        m.slot[j] = -1;
-        m.slot[i] = -1;
-        m.slot[next] = si;
-        m.Tf[sj] = __int_as_float(0x7FC00000);
-      }
-    }
-    cg::this_cluster().sync();
-    // ---- apply: the new node's row sum from the CTA sums
-    if (warp == 0) {
-      USum x;
-      x.u = x.a = 0;
-      x.e = INT_MAX;
-      x.t = INT_MIN;
-      if (lane < C) x = susums[lane];
-      usum_warp(x);
-      if (lane == 0) {
-        if (x.e == INT_MAX) {
-          s_sum = 0.0;
-          s_exact = 1;
-        } else if (x.t - x.e < 48 && x.a < (1ll << 53)) {
-          s_sum = units_to_double(x.u, x.e);
-          s_exact = 1;
-        } else {
-          s_exact = 0;
-        }
-      }
-    }
-    __syncthreads();
-    if (s_exact) {
-      if (tid == 0) {
-        m.Tf[si] = __double2float_rn(s_sum);
-        if (m.owner(si) == rank) m.Tloc[m.local_row(si)] = s_sum;
-      }
-    } else {
-      if (rank == 0 && tid == 0) {
-        double sum = 0.0;   // the reference's loop: active ids ascending, i and j skipped
-        for (int k = 0; k < m_n; ++k) {
-          const int v = act[k];
-          if (v == i || v == j) continue;
-          const int sv = v == next ? si : m.slot[v];
-          sum = __dadd_rn(sum, (double)m.at(m.tvl, m.owner(sv))[m.local_row(sv)]);
-        }
-        const float tf = __double2float_rn(sum);
-        for (int q = 0; q < C; ++q) m.at(m.Tf, q)[si] = tf;
-        m.at(m.Tloc, m.owner(si))[m.local_row(si)] = sum;
-      }
-      cg::this_cluster().sync();
-    }
-    if (rank == 0 && tid == 0) {
-      nwg_join& J = s.joins[step];
-      J.i = i;
-      J.j = j;
-      J.node = next;
-      J.n = m_n;
-      J.d = w.d;
-      J.pad = 0.f;
-      J.q = w.q1;
-      J.ti = w.ta;
-      J.tj = w.tb;
-      s.g32[0] = s.g32[1] = s.g32[2] = 0;
-      record_pick(s, spick);
-    }
-    {
-      int* t = act;
-      act = act2;
-      act2 = t;
-    }
-    // ---- the reference's rebuild schedule (SpeciesBlock.cpp:864, :1206-1247)
-    if (--pq_ck == 0) {
-      pq_ck = 500;
-      if (steps > 0 && (double)(ub / kBinT) / (double)ave0 > 2.0 && rank == 0 && tid == 0) s.stats[3] += 1;
-    }
-    const int m_after = m_n - 1;
-    if (steps == 0) {
-      cg::this_cluster().sync();   // every CTA's own write of the new row sum lands before the broadcasts
-      smem_rowsums(m, act, m_after);
-      if (rank == 0 && tid == 0) s.stats[4] += 1;
-      watermark = next + 1;
-      steps = (m_after < 200) ? INT_MAX : (int)((float)m_after * 0.5f);
-      ave0 = (((long long)(m_after - 1) * m_after) / 2) / kBinT;
-      ub = ((long long)m_after * (m_after - 1)) / 2;
-      cg::this_cluster().sync();
-    } else {
-      --steps;
-      ub += m_after - 1;
-      __syncthreads();
-    }
-  }
-  cg::this_cluster().sync();   // every join record is written; no CTA reads another's shared memory after this
-  if (!failed)
-    for (int k = rank * nth + tid; k < n - 1; k += C * nth) join_lengths(s.joins[k]);
-}
-
 }  // namespace
 
 struct NJState {
   DevBuf D, jobws, desc;
-  // large-n path: row sums, maps, compaction buffers, candidates, grid partials and barrier words
-  DevBuf T, Tf, slot, node, act, na, g32, stats, joins, cand, cbest, tv, grmin, grec, tsnap;
-  DevBuf D2, T2, Tf2, node2, map, act2, part, jsum, jexp, gbar;
+  // whole-GPU form: row sums, maps, compaction buffers, candidates, exchanges and barrier words
+  DevBuf T, Tf, slot, node, act, na, g32, stats, joins, cand, cbest;
+  DevBuf D2, T2, Tf2, node2, map, prow, xrow, tx, gather, gbar;
   ~NJState() {
-    for (DevBuf* b : {&D, &jobws, &desc, &T, &Tf, &slot, &node, &act, &na, &g32, &stats, &joins, &cand, &cbest, &tv, &grmin,
-                      &grec, &tsnap, &D2, &T2, &Tf2, &node2, &map, &act2, &part, &jsum, &jexp, &gbar})
+    for (DevBuf* b : {&D, &jobws, &desc, &T, &Tf, &slot, &node, &act, &na, &g32, &stats, &joins, &cand, &cbest, &D2, &T2,
+                      &Tf2, &node2, &map, &prow, &xrow, &tx, &gather, &gbar})
       b->release();
   }
 };
 
-// Up to this many taxa one cluster runs the whole join loop (the matrix stays
-// in L2); larger matrices take the whole GPU per join.  The environment
-// variable NWG_NJ_CLUSTER_MAX_N overrides the threshold (both forms give the
-// same joins; the tests run each form on the same inputs).
+// Up to this many taxa one cluster runs the whole join loop; larger matrices
+// take the whole GPU.  A cluster's exchange is the cheaper one, the whole GPU
+// has fewer rows to rescan per CTA: 5.94 / 6.15 us a join (cluster / GPU) at 500
+// taxa, 6.18 / 6.12 at 600, 6.30 / 6.12 at 768, 7.19 / 6.32 at 1,100.  The
+// environment variable NWG_NJ_CLUSTER_MAX_N overrides the threshold (both forms
+// give the same joins; the tests run each form on the same inputs).
 int cluster_nj_max_n() {
   static const int v = [] {
     const char* e = std::getenv("NWG_NJ_CLUSTER_MAX_N");
-    return e ? std::atoi(e) : 2048;
+    return e ? std::atoi(e) : 600;
   }();
   return v;
 }
@@ -2348,30 +2042,25 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     // the descriptor travels in the stream (a pageable copy is staged at once)
     if ((rc = cuda(cudaMemcpyAsync(S.desc.p, &J, sizeof(J), cudaMemcpyHostToDevice, s), "nj upload"))) return rc;
     if (st) cudaEventRecord(ev0, s);
-    const int csm = smem_nj_cluster(n);
     if ((rc = cuda(n <= cta_nj_max_n() ? launch_nj_cta(S.desc.p, 1, n, s)
-                   : csm               ? launch_nj_smem(S.desc.p, 1, n, csm, s)
-                                       : launch_nj_cluster(S.desc.p, 1, nj_cluster_size(), s),
+                                       : launch_nj_cluster(S.desc.p, 1, n, nj_cluster_size(), s),
                    "nj launch")))
       return rc;
     ++launches;
   } else {
-    // one CTA of 1024 threads per SM (cooperative launch); every join share
-    // then holds at most one slot per thread
-    const int grid = std::min(sms, kGridMax);
+    // one CTA per SM (cooperative launch)
+    const int grid = std::min(sms, kLazyMaxCtas);
     if ((rc = S.T.ensure(sizeof(double) * n)) || (rc = S.Tf.ensure(sizeof(float) * ldd)) ||
         (rc = S.slot.ensure(sizeof(int) * nn)) || (rc = S.node.ensure(sizeof(int) * n)) ||
         (rc = S.act.ensure(sizeof(int) * (n + 1))) || (rc = S.na.ensure(sizeof(int))) ||
         (rc = S.g32.ensure(sizeof(int) * 4)) || (rc = S.stats.ensure(sizeof(unsigned long long) * 5)) ||
         (rc = S.joins.ensure(sizeof(nwg_join) * (n - 1))) || (rc = S.cand.ensure(sizeof(KCand) * kCandCap)) ||
-        (rc = S.cbest.ensure(sizeof(KCand) * grid)) ||
-        (rc = S.tv.ensure(sizeof(float) * n)) || (rc = S.grmin.ensure(sizeof(int) * n)) ||
-        (rc = S.grec.ensure(sizeof(int4) * n)) || (rc = S.tsnap.ensure(sizeof(double) * n)) || (rc = S.D2.ensure(sizeof(float) * (size_t)n * ldd)) ||
+        (rc = S.cbest.ensure(sizeof(KCand) * grid)) || (rc = S.D2.ensure(sizeof(float) * (size_t)n * ldd)) ||
         (rc = S.T2.ensure(sizeof(double) * n)) || (rc = S.Tf2.ensure(sizeof(float) * ldd)) ||
         (rc = S.node2.ensure(sizeof(int) * n)) || (rc = S.map.ensure(sizeof(int) * n)) ||
-        (rc = S.act2.ensure(sizeof(int) * (n + 1))) || (rc = S.part.ensure(sizeof(float) * 2 * grid)) ||
-        (rc = S.jsum.ensure(sizeof(long long) * 2 * grid)) || (rc = S.jexp.ensure(sizeof(int) * 2 * grid)) ||
-        (rc = S.gbar.ensure(sizeof(int) * 4)))
+        (rc = S.prow.ensure(sizeof(int) * (n + 1))) || (rc = S.xrow.ensure(sizeof(float) * ldd)) ||
+        (rc = S.tx.ensure(sizeof(double) * 2 * n)) ||
+        (rc = S.gather.ensure(sizeof(float4) * 2 * grid)) || (rc = S.gbar.ensure(sizeof(int) * 4)))
       return fail(rc, "nj allocation");
     NJDev d{};
     d.D = (float*)S.D.p;
@@ -2384,28 +2073,35 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     d.g32 = (int*)S.g32.p;
     d.stats = (unsigned long long*)S.stats.p;
     d.joins = (nwg_join*)S.joins.p;
+    d.prow = (int*)S.prow.p;
+    d.xrow = (float*)S.xrow.p;
+    d.tx = (double*)S.tx.p;
     d.n0 = n;
     d.ld = ldd;
     d.cand_cap = kCandCap;
     jsrc = S.joins.p;
     ssrc = S.stats.p;
-    std::vector<int> slot0(nn, -1), act0(n + 1, 0);
+    std::vector<int> slot0(nn, -1), act0(n + 1, n);   // act0: the identity, for the lists and maps
     for (int k = 0; k < n; ++k) slot0[k] = k, act0[k] = k;
     const int na0 = n;
     const int g0[4] = {0, 0, 0, 0};
     if ((rc = cuda(cudaMemcpyAsync(S.slot.p, slot0.data(), sizeof(int) * nn, cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.node.p, act0.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.act.p, act0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s), "nj upload")) ||
+        (rc = cuda(cudaMemcpyAsync(S.prow.p, act0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.na.p, &na0, sizeof(int), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.g32.p, g0, sizeof(g0), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemsetAsync(S.stats.p, 0, sizeof(unsigned long long) * 5, s), "nj upload")) ||
         (rc = cuda(cudaStreamSynchronize(s), "nj upload")))   // the host vectors above are local
       return rc;
+    const int smem = (int)lazy_layout(n, ldd, grid).bytes;   // the first segment's: later ones have fewer slots
     int blocks_per_sm = 0;
-    if ((rc = cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, nj_grid_kernel, 1024, 0),
+    if ((rc = cuda(cudaFuncSetAttribute(nj_lazy_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                   "nj occupancy")) ||
+        (rc = cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, nj_lazy_grid_kernel, kLazyThreads, smem),
                    "nj occupancy")))
       return rc;
-    if (blocks_per_sm < 1 || grid * 1024 < n) return fail(NWG_ERR_CUDA, "neighbor-joining grid kernel does not fit");
+    if (blocks_per_sm < 1) return fail(NWG_ERR_CUDA, "neighbor-joining grid kernel does not fit");
     float* Dalt = (float*)S.D2.p;
     double* Talt = (double*)S.T2.p;
     float* Tfalt = (float*)S.Tf2.p;
@@ -2413,15 +2109,8 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     GridNJ g{};
     g.bar = (unsigned*)S.gbar.p;
     g.abort = (int*)S.gbar.p + 2;
-    g.act2 = (int*)S.act2.p;
-    g.grmin = (int*)S.grmin.p;
-    g.grec = (int4*)S.grec.p;
-    g.tsnap = (double*)S.tsnap.p;
+    g.gather = (float4*)S.gather.p;
     g.cbest = (KCand*)S.cbest.p;
-    g.tv = (float*)S.tv.p;
-    g.part = (float*)S.part.p;
-    g.jsum = (long long*)S.jsum.p;
-    g.jexp = (int*)S.jexp.p;
     g.cand = (KCand*)S.cand.p;
     // NaN (all bits set) float row sums at the padding slots; rowsum_kernel
     // fills the live ones
@@ -2448,7 +2137,8 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
       if ((e = cuda(cudaMemsetAsync(Tfalt, 0xFF, sizeof(float) * ld2, s), "nj launch"))) return e;
       compact_map_kernel<<<1, 1024, 0, s>>>(d, (int*)S.map.p, Talt, Tfalt, nodealt, nn, g.abort);
       compact_copy_kernel<<<d.n0, 256, 0, s>>>(d, (const int*)S.map.p, Dalt, ld2, g.abort);
-      launches += 2;
+      compact_rows_kernel<<<(na + 256) / 256, 256, 0, s>>>(d.prow, na, g.abort);
+      launches += 3;
       std::swap(d.D, Dalt);
       std::swap(d.T, Talt);
       std::swap(d.Tf, Tfalt);
@@ -2457,33 +2147,26 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
       d.ld = ld2;
       return NWG_OK;
     };
-    // Between rebuilds, large matrices are also compacted once a sixteenth of
-    // their slots are dead: the pass streams every column of a live row.
-    constexpr int kCompactMinSlots = 2048, kCompactFrac = 16;
     int step = 0;
     while (step < n - 1) {
-      // the segment ends with the join after which the countdown reaches 0,
-      // or at the next compaction
-      int seg_end = steps == INT_MAX ? n - 1 : std::min(n - 1, step + steps + 1);
-      const bool comp = d.n0 >= kCompactMinSlots && step + d.n0 / kCompactFrac < seg_end;
-      if (comp) seg_end = step + d.n0 / kCompactFrac;
+      // the segment ends with the join after which the countdown reaches 0
+      const int seg_end = steps == INT_MAX ? n - 1 : std::min(n - 1, step + steps + 1);
       if ((rc = cuda(cudaMemsetAsync(S.gbar.p, 0, sizeof(unsigned) * 2, s), "nj launch"))) return rc;
-      // failure injection for the tests (NWG_NJ_INJECT_BARRIER_STALL=1): the
-      // arrival count of the first segment starts one short, so its first
-      // barrier never completes and every CTA gives up after the spin limit
-      if (step == 0 && std::getenv("NWG_NJ_INJECT_BARRIER_STALL") &&
-          std::atoi(std::getenv("NWG_NJ_INJECT_BARRIER_STALL")) == 1 &&
-          (rc = cuda(cudaMemsetAsync(S.gbar.p, 0xFF, sizeof(unsigned), s), "nj launch")))
-        return rc;
+      // failure injection for the tests (NWG_NJ_INJECT_BARRIER_STALL=1): in the
+      // first segment the first CTA never publishes, so the first exchange never
+      // completes and every CTA gives up after the spin limit
+      const char* inject = std::getenv("NWG_NJ_INJECT_BARRIER_STALL");
+      g.stall = step == 0 && inject && std::atoi(inject) == 1 ? 1 : 0;
       {
         int a0 = step, a1 = seg_end, an = n, aw = watermark;
+        const int threads = lazy_threads(d.ld, (d.n0 + grid - 1) / grid, grid);
         void* args[] = {&d, &g, &a0, &a1, &an, &aw};
-        if ((rc = cuda(cudaLaunchCooperativeKernel((const void*)nj_grid_kernel, dim3(grid), dim3(1024), args, 0, s),
+        if ((rc = cuda(cudaLaunchCooperativeKernel((const void*)nj_lazy_grid_kernel, dim3(grid), dim3(threads), args,
+                                                   (size_t)smem, s),
                        "nj launch")))
           return rc;
         ++launches;
       }
-      if ((seg_end - step) & 1) std::swap(d.act, g.act2);   // each join writes the other list
       bool rebuild = false;
       for (; step < seg_end; ++step) {
         if (--pq_ck == 0) {
@@ -2510,8 +2193,6 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
         steps = (m_n < 200) ? INT_MAX : (int)((float)m_n * 0.5f);
         ave0 = (((long long)(m_n - 1) * m_n) / 2) / kBinT;
         ub = ((long long)m_n * (m_n - 1)) / 2;
-      } else if (comp) {
-        if ((rc = compact(m_n))) return rc;
       }
       if ((rc = cuda(cudaGetLastError(), "nj launch"))) return rc;
     }
@@ -2549,12 +2230,12 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
 
 // Workspace of one job of the cluster forms, laid out from `base` (256-byte
 // aligned pieces); fills *J when given.  The job's matrix is separate (n rows
-// of ld floats, ld a multiple of 4; the form over L2 modifies it in place,
-// the shared-memory form only reads it).
+// of ld floats, ld a multiple of 4; the cluster form modifies it in place, the
+// one-CTA form only reads it).
 static size_t job_layout(int n, int ld, char* base, NJJob* J) {
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   const size_t cap = std::min<size_t>(kCandCap, (size_t)n * (n - 1) / 2 + 1);
-  constexpr int kC = 16;   // partials for the largest cluster
+  constexpr int kC = 16;   // the largest cluster
   size_t off = 0;
   auto take = [&](size_t bytes) {
     char* q = base ? base + off : nullptr;
@@ -2566,21 +2247,19 @@ static size_t job_layout(int n, int ld, char* base, NJJob* J) {
   char* slot = take(sizeof(int) * (2 * n));
   char* node = take(sizeof(int) * n);
   char* act = take(sizeof(int) * (n + 1));
-  char* act2 = take(sizeof(int) * (n + 1));
   char* na = take(sizeof(int) * 4);
   char* g32 = take(sizeof(int) * 4);
   char* stats = take(sizeof(unsigned long long) * 5);
-  char* grmin = take(sizeof(int) * n);
-  char* grec = take(sizeof(int4) * n);
-  char* tsnap = take(sizeof(double) * n);
-  char* tv = take(sizeof(float) * n);
-  char* part = take(sizeof(float) * 2 * kC);
-  char* jsum = take(sizeof(long long) * 2 * kC);
-  char* jexp = take(sizeof(int) * 2 * kC);
   char* cand = take(sizeof(KCand) * cap);
   char* cbest = take(sizeof(KCand) * kC);
   char* joins = take(sizeof(nwg_join) * (n > 1 ? n - 1 : 1));
+  char* prow = take(sizeof(int) * (n + 1));
+  char* xrow = take(sizeof(float) * ld);
+  char* tx = take(sizeof(double) * 2 * n);
   if (J) {
+    J->s.prow = (int*)prow;
+    J->s.xrow = (float*)xrow;
+    J->s.tx = (double*)tx;
     J->s.T = (double*)T;
     J->s.Tf = (float*)Tf;
     J->s.slot = (int*)slot;
@@ -2593,14 +2272,6 @@ static size_t job_layout(int n, int ld, char* base, NJJob* J) {
     J->s.n0 = n;
     J->s.ld = ld;
     J->s.cand_cap = (int)cap;
-    J->g.act2 = (int*)act2;
-    J->g.grmin = (int*)grmin;
-    J->g.grec = (int4*)grec;
-    J->g.tsnap = (double*)tsnap;
-    J->g.tv = (float*)tv;
-    J->g.part = (float*)part;
-    J->g.jsum = (long long*)jsum;
-    J->g.jexp = (int*)jexp;
     J->g.cand = (KCand*)cand;
     J->g.cbest = (KCand*)cbest;
     J->n = n;
@@ -2624,16 +2295,23 @@ void nj_job_setup(void* job_out, float* D, int n, int ld, char* base, nwg_join**
 
 size_t nj_job_desc_bytes() { return sizeof(NJJob); }
 
-// One job per cluster of C CTAs (C = 8 or 16).
-cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int C, cudaStream_t s) {
+// One job per cluster of C CTAs (C = 8 or 16); nmax: the largest job.
+cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   const NJJob* jobs = reinterpret_cast<const NJJob*>(d_jobs);
+  const int ld = nj_row_stride(nmax);
+  const int bytes = (int)lazy_layout(nmax, ld, C).bytes;
+  const int rows = (nmax + C - 1) / C;
+  const int threads = lazy_threads(ld, rows, C);
+  cudaError_t e;
   if (C == 16) {
-    cudaError_t e = cudaFuncSetAttribute(nj_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    nj_cluster_kernel<16><<<njobs * 16, 1024, 0, s>>>(jobs, njobs);
+    if ((e = cudaFuncSetAttribute(nj_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) ||
+        (e = cudaFuncSetAttribute(nj_cluster_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+      return e;
+    nj_cluster_kernel<16><<<njobs * 16, threads, bytes, s>>>(jobs, njobs);
   } else {
-    nj_cluster_kernel<8><<<njobs * 8, 1024, 0, s>>>(jobs, njobs);
+    if ((e = cudaFuncSetAttribute(nj_cluster_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))) return e;
+    nj_cluster_kernel<8><<<njobs * 8, threads, bytes, s>>>(jobs, njobs);
   }
   return cudaGetLastError();
 }
@@ -2643,7 +2321,7 @@ cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int C, cudaStream_t
 int cta_nj_max_n() {
   static const int v = [] {
     const char* e = std::getenv("NWG_NJ_CTA_MAX_N");
-    return e ? std::min(std::atoi(e), kCtaNJMax) : kCtaNJMax;
+    return e ? std::min(std::atoi(e), kCtaNJMax) : kCtaNJDefault;
   }();
   return v;
 }
@@ -2654,45 +2332,6 @@ cudaError_t launch_nj_cta(const void* d_jobs, int njobs, int nmax, cudaStream_t 
   cudaError_t e = cudaFuncSetAttribute(nj_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
   nj_cta_kernel<<<njobs, kCtaThreads, bytes, s>>>(reinterpret_cast<const NJJob*>(d_jobs), njobs);
-  return cudaGetLastError();
-}
-
-// Jobs of at most this many taxa run the join loop in the cluster's shared
-// memory (nj_smem_kernel); NWG_NJ_SMEM_MAX_N overrides it (0: never).
-int smem_nj_max_n() {
-  static const int v = [] {
-    const char* e = std::getenv("NWG_NJ_SMEM_MAX_N");
-    return e ? std::min(std::atoi(e), kSmemNJMax) : kSmemNJMax;
-  }();
-  return v;
-}
-
-// The shared-memory form's cluster size for a launch whose largest job has
-// nmax taxa (0 when it does not fit either size).
-int smem_nj_cluster(int nmax) {
-  const size_t cap = 200 * 1024;   // dynamic shared memory per CTA
-  if (nmax > smem_nj_max_n()) return 0;
-  const bool fit8 = smem_layout(nmax, 8).bytes <= cap;
-  const bool fit16 = nj_cluster_size() == 16 && smem_layout(nmax, 16).bytes <= cap;
-  if (nmax < 256 && fit8) return 8;
-  if (fit16) return 16;
-  return fit8 ? 8 : 0;
-}
-
-cudaError_t launch_nj_smem(const void* d_jobs, int njobs, int nmax, int C, cudaStream_t s) {
-  if (njobs <= 0) return cudaSuccess;
-  const NJJob* jobs = reinterpret_cast<const NJJob*>(d_jobs);
-  const int bytes = (int)smem_layout(std::max(nmax, 2), C).bytes;
-  cudaError_t e;
-  if (C == 16) {
-    if ((e = cudaFuncSetAttribute(nj_smem_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) ||
-        (e = cudaFuncSetAttribute(nj_smem_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    nj_smem_kernel<16><<<njobs * 16, 1024, bytes, s>>>(jobs, njobs);
-  } else {
-    if ((e = cudaFuncSetAttribute(nj_smem_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))) return e;
-    nj_smem_kernel<8><<<njobs * 8, 1024, bytes, s>>>(jobs, njobs);
-  }
   return cudaGetLastError();
 }
 
