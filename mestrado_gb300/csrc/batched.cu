@@ -192,7 +192,7 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
       groups.push_back({y, y2, nxg, tc.R, tc.V, tc.W, 2, check});
       y = last + 1;
     } else {
-      const TuneChoice t32 = int32_choice(tc);
+      const TuneChoice t32 = int32_choice(tc, c->plain7(std::max(X.maxlen, Y.maxlen)));
       groups.push_back({y, -1, triangle ? y + 1 : X.n, t32.R, t32.V, 32, 1, 0});
       ++y;
     }
@@ -258,7 +258,7 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   // boundary scratch: buckets run concurrently, so every bucket with more than
   // one band gets its own region
   p->scols = std::max(X.maxlen, 1);
-  size_t scratch_words = 1;
+  size_t scratch_words = 2;   // regions start on 8 bytes
   for (auto& b : p->buckets) {
     b.grid = (int)std::min<int64_t>(b.njobs, (int64_t)c->sms * wave_max_ctas_per_sm(b.R, b.P, b.V, b.W));
     b.grid = std::max(b.grid, 1);

@@ -32,8 +32,8 @@ const int8_t* builtin_matrix();
 const char* letter_order();
 
 struct TuneChoice {
-  int R;   // rows per lane (4 to 32, even; not a multiple of 4, or 28: layouts 2 to 4 on int16x2 lanes only)
-  int V;   // register layout (0 to 6)
+  int R;   // rows per lane (4 to 32, even; not a multiple of 4, or 28: layouts 2 to 4 and 7 on int16x2 lanes only)
+  int V;   // register layout (0 to 7)
   int W;   // lanes per wavefront (32, 16, 8): band of W*R rows; 1: one pair per thread, bands of R rows
 };
 // Rows a Y of `rows` residues occupies under choice t (whole bands).
@@ -44,8 +44,11 @@ inline int padded_rows(const TuneChoice& t, int rows) {
 // The same band on full-width fronts, for groups that run on int32 lanes
 // (the narrow fronts and the rows per lane that are not multiples of 4 exist
 // for int16x2 lanes only).
-inline TuneChoice int32_choice(TuneChoice t) {
+// Layout 7 has no sentinel at the borders, which on int32 lanes the reference's
+// -32768 + ge can reach: it needs ge * length + go below it (plain7).
+inline TuneChoice int32_choice(TuneChoice t, bool plain7) {
   if (t.V == 6) t.V = 3;   // the split strips exist for int16x2 lanes only
+  if (t.V == 3 || t.V == 7) t.V = plain7 ? 7 : 3;
   if (t.W == 32 && t.R % 4 == 0 && t.R != 28) return t;
   const int band = t.W * t.R;
   int R = 32;
@@ -57,15 +60,44 @@ constexpr int kTuneClasses = NWG_TUNE_CLASSES;
 // Upper bound of the Y rows of each class; the last class takes every longer Y.
 constexpr int kClassRows[kTuneClasses] = {64,  96,  128, 160, 192, 224, 256,  320,
                                           384, 448, 512, 640, 768, 1024, 1536, 1 << 30};
-// Defaults before tuning (the table measured on a GB300): one pair per thread
-// (W = 1) for the classes up to 96 rows, wavefronts above, mostly the
-// layouts with 1.5 ALU operations per cell (3, and 6 where R is a multiple of 8).
+// Defaults before tuning, measured on a GB300.  Where layout 7 is exact (go >=
+// ge, see Int16Limits), each class has the candidates that are the fastest for
+// some Y of the class, with their rates in GCUPS over band-padded rows: the plan
+// takes the one with the least estimated time per Y group, as after tuning.
+// Layout 7 is the fastest in every class (at 450 rows 9.1 TCUPS against 7.6 for
+// layout 3, at 2,000 10.1 against 8.4); up to 64 rows with one pair per thread.
+struct RatedChoice {
+  int R, W, gcups;
+};
+constexpr int kRatedMax = 6;
+constexpr RatedChoice kDefaultRated[kTuneClasses][kRatedMax] = {
+    {{32, 1, 6324}, {16, 1, 5010}, {24, 1, 6110}},
+    {{12, 8, 7298}, {24, 1, 5742}},
+    {{16, 8, 8474}},
+    {{20, 8, 8907}, {18, 8, 8672}},
+    {{24, 8, 8996}, {22, 8, 8823}},
+    {{28, 8, 8907}, {26, 8, 9161}},
+    {{16, 8, 8898}},
+    {{20, 8, 8838}, {18, 16, 8816}},
+    {{24, 16, 9266}, {22, 16, 9102}},
+    {{28, 16, 9143}, {26, 16, 9148}, {18, 8, 8907}},
+    {{16, 32, 8755}, {30, 16, 8620}},
+    {{20, 16, 9461}, {18, 16, 9409}},
+    {{24, 16, 9875}, {22, 16, 9778}},
+    {{32, 32, 9808}, {30, 32, 9791}, {26, 16, 9804}, {18, 16, 9678}, {28, 16, 9787}},
+    {{24, 16, 10136}, {22, 16, 10060}, {26, 16, 9923}, {28, 16, 9915}, {20, 32, 9635}, {30, 16, 9669}},
+    {{30, 32, 10106}, {26, 32, 10082}, {32, 32, 10066}, {28, 32, 10032}, {22, 32, 9952}, {24, 32, 9909}}};
+// The wavefronts for latency-bound callers (the serving loop): one pair per
+// thread needs 256 X per CTA and streams a Y in bands, so it wins on throughput
+// over many X but lengthens a small job; one band per Y up to 1,024 rows.
+constexpr TuneChoice kDefaultTuneWave7[kTuneClasses] = {
+    {8, 7, 8},   {12, 7, 8},  {16, 7, 8},  {20, 7, 8},  {24, 7, 8},  {28, 7, 8},  {16, 7, 16}, {20, 7, 16},
+    {24, 7, 16}, {28, 7, 16}, {16, 7, 32}, {20, 7, 32}, {24, 7, 32}, {32, 7, 32}, {24, 7, 32}, {32, 7, 32}};
+// Without layout 7: one choice per class, mostly the layouts with 1.5 ALU
+// operations per cell (3, and 6 where R is a multiple of 8).
 constexpr TuneChoice kDefaultTune[kTuneClasses] = {
     {32, 4, 1},  {32, 4, 1},  {16, 5, 8},  {20, 3, 8},  {24, 6, 8},  {28, 3, 8},  {32, 6, 8},  {20, 3, 16},
     {24, 6, 16}, {28, 3, 16}, {32, 6, 16}, {20, 3, 32}, {24, 6, 16}, {32, 3, 32}, {24, 6, 16}, {32, 3, 32}};
-// The best wavefront (W >= 8) per class before tuning, for latency-bound
-// callers: one pair per thread needs 256 X per CTA and streams a Y in bands,
-// so it wins on throughput over many X but lengthens a small job.
 constexpr TuneChoice kDefaultTuneWave[kTuneClasses] = {
     {8, 5, 8},   {12, 0, 8},  {16, 5, 8},  {20, 3, 8},  {24, 6, 8},  {28, 3, 8},  {32, 6, 8},  {20, 3, 16},
     {24, 6, 16}, {28, 3, 16}, {32, 6, 16}, {20, 3, 32}, {24, 6, 16}, {32, 3, 32}, {24, 6, 16}, {32, 3, 32}};
@@ -78,7 +110,7 @@ void destroy_plans(Ctx* c);
 struct Ctx {
   int go = 10, ge = 2;
   int8_t sub[kLetters * kLetters];
-  Int16Limits i16{kInt16MaxLen, 32756 - 11};   // set from (go, ge, sub) at creation
+  Int16Limits i16{kInt16MaxLen, 32756 - 11, 0};   // set from (go, ge, sub) at creation
   int device = 0, sms = 1;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
@@ -92,17 +124,31 @@ struct Ctx {
   // small jobs are latency-bound (one pair per thread lengthens them).
   TuneChoice tune_wave[kTuneClasses];
   // Every candidate the autotuner timed per class, with its rate in computed
-  // cells per second (band-padded rows x columns / time).  Empty when the
-  // table was set by hand or not tuned: tune[] is then used as it is.
+  // cells per second (band-padded rows x columns / time); before tuning the
+  // defaults' rates.  Empty when the table was set by hand (or without layout 7
+  // before tuning): tune[] is then used as it is.
   struct Cand {
     TuneChoice t;
     double rate;
   };
   std::vector<Cand> cands[kTuneClasses];
+  // The tables before tuning.
+  void default_tuning() {
+    for (int k = 0; k < kTuneClasses; ++k) {
+      const bool seven = i16.max_len7 > 0;
+      cands[k].clear();
+      tune[k] = seven ? TuneChoice{kDefaultRated[k][0].R, 7, kDefaultRated[k][0].W} : kDefaultTune[k];
+      tune_wave[k] = seven ? kDefaultTuneWave7[k] : kDefaultTuneWave[k];
+      if (!seven) continue;
+      for (const RatedChoice& r : kDefaultRated[k])
+        if (r.R > 0) cands[k].push_back({{r.R, 7, r.W}, 1e9 * r.gcups});
+    }
+  }
   // The choice for a Y group of this many rows: the class's candidate with
   // the least estimated time (its padded rows / its rate), the class's
   // fastest at the class bound unless another is estimated 2 % faster.
-  // Layout 4 is exact only when go >= ge and falls back to layout 2.
+  // Layout 4 is exact only when go >= ge and falls back to layout 2; layout 7
+  // falls back to layout 3 beyond its range.
   TuneChoice choice(int rows) const {
     const int k = tune_class(rows);
     TuneChoice t = tune[k], fastest = t;
@@ -116,13 +162,18 @@ struct Ctx {
       }
     }
     if (pick_est > 0.0 && min_est < 0.98 * pick_est) t = fastest;
+    return allowed(t, rows);
+  }
+  TuneChoice allowed(TuneChoice t, int rows) const {
     if (t.V == 4 && go < ge) t.V = 2;
+    if (t.V == 7 && rows > i16.max_len7) t.V = 3;
     return t;
   }
+  // Layout 7 on int32 lanes: no border value of sequences up to maxlen falls to
+  // the reference's sentinel.
+  bool plain7(int maxlen) const { return go >= ge && (int64_t)ge * maxlen + go < 32700; }
   TuneChoice choice_wave(int rows) const {
-    TuneChoice t = tune_wave[tune_class(rows)];
-    if (t.V == 4 && go < ge) t.V = 2;
-    return t;
+    return allowed(tune_wave[tune_class(rows)], rows);
   }
   uint64_t tune_version = 0;        // bumped on every change (part of the plan key)
   bool tuned = false;

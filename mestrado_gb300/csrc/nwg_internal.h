@@ -32,9 +32,15 @@ constexpr int kPlainRows = 16;            // rows per thread strip in the plain 
 //    optimistically, are checked against the device-side bounds and re-run on
 //    int32 lanes when the check fails.
 constexpr int kInt16MaxLen = 6900;
+// Layout 7 of the wave kernel keeps H~ = H + ge (r + c + 2) instead: 0 on the
+// borders and never below -(go - ge), so the halves start there.  A diagonal
+// step adds 2 ge more than to H, a gap adds nothing, so H~ of a pair is at most
+// its H bound + 2 ge times its shorter length.
+constexpr int layout7_zero(int go, int ge) { return 2 * (go - ge) + 136; }   // H~ = 0; below: g twice, an int8 entry
 struct Int16Limits {
   int max_len;   // longest sequence of a set that may use int16 lanes (0: none)
   int max_h;     // largest H an int16 pair may reach
+  int max_len7;  // longest shorter sequence of a pair on layout 7 (0: go < ge, or no room)
 };
 inline Int16Limits int16_limits(int go, int ge, const int8_t* sub) {
   int smin = 127, smax = -128;
@@ -47,7 +53,10 @@ inline Int16Limits int16_limits(int go, int ge, const int8_t* sub) {
   const int slack = go + ge + (smin < 0 ? -smin : 0);
   int len = (32764 - slack) / w - 2 - 32 * 32;
   len = len < 0 ? 0 : (len > kInt16MaxLen ? kInt16MaxLen : len);
-  return {len, 32756 - (smax > 0 ? smax : 0)};
+  const int max_h = 32756 - (smax > 0 ? smax : 0);
+  const long long room = 65535ll - 256 - max_h - layout7_zero(go, ge) - 2ll * ge;
+  const int len7 = go < ge || room <= 0 ? 0 : ge == 0 ? kInt16MaxLen : (int)(room / (2ll * ge));
+  return {len, max_h, len7 < kInt16MaxLen ? len7 : kInt16MaxLen};
 }
 
 // Sequence set laid out on the device for one call: sorted by length

@@ -186,7 +186,7 @@ int Server::launch_batch(Slot& S) {
         groups.push_back({gyi, y2, last + 1, (int)base, tc.R, tc.V, tc.W, 2, (int64_t)J->d_off, ldp});
         y = last + 1;
       } else {
-        const TuneChoice t32 = int32_choice(tc);
+        const TuneChoice t32 = int32_choice(tc, c.plain7(len[base]));
         groups.push_back({gyi, -1, y + 1, (int)base, t32.R, t32.V, 32, 1, (int64_t)J->d_off, ldp});
         ++y;
       }
@@ -221,7 +221,7 @@ int Server::launch_batch(Slot& S) {
     buckets.push_back(b);
     k = e;
   }
-  size_t scratch_words = 1;
+  size_t scratch_words = 2;   // regions start on 8 bytes
   for (auto& b : buckets) {
     b.grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(b.njobs, (int64_t)c.sms * wave_max_ctas_per_sm(b.R, b.P, b.V, b.W)));

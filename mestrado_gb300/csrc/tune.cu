@@ -68,7 +68,7 @@ int probe_rows(int k, const TuneChoice& t) {
   return whole > lo ? whole : hi;
 }
 
-const char kCacheTag[] = "nwgpu-tune-7";   // bumped whenever the candidate set changes
+const char kCacheTag[] = "nwgpu-tune-8";   // bumped whenever the candidate set changes
 
 }  // namespace
 
@@ -176,10 +176,12 @@ int Ctx::autotune(bool force, nwg_tune_result* out) {
     TuneChoice pick = kDefaultTune[k], pick_wave = kDefaultTuneWave[k];
     for (int W : {32, 16, 8, 1})
     for (int R : kCandR) {
-      for (int V = 0; V <= 6; ++V) {
+      for (int V = 0; V <= 7; ++V) {
         const TuneChoice cand{R, V, W};
         const int Lyc = probe_rows(k, cand);
-        if (Lyc == 0 || !wave_exists(R, 2, V, W) || (V == 4 && go < ge)) continue;
+        if (Lyc == 0 || !wave_exists(R, 2, V, W) || (V == 4 && go < ge) ||
+            (V == 7 && Lyc > i16.max_len7))
+          continue;
         for (int j = 0; j <= ny; ++j) yoff[j] = (int64_t)nx * Lx + (int64_t)j * Lyc;
         tune[k] = cand;
         ++tune_version;
@@ -221,10 +223,7 @@ int Ctx::autotune(bool force, nwg_tune_result* out) {
   use_graphs = saved_graphs;
   ++tune_version;
   if (rc) {
-    for (int k = 0; k < kTuneClasses; ++k) {
-      tune[k] = kDefaultTune[k];
-      tune_wave[k] = kDefaultTuneWave[k];
-    }
+    default_tuning();
     return rc;
   }
   for (int k = 0; k < kTuneClasses; ++k) cands[k] = std::move(found[k]);

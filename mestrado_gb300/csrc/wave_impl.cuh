@@ -44,6 +44,15 @@
 // before.  The two halves are independent within a step, so the lane has two
 // dependency chains of R/2 rows instead of one of R, with layout 3's 3 ALU
 // operations per word; the skew between lanes becomes two columns.
+// V = 7 scores the alignment with the extension cost taken out: with
+// H~ = H + ge (r + c + 2), and E~, F~ alike, and g = go - ge,
+//   F~[r+1][c] = max(F~[r][c], H~[r][c] - g),  E~[r][c+1] = max(E~[r][c], H~[r][c] - g),
+//   H~ = max(E~, F~, H~[r-1][c-1] + (S + 2 ge)),
+// the same values again, with H~ = 0 and E~ = F~ = -g all along both borders.
+// Three ALU operations per word as in layout 3, but one add instead of two
+// (S + 2 ge is in the profile), two dependent operations from row to row, and
+// nothing to carry along the border.  Nothing falls below -g, so the halves
+// hold [0, 65535) from there up; rows past a Y add 0 instead of S + 2 ge.
 // V = 5 is layout 3 with two X per front: every lane runs the strips of two
 // X (adjacent in length order) against the same band, row by row
 // interleaved, so two independent dependency chains share the lane's issue
@@ -267,6 +276,31 @@ __device__ __forceinline__ uint32_t strip_column(BandState<R, P, V>& s, const ui
         hd = hn;
       }
       pv = pn;
+    }
+    return f;
+  }
+  if (V == 7) {
+    // fin is F~ of the strip's first row, NGO the per-half operand -g; s.E holds
+    // E~ of the column at hand, and of the next one after it.  The diagonal
+    // terms of all rows replace H first, from the last row up: every value then
+    // stays in its register (an order that keeps two rows' H alive costs a
+    // register move per word, 1.92 instead of 1.5 IMAD).
+#pragma unroll
+    for (int q = Q - 1; q >= 0; --q) {
+      const uint4 pv = pp[q * W];
+      const uint32_t sv[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+      for (int w = 3; w >= 0; --w) {
+        const int r = q * 4 + w;
+        if (r >= R) continue;
+        s.H[r] = L::add(r > 0 ? s.H[r > 0 ? r - 1 : 0] : diag, sv[w]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      s.H[r] = L::max3(s.E[r], f, s.H[r]);
+      f = L::addmax(s.H[r], NGO, f);
+      s.E[r] = L::addmax(s.H[r], NGO, s.E[r]);
     }
     return f;
   }
@@ -510,6 +544,128 @@ __device__ __forceinline__ void wave_band_split(const WaveArgs& a, int sl, int b
   }
 }
 
+// Layout 7 on wavefronts (W > 1): the step's own work is what the strip leaves,
+// so little is left of it.  The codes of the next 32 columns and the boundary row
+// under which they run are staged in shared memory, the codes as byte offsets
+// into the profile, one block of columns ahead of their use in registers.  A
+// step is then two shuffles, the lane's profile offset, the boundary of the
+// first lane, the strip, and the store of the last lane; nothing is clamped,
+// selected by band or addressed per step.  Columns before the first carry the
+// offset of a profile row of zeros, which leaves the border's state as it is:
+// the ramp up needs no checks.
+constexpr int kStageCols = 32;
+template <int W>
+struct Stage {
+  static constexpr int kFronts = kWaveWarps * (32 / W);
+  static constexpr int kCodes = W + kStageCols;                       // words per front, W of the block before
+  static constexpr size_t kBytes = (size_t)kFronts * (kStageCols * sizeof(int2) + kCodes * sizeof(uint32_t));
+};
+
+// One band of layout 7; arguments as wave_band's.  border / codes: the front's
+// staging buffers.
+template <int R, int P, int W>
+__device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int nb, const int8_t* __restrict__ X,
+                                           int Lx, int Lmin, int Lmax, const uint32_t* __restrict__ prof,
+                                           int2* __restrict__ border, uint32_t* __restrict__ codes,
+                                           int32_t* __restrict__ scratch, int rowA, int rowB, bool wantA, bool wantB,
+                                           int xo, int yoA, int yoB, float* jobD, int64_t jobld) {
+  using L = Lanes<P>;
+  constexpr int BAND = W * R;
+  constexpr int LSB = Profile<R, W>::kLetterStride * 16;   // bytes per letter
+  constexpr int KS = kStageCols / W;                        // staged columns per lane
+  const uint32_t NG = L::packed(a.ge - a.go);
+  const int zero = P == 2 ? layout7_zero(a.go, a.ge) - 32768 : 0;   // the border's H~
+  const uint32_t ZERO = L::splat(zero), GAP = L::splat(zero + a.ge - a.go);
+  BandState<R, P, 7> s;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    s.H[r] = ZERO;
+    s.E[r] = GAP;
+  }
+  uint32_t hprev = ZERO, hbot = ZERO, fbot = GAP;
+  const bool top = b == 0;
+  const int2* rd = reinterpret_cast<const int2*>(scratch) + (size_t)((b + 1) & 1) * a.scratch_cols;   // band b-1
+  int2* wr = reinterpret_cast<int2*>(scratch) + (size_t)(b & 1) * a.scratch_cols - sl;
+  const bool store = sl == W - 1 && b + 1 < nb && Lx > 0;
+  const char* pl = reinterpret_cast<const char*>(prof) + 16 * sl;
+
+  int nx[KS];
+  int2 nb2[KS];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      const int c = t0 + sl + W * k;
+      nx[k] = c < Lx ? (int)X[c] : 0;
+      nb2[k] = !top && c < Lx ? rd[c] : make_int2((int)ZERO, (int)GAP);
+    }
+  };
+  uint32_t last = kLetters * LSB;   // columns before the first: the row of zeros
+  fetch(0);
+
+  auto step = [&](int t0, int i, auto checked) {
+    constexpr bool kChecked = decltype(checked)::value;
+    const int c = t0 + i - sl;
+    uint32_t hin = __shfl_up_sync(0xffffffffu, hbot, 1, W);
+    uint32_t fin = __shfl_up_sync(0xffffffffu, fbot, 1, W);
+    const uint32_t off = codes[W - sl + i];
+    if (sl == 0) {
+      const int2 bd = border[i];
+      hin = (uint32_t)bd.x;
+      fin = (uint32_t)bd.y;
+    }
+    if (!kChecked || c < Lx) {
+      const uint32_t diag = hprev;
+      hprev = hin;
+      fbot = strip_column<R, P, 7, W>(s, reinterpret_cast<const uint4*>(pl + off), diag, hin, fin, 0u, NG, 0u);
+      hbot = s.H[R - 1];
+      if (store && (!kChecked || c >= 0)) wr[t0 + i] = make_int2((int)hbot, (int)fbot);
+    }
+  };
+  const int nt = Lmax + W - 1;
+  for (int t0 = 0; t0 < nt; t0 += kStageCols) {
+    __syncwarp();
+    codes[sl] = last;
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      last = clamp_code(nx[k]) * LSB;
+      codes[W + W * k + sl] = last;
+      border[W * k + sl] = nb2[k];
+    }
+    __syncwarp();
+    fetch(t0 + kStageCols);
+    const int ne = min(nt - t0, kStageCols);
+    const int ns = min(Lmin - t0, kStageCols);   // steps below it leave no lane past its last column
+    for (int i = 0; i < ne;) {
+      if (t0 + i >= W - 1 && i < ns) {   // every lane on a column
+#pragma unroll 8   // 1: 8.2, 4: 9.6, 8: 10.0, 16: 9.8 TCUPS (R = 24, W = 16): fewer register moves
+        for (; i < ns; ++i) step(t0, i, std::false_type{});
+      } else {
+        step(t0, i, std::true_type{});
+        ++i;
+      }
+    }
+  }
+
+  // H[] now holds the last column; the lane owning a pair's last row reports.
+  const int csh = -zero - a.ge * (Lx + 1);
+  if (wantA) {
+    const int rr = rowA - b * BAND;
+    if (rr >= 0 && rr < BAND && sl == rr / R) {
+      const int v = L::lo(pick<R>(s.H, rr % R)) + csh - a.ge * rowA;
+      if (jobD) put_score_job(a, jobD, jobld, xo, yoA, v);
+      else put_score(a, xo, yoA, v);
+    }
+  }
+  if (P == 2 && wantB) {
+    const int rr = rowB - b * BAND;
+    if (rr >= 0 && rr < BAND && sl == rr / R) {
+      const int v = L::hi(pick<R>(s.H, rr % R)) + csh - a.ge * rowB;
+      if (jobD) put_score_job(a, jobD, jobld, xo, yoB, v);
+      else put_score(a, xo, yoB, v);
+    }
+  }
+}
+
 // One band (W*R rows starting at b*W*R) of the front's K X (K = 2 for V = 5).
 // sl: lane within the front; Lx[k]: length of X k, 0 when it has no pair to
 // report (its strip is then not computed; the lanes still take part in the
@@ -529,22 +685,26 @@ __device__ __forceinline__ void wave_band(const WaveArgs& a, int sl, int b, int 
   constexpr int VL = Layout<V>::L;
   constexpr int BAND = W * R;
   const uint32_t NGE = L::packed(-a.ge);        // per-half operand of addmax
-  const uint32_t NGO = L::arith(-a.go, -a.go);   // word added to H to get H - go
+  // word added to H to get H - go (layout 7: the per-half operand -(go - ge))
+  const uint32_t NGO = VL == 7 ? L::packed(a.ge - a.go) : L::arith(-a.go, -a.go);
   const uint32_t NGOP = L::packed(-a.go);        // per-half operand: - go
-  const uint32_t NGEA = L::arith(-a.ge, -a.ge);  // word added to H[-1][c] to get H[-1][c+1]
+  const int zero7 = P == 2 ? layout7_zero(a.go, a.ge) - 32768 : 0;   // layout 7: the border's H~
+  const int nge = VL == 7 ? 0 : -a.ge;           // H's slope along the borders
+  const uint32_t NGEA = L::arith(nge, nge);      // word added to H[-1][c] to get H[-1][c+1]
   // E[r][-1] = F[-1][c] = -32768 + ge; layouts 2 and 4 keep them shifted by go
-  const uint32_t SENT = L::splat(kShortMin + a.ge + ((VL == 2 || VL == 4) ? a.go : 0));
+  const uint32_t SENT = VL == 7 ? L::splat(zero7 + a.ge - a.go)
+                                : L::splat(kShortMin + a.ge + ((VL == 2 || VL == 4) ? a.go : 0));
 
   constexpr int SST = scratch_stride<W>();
   constexpr int LS = Profile<R, W>::kLetterStride;
   BandState<R, P, VL> s[K];
   const int rowbase = b * BAND + sl * R;
-  const int gsh = VL == 3 ? a.go : 0;               // layout 3 carries T = H - go instead of H
+  const int gsh = VL == 3 ? a.go : VL == 7 ? -zero7 : 0;   // layout 3 carries T = H - go instead of H
 #pragma unroll
   for (int k = 0; k < K; ++k)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      s[k].H[r] = L::splat(-a.ge * (rowbase + r + 1) - gsh);   // H[row][-1] (T for layout 3)
+      s[k].H[r] = L::splat(nge * (rowbase + r + 1) - gsh);     // H[row][-1] (T for layout 3)
       s[k].E[r] = SENT;                                         // E[row][-1]
       if (VL == 0) s[k].T[(VL == 0) ? r : 0] = L::add(s[k].H[r], NGO);
     }
@@ -557,14 +717,14 @@ __device__ __forceinline__ void wave_band(const WaveArgs& a, int sl, int b, int 
   const uint4* pl = reinterpret_cast<const uint4*>(prof) + sl;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    hprev[k] = L::splat(-a.ge * rowbase - gsh);     // H[rowbase-1][-1]: diag of column 0
+    hprev[k] = L::splat(nge * rowbase - gsh);       // H[rowbase-1][-1]: diag of column 0
     hbot[k] = fbot[k] = 0;
     work[k] = Lx[k] > 0;
     rd[k] = scratch + ((size_t)k * 4 * a.scratch_cols + ((b + 1) & 1) * 2 * a.scratch_cols) * SST;   // band b-1
     wr[k] = scratch + ((size_t)k * 4 * a.scratch_cols + (b & 1) * 2 * a.scratch_cols) * SST;
     xnext[k] = (sl == 0 && work[k]) ? (int)X[k][0] : 0;
   }
-  uint32_t hb = L::splat(-a.ge - gsh);              // H[-1][c] of the column lane 0 works on (band 0)
+  uint32_t hb = L::splat(nge - gsh);                // H[-1][c] of the column lane 0 works on (band 0)
   const bool last_band = b + 1 >= nb;
 
   auto step = [&](int t, auto checked) {
@@ -594,7 +754,7 @@ __device__ __forceinline__ void wave_band(const WaveArgs& a, int sl, int b, int 
         fin[k] = top ? SENT : (uint32_t)rd[k][(size_t)(2 * c + 1) * SST];
       }
     }
-    if (!kChecked || c >= 0) hb = L::add(hb, NGEA);
+    if (VL != 7 && (!kChecked || c >= 0)) hb = L::add(hb, NGEA);
     bool paired = false;
     if constexpr (K == 2) {
       if (!kChecked && on[0] && on[1]) {
@@ -644,10 +804,11 @@ __device__ __forceinline__ void wave_band(const WaveArgs& a, int sl, int b, int 
   // H[] now holds the last column; the lane owning a pair's last row reports.
 #pragma unroll
   for (int k = 0; k < K; ++k) {
+    const int csh = VL == 7 ? gsh - a.ge * (Lx[k] + 1) : gsh;   // layout 7: less ge (r + 1) below
     if (wantA[k]) {
       const int rr = rowA - b * BAND;
       if (rr >= 0 && rr < BAND && sl == rr / R) {
-        const int v = L::lo(pick<R>(s[k].H, rr % R)) + gsh;
+        const int v = L::lo(pick<R>(s[k].H, rr % R)) + csh - (VL == 7 ? a.ge * rowA : 0);
         if (jobD) put_score_job(a, jobD, jobld, xo[k], yoA, v);
         else put_score(a, xo[k], yoA, v);
       }
@@ -655,7 +816,7 @@ __device__ __forceinline__ void wave_band(const WaveArgs& a, int sl, int b, int 
     if (P == 2 && wantB[k]) {
       const int rr = rowB - b * BAND;
       if (rr >= 0 && rr < BAND && sl == rr / R) {
-        const int v = L::hi(pick<R>(s[k].H, rr % R)) + gsh;
+        const int v = L::hi(pick<R>(s[k].H, rr % R)) + csh - (VL == 7 ? a.ge * rowB : 0);
         if (jobD) put_score_job(a, jobD, jobld, xo[k], yoB, v);
         else put_score(a, xo[k], yoB, v);
       }
@@ -695,10 +856,22 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// Dynamic shared memory: the profile (layout 7 on wavefronts: a letter of zeros
+// more, and the staging buffers).
+template <int R, int V, int W>
+constexpr size_t wave_smem() {
+  if constexpr (V == 7 && W > 1)
+    return Profile<R, W>::kBytes + (size_t)Profile<R, W>::kLetterStride * 16 + Stage<W>::kBytes;
+  else
+    return Profile<R, W>::kBytes;
+}
+
 template <int R, int P, int V>
 struct MinBlocks {
   static constexpr int rows = V == 5 ? 2 * R : R;   // register rows per lane
-  static constexpr int value = V == 0 ? 1 : (rows <= 8 ? 4 : (rows <= 16 ? 3 : 2));
+  // layout 7, 8 to 16 rows: the registers that keep the unrolled columns free of
+  // moves are worth more than a third CTA (16 rows: 9.1 against 8.0 TCUPS)
+  static constexpr int value = V == 0 ? 1 : V == 7 ? (rows <= 4 ? 3 : 2) : (rows <= 8 ? 4 : (rows <= 16 ? 3 : 2));
 };
 
 template <int R, int P, int V, int W>
@@ -723,6 +896,8 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
   // the substitution matrix, staged by cp.async (visible after the job loop's first barrier)
   stage_bytes(s_sub, a.sub, kLetters * kLetters, a.sub, a.sub + kLetters * kLetters, threadIdx.x, blockDim.x);
   cp_async_wait_all();
+  if constexpr (V == 7 && W > 1)
+    for (int e = threadIdx.x; e < Profile<R, W>::kLetterStride * 4; e += blockDim.x) prof[Profile<R, W>::kWords + e] = 0;
   // band-boundary scratch of the front: its own block of 4 x scratch_cols
   // words per X, or (W = 1) one column of the CTA's interleaved block
   int32_t* scratch =
@@ -808,11 +983,13 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
         const int x = e / BAND;
         const int row = e - x * BAND;
         const int grow = b * BAND + row;
-        const int gsh = Layout<V>::L == 3 ? a.go : 0;   // layout 3 adds the profile to T = H - go
-        const int sa = (grow < LyA ? (int)s_sub[clamp_code(s_ytile[0][leadA + row]) * kLetters + x] : 0) + gsh;
+        // layout 3 adds the profile to T = H - go, layout 7 to H~ (and 0 past the Y)
+        const int gsh = Layout<V>::L == 3 ? a.go : V == 7 ? 2 * a.ge : 0;
+        const int pad = V == 7 ? -gsh : 0;
+        const int sa = (grow < LyA ? (int)s_sub[clamp_code(s_ytile[0][leadA + row]) * kLetters + x] : pad) + gsh;
         uint32_t w;
         if (P == 2) {
-          const int sb = (grow < LyB ? (int)s_sub[clamp_code(s_ytile[1][leadB + row]) * kLetters + x] : 0) + gsh;
+          const int sb = (grow < LyB ? (int)s_sub[clamp_code(s_ytile[1][leadB + row]) * kLetters + x] : pad) + gsh;
           w = Lanes<2>::arith(sa, sb);
         } else {
           w = (uint32_t)sa;
@@ -821,7 +998,14 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
       }
       __syncthreads();
       if (Lmax > 0) {
-        if constexpr (V == 6)
+        if constexpr (V == 7 && W > 1) {
+          const int front = warp * S + seg;
+          int2* border = reinterpret_cast<int2*>(prof + Profile<R, W>::kWords + Profile<R, W>::kLetterStride * 4);
+          uint32_t* codes = reinterpret_cast<uint32_t*>(border + Stage<W>::kFronts * kStageCols);
+          wave_band7<R, P, W>(a, sl, b, nb, X[0], Lx[0], Lmin, Lmax, prof, border + front * kStageCols,
+                              codes + front * Stage<W>::kCodes, scratch, LyA - 1, LyB - 1, wantA[0], wantB[0], xo[0],
+                              yoA, yoB, jobD, jobld);
+        } else if constexpr (V == 6)
           wave_band_split<R, P, W>(a, sl, b, nb, X[0], Lx[0], Lmin, Lmax, prof, scratch, LyA - 1, LyB - 1, wantA[0],
                                    wantB[0], xo[0], yoA, yoB, jobD, jobld);
         else
@@ -834,20 +1018,20 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
 
 template <int R, int P, int V, int W>
 void prepare_one() {
-  const size_t smem = Profile<R, W>::kBytes;
+  const size_t smem = wave_smem<R, V, W>();
   cudaFuncSetAttribute(wave_kernel<R, P, V, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
 template <int R, int P, int V, int W>
 cudaError_t launch_one(const WaveArgs& a, int grid, cudaStream_t s) {
-  const size_t smem = Profile<R, W>::kBytes;
+  const size_t smem = wave_smem<R, V, W>();
   wave_kernel<R, P, V, W><<<grid, kWaveThreads, smem, s>>>(a);
   return cudaGetLastError();
 }
 
 template <int R, int P, int V, int W>
 int occupancy_one() {
-  const size_t smem = Profile<R, W>::kBytes;
+  const size_t smem = wave_smem<R, V, W>();
   cudaFuncSetAttribute(wave_kernel<R, P, V, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int n = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wave_kernel<R, P, V, W>, kWaveThreads, smem) != cudaSuccess)
@@ -856,20 +1040,20 @@ int occupancy_one() {
 }
 
 // Rows per lane that exist only in the most used forms (int16x2 wavefronts,
-// layouts 2 to 4): they refine the band sizes between the multiples of 4.
+// layouts 2 to 4 and 7): they refine the band sizes between the multiples of 4.
 constexpr bool extra_rows(int R) { return R % 4 != 0 || R == 28; }
 
 // The (P, V, W) combinations that exist for R rows per lane.  For R a multiple
 // of 4 (not 28): W = 32 with every P and V; the narrow fronts (W = 16, 8) on
-// int16x2 lanes with V = 0, 2, 3, 4 or 5; one pair per thread (W = 1: every
-// lane its own front, bands of R rows) on int16x2 lanes with V = 0, 2, 3 or 4.
-// The other R: int16x2 wavefronts of 32, 16 or 8 lanes with V = 2, 3 or 4.
+// int16x2 lanes with V = 0, 2, 3, 4, 5 or 7; one pair per thread (W = 1: every
+// lane its own front, bands of R rows) on int16x2 lanes with V = 0, 2, 3, 4 or 7.
+// The other R: int16x2 wavefronts of 32, 16 or 8 lanes with V = 2, 3, 4 or 7.
 inline bool wave_variant_exists(int R, int P, int V, int W) {
   if (V == 6) return !extra_rows(R) && R % 8 == 0 && P == 2 && (W == 32 || W == 16 || W == 8);
-  if (extra_rows(R)) return P == 2 && (W == 32 || W == 16 || W == 8) && V >= 2 && V <= 4;
-  if (W == 32) return (P == 1 || P == 2) && V >= 0 && V <= 5;
-  if (W == 1) return P == 2 && (V == 0 || V == 2 || V == 3 || V == 4);
-  return (W == 16 || W == 8) && P == 2 && (V == 0 || V == 2 || V == 3 || V == 4 || V == 5);
+  if (extra_rows(R)) return P == 2 && (W == 32 || W == 16 || W == 8) && ((V >= 2 && V <= 4) || V == 7);
+  if (W == 32) return (P == 1 || P == 2) && ((V >= 0 && V <= 5) || V == 7);
+  if (W == 1) return P == 2 && (V == 0 || V == 2 || V == 3 || V == 4 || V == 7);
+  return (W == 16 || W == 8) && P == 2 && (V == 0 || V == 2 || V == 3 || V == 4 || V == 5 || V == 7);
 }
 
 // Entry points of one rows-per-lane template (every existing P, V, W).
@@ -885,6 +1069,7 @@ struct Entry {
     if constexpr (W > 1 && !kExtra && P == 2 && R % 8 == 0) {
       if (V == 6) return fn(integral_constant<int, P>{}, integral_constant<int, 6>{}, integral_constant<int, W>{});
     }
+    if (V == 7) return fn(integral_constant<int, P>{}, integral_constant<int, 7>{}, integral_constant<int, W>{});
     if (V == 4) return fn(integral_constant<int, P>{}, integral_constant<int, 4>{}, integral_constant<int, W>{});
     if (V == 3) return fn(integral_constant<int, P>{}, integral_constant<int, 3>{}, integral_constant<int, W>{});
     if constexpr (kExtra) {
