@@ -177,11 +177,19 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   for (int k = 0; k < kLetters * kLetters; ++k) maxs = std::max<int>(maxs, c->sub[k]);
   const int certain_len = maxs > 0 ? c->i16.max_h / maxs : 1 << 30;
 
+  double cells = 0.0, xsum = 0.0;
+  for (int i = 0; i < X.n; ++i) {
+    xsum += X.len[i];
+    if (triangle) cells += xsum * X.len[i];
+  }
+  if (!triangle)
+    for (int k = 0; k < Y.n; ++k) cells += xsum * Y.len[k];
+
   struct Group { int y, y2, nx, R, V, W, P, check; };
   std::vector<Group> groups;
   groups.reserve((size_t)Y.n / 2 + 1);
   for (int y = 0; y < Y.n;) {
-    const TuneChoice tc = c->choice(Y.len[y]);
+    const TuneChoice tc = c->choice_set(Y.len[y], X.maxlen, cells);
     if (!force32) {
       const int y2 = y + 1 < Y.n ? y + 1 : -1;
       const int last = y2 >= 0 ? y2 : y;

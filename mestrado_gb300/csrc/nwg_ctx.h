@@ -1,6 +1,7 @@
 // nwg_ctx.h -- the context behind the opaque nwg_ctx handle (not installed).
 #pragma once
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -163,6 +164,40 @@ struct Ctx {
     }
     if (pick_est > 0.0 && min_est < 0.98 * pick_est) t = fastest;
     return allowed(t, rows);
+  }
+  // The choice when the whole set is `cells` cells over columns up to `cols`: a
+  // small set does not fill the GPU with warps, and what counts is how long one
+  // warp takes for its Y, a chain of two maxima per row (10 cycles) and about 90
+  // cycles per column.  The wavefronts with few rows per lane are then the
+  // faster ones; the estimate is the longer of that chain and the set's time at
+  // the candidate's rate, and a quarter of the shorter.  All pairs of 64 x 300
+  // residues: 52 us with 12 rows on 32 lanes, 62 with 18 on 16, 86 with two
+  // bands of 20 on 8.
+  TuneChoice choice_set(int rows, int cols, double cells) const {
+    const TuneChoice t = choice(rows);
+    if (t.V != 7 || cands[tune_class(rows)].empty()) return t;
+    constexpr double kHz = 2.0e9, kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // cells/s at 4, 8, 12, 16 rows
+    const auto est = [&](const TuneChoice& c, double rate) {
+      const int bands = padded_rows(c, rows) / (c.W * c.R);
+      const double chain = bands * (cols + c.W - 1) * (10.0 * c.R + 90.0) / kHz;
+      const double whole = cells * padded_rows(c, rows) / rows / rate;
+      return std::max(chain, whole) + 0.25 * std::min(chain, whole);
+    };
+    double rate = 9.0e12;
+    for (const Cand& c : cands[tune_class(rows)])
+      if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) rate = c.rate;
+    TuneChoice best = t;
+    double best_est = 0.95 * est(t, rate);   // not for less than a twentieth
+    for (int W : {8, 16, 32})
+      for (int R : {4, 8, 12, 16, 20, 24, 28, 32}) {
+        const TuneChoice c{R, 7, W};
+        const double e = est(c, R < 20 ? kSlow[R / 4 - 1] : 9.0e12);
+        if (e < best_est) {
+          best_est = e;
+          best = c;
+        }
+      }
+    return best;
   }
   TuneChoice allowed(TuneChoice t, int rows) const {
     if (t.V == 4 && go < ge) t.V = 2;

@@ -904,16 +904,24 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
       W == 1 ? a.scratch + (size_t)blockIdx.x * kWaveThreads * K * 4 * (size_t)a.scratch_cols + threadIdx.x
              : a.scratch + ((size_t)(blockIdx.x * kWaveWarps + warp) * S + seg) * K * 4 * (size_t)a.scratch_cols;
 
+  long long next = 0;   // thread 0: the job after this one, taken while this one runs
+  if (threadIdx.x == 0) next = (long long)atomicAdd(a.counter, 1ull);
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_job = (long long)atomicAdd(a.counter, 1ull);
+    if (threadIdx.x == 0) s_job = next;
     __syncthreads();
     const long long job = s_job;
     if (job >= a.njobs) break;
-    int lo = 0, hi = a.ngroups - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (a.job_prefix[mid] <= job) lo = mid; else hi = mid - 1;
+    if (threadIdx.x == 0) next = (long long)atomicAdd(a.counter, 1ull);
+    // the last group whose first job is at most this one: 32 probes at a time
+    int lo = 0;
+    for (int n = a.ngroups; n > 1;) {   // it is one of the n from lo
+      const int step = (n + 31) >> 5;
+      const int at = lane * step;
+      const unsigned le = __ballot_sync(0xffffffffu, at < n && a.job_prefix[lo + at] <= job);
+      const int k = 31 - __clz(le);     // lane 0's always holds
+      lo += k * step;
+      n = min(step, n - k * step);
     }
     const long long chunk = job - a.job_prefix[lo];
     const int g = a.g_begin + lo;
