@@ -437,8 +437,7 @@ int nwg_score_all(nwg_ctx* ctx, const int8_t* codes, const int64_t* offsets, int
   int rc;
   for (int s = 0; s < n; ++s)
     if (offsets[s + 1] <= offsets[s]) return c->fail(NWG_ERR_EMPTY_SEQ, "zero-length sequence");
-  for (int64_t k = 0; k < total; ++k)
-    if ((unsigned)codes[k] >= (unsigned)nwg::kLetters) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code outside 0..23");
+  if (!nwg::residues_ok(codes, total)) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code outside 0..23");
   if ((rc = c->b_codes.ensure((size_t)std::max<int64_t>(total, 1))) ||
       (rc = c->b_D.ensure(sizeof(float) * (size_t)n * (size_t)n)))
     return c->fail(rc, "score_all allocation");
@@ -486,10 +485,8 @@ int nwg_score_block(nwg_ctx* ctx, const int8_t* xcodes, const int64_t* xoff, int
   if ((rc = c->cuda(cudaMemcpyAsync(dc, xcodes, (size_t)tx, cudaMemcpyHostToDevice, c->stream), "upload")) ||
       (rc = c->cuda(cudaMemcpyAsync(dc + tx, ycodes, (size_t)ty, cudaMemcpyHostToDevice, c->stream), "upload")))
     return rc;
-  for (int64_t k = 0; k < tx; ++k)
-    if ((unsigned)xcodes[k] >= (unsigned)nwg::kLetters) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
-  for (int64_t k = 0; k < ty; ++k)
-    if ((unsigned)ycodes[k] >= (unsigned)nwg::kLetters) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
+  if (!nwg::residues_ok(xcodes, tx)) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
+  if (!nwg::residues_ok(ycodes, ty)) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
   std::vector<int64_t> yo2(ny + 1);
   for (int k = 0; k <= ny; ++k) yo2[k] = yoff[k] + tx;
   if (stats) {
@@ -542,8 +539,7 @@ int nwg_score_pairs(nwg_ctx* ctx, const int8_t* codes, const int64_t* offsets, i
   for (int s = 0; s < n; ++s)
     if (offsets[s + 1] <= offsets[s]) return c->fail(NWG_ERR_EMPTY_SEQ, "zero-length sequence");
   if (npairs == 0) return NWG_OK;
-  for (int64_t k = 0; k < offsets[n]; ++k)
-    if ((unsigned)codes[k] >= (unsigned)nwg::kLetters) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
+  if (!nwg::residues_ok(codes, offsets[n])) return c->fail(NWG_ERR_BAD_RESIDUE, "residue code");
   int64_t pairs16 = 0;
   const int rc = c->score_pairs(codes, offsets, n, pi, pj, npairs, out, &pairs16);
   if (rc) return rc;

@@ -537,8 +537,7 @@ int Ctx::align_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
   }
   if (npairs == 0) return NWG_OK;
   const int64_t total = offsets[n];
-  for (int64_t k = 0; k < total; ++k)
-    if ((unsigned)codes[k] >= (unsigned)kLetters) return fail(NWG_ERR_BAD_RESIDUE, "residue code outside 0..23");
+  if (!residues_ok(codes, total)) return fail(NWG_ERR_BAD_RESIDUE, "residue code outside 0..23");
   if (!trace_state) trace_state = new TraceState();
   TraceState& T = *reinterpret_cast<TraceState*>(trace_state);
   std::vector<int32_t> len(n);
