@@ -81,7 +81,7 @@ struct BatchPlan {
   DevBuf gy, gy2, gx, jobs, counters, rerun, rerun_scratch, wscratch;
   int64_t rerun_cap = 0, rerun_threads = 0;
   int64_t pairs16 = 0, pairs32 = 0, pairs_checked = 0;
-  int scols = 1;
+  int scols = 1, rebase_rows = 0;
   int64_t codes_len = 0;   // bytes of the codes buffer the sets reach (one past the last residue)
   // graph
   cudaGraphExec_t exec = nullptr;
@@ -169,8 +169,16 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   const SetView& Y = p->Y;
   for (int k = 0; k < X.n; ++k) p->codes_len = std::max<int64_t>(p->codes_len, X.start[k] + X.len[k]);
   for (int k = 0; k < Y.n; ++k) p->codes_len = std::max<int64_t>(p->codes_len, Y.start[k] + Y.len[k]);
-  const bool force32 = mode == NWG_MODE_BATCHED_INT32 ||
-                       std::max(X.maxlen, Y.maxlen) > c->i16.max_len;
+  // A set with sequences beyond the 16-bit lanes' length runs on int32 lanes when
+  // that is one CTA per SM at most (two Y per word then only leave SMs idle), else
+  // its long Y on layout 8 and the others, whose length bounds every score, on
+  // layout 7.
+  const int longest = std::max(X.maxlen, Y.maxlen);
+  const bool over = longest > c->i16.max_len;
+  int64_t jobs32 = 0;
+  for (int y = 0; y < Y.n; ++y) jobs32 += ((triangle ? y + 1 : X.n) + kWaveWarps - 1) / kWaveWarps;
+  const bool rebase = over && c->i16.rebased && c->plain7(longest) && jobs32 > c->sms;
+  const bool force32 = mode == NWG_MODE_BATCHED_INT32 || (over && !rebase);
   // certain int16: the shorter sequence of every pair is short enough that
   // even its best-case score fits (max matrix entry * length)
   int maxs = 0;
@@ -190,7 +198,14 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   groups.reserve((size_t)Y.n / 2 + 1);
   for (int y = 0; y < Y.n;) {
     const TuneChoice tc = c->choice_set(Y.len[y], X.maxlen, cells);
-    if (!force32) {
+    if (!force32 && rebase) {
+      const int y2 = y + 1 < Y.n ? y + 1 : -1;
+      const int last = y2 >= 0 ? y2 : y;
+      const bool seven = tc.V == 7 && Y.len[y] <= std::min(certain_len, c->i16.max_len7);
+      const TuneChoice t = seven ? tc : TuneChoice{Y.len[y] <= 768 ? 24 : 32, 8, 32};
+      groups.push_back({y, y2, triangle ? last + 1 : X.n, t.R, t.V, t.W, 2, 0});
+      y = last + 1;
+    } else if (!force32) {
       const int y2 = y + 1 < Y.n ? y + 1 : -1;
       const int last = y2 >= 0 ? y2 : y;
       const int nxg = triangle ? last + 1 : X.n;
@@ -266,13 +281,15 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   // boundary scratch: buckets run concurrently, so every bucket with more than
   // one band gets its own region
   p->scols = std::max(X.maxlen, 1);
+  p->rebase_rows = (p->scols + 31) / kRebase + 1;   // layout 8: blocks of steps in a band
   size_t scratch_words = 2;   // regions start on 8 bytes
   for (auto& b : p->buckets) {
     b.grid = (int)std::min<int64_t>(b.njobs, (int64_t)c->sms * wave_max_ctas_per_sm(b.R, b.P, b.V, b.W));
     b.grid = std::max(b.grid, 1);
     b.scratch_off = scratch_words;
     if (b.maxrows > b.W * b.R)
-      scratch_words += (size_t)b.grid * kWaveWarps * (32 / b.W) * wave_x_per_front(b.V) * 4 * p->scols;
+      scratch_words += (size_t)b.grid * kWaveWarps * (32 / b.W) * wave_x_per_front(b.V) * 4 *
+                       (p->scols + (b.V == 8 ? p->rebase_rows : 0));
   }
   if ((rc = p->wscratch.ensure(sizeof(int32_t) * scratch_words))) {
     delete p;
@@ -324,6 +341,8 @@ static int enqueue_step(Ctx* c, BatchPlan* p, const int8_t* d_codes, float* d_D,
   a.nx = p->X.n; a.ny = p->Y.n;
   a.triangle = p->triangle ? 1 : 0;
   a.go = c->go; a.ge = c->ge;
+  a.rebase_at = p->scols;
+  a.best_step = c->i16.best_step;
   a.sub = (const int8_t*)c->b_sub.p;
   a.xbound = (const int32_t*)p->bxb.p;
   a.ybound = (const int32_t*)(p->triangle ? p->bxb.p : p->byb.p);
@@ -351,6 +370,7 @@ static int enqueue_step(Ctx* c, BatchPlan* p, const int8_t* d_codes, float* d_D,
     a.check_bound = b.check;
     a.max_h = c->i16.max_h;
     a.scratch = (int32_t*)p->wscratch.p + b.scratch_off;
+    a.scratch_cols = p->scols + (b.V == 8 ? p->rebase_rows : 0);
     int ri = -1;
     if (timed) {
       nwg_launch_rec r{0, b.R, b.P == 2 ? 1 : 0, b.grid, b.pairs, (int64_t)b.cells, 0.0, b.V, b.W};

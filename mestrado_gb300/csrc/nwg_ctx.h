@@ -111,7 +111,7 @@ void destroy_plans(Ctx* c);
 struct Ctx {
   int go = 10, ge = 2;
   int8_t sub[kLetters * kLetters];
-  Int16Limits i16{kInt16MaxLen, 32756 - 11, 0};   // set from (go, ge, sub) at creation
+  Int16Limits i16{kInt16MaxLen, 32756 - 11, 0, 0, false};   // set from (go, ge, sub) at creation
   int device = 0, sms = 1;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;

@@ -37,10 +37,15 @@ constexpr int kInt16MaxLen = 6900;
 // step adds 2 ge more than to H, a gap adds nothing, so H~ of a pair is at most
 // its H bound + 2 ge times its shorter length.
 constexpr int layout7_zero(int go, int ge) { return 2 * (go - ge) + 136; }   // H~ = 0; below: g twice, an int8 entry
+// Layout 8 moves every lane's values down each kRebase steps: no limit of
+// length, but of the entries (the bound is derived at wave_band7).
+constexpr int kRebase = 1024;
 struct Int16Limits {
   int max_len;   // longest sequence of a set that may use int16 lanes (0: none)
   int max_h;     // largest H an int16 pair may reach
   int max_len7;  // longest shorter sequence of a pair on layout 7 (0: go < ge, or no room)
+  int best_step;  // best matrix entry (at least 0) + 2 ge
+  bool rebased;   // layout 8 holds
 };
 inline Int16Limits int16_limits(int go, int ge, const int8_t* sub) {
   int smin = 127, smax = -128;
@@ -56,7 +61,9 @@ inline Int16Limits int16_limits(int go, int ge, const int8_t* sub) {
   const int max_h = 32756 - (smax > 0 ? smax : 0);
   const long long room = 65535ll - 256 - max_h - layout7_zero(go, ge) - 2ll * ge;
   const int len7 = go < ge || room <= 0 ? 0 : ge == 0 ? kInt16MaxLen : (int)(room / (2ll * ge));
-  return {len, max_h, len7 < kInt16MaxLen ? len7 : kInt16MaxLen};
+  const int step = (smax > 0 ? smax : 0) + 2 * ge, g = go - ge;
+  const bool rebased = g >= 0 && layout7_zero(go, ge) + 6 * g + (kRebase + 98) * step <= 65000;
+  return {len, max_h, len7 < kInt16MaxLen ? len7 : kInt16MaxLen, step, rebased};
 }
 
 // Sequence set laid out on the device for one call: sorted by length
@@ -104,6 +111,8 @@ struct WaveArgs {
   int triangle;
   int go, ge;
   int scratch_cols;
+  int rebase_at;              // layout 8: the bases' table within a boundary buffer (in columns)
+  int best_step;              // layout 8: best matrix entry (at least 0) + 2 ge
   const int8_t* sub;          // 24*24 on device, 4-byte aligned (staged by cp.async)
   // overflow guard (optimistic int16 buckets)
   int check_bound;

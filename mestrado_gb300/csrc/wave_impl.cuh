@@ -53,6 +53,11 @@
 // (S + 2 ge is in the profile), two dependent operations from row to row, and
 // nothing to carry along the border.  Nothing falls below -g, so the halves
 // hold [0, 65535) from there up; rows past a Y add 0 instead of S + 2 ge.
+// V = 8 is layout 7 for sequences of any length: every kRebase steps each lane
+// takes what its last row has grown by out of its strip, per half, and keeps the
+// sum in a 32-bit base.  What the lanes hand down is shifted by the difference of
+// their bases (one add each); the boundary row between bands goes with its
+// bases, a row of the table per block of steps.
 // V = 5 is layout 3 with two X per front: every lane runs the strips of two
 // X (adjacent in length order) against the same band, row by row
 // interleaved, so two independent dependency chains share the lane's issue
@@ -231,6 +236,7 @@ template <int V>
 struct Layout {
   static constexpr int K = V == 5 ? 2 : 1;                // X per front
   static constexpr int L = (V == 5 || V == 6) ? 3 : V;    // register layout of each strip
+  static constexpr bool seven = V == 7 || V == 8;
 };
 
 template <int R, int P, int V>
@@ -561,9 +567,17 @@ struct Stage {
   static constexpr size_t kBytes = (size_t)kFronts * (kStageCols * sizeof(int2) + kCodes * sizeof(uint32_t));
 };
 
-// One band of layout 7; arguments as wave_band's.  border / codes: the front's
-// staging buffers.
-template <int R, int P, int W>
+// One band of layout 7 (RB: 8); arguments as wave_band's.  border / codes: the
+// front's staging buffers.
+//
+// The bases (RB).  A value never falls by more than g along a row, and over R
+// rows or kRebase columns it rises by at most s = best entry + 2 ge per row or
+// column.  So with the last row of the strip moved down to `target` = zero + 34 s
+// + 4 g, everything the lane holds or is handed stays above 0 until the next
+// move, and below 65536 where the host has checked zero + 6 g + (kRebase + 98) s
+// against it.  A move never goes up: lanes before their first column, and those
+// of the first rows, keep base 0 and the constant borders.
+template <int R, int P, int W, bool RB>
 __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int nb, const int8_t* __restrict__ X,
                                            int Lx, int Lmin, int Lmax, const uint32_t* __restrict__ prof,
                                            int2* __restrict__ border, uint32_t* __restrict__ codes,
@@ -590,16 +604,22 @@ __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int
   const char* pl = reinterpret_cast<const char*>(prof) + 16 * sl;
 
   int nx[KS];
-  int2 nb2[KS];
+  int2 nb2[KS], tab[RB ? KS : 1];   // tab: the bases that go with the boundary's column
   auto fetch = [&](int t0) {
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       const int c = t0 + sl + W * k;
       nx[k] = c < Lx ? (int)X[c] : 0;
       nb2[k] = !top && c < Lx ? rd[c] : make_int2((int)ZERO, (int)GAP);
+      if constexpr (RB) {
+        const int p = (c + W - 1) / kRebase;   // the block of the step in which the last lane wrote it
+        tab[k] = !top && c < Lx && p > 0 ? rd[a.rebase_at + p] : make_int2(0, 0);
+      }
     }
   };
   uint32_t last = kLetters * LSB;   // columns before the first: the row of zeros
+  int baseA = 0, baseB = 0;         // RB: what is taken out of the halves so far
+  uint32_t adj = 0;                 // RB: the lane above's bases less this lane's
   fetch(0);
 
   auto step = [&](int t0, int i, auto checked) {
@@ -608,6 +628,10 @@ __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int
     uint32_t hin = __shfl_up_sync(0xffffffffu, hbot, 1, W);
     uint32_t fin = __shfl_up_sync(0xffffffffu, fbot, 1, W);
     const uint32_t off = codes[W - sl + i];
+    if constexpr (RB) {
+      hin += adj;
+      fin += adj;
+    }
     if (sl == 0) {
       const int2 bd = border[i];
       hin = (uint32_t)bd.x;
@@ -623,12 +647,39 @@ __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int
   };
   const int nt = Lmax + W - 1;
   for (int t0 = 0; t0 < nt; t0 += kStageCols) {
+    if constexpr (RB) {
+      if (t0 > 0 && t0 % kRebase == 0) {
+        const int g = a.go - a.ge;
+        const int target = layout7_zero(a.go, a.ge) + 34 * a.best_step + 4 * g;
+        const int dA = max((int)(s.H[R - 1] & 0xFFFFu) - target, 0), dB = max((int)(s.H[R - 1] >> 16) - target, 0);
+        const uint32_t d = (uint32_t)dA | ((uint32_t)dB << 16);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          s.H[r] -= d;
+          s.E[r] -= d;
+        }
+        hprev -= d;
+        hbot -= d;
+        fbot -= d;
+        baseA += dA;
+        baseB += dB;
+        const int uA = __shfl_up_sync(0xffffffffu, baseA, 1, W), uB = __shfl_up_sync(0xffffffffu, baseB, 1, W);
+        adj = (uint32_t)(uA - baseA) + ((uint32_t)(uB - baseB) << 16);
+        if (store) wr[sl + a.rebase_at + t0 / kRebase] = make_int2(baseA, baseB);
+      }
+    }
     __syncwarp();
     codes[sl] = last;
 #pragma unroll
     for (int k = 0; k < KS; ++k) {
       last = clamp_code(nx[k]) * LSB;
       codes[W + W * k + sl] = last;
+      if constexpr (RB) {
+        const uint32_t to0 = (uint32_t)(tab[k].x - __shfl_sync(0xffffffffu, baseA, 0, W)) +
+                             ((uint32_t)(tab[k].y - __shfl_sync(0xffffffffu, baseB, 0, W)) << 16);
+        nb2[k].x = (int)((uint32_t)nb2[k].x + to0);
+        nb2[k].y = (int)((uint32_t)nb2[k].y + to0);
+      }
       border[W * k + sl] = nb2[k];
     }
     __syncwarp();
@@ -651,7 +702,7 @@ __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int
   if (wantA) {
     const int rr = rowA - b * BAND;
     if (rr >= 0 && rr < BAND && sl == rr / R) {
-      const int v = L::lo(pick<R>(s.H, rr % R)) + csh - a.ge * rowA;
+      const int v = L::lo(pick<R>(s.H, rr % R)) + baseA + csh - a.ge * rowA;
       if (jobD) put_score_job(a, jobD, jobld, xo, yoA, v);
       else put_score(a, xo, yoA, v);
     }
@@ -659,7 +710,7 @@ __device__ __forceinline__ void wave_band7(const WaveArgs& a, int sl, int b, int
   if (P == 2 && wantB) {
     const int rr = rowB - b * BAND;
     if (rr >= 0 && rr < BAND && sl == rr / R) {
-      const int v = L::hi(pick<R>(s.H, rr % R)) + csh - a.ge * rowB;
+      const int v = L::hi(pick<R>(s.H, rr % R)) + baseB + csh - a.ge * rowB;
       if (jobD) put_score_job(a, jobD, jobld, xo, yoB, v);
       else put_score(a, xo, yoB, v);
     }
@@ -860,7 +911,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // more, and the staging buffers).
 template <int R, int V, int W>
 constexpr size_t wave_smem() {
-  if constexpr (V == 7 && W > 1)
+  if constexpr (Layout<V>::seven && W > 1)
     return Profile<R, W>::kBytes + (size_t)Profile<R, W>::kLetterStride * 16 + Stage<W>::kBytes;
   else
     return Profile<R, W>::kBytes;
@@ -871,7 +922,7 @@ struct MinBlocks {
   static constexpr int rows = V == 5 ? 2 * R : R;   // register rows per lane
   // layout 7, 8 to 16 rows: the registers that keep the unrolled columns free of
   // moves are worth more than a third CTA (16 rows: 9.1 against 8.0 TCUPS)
-  static constexpr int value = V == 0 ? 1 : V == 7 ? (rows <= 4 ? 3 : 2) : (rows <= 8 ? 4 : (rows <= 16 ? 3 : 2));
+  static constexpr int value = V == 0 ? 1 : V >= 7 ? (rows <= 4 ? 3 : 2) : (rows <= 8 ? 4 : (rows <= 16 ? 3 : 2));
 };
 
 template <int R, int P, int V, int W>
@@ -896,7 +947,7 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
   // the substitution matrix, staged by cp.async (visible after the job loop's first barrier)
   stage_bytes(s_sub, a.sub, kLetters * kLetters, a.sub, a.sub + kLetters * kLetters, threadIdx.x, blockDim.x);
   cp_async_wait_all();
-  if constexpr (V == 7 && W > 1)
+  if constexpr (Layout<V>::seven && W > 1)
     for (int e = threadIdx.x; e < Profile<R, W>::kLetterStride * 4; e += blockDim.x) prof[Profile<R, W>::kWords + e] = 0;
   // band-boundary scratch of the front: its own block of 4 x scratch_cols
   // words per X, or (W = 1) one column of the CTA's interleaved block
@@ -996,8 +1047,8 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
         const int row = e - x * BAND;
         const int grow = b * BAND + row;
         // layout 3 adds the profile to T = H - go, layout 7 to H~ (and 0 past the Y)
-        const int gsh = Layout<V>::L == 3 ? a.go : V == 7 ? 2 * a.ge : 0;
-        const int pad = V == 7 ? -gsh : 0;
+        const int gsh = Layout<V>::L == 3 ? a.go : Layout<V>::seven ? 2 * a.ge : 0;
+        const int pad = Layout<V>::seven ? -gsh : 0;
         const int sa = (grow < LyA ? (int)s_sub[clamp_code(s_ytile[0][leadA + row]) * kLetters + x] : pad) + gsh;
         uint32_t w;
         if (P == 2) {
@@ -1010,11 +1061,11 @@ __global__ void __launch_bounds__(kWaveThreads, (MinBlocks<R, P, V>::value)) wav
       }
       __syncthreads();
       if (Lmax > 0) {
-        if constexpr (V == 7 && W > 1) {
+        if constexpr (Layout<V>::seven && W > 1) {
           const int front = warp * S + seg;
           int2* border = reinterpret_cast<int2*>(prof + Profile<R, W>::kWords + Profile<R, W>::kLetterStride * 4);
           uint32_t* codes = reinterpret_cast<uint32_t*>(border + Stage<W>::kFronts * kStageCols);
-          wave_band7<R, P, W>(a, sl, b, nb, X[0], Lx[0], Lmin, Lmax, prof, border + front * kStageCols,
+          wave_band7<R, P, W, V == 8>(a, sl, b, nb, X[0], Lx[0], Lmin, Lmax, prof, border + front * kStageCols,
                               codes + front * Stage<W>::kCodes, scratch, LyA - 1, LyB - 1, wantA[0], wantB[0], xo[0],
                               yoA, yoB, jobD, jobld);
         } else if constexpr (V == 6)
@@ -1069,6 +1120,9 @@ inline bool wave_variant_exists(int R, int P, int V, int W) {
   return (W == 16 || W == 8) && P == 2 && (V == 0 || V == 2 || V == 3 || V == 4 || V == 5 || V == 7);
 }
 
+// Layout 8 (not a choice of the tables: the plan takes it for long sequences).
+constexpr bool rebased_exists(int R, int P, int V, int W) { return V == 8 && P == 2 && W == 32 && (R == 24 || R == 32); }
+
 // Entry points of one rows-per-lane template (every existing P, V, W).
 template <int R>
 struct Entry {
@@ -1081,6 +1135,9 @@ struct Entry {
     }
     if constexpr (W > 1 && !kExtra && P == 2 && R % 8 == 0) {
       if (V == 6) return fn(integral_constant<int, P>{}, integral_constant<int, 6>{}, integral_constant<int, W>{});
+    }
+    if constexpr (rebased_exists(R, P, 8, W)) {
+      if (V == 8) return fn(integral_constant<int, P>{}, integral_constant<int, 8>{}, integral_constant<int, W>{});
     }
     if (V == 7) return fn(integral_constant<int, P>{}, integral_constant<int, 7>{}, integral_constant<int, W>{});
     if (V == 4) return fn(integral_constant<int, P>{}, integral_constant<int, 4>{}, integral_constant<int, W>{});
@@ -1110,20 +1167,20 @@ struct Entry {
     }
   }
   static cudaError_t launch(int P, int V, int W, const WaveArgs& a, int grid, cudaStream_t s) {
-    if (!wave_variant_exists(R, P, V, W)) return cudaErrorInvalidValue;
+    if (!wave_variant_exists(R, P, V, W) && !rebased_exists(R, P, V, W)) return cudaErrorInvalidValue;
     return with(P, V, W, [&](auto p, auto v, auto w) {
       return launch_one<R, decltype(p)::value, decltype(v)::value, decltype(w)::value>(a, grid, s);
     });
   }
   static void prepare(int P, int V, int W) {
-    if (!wave_variant_exists(R, P, V, W)) return;
+    if (!wave_variant_exists(R, P, V, W) && !rebased_exists(R, P, V, W)) return;
     with(P, V, W, [&](auto p, auto v, auto w) {
       prepare_one<R, decltype(p)::value, decltype(v)::value, decltype(w)::value>();
       return 0;
     });
   }
   static int occupancy(int P, int V, int W) {
-    if (!wave_variant_exists(R, P, V, W)) return 1;
+    if (!wave_variant_exists(R, P, V, W) && !rebased_exists(R, P, V, W)) return 1;
     return with(P, V, W, [&](auto p, auto v, auto w) {
       return occupancy_one<R, decltype(p)::value, decltype(v)::value, decltype(w)::value>();
     });

@@ -4,7 +4,10 @@ template and front width; column counts around the staged blocks of 32 columns
 and the ramps; bands that end in or before the second Y of a pair; gap models
 down to go = ge and beyond its range (go < ge); scores at the top of the 16-bit
 range; lengths where the 16-bit or the border's range ends; sets too small to
-fill the GPU, which take other templates; and the job search over many groups.
+fill the GPU, which take other templates; the job search over many groups; and
+sets with sequences beyond the 16-bit lanes' length, whose lanes move their
+values down as they grow (columns and bands around the steps of the move, the
+steepest growth, growth of only one of two Y in a word).
 Scores are whole numbers: equality."""
 import os
 
@@ -71,3 +74,21 @@ def test_lengths_at_the_ends_of_the_ranges(go, ge, n):
 def test_small_sets_and_many_groups(n):
     rng = np.random.default_rng(n)
     _check(_seqs(rng, rng.integers(1, 330 if n > 2 else 1500, n), 20))
+
+
+@pytest.mark.parametrize("go,ge", [(10, 2), (11, 1), (0, 0), (12, 3)])
+def test_sets_with_very_long_sequences(go, ge):
+    rng = np.random.default_rng(go)
+    long = LETTERS[rng.integers(0, 20, 9100)]
+    near = long[40:8300].copy()
+    near[::4] = LETTERS[rng.integers(0, 20, len(near[::4]))]
+    seqs = [b"W" * 7168, b"W" * 7137, b"P" * 7169, long.tobytes(), near.tobytes(), b"W" * 2100 + b"P" * 5000,
+            b"W" * 3100, LETTERS[rng.integers(0, 20, 1025)].tobytes()] + _seqs(rng, rng.integers(1, 300, 48), 20)
+    ref = O.score_all(seqs, go, ge, threads=os.cpu_count())
+    with Context(go, ge) as c:
+        D, st = c.score_all(seqs, mode=MODE_BATCHED, stats=True)
+        assert np.array_equal(D, ref)
+        assert st["pairs_int16"] == len(seqs) * (len(seqs) + 1) // 2   # enough work: no int32 lanes
+        # columns short and long against long rows, as a block
+        xs = seqs[:4] + seqs[30:]
+        assert np.array_equal(c.score_block(xs * 40, seqs[:8])[: len(xs)], ref[np.r_[0:4, 30:len(seqs)]][:, :8])
