@@ -9,13 +9,14 @@
 // two pairs share a Y, so there is no profile to share: each warp builds its
 // own, one byte per (letter, row), with its scores made non-negative by a bias
 // so that one byte permute yields the word of both pairs.
-// Bound by integer issue (about 3.9 instructions a cell with the shuffles and
-// loads of a step spread over R = 8 rows).  R = 8 needs 12 KB of profile per
-// warp, which leaves 18 warps per SM; R = 4 is for pairs whose Y fits one band
-// of 128 rows.  20,000 pairs of about 245 residues, the whole call on a GB300:
-// 13.8 ms with one pair per thread and the (H, F) row in global memory (157
-// CTAs, one 4-byte-gather chain per cell), 0.99 ms here.
+// Bound by integer issue and the latency of a step (two shuffles, the profile's
+// loads, two dependent maxima per row) at 10 to 16 warps per SM, which the
+// profiles' shared memory allows.  20,000 pairs of about 245 residues, the whole
+// call on a GB300: 13.8 ms with one pair per thread and the (H, F) row in global
+// memory (157 CTAs, one 4-byte-gather chain per cell), 0.75 ms on layout 3 (its
+// kernels 0.68), 0.64 ms on layout 7 (0.47).
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "nwg_ctx.h"
@@ -199,17 +200,207 @@ __global__ void __launch_bounds__(32 * kPWarps) pair_wave_kernel(const PairWaveA
   }
 }
 
+// The same jobs on layout 7 of wave_impl.cuh (the extension cost taken out: three
+// DPX operations and one add per word, two dependent ones per row, constant
+// borders), where go >= ge, the scores fit the profile's bytes and the borders stay
+// above the reference's sentinel.  The codes of the next 32 columns are staged as
+// offsets into the profile, as in wave_band7, and R = 12 serves pairs of up to 384
+// rows in one band: of 20,000 pairs of 245 residues a quarter have more than 256
+// rows, which two bands of 256 computed as 512.  A profile byte is S + 2 ge +
+// lift, lift making the least of them 0; rows past a Y and columns past an X have
+// the byte `lift`, which adds nothing.
 template <int R, int P>
+__global__ void __launch_bounds__(32 * kPWarps) pair7_kernel(const PairWaveArgs a) {
+  using L = Lanes<P>;
+  constexpr int BAND = 32 * R, Q = R / 4;
+  constexpr int PW = (kLetters + 1) * BAND / 4;                 // profile words of one pair, a row of `lift` last
+  constexpr int SC = 32;                                        // staged columns
+  __shared__ __align__(16) int8_t s_sub[kLetters * kLetters];
+  __shared__ __align__(16) uint32_t s_prof[kPWarps][P][PW];
+  __shared__ __align__(16) int2 s_border[kPWarps][SC];
+  __shared__ uint32_t s_codes[kPWarps][P][2 * SC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < kLetters * kLetters; e += blockDim.x) s_sub[e] = (int8_t)(a.sub[e] + 2 * a.ge + a.bias);
+  const uint32_t lifts = 0x01010101u * (uint32_t)a.bias;
+#pragma unroll
+  for (int k = 0; k < P; ++k)
+    for (int e = lane; e < BAND / 4; e += 32) s_prof[warp][k][kLetters * BAND / 4 + e] = lifts;
+  __syncthreads();
+  const uint32_t NG = L::packed(a.ge - a.go);
+  const int zero = P == 2 ? layout7_zero(a.go, a.ge) - 32768 : 0;
+  const uint32_t ZERO = L::splat(zero), GAP = L::splat(zero + a.ge - a.go);
+  const uint32_t CORR = L::arith(-a.bias, -a.bias);
+  int2* scratch = reinterpret_cast<int2*>(a.scratch) + (size_t)(blockIdx.x * kPWarps + warp) * 2 * a.scratch_cols;
+  int2* border = s_border[warp];
+  const int njobs = (a.npairs + P - 1) / P;
+  for (;;) {
+    unsigned job = 0;
+    if (lane == 0) job = atomicAdd(a.counter, 1u);
+    job = __shfl_sync(0xffffffffu, job, 0);
+    if (job >= (unsigned)njobs) break;
+    const int8_t* X[P];
+    const int8_t* Y[P];
+    int Lx[P], Ly[P], id[P];
+    int cols = 0, rows = 0, Lmin = 0x7fffffff;
+#pragma unroll
+    for (int k = 0; k < P; ++k) {
+      const int s = (int)job * P + k;
+      id[k] = a.order[s < a.npairs ? s : s - 1];               // the odd one out runs in both halves
+      const int ix = a.pi[id[k]], iy = a.pj[id[k]];
+      X[k] = a.codes + a.start[ix];
+      Y[k] = a.codes + a.start[iy];
+      Lx[k] = a.len[ix];
+      Ly[k] = a.len[iy];
+      cols = max(cols, Lx[k]);
+      rows = max(rows, Ly[k]);
+      Lmin = min(Lmin, Lx[k]);
+    }
+    const int nb = (rows + BAND - 1) / BAND;
+    for (int b = 0; b < nb; ++b) {
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < P; ++k)
+        build_profile<R>(s_prof[warp][k], s_sub, Y[k], b * BAND + lane * R, Ly[k], lifts, lane);
+      uint32_t H[R], E[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        H[r] = ZERO;
+        E[r] = GAP;
+      }
+      // the column after which this lane holds a pair's score in row rr[k], or none
+      int endc[P], rr[P];
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const int r = Ly[k] - 1 - (b * BAND + lane * R);
+        endc[k] = r >= 0 && r < R ? Lx[k] - 1 : INT_MIN;
+        rr[k] = r;
+      }
+      uint32_t hprev = ZERO, hbot = ZERO, fbot = GAP;
+      const int2* rd = scratch + (size_t)((b + 1) & 1) * a.scratch_cols;
+      int2* wr = scratch + (size_t)(b & 1) * a.scratch_cols - lane;
+      const bool store = lane == 31 && b + 1 < nb;
+      int nx[P];
+      int2 nbd;
+      uint32_t last[P];
+      auto fetch = [&](int t0) {
+        const int c = t0 + lane;
+#pragma unroll
+        for (int k = 0; k < P; ++k) nx[k] = c < Lx[k] ? (int)clamp_code(X[k][c]) : kLetters;
+        nbd = b > 0 && c < cols ? rd[c] : make_int2((int)ZERO, (int)GAP);
+      };
+#pragma unroll
+      for (int k = 0; k < P; ++k) last[k] = kLetters * BAND;     // columns before the first
+      fetch(0);
+      auto step = [&](int t0, int i, auto tail) {
+        constexpr bool kTail = decltype(tail)::value;
+        const int c = t0 + i - lane;
+        uint32_t hin = __shfl_up_sync(0xffffffffu, hbot, 1);
+        uint32_t f = __shfl_up_sync(0xffffffffu, fbot, 1);
+        uint32_t w[P][Q];
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          const uint32_t* p = s_prof[warp][k] + (s_codes[warp][k][SC - lane + i] >> 2) + lane * Q;
+          if constexpr (R == 8) {
+            const uint2 v = *reinterpret_cast<const uint2*>(p);
+            w[k][0] = v.x;
+            w[k][Q - 1] = v.y;
+          } else {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) w[k][q] = p[q];
+          }
+        }
+        if (lane == 0) {
+          const int2 bd = border[i];
+          hin = (uint32_t)bd.x;
+          f = (uint32_t)bd.y;
+        }
+        if (kTail && c >= cols) return;
+        auto score = [&](int r) -> uint32_t {   // the word of row r: byte r of each pair
+          const uint32_t i4 = r & 3;
+          if constexpr (P == 2)
+            return perm(w[0][r >> 2], w[P - 1][r >> 2], i4 | (i4 | 8) << 4 | (i4 + 4) << 8 | (i4 + 4 | 8) << 12);
+          else
+            return perm(w[0][r >> 2], 0u, i4 | (i4 | 8) << 4 | (i4 | 8) << 8 | (i4 | 8) << 12);
+        };
+#pragma unroll
+        for (int r = R - 1; r >= 0; --r) H[r] = (r > 0 ? H[r > 0 ? r - 1 : 0] : hprev) + score(r) + CORR;
+        hprev = hin;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          H[r] = L::max3(E[r], f, H[r]);
+          f = L::addmax(H[r], NG, f);
+          E[r] = L::addmax(H[r], NG, E[r]);
+        }
+        hbot = H[R - 1];
+        fbot = f;
+        if (store && (!kTail || c >= 0)) wr[t0 + i] = make_int2((int)hbot, (int)fbot);
+        if (kTail) {
+#pragma unroll
+          for (int k = 0; k < P; ++k)
+            if (c == endc[k]) {
+              const uint32_t v = pick<R>(H, rr[k]);
+              a.out[id[k]] = (k == 0 ? L::lo(v) : L::hi(v)) - zero - a.ge * (Lx[k] + Ly[k]);
+            }
+        }
+      };
+      const int nt = cols + 31;
+      for (int t0 = 0; t0 < nt; t0 += SC) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          s_codes[warp][k][lane] = last[k];
+          last[k] = (uint32_t)nx[k] * BAND;
+          s_codes[warp][k][SC + lane] = last[k];
+        }
+        border[lane] = nbd;
+        __syncwarp();
+        fetch(t0 + SC);
+        const int ne = min(nt - t0, SC), ns = min(Lmin - 1 - t0, SC);   // below ns no pair's last column
+        for (int i = 0; i < ne;) {
+          if (t0 + i >= 31 && i < ns) {
+#pragma unroll 4
+            for (; i < ns; ++i) step(t0, i, std::false_type{});
+          } else {
+            step(t0, i, std::true_type{});
+            ++i;
+          }
+        }
+      }
+    }
+  }
+}
+
+template <int R, int P, bool Seven>
 int pair_ctas_per_sm() {
   static const int n = [] {
     int k = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, pair_wave_kernel<R, P>, 32 * kPWarps, 0) != cudaSuccess) {
+    const void* fn = nullptr;
+    if constexpr (Seven) fn = (const void*)pair7_kernel<R, P>;
+    else fn = (const void*)pair_wave_kernel<R, P>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, 32 * kPWarps, 0) != cudaSuccess) {
       cudaGetLastError();
       return 4;
     }
     return k > 0 ? k : 1;
   }();
   return n;
+}
+
+// fn(rows per lane, pairs per word, layout 7) as constants.
+template <class Fn>
+void pair_dispatch(int R, int P, bool seven, Fn&& fn) {
+  using std::integral_constant;
+  auto with_p = [&](auto p) {
+    using B7 = integral_constant<bool, true>;
+    using B3 = integral_constant<bool, false>;
+    if (seven && R == 12) fn(integral_constant<int, 12>{}, p, B7{});
+    else if (seven && R == 8) fn(integral_constant<int, 8>{}, p, B7{});
+    else if (seven) fn(integral_constant<int, 4>{}, p, B7{});
+    else if (R == 8) fn(integral_constant<int, 8>{}, p, B3{});
+    else fn(integral_constant<int, 4>{}, p, B3{});
+  };
+  if (P == 2) with_p(integral_constant<int, 2>{});
+  else with_p(integral_constant<int, 1>{});
 }
 
 }  // namespace
@@ -239,19 +430,28 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
     smin = std::min<int>(smin, sub[k]);
     smax = std::max<int>(smax, sub[k]);
   }
+  int maxlen = 1;
+  for (int64_t k = 0; k < npairs; ++k) maxlen = std::max(maxlen, std::max(len[pi[k]], len[pj[k]]));
+  // layout 7: its bytes are S + 2 ge, lifted to 0 where the least is below
+  const int lift = std::max(0, -(smin + 2 * ge));
+  const bool seven = plain7(maxlen) && std::max(smax, 0) + 2 * ge + lift <= 127;
   const bool bytes7 = smax - std::min(smin, 0) <= 127 && smin >= -127;
-  const int bias = -std::min(smin, 0);
-  auto kind = [&](int64_t k) {   // bucket: (P, R)
+  const int bias = seven ? lift : -std::min(smin, 0);
+  // Bucket of a pair: lanes (int16x2 or int32) and rows per lane, with the fewest
+  // rows computed; at equal rows the wider lanes (fewer bands).  12 rows exist on
+  // layout 7.
+  struct Kind { int R, P; };
+  const Kind kinds[6] = {{12, 2}, {8, 2}, {4, 2}, {12, 1}, {8, 1}, {4, 1}};
+  auto kind = [&](int64_t k) {
     const int Lx = len[pi[k]], Ly = len[pj[k]];
-    const bool p2 = bytes7 && std::max(Lx, Ly) <= i16.max_len &&
+    const bool p2 = bytes7 && std::max(Lx, Ly) <= i16.max_len && (!seven || Ly <= i16.max_len7) &&
                     (smax <= 0 || (int64_t)Ly * smax <= i16.max_h);
-    return (p2 ? 0 : 2) + (Ly > 128 ? 0 : 1);
+    const int padded12 = (Ly + 383) / 384 * 384, padded8 = (Ly + 255) / 256 * 256;
+    return (p2 ? 0 : 3) + (Ly <= 128 ? 2 : seven && padded12 <= padded8 ? 0 : 1);
   };
   // Order of the list: by bucket, then bands, then X length, longest first
   // (counting sort on X length, then a stable one on the other two), so that
   // the pairs of a word are alike and the long jobs start first.
-  int maxlen = 1;
-  for (int64_t k = 0; k < npairs; ++k) maxlen = std::max(maxlen, std::max(len[pi[k]], len[pj[k]]));
   const int maxb = (maxlen + 255) / 256;
   const int m = (int)npairs;
   std::vector<int32_t> by_x(m), order(m), slot;
@@ -259,41 +459,44 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
   for (int k = 0; k < m; ++k) ++slot[(size_t)(maxlen - len[pi[k]]) + 1];
   for (size_t k = 1; k < slot.size(); ++k) slot[k] += slot[k - 1];
   for (int k = 0; k < m; ++k) by_x[(size_t)slot[(size_t)(maxlen - len[pi[k]])]++] = k;
-  auto key = [&](int k) {
-    const int b = kind(k);
-    return (size_t)b * (maxb + 1) + (size_t)(maxb - (len[pj[k]] + 255) / 256);
-  };
-  slot.assign((size_t)4 * (maxb + 1) + 1, 0);
-  PairBucket bucket[4] = {{8, 2, 0, 0, 1, 1}, {4, 2, 0, 0, 1, 1}, {8, 1, 0, 0, 1, 1}, {4, 1, 0, 0, 1, 1}};
+  std::vector<int32_t> key(m);
+  slot.assign((size_t)6 * (maxb + 1) + 1, 0);
+  PairBucket bucket[6];
+  for (int q = 0; q < 6; ++q) bucket[q] = {kinds[q].R, kinds[q].P, 0, 0, 1, 1};
   for (int k = 0; k < m; ++k) {
-    ++slot[key(k) + 1];
-    PairBucket& b = bucket[kind(k)];
+    const int q = kind(k);
+    PairBucket& b = bucket[q];
+    key[(size_t)k] = q * (maxb + 1) + (maxb - (len[pj[k]] + 32 * b.R - 1) / (32 * b.R));
+    ++slot[(size_t)key[(size_t)k] + 1];
     ++b.count;
     b.maxrows = std::max(b.maxrows, len[pj[k]]);
     b.maxcols = std::max(b.maxcols, len[pi[k]]);
   }
   for (size_t k = 1; k < slot.size(); ++k) slot[k] += slot[k - 1];
-  *pairs16 += bucket[0].count + bucket[1].count;
-  for (int k = 1; k < 4; ++k) bucket[k].first = bucket[k - 1].first + bucket[k - 1].count;
-  for (int k = 0; k < m; ++k) order[(size_t)slot[key(by_x[k])]++] = by_x[k];
+  *pairs16 += bucket[0].count + bucket[1].count + bucket[2].count;
+  for (int k = 1; k < 6; ++k) bucket[k].first = bucket[k - 1].first + bucket[k - 1].count;
+  for (int k = 0; k < m; ++k) order[(size_t)slot[(size_t)key[(size_t)by_x[k]]]++] = by_x[k];
   // grids and band-boundary scratch
-  int grid[4] = {};
-  size_t scratch_words = 1;
-  for (int q = 0; q < 4; ++q) {
+  int grid[6] = {}, kinds_used = 0;
+  size_t scratch_words = 2, scratch_at[6] = {};   // regions of their own: the buckets run side by side
+  for (int q = 0; q < 6; ++q) {
     const PairBucket& b = bucket[q];
     if (!b.count) continue;
-    const int occ = b.P == 2 ? (b.R == 8 ? pair_ctas_per_sm<8, 2>() : pair_ctas_per_sm<4, 2>())
-                             : (b.R == 8 ? pair_ctas_per_sm<8, 1>() : pair_ctas_per_sm<4, 1>());
+    ++kinds_used;
+    int occ = 1;
+    pair_dispatch(b.R, b.P, seven, [&](auto r, auto p, auto s7) {
+      occ = pair_ctas_per_sm<decltype(r)::value, decltype(p)::value, decltype(s7)::value>();
+    });
     const int jobs = (b.count + b.P - 1) / b.P;
     grid[q] = std::min((jobs + kPWarps - 1) / kPWarps, sms * occ);
-    if (b.maxrows > 32 * b.R)
-      scratch_words = std::max(scratch_words, (size_t)grid[q] * kPWarps * 4 * (size_t)b.maxcols);
+    scratch_at[q] = scratch_words;
+    if (b.maxrows > 32 * b.R) scratch_words += (size_t)grid[q] * kPWarps * 4 * (size_t)b.maxcols;
   }
   int rc;
   if ((rc = b_codes.ensure((size_t)total)) || (rc = b_start.ensure(sizeof(int64_t) * n)) ||
       (rc = b_len.ensure(sizeof(int32_t) * n)) || (rc = b_pi.ensure(sizeof(int32_t) * npairs)) ||
       (rc = b_pj.ensure(sizeof(int32_t) * npairs)) || (rc = b_out.ensure(sizeof(int32_t) * npairs)) ||
-      (rc = b_orig.ensure(sizeof(int32_t) * npairs)) || (rc = b_counter.ensure(sizeof(unsigned) * 4)) ||
+      (rc = b_orig.ensure(sizeof(int32_t) * npairs)) || (rc = b_counter.ensure(sizeof(unsigned) * 6)) ||
       (rc = b_pscratch.ensure(sizeof(uint32_t) * scratch_words)))
     return fail(rc, "pair-list allocation");
   cudaStream_t s = stream;
@@ -303,7 +506,7 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
       (rc = cuda(cudaMemcpyAsync(b_pi.p, pi, sizeof(int32_t) * npairs, cudaMemcpyHostToDevice, s), "upload")) ||
       (rc = cuda(cudaMemcpyAsync(b_pj.p, pj, sizeof(int32_t) * npairs, cudaMemcpyHostToDevice, s), "upload")) ||
       (rc = cuda(cudaMemcpyAsync(b_orig.p, order.data(), sizeof(int32_t) * npairs, cudaMemcpyHostToDevice, s), "upload")) ||
-      (rc = cuda(cudaMemsetAsync(b_counter.p, 0, sizeof(unsigned) * 4, s), "pair-list counters")))
+      (rc = cuda(cudaMemsetAsync(b_counter.p, 0, sizeof(unsigned) * 6, s), "pair-list counters")))
     return rc;
   PairWaveArgs a{};
   a.codes = (const int8_t*)b_codes.p;
@@ -312,25 +515,37 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
   a.pi = (const int32_t*)b_pi.p;
   a.pj = (const int32_t*)b_pj.p;
   a.out = (int32_t*)b_out.p;
-  a.scratch = (uint32_t*)b_pscratch.p;
   a.go = go;
   a.ge = ge;
   a.bias = bias;
   a.sub = (const int8_t*)b_sub.p;
-  for (int q = 0; q < 4; ++q) {
+  // one launch's last jobs beside the next one's first
+  const int sides = std::max(0, std::min(kinds_used - 1, (int)branch.size()));
+  if (sides > 0 && (rc = cuda(cudaEventRecord(fork_ev, s), "pair-list streams"))) return rc;
+  for (int k = 0; k < sides; ++k)
+    if ((rc = cuda(cudaStreamWaitEvent(branch[k], fork_ev, 0), "pair-list streams"))) return rc;
+  int at = 0;
+  for (int q = 0; q < 6; ++q) {
     const PairBucket& b = bucket[q];
     if (!b.count) continue;
+    const int on = at++ % (sides + 1);
+    cudaStream_t bs = on ? branch[on - 1] : s;
+    a.scratch = (uint32_t*)b_pscratch.p + scratch_at[q];
     a.order = (const int32_t*)b_orig.p + b.first;
     a.npairs = b.count;
     a.scratch_cols = b.maxrows > 32 * b.R ? b.maxcols : 0;
     a.counter = (unsigned*)b_counter.p + q;
-    if (b.P == 2 && b.R == 8) pair_wave_kernel<8, 2><<<grid[q], 32 * kPWarps, 0, s>>>(a);
-    else if (b.P == 2) pair_wave_kernel<4, 2><<<grid[q], 32 * kPWarps, 0, s>>>(a);
-    else if (b.R == 8) pair_wave_kernel<8, 1><<<grid[q], 32 * kPWarps, 0, s>>>(a);
-    else pair_wave_kernel<4, 1><<<grid[q], 32 * kPWarps, 0, s>>>(a);
+    pair_dispatch(b.R, b.P, seven, [&](auto r, auto p, auto s7) {
+      if constexpr (decltype(s7)::value) pair7_kernel<decltype(r)::value, decltype(p)::value><<<grid[q], 32 * kPWarps, 0, bs>>>(a);
+      else pair_wave_kernel<decltype(r)::value, decltype(p)::value><<<grid[q], 32 * kPWarps, 0, bs>>>(a);
+    });
     if ((rc = cuda(cudaGetLastError(), "pair-list launch"))) return rc;
     ++launches;
   }
+  for (int k = 0; k < sides; ++k)
+    if ((rc = cuda(cudaEventRecord(join_ev[k], branch[k]), "pair-list streams")) ||
+        (rc = cuda(cudaStreamWaitEvent(s, join_ev[k], 0), "pair-list streams")))
+      return rc;
   if ((rc = cuda(cudaMemcpyAsync(out, b_out.p, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, s), "download")) ||
       (rc = cuda(cudaStreamSynchronize(s), "pair-list sync")))
     return rc;

@@ -47,8 +47,12 @@ __device__ __forceinline__ void build_profile(uint32_t* prof, const int8_t* s_su
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       uint32_t* d = prof + ((x4 + k) * 32 + lane) * (R / 4);
-      if constexpr (R == 8) *reinterpret_cast<uint2*>(d) = make_uint2(w[k][0], w[k][1]);
-      else *d = w[k][0];
+      if constexpr (R == 8) {
+        *reinterpret_cast<uint2*>(d) = make_uint2(w[k][0], w[k][1]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < R / 4; ++q) d[q] = w[k][q];
+      }
     }
   }
 }
