@@ -46,8 +46,8 @@
 //  * one CTA with the job in its shared memory (up to 136 taxa);
 //  * one thread-block cluster, the matrix in L2 (up to 600 taxa, and every larger
 //    job of the serving loop);
-//  * the whole GPU, one cooperative launch per segment between rebuilds
-//    (compacted to the live slots, in slot order), above that.
+//  * the whole GPU, one cooperative launch per segment between compactions (to
+//    the live slots, in slot order), above that.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -536,8 +536,8 @@ __device__ __forceinline__ void usum_warp(USum& x) {
 // barrier or an L2 round trip; 5.5-10 us.  Against one streaming pass over the
 // whole live triangle per join with three to four barriers, which it replaced
 // (bounded by L2 and HBM bandwidth at 8,000 taxa, by its barriers below 2,000),
-// whole job, matrix on the device: 15.1 -> 7.8 ms at 1,200 taxa, 131 -> 78.6 ms
-// at 8,000.
+// whole job, matrix on the device: 15.1 -> 7.8 ms at 1,200 taxa, 131 -> 73 ms at
+// 8,000.
 //
 // The pick is exact as with a full pass: every float q is within E of the exact
 // q; every pair whose float q is at most the smallest + 3E lies in a row whose
@@ -548,6 +548,12 @@ __device__ __forceinline__ void usum_warp(USum& x) {
 // threshold into the candidate list.
 constexpr int kLazyThreads = 1024;
 constexpr int kLazyMaxCtas = 160;         // team size, at most
+// From kCompactN slots on, the matrix is also compacted whenever one in
+// kCompactPart of them is dead: every CTA reads and updates all slots for every
+// join, and a new segment costs one scan of all rows.  8,000 taxa: 78.1 ms at
+// rebuilds only, 73.5 / 72.9 / 74.0 / 75.2 with a part of 4 / 8 / 16 / 24; 2,100:
+// 14.57 / 14.28 / 14.30 / 14.42 / 14.65.
+constexpr int kCompactN = 2048, kCompactPart = 8;
 
 struct LazyLayout {
   size_t tf, tl, tv, node, prow, ord, made, row, town, parts, bytes;
@@ -2150,7 +2156,8 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     int step = 0;
     while (step < n - 1) {
       // the segment ends with the join after which the countdown reaches 0
-      const int seg_end = steps == INT_MAX ? n - 1 : std::min(n - 1, step + steps + 1);
+      const int sched_end = steps == INT_MAX ? n - 1 : std::min(n - 1, step + steps + 1);
+      const int seg_end = d.n0 >= kCompactN ? std::min(sched_end, step + d.n0 / kCompactPart) : sched_end;
       if ((rc = cuda(cudaMemsetAsync(S.gbar.p, 0, sizeof(unsigned) * 2, s), "nj launch"))) return rc;
       // failure injection for the tests (NWG_NJ_INJECT_BARRIER_STALL=1): in the
       // first segment the first CTA never publishes, so the first exchange never
@@ -2193,6 +2200,8 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
         steps = (m_n < 200) ? INT_MAX : (int)((float)m_n * 0.5f);
         ave0 = (((long long)(m_n - 1) * m_n) / 2) / kBinT;
         ub = ((long long)m_n * (m_n - 1)) / 2;
+      } else if (step < n - 1 && (rc = compact(m_n))) {
+        return rc;
       }
       if ((rc = cuda(cudaGetLastError(), "nj launch"))) return rc;
     }

@@ -62,3 +62,11 @@ def test_lazy_search_matches_oracle(form):
     r = subprocess.run([sys.executable, "-c", _CODE], cwd=ROOT, env=dict(os.environ, **_FORMS[form]),
                        capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+def test_compaction_between_rebuilds_matches_oracle():
+    # above 2,048 slots the matrix is compacted every eighth of them: three times before the first rebuild here
+    code = _CODE[: _CODE.index("rng = ")] + "\nrng = np.random.default_rng(8)\nn = 2200\n" \
+        "check(sym(rng.integers(1, 100000, (n, n)) / 8))\nprint('ok')\n"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
