@@ -223,7 +223,7 @@ int64_t nwg_newick(const nwg_join* joins, int n, const char* const* names, char*
  * library call cudaMalloc or cudaFree -- code running while a stream is
  * captured in the global capture mode, or hosts that hand out all device
  * memory from their own pool and must not have a cudaFree synchronize the
- * device under them.  Same scores as nwg_score_pairs (one pair per thread,
+ * device under them.  Same scores as nwg_score_pairs (here one pair per thread,
  * int32), but every input and output is caller-provided device memory, no
  * context is used, and the only work memory is a fixed 32 MiB static device
  * array that every GPU loading the library holds until exit.
@@ -272,7 +272,7 @@ typedef struct {
   int64_t pairs;        /* pairs (i<j) this launch computes                    */
   int64_t cells;        /* their L_i*L_j sum                                   */
   double ms;            /* device time (events around this launch alone)       */
-  int32_t variant;      /* register layout of the wave kernel (0..6)          */
+  int32_t variant;      /* register layout of the wave kernel (0..8)          */
   int32_t lanes;        /* lanes per wavefront (32, 16, 8)                    */
 } nwg_launch_rec;
 
@@ -342,9 +342,9 @@ int nwg_msa_rows(nwg_ctx* ctx, char* out, int64_t row_stride);
  * (n^2 floats of matrix + NJ workspace + codes) fits hbm_budget_bytes and puts
  * up to max_batch_jobs of them into one batch: one persistent launch per
  * length bucket with pairs of all the batch's jobs interleaved, then the
- * join loops, one launch per form: one CTA per job up to 160 sequences, a
- * cluster per job (8 CTAs, 16 from 256 sequences on) with the matrix in its
- * shared memory up to 768, a cluster over L2 above.  Up to four batches
+ * join loops, one launch per form, side by side: one CTA per job up to 136
+ * sequences, a cluster per job above (8 CTAs, 16 when the batch's largest has
+ * 256 sequences or more).  Up to four batches
  * can be on the device at once (own streams), so jobs arriving while one batch runs
  * are admitted and overlap it, and each batch is returned as soon as it is done.  Each job's matrix and join list equal what
  * nwg_score_all and nwg_nj return for that job alone.

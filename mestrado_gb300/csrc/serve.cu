@@ -10,10 +10,9 @@
 // device arenas, pinned staging):
 //   residues in (ASCII; encoded and reversed on the device) -> one
 //   multi-job plan: every job's Y groups in shared length buckets, so one
-//   persistent launch per bucket interleaves pairs of different jobs ->
-//   matrices out -> the join loops, one thread-block cluster per job (jobs
-//   that fit, with the matrix in the cluster's shared memory) -> join lists
-//   out.
+//   persistent launch per bucket interleaves pairs of different jobs (the
+//   buckets on three streams) -> matrices out -> the join loops, one CTA or
+//   one thread-block cluster per job -> join lists out.
 // While one slot's batch is on the device the next batch is formed and queued
 // on another free slot, so arrivals overlap the work in flight.  Each slot has
 // its own completion thread that waits for that slot's event, hands results

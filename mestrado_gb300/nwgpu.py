@@ -275,7 +275,7 @@ class Context:
         return off, int(bad[0])
 
     def score_pairs(self, codes, offsets, pi, pj):
-        """Scores of explicit pairs (int32 lanes, one thread per pair)."""
+        """Scores of explicit pairs (a warp per two pairs)."""
         pi = np.ascontiguousarray(pi, dtype=np.int32)
         pj = np.ascontiguousarray(pj, dtype=np.int32)
         out = np.zeros(len(pi), dtype=np.int32)
