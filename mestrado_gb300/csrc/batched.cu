@@ -196,8 +196,13 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   struct Group { int y, y2, nx, R, V, W, P, check; };
   std::vector<Group> groups;
   groups.reserve((size_t)Y.n / 2 + 1);
+  TuneChoice tc{};
+  int tc_rows = 0;   // the rows of tc: groups of equal length share the choice
   for (int y = 0; y < Y.n;) {
-    const TuneChoice tc = c->choice_set(Y.len[y], X.maxlen, cells);
+    if (Y.len[y] != tc_rows) {
+      tc_rows = Y.len[y];
+      tc = c->choice_set(tc_rows, X.maxlen, cells);
+    }
     if (!force32 && rebase) {
       const int y2 = y + 1 < Y.n ? y + 1 : -1;
       const int last = y2 >= 0 ? y2 : y;

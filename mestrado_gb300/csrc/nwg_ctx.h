@@ -186,6 +186,9 @@ struct Ctx {
     double rate = 9.0e12;
     for (const Cand& c : cands[tune_class(rows)])
       if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) rate = c.rate;
+    // a set of many waves of jobs: the shortest chain would not show
+    const int bands = padded_rows(t, rows) / (t.W * t.R);
+    if (cells * padded_rows(t, rows) / rows / rate > 20.0 * bands * (cols + t.W - 1) * (10.0 * t.R + 90.0) / kHz) return t;
     TuneChoice best = t;
     double best_est = 0.95 * est(t, rate);   // not for less than a twentieth
     for (int W : {8, 16, 32})
