@@ -196,10 +196,19 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   struct Group { int y, y2, nx, R, V, W, P, check; };
   std::vector<Group> groups;
   groups.reserve((size_t)Y.n / 2 + 1);
-  TuneChoice tc{};
-  int tc_rows = 0;   // the rows of tc: groups of equal length share the choice
+  // A set that takes a fraction of the longest Y's chain runs on that Y's template
+  // throughout: one launch, and one kernel to load on its first use.
+  TuneChoice tc = c->choice_set(Y.len[0], X.maxlen, cells);
+  int tc_rows = Y.len[0];   // the rows of tc: groups of equal length share the choice
+  double padded = 0.0, xcols = 0.0;
+  for (int y = 0; y < Y.n; ++y) {
+    if (triangle) xcols += X.len[y];
+    padded += (double)padded_rows(tc, Y.len[y]) * (triangle ? xcols : xsum);
+  }
+  const bool one = tc.V == 7 && padded / 7.0e12 < 0.25 * Ctx::chain_s(tc, Y.len[0], X.maxlen) &&
+                   !c->cands[tune_class(Y.len[0])].empty();
   for (int y = 0; y < Y.n;) {
-    if (Y.len[y] != tc_rows) {
+    if (!one && Y.len[y] != tc_rows) {
       tc_rows = Y.len[y];
       tc = c->choice_set(tc_rows, X.maxlen, cells);
     }

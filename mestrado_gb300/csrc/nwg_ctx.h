@@ -173,13 +173,15 @@ struct Ctx {
   // the candidate's rate, and a quarter of the shorter.  All pairs of 64 x 300
   // residues: 52 us with 12 rows on 32 lanes, 62 with 18 on 16, 86 with two
   // bands of 20 on 8.
+  static double chain_s(const TuneChoice& t, int rows, int cols) {   // seconds
+    return padded_rows(t, rows) / (t.W * t.R) * (cols + t.W - 1) * (10.0 * t.R + 90.0) / 2.0e9;
+  }
   TuneChoice choice_set(int rows, int cols, double cells) const {
     const TuneChoice t = choice(rows);
     if (t.V != 7 || cands[tune_class(rows)].empty()) return t;
-    constexpr double kHz = 2.0e9, kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // cells/s at 4, 8, 12, 16 rows
+    constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // cells/s at 4, 8, 12, 16 rows
     const auto est = [&](const TuneChoice& c, double rate) {
-      const int bands = padded_rows(c, rows) / (c.W * c.R);
-      const double chain = bands * (cols + c.W - 1) * (10.0 * c.R + 90.0) / kHz;
+      const double chain = chain_s(c, rows, cols);
       const double whole = cells * padded_rows(c, rows) / rows / rate;
       return std::max(chain, whole) + 0.25 * std::min(chain, whole);
     };
@@ -187,12 +189,11 @@ struct Ctx {
     for (const Cand& c : cands[tune_class(rows)])
       if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) rate = c.rate;
     // a set of many waves of jobs: the shortest chain would not show
-    const int bands = padded_rows(t, rows) / (t.W * t.R);
-    if (cells * padded_rows(t, rows) / rows / rate > 20.0 * bands * (cols + t.W - 1) * (10.0 * t.R + 90.0) / kHz) return t;
+    if (cells * padded_rows(t, rows) / rows / rate > 20.0 * chain_s(t, rows, cols)) return t;
     TuneChoice best = t;
     double best_est = 0.95 * est(t, rate);   // not for less than a twentieth
-    for (int W : {8, 16, 32})
-      for (int R : {4, 8, 12, 16, 20, 24, 28, 32}) {
+    for (int W : {8, 32})   // few templates: the first use of each in a process loads it (0.5 to 1 ms)
+      for (int R : {4, 8, 12, 16, 24, 32}) {
         const TuneChoice c{R, 7, W};
         const double e = est(c, R < 20 ? kSlow[R / 4 - 1] : 9.0e12);
         if (e < best_est) {
