@@ -211,7 +211,7 @@ struct KCand {
 
 struct GridNJ {
   unsigned* bar;        // [0] barrier arrivals, [1] publications (both count up from 0 per launch)
-  int* abort;           // set when a barrier wait gave up; every CTA then leaves
+  int* abort;           // set when a wait gave up or a pick failed; every CTA and queued kernel then leaves
   float4* gather;       // [2 * CTAs]: the grid's exchanges
   KCand* cand;          // the candidate list of the fallback scan
   KCand* cbest;         // [CTAs]: per CTA its first candidate of the fallback scan
@@ -219,6 +219,7 @@ struct GridNJ {
   int pad;
 };
 
+constexpr int kAbortWait = 1, kAbortPick = 2;
 constexpr long long kBarrierSpinCycles = 4000000000ll;   // about two seconds: no phase takes a millisecond
 constexpr int kFastRows = 32;                             // candidate rows the direct pick evaluates
 
@@ -252,7 +253,7 @@ __device__ bool grid_barrier(const GridNJ& g, unsigned& target) {
         break;
       }
       if (clock64() - t0 > kBarrierSpinCycles) {
-        atomicExch(g.abort, 1);
+        atomicExch(g.abort, kAbortWait);
         ok = 0;
         break;
       }
@@ -765,7 +766,7 @@ __device__ bool grid_gather(const GridNJ& g, Team tm, unsigned seq, float4* part
     while ((int)(ld_acquire_u32(&g.bar[1]) - target) < 0) {
       if (*(volatile int*)g.abort) bad = 1;
       else if (clock64() - t0 > kBarrierSpinCycles) {
-        atomicExch(g.abort, 1);
+        atomicExch(g.abort, kAbortWait);
         bad = 1;
       }
       if (bad) break;
@@ -1105,8 +1106,13 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
                               &spick, target))
         return false;
       __syncthreads();
-      if (spick.error) {
-        if (tm.rank == 0 && tid == 0) record_pick(s, spick);
+      if (spick.error) {   // the same in every CTA
+        if (tm.rank == 0 && tid == 0) {
+          record_pick(s, spick);
+          // nothing goes back to global memory: what is queued behind this
+          // segment must not read the lists, it leaves as after a wait that ran out
+          if constexpr (!CL) atomicExch(g.abort, kAbortPick);
+        }
         return false;
       }
       i = swin.a;
@@ -2219,7 +2225,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
   if (big) {
     int gb[4];
     if ((rc = cuda(cudaMemcpy(gb, S.gbar.p, sizeof(gb), cudaMemcpyDeviceToHost), "nj download"))) return rc;
-    if (gb[2]) return fail(NWG_ERR_CUDA, "neighbor-joining grid barrier timed out");
+    if (gb[2] == kAbortWait) return fail(NWG_ERR_CUDA, "neighbor-joining grid barrier timed out");
   }
   stats.ambiguous_steps = (int64_t)dst[0];
   stats.tie_steps = (int64_t)dst[1];
