@@ -204,7 +204,11 @@ typedef struct {
  * layouts and on which tied candidates its library's cut keeps (duplicated
  * sequences: tens of tied pairs).  stats.reference_identical is 1 exactly
  * when no step was ambiguous, i.e. when the returned tree is guaranteed to be
- * the reference's. */
+ * the reference's.
+ *
+ * Distances are meant to be finite, of any magnitude.  Infinite and undefined
+ * ones follow IEEE comparisons: a pair whose q is undefined or +infinity is
+ * never joined, and when no other is left the call returns NWG_ERR_CUDA. */
 int nwg_nj(nwg_ctx* ctx, const float* D, int64_t ld, int n, nwg_join* joins, nwg_nj_stats* stats);
 
 /* Same with D already on the device (d_D). */

@@ -56,6 +56,7 @@
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <math_constants.h>
 
 #include "nwg_ctx.h"
 
@@ -64,6 +65,7 @@ namespace nwg {
 namespace {
 
 constexpr int kNJMaxN = 8192;
+constexpr float kFloatTop = 1.329228e36f;   // 2^120: the float search holds q and T up to here
 constexpr int kCandCap = 2048;         // candidate list capacity per join (longer lists are not read)
 
 struct NJDev {
@@ -620,6 +622,13 @@ __device__ __forceinline__ float lazy_err(const LazyRep& k, float nm2f) {   // E
   return __fadd_ru(__fmul_ru(8.f * 5.9604645e-8f, m), 1e-30f);
 }
 
+// Whether floats do not hold this join's q and T (undefined or infinite values
+// among them, or too near the overflow for one more join's growth): the search
+// is then exact, over every pair.
+__device__ __forceinline__ bool lazy_wide(const LazyRep& k, float nm2f) {
+  return !(__fadd_ru(__fmul_ru(k.dabs, fmaxf(nm2f, 1.f)), __fmul_ru(2.f, k.tabs)) <= kFloatTop);
+}
+
 __device__ __forceinline__ float lazy_q(float d, float tr, float tc, float nm2f) {
   return __fsub_rn(__fsub_rn(__fmul_rn(d, nm2f), tr), tc);
 }
@@ -818,14 +827,16 @@ __device__ __forceinline__ float4 cta_best(const LazyMem& m, Team tm, int rows) 
 }
 
 // Candidate scan of the fallback: this CTA's own rows within the threshold,
-// visit(pred, candidate) by whole warps.  tx: every slot's exact T.
+// visit(pred, candidate) by whole warps.  tx: every slot's exact T.  wide: every
+// live row's pairs, without a look at the floats; a pair whose q is undefined or
+// +infinity is none, as in the reference's comparisons.
 template <class Visit>
 __device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int rows, const double* tx, float nm2f,
-                               double nm2, int watermark, float thr, Visit&& visit) {
+                               double nm2, int watermark, float thr, bool wide, Visit&& visit) {
   const int lane = threadIdx.x & 31;
   for (int l = (int)threadIdx.x >> 5; l < rows; l += (int)blockDim.x >> 5) {
     const int r = l * tm.size + tm.rank;
-    if (m.U[l] > thr) continue;
+    if (wide ? r >= s.n0 || m.node[r] < 0 : m.U[l] > thr) continue;
     const int ur = m.node[r];
     const float tr = m.Tf[r];
     const double Tr = m.To[l];
@@ -836,10 +847,10 @@ __device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int ro
       KCand kc = kc_none();
       if (c < s.n0 && m.node[c] >= 0) {
         const float d = __ldcg(row + c);
-        if (lazy_q(d, tr, m.Tf[c], nm2f) <= thr) {
+        if (wide || lazy_q(d, tr, m.Tf[c], nm2f) <= thr) {
           const GCand cd = make_cand(r, c, ur, m.node[c], Tr, __ldcg(tx + c), d, nm2, watermark);
           kc = KCand{cd.k1, cd.k2, cd.a, cd.b};
-          pred = true;
+          pred = !wide || cd.q1 < DBL_MAX;
         }
       }
       visit(pred, kc);
@@ -852,8 +863,8 @@ __device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int ro
 // CTA.  False when a wait ran out.
 template <bool CL>
 __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m, Team tm, int rows,
-                               const float4* parts, const double* tx, float thr, bool listed, float nm2f, double nm2,
-                               int watermark, GCand* win, PickOut* pk, unsigned& target) {
+                               const float4* parts, const double* tx, float thr, bool listed, bool wide, float nm2f,
+                               double nm2, int watermark, GCand* win, PickOut* pk, unsigned& target) {
   __shared__ GCand fc[32];
   const int lane = threadIdx.x & 31;
   if (listed) {   // at most 32 published pairs are all the candidates
@@ -861,7 +872,7 @@ __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m
       int base = 0;
       for (int b0 = 0; b0 < tm.size; b0 += 32) {
         const float4 v = b0 + lane < tm.size ? parts[b0 + lane] : make_float4(FLT_MAX, FLT_MAX, 0.f, 0.f);
-        const bool in = v.x <= thr;
+        const bool in = b0 + lane < tm.size && v.x <= thr;
         const unsigned bal = __ballot_sync(0xffffffffu, in);
         if (in) {
           const unsigned rc = __float_as_uint(v.z);
@@ -883,7 +894,7 @@ __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m
   }
   KCand first = kc_none();
   bool full = false;
-  lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
+  lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, wide, [&](bool pred, const KCand& c) {
     list_push(s, g, pred, c, full);
     if (pred && kc_first(c, first)) first = c;
   });
@@ -917,7 +928,7 @@ __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m
     __syncthreads();
     const KCand w = sfirst;
     unsigned ties = 0, amb = 0;
-    lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, [&](bool pred, const KCand& c) {
+    lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, wide, [&](bool pred, const KCand& c) {
       if (pred) count_vs(c, w, ties, amb);
     });
     add_counts(ties, amb, s.g32);
@@ -1002,10 +1013,10 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     if (p < n0) m.prow[p] = (int16_t)__ldcg(s.prow + p);
     const double t = v >= 0 ? __ldcg(s.T + p) : 0.0;
     const float hi = __double2float_rn(t);
+    ta = fmaxf(ta, fabsf(hi) <= FLT_MAX ? fabsf(hi) : CUDART_INF_F);
     m.Tf[p] = v >= 0 ? hi : __int_as_float(0x7FC00000);
     m.Tl[p] = __double2float_rn(__dsub_rn(t, (double)hi));
     m.tv[p] = 0.f;
-    ta = fmaxf(ta, fabsf(hi));
   }
   for (int k = tid; k < n_ord; k += nth) m.ord[k] = (int16_t)__ldcg(s.slot + __ldcg(s.act + k));
   for (int l = tid; l < rows; l += nth) {
@@ -1056,6 +1067,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     const float4* const parts = m.parts + (seq & 1) * tm.size;
     const double* const tx = s.tx + (size_t)(seq & 1) * n0;
     // ---- pick: the published pairs within the threshold
+    const bool wide = lazy_wide(rep, nm2f);   // the same in every thread of the team
     if (warp == 0) {
       const float E = lazy_err(rep, nm2f);
       constexpr int kPer = kLazyMaxCtas / 32;
@@ -1075,7 +1087,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
       bool second = false;
 #pragma unroll
       for (int t = 0; t < kPer; ++t) {
-        const bool in = x[t] <= thr;
+        const bool in = lane + 32 * t < tm.size && x[t] <= thr;
         if (in) second |= parts[lane + 32 * t].y <= thr;
         cands += __popc(__ballot_sync(0xffffffffu, in));
       }
@@ -1093,7 +1105,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     const unsigned rc = __float_as_uint(s_pair.z);
     float dmin = s_pair.w;
     int i, j, si, sj;
-    const bool fast = cands == 1;
+    const bool fast = cands == 1 && !wide;
     if (fast) {
       const int r = rc & 0xFFFFu, c = rc >> 16;
       const int ur = m.node[r], uc = m.node[c];
@@ -1102,8 +1114,8 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
       si = ur < uc ? r : c;
       sj = ur < uc ? c : r;
     } else {
-      if (!lazy_pick_slow<CL>(s, g, m, tm, rows, parts, tx, thr, cands >= 1 && cands <= 32, nm2f, nm2, watermark, &swin,
-                              &spick, target))
+      if (!lazy_pick_slow<CL>(s, g, m, tm, rows, parts, tx, thr, cands >= 1 && cands <= 32 && !wide, wide, nm2f, nm2,
+                              watermark, &swin, &spick, target))
         return false;
       __syncthreads();
       if (spick.error) {   // the same in every CTA
@@ -1130,8 +1142,8 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     // every new value is a multiple of 2^eu, and at most 1.5 dabs (rounding aside)
     const int eu = rep.elow == INT_MAX ? 0 : rep.elow - 1;
     const int span_max = rep.dabs > 0.f ? top_bit_exp(rep.dabs) + 3 - eu : 0;
-    const bool u32 = span_max <= 30 && eu >= -100 && eu <= 100;
-    const bool u64 = span_max < 47;
+    const bool u32 = !wide && span_max <= 30 && eu >= -100 && eu <= 100;
+    const bool u64 = !wide && span_max < 47;
     const float scale = u32 ? __int_as_float((127 - eu) << 23) : 0.f;
     long long u = 0;
     int x_el = INT_MAX, x_or = 0;
@@ -1218,7 +1230,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     // sequential double sum is exact (all terms multiples of 2^eu, together
     // below 2^53 of them), else the sequential sum itself
     const int span = x_el == INT_MAX ? 0 : top_bit_exp(x_d) + 1 - eu;
-    if (x_el == INT_MAX) {
+    if (!wide && x_el == INT_MAX) {
       // every value is zero
     } else if (u64 && x_el >= eu && span <= span_max && span + 32 - __clz(m_n) <= 53) {
       tsum = units_to_double(u, eu);
@@ -1228,7 +1240,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
       tsum = s_seq;
     }
     if (lead) {
-      rep.dabs = fmaxf(rep.dabs, x_d);
+      rep.dabs = wide ? CUDART_INF_F : fmaxf(rep.dabs, x_d);   // wide up to the segment's end: Tf no longer says who lives
       rep.elow = min(rep.elow, x_el);
       tsf = __double2float_rn(tsum);
       rep.tabs = __fmul_ru(fmaxf(x_t, fabsf(tsf)), 1.000001f);
@@ -1321,11 +1333,12 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     if (step + 1 == step1) break;
     // ---- the rows whose bound reaches it, counted by every warp for itself
     rep = s_rep;
+    const bool search = !lazy_wide(rep, nm2f);
     const float E = lazy_err(rep, nm2f);
     const float best = unford(s_hint);
     const float reach = best < FLT_MAX ? __fadd_ru(best, __fmul_ru(5.f, E)) : FLT_MAX;
     int cnt = 0;
-    for (int l0 = 0; l0 < rows; l0 += 32) {
+    for (int l0 = 0; search && l0 < rows; l0 += 32) {
       const float L = l0 + lane < rows ? m.L[l0 + lane] : FLT_MAX;
       cnt += __popc(__ballot_sync(0xffffffffu, L <= reach && L < FLT_MAX));
     }
