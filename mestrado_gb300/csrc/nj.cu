@@ -66,6 +66,7 @@ namespace {
 
 constexpr int kNJMaxN = 8192;
 constexpr float kFloatTop = 1.329228e36f;   // 2^120: the float search holds q and T up to here
+constexpr int kNoPair = 0x7F7FFFFF;    // ford(FLT_MAX): a row without a pair
 constexpr int kCandCap = 2048;         // candidate list capacity per join (longer lists are not read)
 
 struct NJDev {
@@ -1684,6 +1685,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
   __shared__ PickOut spick;
   __shared__ GCand swin;
   __shared__ float sthr;
+  __shared__ bool s_wide;   // floats do not hold this join's q: every live pair is looked at, exactly
   if ((int)blockIdx.x >= njobs) return;
   if (threadIdx.x == 0) sjob = jobs[blockIdx.x];
   __syncthreads();
@@ -1752,7 +1754,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
         if (h && r == tid) break;
         const float tr = Tf[r];
         if (tr != tr) {   // dead
-          grm[r] = 0x7F7FFFFF;
+          grm[r] = kNoPair;
           continue;
         }
         const float* row = rows + (size_t)r * ldl;
@@ -1795,14 +1797,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
         mm = fmaxf(mm, wm[w]);
       }
       sthr = q + 3.f * (8.f * 5.9604645e-8f * mm) + 1e-30f;
+      s_wide = !(mm <= kFloatTop);
       nsel = 0;
     }
     __syncthreads();
     // ---- pick
     const float thr = sthr;
+    const bool wide = s_wide;
     const int othr = ford(thr);
     for (int r = tid; r < n; r += nth) {
-      if (grm[r] <= othr) {
+      if (grm[r] <= othr && grm[r] != kNoPair) {
         const int k = atomicAdd(&nsel, 1);
         if (k < kFastRows) rows_sel[k] = r;
       }
@@ -1810,7 +1814,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
     __syncthreads();
     const int nr = nsel;
     if (warp == 0) {
-      int ok = nr >= 1 && nr <= kFastRows;
+      int ok = nr >= 1 && nr <= kFastRows && !wide;
       if (ok && lane < nr) {
         const int r = rows_sel[lane];
         const int4 rec = grc[r];
@@ -1846,8 +1850,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
       // then the ties and ambiguous pairs against it (pick_keys' rule)
       auto scan = [&](auto&& visit) {
         for (int r = 0; r < n; ++r) {
-          if (grm[r] > othr) continue;
           const int ur = node[r];
+          if (ur < 0 || !(wide || grm[r] <= othr)) continue;
           const float tr = Tf[r];
           const float* row = rows + (size_t)r * ldl;
           for (int c = r + 1 + tid; c < n; c += nth) {
@@ -1855,8 +1859,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
             if (uc < 0) continue;
             const float d = row[c];
             const float q = __fsub_rn(__fsub_rn(__fmul_rn(d, nm2f), tr), Tf[c]);
-            if (q > thr) continue;
+            if (!wide && !(q <= thr)) continue;
             const GCand cd = make_cand(r, c, ur, uc, T[r], T[c], d, nm2, watermark);
+            if (wide && !(cd.q1 < DBL_MAX)) continue;
             visit(KCand{cd.k1, cd.k2, cd.a, cd.b});
           }
         }
@@ -1940,7 +1945,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
       double sum;
       if (x.e == INT_MAX) {
         sum = 0.0;
-      } else if (x.t - x.e < 48 && x.a < (1ll << 53)) {
+      } else if (x.t - x.e < 48 && x.a < (1ll << 53) && x.t < 128) {   // 128: infinite or undefined
         sum = units_to_double(x.u, x.e);   // exact: the sequential sum's value
       } else {
         sum = 0.0;   // the reference's loop: active ids ascending, i and j skipped

@@ -29,7 +29,7 @@ def _check(ctx, D):
         assert np.array_equal(np.array([x[f] for x in oj], j[f].dtype), j[f], equal_nan=True), f
 
 
-@pytest.mark.parametrize("n,undefined", [(300, 150), (700, 400), (2200, 900)])
+@pytest.mark.parametrize("n,undefined", [(9, 4), (130, 40), (300, 150), (700, 400), (2200, 900)])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_no_pair_left_to_join(ctx, n, undefined, value):
     # the defined taxa join, then no pair has a value: a status, with row sums and
@@ -56,7 +56,7 @@ import numpy as np, oracle_py as O, pytest
 from mestrado_gb300 import Context
 from test_nj_range_gpu import _check, _overflowing, _sym
 c = Context(10, 2)
-for n in (139, 170, 290, 650):
+for n in (40, 139, 170, 290, 650):
     _check(c, _overflowing(n, 2.0 ** 126, n))            # T and q overflow floats throughout
     _check(c, _overflowing(n, 2.0 ** 116, n))
     _check(c, _overflowing(n, 2.0 ** 112, n))            # exact at first, held by floats once few taxa are left
