@@ -1003,6 +1003,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
   __shared__ float4 s_pair;
   __shared__ LazyRep s_rep;
   __shared__ long long w_u[32];            // per warp: the join's integer sum,
+  __shared__ long long w_u2[32], w_a2[32]; // the second sum and its values' magnitudes
   __shared__ int4 w_x[32];                 // largest dT (ordered), |T|, |tmp|, lowest exponent
   const int id0 = n + step0;               // ids from here on are made in this segment
   const int n_ord = __ldcg(s.na);
@@ -1229,16 +1230,54 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
     }
     // the new node's row sum: the integer sum when every partial sum of the
     // sequential double sum is exact (all terms multiples of 2^eu, together
-    // below 2^53 of them), else the sequential sum itself
+    // below 2^53 of them), else a sum in finer units or the sequential sum itself
     const int span = x_el == INT_MAX ? 0 : top_bit_exp(x_d) + 1 - eu;
     if (!wide && x_el == INT_MAX) {
       // every value is zero
     } else if (u64 && x_el >= eu && span <= span_max && span + 32 - __clz(m_n) <= 53) {
       tsum = units_to_double(u, eu);
     } else {
-      if (tid == 0) s_seq = lazy_seq_sum(m, n_ord, id0, step - step0, si, sj);
-      __syncthreads();
-      tsum = s_seq;
+      // Real-valued distances: halving every join takes elow below what the job's
+      // largest value leaves room for, but the values of one join span less.  A
+      // second sum in units of their own lowest bit, exact under the same rule:
+      // 16 ms instead of 75 (a sequential sum per join) for 1,200 taxa.
+      bool exact = false;
+      if (!wide && top_bit_exp(x_d) - x_el < 48) {   // |value| < 2^49 units, 8,192 of them
+        long long u2 = 0, a2 = 0;
+        for (int v = tid; v < nv; v += nth) {   // the slots that this thread has just updated
+          const float4 h4 = reinterpret_cast<const float4*>(m.Tf)[v], t4 = reinterpret_cast<const float4*>(m.tv)[v];
+          const float hi[4] = {h4.x, h4.y, h4.z, h4.w}, val[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (hi[k] == hi[k] && 4 * v + k != si && 4 * v + k != sj) {
+              const long long y = float_units(val[k], x_el);
+              u2 += y;
+              a2 += y < 0 ? -y : y;
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+          u2 += __shfl_xor_sync(0xffffffffu, u2, o);
+          a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+        }
+        if (lane == 0) {
+          w_u2[warp] = u2;
+          w_a2[warp] = a2;
+        }
+        __syncthreads();
+        u2 = lane < nw ? w_u2[lane] : 0;
+        a2 = lane < nw ? w_a2[lane] : 0;
+        for (int o = 16; o > 0; o >>= 1) {
+          u2 += __shfl_xor_sync(0xffffffffu, u2, o);
+          a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+        }
+        exact = a2 < (1ll << 53);
+        if (exact) tsum = units_to_double(u2, x_el);
+      }
+      if (!exact) {   // the same in the CTA
+        if (tid == 0) s_seq = lazy_seq_sum(m, n_ord, id0, step - step0, si, sj);
+        __syncthreads();
+        tsum = s_seq;
+      }
     }
     if (lead) {
       rep.dabs = wide ? CUDART_INF_F : fmaxf(rep.dabs, x_d);   // wide up to the segment's end: Tf no longer says who lives

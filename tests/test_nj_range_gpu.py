@@ -76,3 +76,17 @@ print('ok')
         env.update(NWG_NJ_CTA_MAX_N="0", NWG_NJ_CLUSTER_MAX_N="100000" if form == "cluster" else "0")
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+def test_real_valued_distances_cost_what_whole_ones_do(ctx):
+    # sums of one join's values in their own units: a sequential sum per join took nine times as long
+    rng = np.random.default_rng(2)
+    whole, real = _sym(rng.integers(1, 1000, (1200, 1200))), _sym(rng.random((1200, 1200)) * 100)
+    for D in (whole, real):
+        ctx.nj(D)
+    ms = [min(ctx.nj(D, stats=True)[1]["device_ms"] for _ in range(3)) for D in (whole, real)]
+    assert ms[1] < 4 * ms[0]
+    p = np.sort(rng.random(700)) * 1000
+    _check(ctx, _sym(np.abs(p[:, None] - p[None, :])))
+    _check(ctx, _sym(rng.random((700, 700)) * 100))
+    _check(ctx, _sym(rng.random((330, 330)) * 100))
