@@ -77,7 +77,7 @@ struct NJDev {
   int* node;           // per slot: node id, -1 dead
   int* act;            // active node ids ascending [n0 + 1]
   int* na;             // active count
-  int* g32;            // [2] candidates of the fallback scan
+  int* g32;            // [2][4]: ties, ambiguous pairs and candidates of the fallback scan
   unsigned long long* stats;  // [0] ambiguous steps, [1] tie steps, [2] internal errors,
                               // [3] open heap-size checks, [4] rebuilds (cluster form)
   nwg_join* joins;
@@ -205,12 +205,19 @@ struct GCand {
   int pad;
 };
 
-// An entry of the fallback scan's list: the keys and the node ids (the
-// winner's slots, d and row sums are read again after the pick).
+// An entry of the fallback scan's list: the keys and the nodes, each as its id
+// above its slot (in the order of the ids; the winner's d and row sums are read
+// again after the pick).
 struct KCand {
   long long k1, k2;
   int a, b;
 };
+constexpr int kSlotBits = 13;
+static_assert(kNJMaxN <= 1 << kSlotBits, "slots");
+__device__ __forceinline__ int slot_of(int packed) { return packed & ((1 << kSlotBits) - 1); }
+__device__ __forceinline__ KCand kc_of(const GCand& c) {
+  return KCand{c.k1, c.k2, c.a << kSlotBits | c.sa, c.b << kSlotBits | c.sb};
+}
 
 struct GridNJ {
   unsigned* bar;        // [0] barrier arrivals, [1] publications (both count up from 0 per launch)
@@ -444,28 +451,16 @@ __device__ __forceinline__ void count_vs(const KCand& c, const KCand& w, unsigne
   else ++amb;
 }
 
-// The CTA's counts into cnt[0] (ties) and cnt[1] (ambiguous pairs).
-__device__ __forceinline__ void add_counts(unsigned ties, unsigned amb, int* cnt) {
-  for (int o = 16; o > 0; o >>= 1) {
-    ties += __shfl_xor_sync(0xffffffffu, ties, o);
-    amb += __shfl_xor_sync(0xffffffffu, amb, o);
-  }
-  if ((threadIdx.x & 31) == 0 && (ties | amb)) {
-    atomicAdd(&cnt[0], (int)ties);
-    atomicAdd(&cnt[1], (int)amb);
-  }
-}
-
 // A warp's candidates of one scan step into the list, one atomic per warp.
-// s.g32[2] ends at the number of candidates when that is at most
+// *count ends at the number of candidates when that is at most
 // kListPickMax, else above kListPickMax: a warp that saw the count pass it
 // stops counting (full, the same in the warp).
-__device__ __forceinline__ void list_push(const NJDev& s, const GridNJ& g, bool pred, const KCand& c, bool& full) {
+__device__ __forceinline__ void list_push(const NJDev& s, const GridNJ& g, int* count, bool pred, const KCand& c, bool& full) {
   const unsigned bal = __ballot_sync(0xffffffffu, pred);
   if (bal == 0 || full) return;
   const int lane = threadIdx.x & 31;
   int base = 0;
-  if (lane == 0) base = atomicAdd(&s.g32[2], __popc(bal));
+  if (lane == 0) base = atomicAdd(count, __popc(bal));
   base = __shfl_sync(0xffffffffu, base, 0);
   const int idx = base + __popc(bal & ((1u << lane) - 1u));
   if (pred && idx < s.cand_cap) g.cand[idx] = c;
@@ -537,11 +532,14 @@ __device__ __forceinline__ void usum_warp(USum& x) {
 //
 // What bounds it: a chain of a few dependent steps per join (pick, the two rows
 // through L2, the update and its reduction, the scan, the exchange), each a CTA
-// barrier or an L2 round trip; 5.5-10 us.  Against one streaming pass over the
+// barrier or an L2 round trip; 5-9 us.  Against one streaming pass over the
 // whole live triangle per join with three to four barriers, which it replaced
 // (bounded by L2 and HBM bandwidth at 8,000 taxa, by its barriers below 2,000),
-// whole job, matrix on the device: 15.1 -> 7.8 ms at 1,200 taxa, 131 -> 73 ms at
-// 8,000.
+// whole job, matrix on the device: 15.3 -> 7.7 ms at 1,200 taxa, 130 -> 70.5 ms at
+// 8,000.  Where many pairs tie, exactly or within rounding, the candidate scan
+// decides: 16-byte loads, several in flight, few rows split over the warps, and a
+// count that stops at five ties (400 taxa in copies 8.1 -> 5.5 ms, the full pass
+// 6.2; 8,000 taxa that tie within rounding 1,030 -> 367, the full pass 730).
 //
 // The pick is exact as with a full pass: every float q is within E of the exact
 // q; every pair whose float q is at most the smallest + 3E lies in a row whose
@@ -550,7 +548,12 @@ __device__ __forceinline__ void usum_warp(USum& x) {
 // row); when no second is within the threshold, the published pairs within it
 // are all the candidates.  Otherwise the CTAs scan their rows within the
 // threshold into the candidate list.
-constexpr int kLazyThreads = 1024;
+// Threads per CTA, at most.  A thread per own row, so 512 do for 16 CTAs or more
+// and for 8 up to 4,096 taxa, with 128 registers.  Bounded at 1,024 the kernels
+// have 64 registers and spill in the candidate scan (400 taxa: 2.5 instead of 2.2
+// ms), but four CTAs of 256 threads fit an SM: for launches of more clusters than
+// the SMs hold one by one (100 jobs of 140 to 300 taxa: 14.8 instead of 24.7 ms).
+constexpr int kLazyThreads = 512, kLazyThreadsMax = 1024;
 constexpr int kLazyMaxCtas = 160;         // team size, at most
 // From kCompactN slots on, the matrix is also compacted whenever one in
 // kCompactPart of them is dead: every CTA reads and updates all slots for every
@@ -583,12 +586,15 @@ __host__ __device__ inline LazyLayout lazy_layout(int n0, int ld, int size) {
   return L;
 }
 
-// Threads per CTA: one per four slots between 256 and 512 (more make every CTA
-// barrier dearer than their loads in flight save), at least one per own row and
-// per CTA of the team (a multiple of 32).
-inline int lazy_threads(int ld, int rows, int size) {
-  const int t = std::max(std::max(std::min(std::max(ld / 4, 256), 512), rows), size);
-  return std::min((t + 31) / 32 * 32, kLazyThreads);
+// Threads per CTA, between 256 and 512 (more make every CTA barrier dearer than
+// their loads in flight save), at least one per own row and per CTA of the team, a
+// multiple of 32: one per four slots over the whole GPU, one per slot in a
+// cluster with its SMs to itself, whose CTAs have more rows to scan (500 taxa that tie within rounding:
+// 4.7 ms instead of 5.0, with distances of 1 to 999 2.73 instead of 2.82).
+inline int lazy_threads(int ld, int rows, int size, bool crowded) {
+  const int want = size <= 16 && !crowded ? ld : ld / 4;
+  const int t = std::max(std::max(std::min(std::max(want, 256), 512), rows), size);
+  return (t + 31) / 32 * 32;
 }
 
 // The job's state in the CTA's shared memory.
@@ -830,31 +836,69 @@ __device__ __forceinline__ float4 cta_best(const LazyMem& m, Team tm, int rows) 
 // Candidate scan of the fallback: this CTA's own rows within the threshold,
 // visit(pred, candidate) by whole warps.  tx: every slot's exact T.  wide: every
 // live row's pairs, without a look at the floats; a pair whose q is undefined or
-// +infinity is none, as in the reference's comparisons.
+// +infinity is none, as in the reference's comparisons.  A warp stops when visit
+// returns false (the same in the warp).  Every thread calls it.
 template <class Visit>
 __device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int rows, const double* tx, float nm2f,
                                double nm2, int watermark, float thr, bool wide, Visit&& visit) {
-  const int lane = threadIdx.x & 31;
-  for (int l = (int)threadIdx.x >> 5; l < rows; l += (int)blockDim.x >> 5) {
-    const int r = l * tm.size + tm.rank;
-    if (wide ? r >= s.n0 || m.node[r] < 0 : m.U[l] > thr) continue;
-    const int ur = m.node[r];
+  __shared__ int16_t s_rows[1024];
+  const int lane = threadIdx.x & 31, warp = (int)threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  int cnt = 0;   // the rows, counted by every warp for itself
+  for (int l0 = 0; l0 < rows; l0 += 32) {
+    const int l = l0 + lane, r = l * tm.size + tm.rank;
+    const bool in = l < rows && (wide ? r < s.n0 && m.node[r] >= 0 : m.U[l] <= thr);
+    const unsigned bal = __ballot_sync(0xffffffffu, in);
+    if (warp == 0 && in) s_rows[cnt + __popc(bal & ((1u << lane) - 1u))] = (int16_t)l;
+    cnt += __popc(bal);
+  }
+  __syncthreads();
+  if (cnt == 0) return;
+  int wpr = 1;   // few rows are split over the warps
+  while (2 * wpr * cnt <= nw) wpr *= 2;
+  const int per = nw / wpr, sub = warp % wpr, nv = s.ld >> 2;
+  if (warp / wpr >= per) return;
+  constexpr int kAhead = 2;   // 16-byte loads of a lane in flight
+  const float4* Tf4 = reinterpret_cast<const float4*>(m.Tf);
+  for (int k = warp / wpr; k < cnt; k += per) {
+    const int l = s_rows[k], r = l * tm.size + tm.rank, ur = m.node[r];
     const float tr = m.Tf[r];
     const double Tr = m.To[l];
-    const float* row = row_at(s, m.prow[r]);
-    for (int cb = r + 1; cb < s.n0; cb += 32) {
-      const int c = cb + lane;
-      bool pred = false;
-      KCand kc = kc_none();
-      if (c < s.n0 && m.node[c] >= 0) {
-        const float d = __ldcg(row + c);
-        if (wide || lazy_q(d, tr, m.Tf[c], nm2f) <= thr) {
-          const GCand cd = make_cand(r, c, ur, m.node[c], Tr, __ldcg(tx + c), d, nm2, watermark);
-          kc = KCand{cd.k1, cd.k2, cd.a, cd.b};
-          pred = !wide || cd.q1 < DBL_MAX;
+    const float4* row4 = reinterpret_cast<const float4*>(row_at(s, m.prow[r]));
+    for (int v0 = ((r + 1) >> 2) + 32 * sub; v0 < nv; v0 += 32 * wpr * kAhead) {
+      float4 d4[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int v = v0 + 32 * wpr * u + lane;
+        d4[u] = v < nv ? __ldcg(row4 + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int v = v0 + 32 * wpr * u + lane;
+        const float4 t4 = Tf4[min(v, nv - 1)];
+        const float d[4] = {d4[u].x, d4[u].y, d4[u].z, d4[u].w}, tc[4] = {t4.x, t4.y, t4.z, t4.w};
+        unsigned in = 0;   // the candidates among the four columns
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = 4 * v + e;   // q is NaN at dead and padding slots
+          const bool is = wide ? c < s.n0 && m.node[c] >= 0 : lazy_q(d[e], tr, tc[e], nm2f) <= thr;
+          if (v < nv && c > r && is) in |= 1u << e;
+        }
+        if (!__any_sync(0xffffffffu, in)) continue;
+        double Tc[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) Tc[e] = in >> e & 1 ? __ldcg(tx + 4 * v + e) : 0.0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          bool pred = in >> e & 1;
+          KCand kc = kc_none();
+          if (pred) {
+            const GCand cd = make_cand(r, 4 * v + e, ur, m.node[4 * v + e], Tr, Tc[e], d[e], nm2, watermark);
+            kc = kc_of(cd);
+            pred = !wide || cd.q1 < DBL_MAX;
+          }
+          if (!visit(pred, kc)) return;
         }
       }
-      visit(pred, kc);
     }
   }
 }
@@ -865,7 +909,7 @@ __device__ void lazy_cand_scan(const NJDev& s, const LazyMem& m, Team tm, int ro
 template <bool CL>
 __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m, Team tm, int rows,
                                const float4* parts, const double* tx, float thr, bool listed, bool wide, float nm2f,
-                               double nm2, int watermark, GCand* win, PickOut* pk, unsigned& target) {
+                               double nm2, int watermark, GCand* win, PickOut* pk, unsigned& picks, unsigned& target) {
   __shared__ GCand fc[32];
   const int lane = threadIdx.x & 31;
   if (listed) {   // at most 32 published pairs are all the candidates
@@ -893,21 +937,28 @@ __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m
     __syncthreads();
     return true;
   }
+  // the counts alternate between two sets: this pick's are zero, the last one's
+  // are read by nobody any more once every CTA is here
+  int* const cnt = s.g32 + 4 * (picks & 1);
+  int* const old = s.g32 + 4 * (picks + 1 & 1);
+  ++picks;
   KCand first = kc_none();
   bool full = false;
   lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, wide, [&](bool pred, const KCand& c) {
-    list_push(s, g, pred, c, full);
+    list_push(s, g, &cnt[2], pred, c, full);
     if (pred && kc_first(c, first)) first = c;
+    return true;
   });
   if (!team_sync<CL>(g, target)) return false;
+  if (tm.rank == 0 && threadIdx.x == 0) old[0] = old[1] = old[2] = 0;
   // the winner's pair again, as the scan read it (row = the smaller slot)
   auto rederive = [&](const KCand& w) {
-    const int sa = __ldcg(s.slot + w.a), sb = __ldcg(s.slot + w.b);
+    const int sa = slot_of(w.a), sb = slot_of(w.b);
     const int r0 = min(sa, sb), c0 = max(sa, sb);
     *win = make_cand(r0, c0, m.node[r0], m.node[c0], __ldcg(tx + r0), __ldcg(tx + c0),
                      __ldcg(row_at(s, m.prow[r0]) + c0), nm2, watermark);
   };
-  const int ncount = __ldcg(&s.g32[2]);   // the same in every CTA
+  const int ncount = __ldcg(&cnt[2]);   // the same in every CTA
   if (ncount <= min(s.cand_cap, kListPickMax)) {
     if (threadIdx.x < 32) {
       const PickOut r = pick_keys(ncount, [&](int k) { return ld_kcand(&g.cand[k]); });
@@ -930,21 +981,26 @@ __device__ bool lazy_pick_slow(const NJDev& s, const GridNJ& g, const LazyMem& m
     const KCand w = sfirst;
     unsigned ties = 0, amb = 0;
     lazy_cand_scan(s, m, tm, rows, tx, nm2f, nm2, watermark, thr, wide, [&](bool pred, const KCand& c) {
-      if (pred) count_vs(c, w, ties, amb);
+      // one ambiguous pair, or five ties, decide the step's statistics
+      unsigned t = 0, a = 0;
+      if (pred) count_vs(c, w, t, a);
+      ties += __popc(__ballot_sync(0xffffffffu, t));
+      amb |= __any_sync(0xffffffffu, a);
+      return ties <= 4 && !amb;
     });
-    add_counts(ties, amb, s.g32);
+    if (lane == 0 && (ties | amb)) {   // the warp's
+      atomicAdd(&cnt[0], (int)ties);
+      atomicAdd(&cnt[1], (int)amb);
+    }
     if (!team_sync<CL>(g, target)) return false;
     if (threadIdx.x == 0) {
       pk->idx = 0;
-      pk->ties = (unsigned)__ldcg(&s.g32[0]);
-      pk->amb = (unsigned)__ldcg(&s.g32[1]);
+      pk->ties = (unsigned)__ldcg(&cnt[0]);
+      pk->amb = (unsigned)__ldcg(&cnt[1]);
       pk->error = w.b < 0;
       if (!pk->error) rederive(w);
     }
   }
-  // every CTA has read the counts before they are reset for the next scan
-  if (!team_sync<CL>(g, target)) return false;
-  if (tm.rank == 0 && threadIdx.x == 0) s.g32[0] = s.g32[1] = s.g32[2] = 0;
   return true;
 }
 
@@ -1005,6 +1061,8 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
   __shared__ long long w_u[32];            // per warp: the join's integer sum,
   __shared__ long long w_u2[32], w_a2[32]; // the second sum and its values' magnitudes
   __shared__ int4 w_x[32];                 // largest dT (ordered), |T|, |tmp|, lowest exponent
+  unsigned picks = 0;                      // slow picks over the candidate scan so far
+  if (tm.rank == 0 && tid < 8) s.g32[tid] = 0;   // before the first exchange
   const int id0 = n + step0;               // ids from here on are made in this segment
   const int n_ord = __ldcg(s.na);
   int spare = __ldcg(s.prow + n0);         // the free place
@@ -1117,7 +1175,7 @@ __device__ bool lazy_segment(const NJDev& s, const GridNJ& g, Team tm, unsigned 
       sj = ur < uc ? c : r;
     } else {
       if (!lazy_pick_slow<CL>(s, g, m, tm, rows, parts, tx, thr, cands >= 1 && cands <= 32 && !wide, wide, nm2f, nm2,
-                              watermark, &swin, &spick, target))
+                              watermark, &swin, &spick, picks, target))
         return false;
       __syncthreads();
       if (spick.error) {   // the same in every CTA
@@ -1593,8 +1651,8 @@ __device__ void team_rowsums(const NJDev& s, const int* act, int w0, int wstride
   }
 }
 
-template <int C>
-__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kLazyThreads, 1) nj_cluster_kernel(const NJJob* jobs,
+template <int C, int Threads>
+__global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(Threads, 1) nj_cluster_kernel(const NJJob* jobs,
                                                                                               int njobs) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ NJJob sjob;   // the job's descriptor (shared memory keeps registers free)
@@ -1618,7 +1676,6 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kLazyThreads, 1) nj_
   for (int k = t0; k <= n; k += tstride) s.prow[k] = k;
   if (tm.rank == 0 && threadIdx.x == 0) {
     *s.na = n;
-    s.g32[0] = s.g32[1] = s.g32[2] = 0;
     s.stats[0] = s.stats[1] = s.stats[2] = s.stats[3] = s.stats[4] = 0;
   }
   cooperative_groups::this_cluster().sync();
@@ -1673,9 +1730,10 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kLazyThreads, 1) nj_
 // join share's block reduction is.  The arithmetic is that of the other forms.
 
 constexpr int kCtaNJMax = 160;       // at most: shared memory
-// Up to here the CTA is faster than a cluster, whose join costs the same at any
-// small size: 4.94 / 5.63 us a join (CTA / cluster) at 100 taxa, 5.43 / 5.62 at
-// 130, 6.21 / 5.54 at 160.
+// Up to here the CTA is faster than a cluster, whose join costs nearly the same at
+// any small size.  Whole-number distances, ms (CTA / cluster): 0.79 / 0.71 at 137
+// taxa, 0.88 / 0.77 at 150, 1.03 / 0.82 at 160; points on a line 0.72 / 0.74, 0.79 /
+// 0.80, 0.98 / 0.85.
 constexpr int kCtaNJDefault = 136;
 constexpr int kCtaThreads = 256;
 
@@ -1755,7 +1813,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
     act[k] = k;
   }
   if (tid == 0) {
-    s.g32[2] = 0;
     s.stats[0] = s.stats[1] = s.stats[2] = s.stats[3] = s.stats[4] = 0;
   }
   __syncthreads();
@@ -1887,10 +1944,11 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
       // fallback: the selected rows' pairs within the threshold, scanned
       // twice: the first candidate in the pick's order (block reduction),
       // then the ties and ambiguous pairs against it (pick_keys' rule)
-      auto scan = [&](auto&& visit) {
+      auto scan = [&](auto&& visit, auto&& go_on) {
         for (int r = 0; r < n; ++r) {
+          if (!(wide || grm[r] <= othr) || node[r] < 0) continue;
+          if (!go_on()) break;
           const int ur = node[r];
-          if (ur < 0 || !(wide || grm[r] <= othr)) continue;
           const float tr = Tf[r];
           const float* row = rows + (size_t)r * ldl;
           for (int c = r + 1 + tid; c < n; c += nth) {
@@ -1901,7 +1959,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
             if (!wide && !(q <= thr)) continue;
             const GCand cd = make_cand(r, c, ur, uc, T[r], T[c], d, nm2, watermark);
             if (wide && !(cd.q1 < DBL_MAX)) continue;
-            visit(KCand{cd.k1, cd.k2, cd.a, cd.b});
+            visit(kc_of(cd));
           }
         }
       };
@@ -1911,7 +1969,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
       KCand first = kc_none();
       scan([&](const KCand& c) {
         if (kc_first(c, first)) first = c;
-      });
+      }, [] { return true; });
       first = cta_first(first, skw);
       if (tid == 0) {
         sfirst = first;
@@ -1920,7 +1978,10 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
       __syncthreads();
       const KCand wk = sfirst;
       unsigned ties = 0, amb = 0;
-      if (wk.b >= 0) scan([&](const KCand& c) { count_vs(c, wk, ties, amb); });
+      // one ambiguous pair, or five ties, decide the step's statistics
+      if (wk.b >= 0)
+        scan([&](const KCand& c) { count_vs(c, wk, ties, amb); },
+             [&] { return !__any_sync(0xffffffffu, amb) && __popc(__ballot_sync(0xffffffffu, ties)) <= 4; });
       for (int o = 16; o > 0; o >>= 1) {
         ties += __shfl_xor_sync(0xffffffffu, ties, o);
         amb += __shfl_xor_sync(0xffffffffu, amb, o);
@@ -1937,7 +1998,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) nj_cta_kernel(const NJJob* job
         spick.error = wk.b < 0;
         if (!spick.error) {
           // the winner's pair again, as the scan read it (row = the smaller slot)
-          const int sa = slot[wk.a], sb = slot[wk.b];
+          const int sa = slot_of(wk.a), sb = slot_of(wk.b);
           const int r0 = min(sa, sb), c0 = max(sa, sb);
           swin = make_cand(r0, c0, node[r0], node[c0], T[r0], T[c0], rows[(size_t)r0 * ldl + c0], nm2, watermark);
         }
@@ -2058,8 +2119,8 @@ struct NJState {
 
 // Up to this many taxa one cluster runs the whole join loop; larger matrices
 // take the whole GPU.  A cluster's exchange is the cheaper one, the whole GPU
-// has fewer rows to rescan per CTA: 5.94 / 6.15 us a join (cluster / GPU) at 500
-// taxa, 6.18 / 6.12 at 600, 6.30 / 6.12 at 768, 7.19 / 6.32 at 1,100.  The
+// has fewer rows to rescan per CTA: 5.5 us a join in the cluster at 500 taxa, 5.8 at
+// 600, 6.2 on the whole GPU at 650 to 1,000.  The
 // environment variable NWG_NJ_CLUSTER_MAX_N overrides the threshold (both forms
 // give the same joins; the tests run each form on the same inputs).
 int cluster_nj_max_n() {
@@ -2112,7 +2173,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     if ((rc = cuda(cudaMemcpyAsync(S.desc.p, &J, sizeof(J), cudaMemcpyHostToDevice, s), "nj upload"))) return rc;
     if (st) cudaEventRecord(ev0, s);
     if ((rc = cuda(n <= cta_nj_max_n() ? launch_nj_cta(S.desc.p, 1, n, s)
-                                       : launch_nj_cluster(S.desc.p, 1, n, nj_cluster_size(), s),
+                                       : launch_nj_cluster(S.desc.p, 1, n, nj_cluster_size(), sms, s),
                    "nj launch")))
       return rc;
     ++launches;
@@ -2122,7 +2183,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     if ((rc = S.T.ensure(sizeof(double) * n)) || (rc = S.Tf.ensure(sizeof(float) * ldd)) ||
         (rc = S.slot.ensure(sizeof(int) * nn)) || (rc = S.node.ensure(sizeof(int) * n)) ||
         (rc = S.act.ensure(sizeof(int) * (n + 1))) || (rc = S.na.ensure(sizeof(int))) ||
-        (rc = S.g32.ensure(sizeof(int) * 4)) || (rc = S.stats.ensure(sizeof(unsigned long long) * 5)) ||
+        (rc = S.g32.ensure(sizeof(int) * 8)) || (rc = S.stats.ensure(sizeof(unsigned long long) * 5)) ||
         (rc = S.joins.ensure(sizeof(nwg_join) * (n - 1))) || (rc = S.cand.ensure(sizeof(KCand) * kCandCap)) ||
         (rc = S.cbest.ensure(sizeof(KCand) * grid)) || (rc = S.D2.ensure(sizeof(float) * (size_t)n * ldd)) ||
         (rc = S.T2.ensure(sizeof(double) * n)) || (rc = S.Tf2.ensure(sizeof(float) * ldd)) ||
@@ -2153,13 +2214,11 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     std::vector<int> slot0(nn, -1), act0(n + 1, n);   // act0: the identity, for the lists and maps
     for (int k = 0; k < n; ++k) slot0[k] = k, act0[k] = k;
     const int na0 = n;
-    const int g0[4] = {0, 0, 0, 0};
     if ((rc = cuda(cudaMemcpyAsync(S.slot.p, slot0.data(), sizeof(int) * nn, cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.node.p, act0.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.act.p, act0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.prow.p, act0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemcpyAsync(S.na.p, &na0, sizeof(int), cudaMemcpyHostToDevice, s), "nj upload")) ||
-        (rc = cuda(cudaMemcpyAsync(S.g32.p, g0, sizeof(g0), cudaMemcpyHostToDevice, s), "nj upload")) ||
         (rc = cuda(cudaMemsetAsync(S.stats.p, 0, sizeof(unsigned long long) * 5, s), "nj upload")) ||
         (rc = cuda(cudaStreamSynchronize(s), "nj upload")))   // the host vectors above are local
       return rc;
@@ -2229,7 +2288,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
       g.stall = step == 0 && inject && std::atoi(inject) == 1 ? 1 : 0;
       {
         int a0 = step, a1 = seg_end, an = n, aw = watermark;
-        const int threads = lazy_threads(d.ld, (d.n0 + grid - 1) / grid, grid);
+        const int threads = lazy_threads(d.ld, (d.n0 + grid - 1) / grid, grid, false);
         void* args[] = {&d, &g, &a0, &a1, &an, &aw};
         if ((rc = cuda(cudaLaunchCooperativeKernel((const void*)nj_lazy_grid_kernel, dim3(grid), dim3(threads), args,
                                                    (size_t)smem, s),
@@ -2320,7 +2379,7 @@ static size_t job_layout(int n, int ld, char* base, NJJob* J) {
   char* node = take(sizeof(int) * n);
   char* act = take(sizeof(int) * (n + 1));
   char* na = take(sizeof(int) * 4);
-  char* g32 = take(sizeof(int) * 4);
+  char* g32 = take(sizeof(int) * 8);
   char* stats = take(sizeof(unsigned long long) * 5);
   char* cand = take(sizeof(KCand) * cap);
   char* cbest = take(sizeof(KCand) * kC);
@@ -2368,23 +2427,21 @@ void nj_job_setup(void* job_out, float* D, int n, int ld, char* base, nwg_join**
 size_t nj_job_desc_bytes() { return sizeof(NJJob); }
 
 // One job per cluster of C CTAs (C = 8 or 16); nmax: the largest job.
-cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, cudaStream_t s) {
+cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, int sms, cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   const NJJob* jobs = reinterpret_cast<const NJJob*>(d_jobs);
   const int ld = nj_row_stride(nmax);
   const int bytes = (int)lazy_layout(nmax, ld, C).bytes;
-  const int rows = (nmax + C - 1) / C;
-  const int threads = lazy_threads(ld, rows, C);
+  const bool crowded = (int64_t)njobs * C > sms;
+  const int threads = lazy_threads(ld, (nmax + C - 1) / C, C, crowded);
+  const bool most = crowded || threads > kLazyThreads;
+  const auto fn = C == 16 ? (most ? nj_cluster_kernel<16, kLazyThreadsMax> : nj_cluster_kernel<16, kLazyThreads>)
+                          : (most ? nj_cluster_kernel<8, kLazyThreadsMax> : nj_cluster_kernel<8, kLazyThreads>);
   cudaError_t e;
-  if (C == 16) {
-    if ((e = cudaFuncSetAttribute(nj_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) ||
-        (e = cudaFuncSetAttribute(nj_cluster_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
-      return e;
-    nj_cluster_kernel<16><<<njobs * 16, threads, bytes, s>>>(jobs, njobs);
-  } else {
-    if ((e = cudaFuncSetAttribute(nj_cluster_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))) return e;
-    nj_cluster_kernel<8><<<njobs * 8, threads, bytes, s>>>(jobs, njobs);
-  }
+  if ((C == 16 && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) ||
+      (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return e;
+  fn<<<njobs * C, threads, bytes, s>>>(jobs, njobs);
   return cudaGetLastError();
 }
 
@@ -2412,11 +2469,11 @@ int nj_cluster_size() {
   static int best = 0;
   if (best) return best;
   best = 8;
-  const void* fn = (const void*)nj_cluster_kernel<16>;
+  const void* fn = (const void*)nj_cluster_kernel<16, kLazyThreads>;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(1024);
+    cfg.blockDim = dim3(kLazyThreads);
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = 16;
