@@ -4,8 +4,10 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "nwg_ctx.h"
@@ -258,6 +260,24 @@ int Ctx::score_all_dev(const int8_t* d_codes, const int64_t* offsets, int n, flo
     st->kernel_ms += ms;
   }
   return NWG_OK;
+}
+
+cudaError_t allow_smem(const void* fn) {
+  static std::mutex mu;
+  static std::vector<std::pair<int, const void*>> raised;   // (device, function)
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(mu);
+  const std::pair<int, const void*> key{dev, fn};
+  if (std::find(raised.begin(), raised.end(), key) != raised.end()) return cudaSuccess;
+  cudaFuncAttributes fa;
+  if ((e = cudaFuncGetAttributes(&fa, fn)) ||
+      (e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) ||
+      (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes)))
+    return e;
+  raised.push_back(key);
+  return cudaSuccess;
 }
 
 }  // namespace nwg

@@ -507,8 +507,7 @@ cudaError_t launch_msa_wave(const MergeDesc* md, int count, int warps, const int
   cfg.blockDim = dim3((unsigned)(32 * wpc));
   cfg.dynamicSmemBytes = sizeof(MsaScore::Ring) * wpc;
   cfg.stream = s;
-  const cudaError_t e = cudaFuncSetAttribute(msa_wave_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(MsaScore::Ring) * pipe::kWarps);
+  const cudaError_t e = allow_smem((const void*)msa_wave_kernel);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

@@ -2224,8 +2224,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
       return rc;
     const int smem = (int)lazy_layout(n, ldd, grid).bytes;   // the first segment's: later ones have fewer slots
     int blocks_per_sm = 0;
-    if ((rc = cuda(cudaFuncSetAttribute(nj_lazy_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                   "nj occupancy")) ||
+    if ((rc = cuda(allow_smem((const void*)nj_lazy_grid_kernel), "nj occupancy")) ||
         (rc = cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, nj_lazy_grid_kernel, kLazyThreads, smem),
                    "nj occupancy")))
       return rc;
@@ -2439,7 +2438,7 @@ cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, in
                           : (most ? nj_cluster_kernel<8, kLazyThreadsMax> : nj_cluster_kernel<8, kLazyThreads>);
   cudaError_t e;
   if ((C == 16 && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) ||
-      (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+      (e = allow_smem((const void*)fn)))
     return e;
   fn<<<njobs * C, threads, bytes, s>>>(jobs, njobs);
   return cudaGetLastError();
@@ -2458,7 +2457,7 @@ int cta_nj_max_n() {
 cudaError_t launch_nj_cta(const void* d_jobs, int njobs, int nmax, cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   const int bytes = (int)cta_layout(std::max(nmax, 2)).bytes;
-  cudaError_t e = cudaFuncSetAttribute(nj_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  const cudaError_t e = allow_smem((const void*)nj_cta_kernel);
   if (e != cudaSuccess) return e;
   nj_cta_kernel<<<njobs, kCtaThreads, bytes, s>>>(reinterpret_cast<const NJJob*>(d_jobs), njobs);
   return cudaGetLastError();

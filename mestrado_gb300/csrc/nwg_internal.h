@@ -161,6 +161,12 @@ inline bool residues_ok(const int8_t* codes, int64_t n) {
   return true;
 }
 
+// Lets fn's launches ask for all the dynamic shared memory that the device has
+// beside fn's static part.  The limit belongs to the function, not to a context or
+// a thread: set to what one call needs, another thread's smaller call takes it
+// away between the first one's setting and its launch.
+cudaError_t allow_smem(const void* fn);
+
 // Launchers (score_kernels.cu, wave_r*.cu).  R is the rows per lane; P = 2
 // for int16x2 lanes (two pairs per warp), 1 for int32 lanes.
 // V: register layout of the wave kernel (0: H, H-go, E per row; 1: H, E per

@@ -439,8 +439,7 @@ cudaError_t launch_pipe(const TraceArgs& a, int first, int count, int warps, int
   cfg.blockDim = dim3((unsigned)(32 * wpc));
   cfg.dynamicSmemBytes = trace_pipe_smem(wpc, lx_max);
   cfg.stream = s;
-  const cudaError_t e = cudaFuncSetAttribute(trace_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)trace_pipe_smem(pipe::kWarps, lx_max));
+  const cudaError_t e = allow_smem((const void*)trace_pipe_kernel);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
