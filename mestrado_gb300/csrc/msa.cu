@@ -13,16 +13,17 @@
 //
 // Device work per tree level (every merge whose children are done):
 //  1. msa_score_kernel: every cell's score, over the whole GPU;
-//  2. msa_wave_kernel, one CTA per merge: the recurrence as a wavefront of
+//  2. msa_wave_kernel, one cluster per merge: the recurrence as a wavefront of
 //     warps, then the walk over its flags;
 //  3. msa_build_kernel: the merged profile and, for both children, the map of
 //     their columns to the new ones.
-// Merges whose differences between neighbouring cells could leave 32 bits, and
-// gap models with open < extension, take msa_dp_kernel (64-bit cells) in
-// place of 1 and 2.
+// Merges whose differences between neighbouring cells could leave 32 bits or
+// whose scores find no memory, and gap models with open < extension, take
+// msa_dp_kernel (64-bit cells) in place of 1 and 2.
 // At the end the final position of every column is resolved parents first
 // (msa_pos_kernel) and every leaf's residues are scattered into its row.
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -670,6 +671,17 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
   constexpr int64_t kScoreMax = (int64_t)1 << 31;          // of one merge (8 GiB; beyond, the 64-bit form)
   std::vector<MergeDesc> md;
   std::vector<int32_t> nops;
+  // Cell scores that one merge may take.  Where there is no memory for a level's,
+  // its merges beyond a batch, then all, take the 64-bit form, which needs none.
+  int64_t score_max = kScoreMax;
+  // failure injection for the tests: more scores than this do not fit
+  const char* inject = std::getenv("NWG_MSA_INJECT_SCORE_OOM");
+  const int64_t score_room = inject ? std::atoll(inject) : INT64_MAX;
+  // batches of wave merges that share the score buffer (on one stream, so one after another)
+  struct Batch {
+    int first, count, tiles, warps;
+  };
+  std::vector<Batch> batches;
   for (int l = 1; l <= levels; ++l) {
     // wave-form merges first, most supersteps first; then the 64-bit ones
     std::vector<int>& nodes = bylevel[l];
@@ -681,75 +693,81 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
     };
     auto is_wave = [&](int v) {
       return go >= ge && (int64_t)kseq[left[v - n]] * kseq[right[v - n]] * diff_bound < ((int64_t)1 << 31) &&
-             padded(v) <= kScoreMax;
+             padded(v) <= score_max;
     };
-    const int nwave = (int)(std::stable_partition(nodes.begin(), nodes.end(), is_wave) - nodes.begin());
-    std::stable_sort(nodes.begin(), nodes.begin() + nwave, [&](int u, int v) {
-      const int64_t bu = (len[right[u - n]] + kBand - 1) / kBand, bv = (len[right[v - n]] + kBand - 1) / kBand;
-      return bu != bv ? bu > bv : len[left[u - n]] > len[left[v - n]];
-    });
-    md.assign(nm, MergeDesc{});
-    int64_t nib_total = 0, src_total = 0, scr_total = 0, score_cap = 0, bnd_total = 0;
-    // batches of wave merges that share the score buffer (on one stream, so one after another)
-    struct Batch {
-      int first, count, tiles, warps;
-    };
-    std::vector<Batch> batches;
-    int64_t score_used = 0;
-    int maxcols = 1;
-    for (int q = 0; q < nm; ++q) {
-      const int v = nodes[q], a = left[v - n], b = right[v - n];
-      MergeDesc& d = md[q];
-      d.xoff = col[a];
-      d.yoff = col[b];
-      d.lx = (int)len[a];
-      d.ly = (int)len[b];
-      d.kx = kseq[a];
-      d.ky = kseq[b];
-      d.mac32 = (int64_t)d.kx * d.ky * smax < ((int64_t)1 << 31) ? 1 : 0;
-      d.bytes = d.kx > 255 ? 0 : d.ky * smax <= 127 ? 1 : d.ky * smax <= 32767 ? 2 : 0;
-      d.xmap = col[a];
-      d.ymap = col[b];
-      d.ooff = pool;
-      col[v] = pool;
-      pool += len[a] + len[b];   // capacity; the walk's length is read back below
-      d.nib = nib_total;
-      d.src = src_total;
-      src_total += d.lx + d.ly;
-      maxcols = std::max(maxcols, d.lx + d.ly);
-      cells += (int64_t)d.lx * d.ly;
-      if (q < nwave) {
-        const int64_t bands = (d.ly + kBand - 1) / kBand, nsup = pipe::supersteps_of(d.lx);
-        const int64_t words = padded(v);
-        if (batches.empty() || score_used + words > kScoreBatch) {
-          batches.push_back({q, 0, 0, 1});
-          score_used = 0;
+    int nwave = 0, maxcols = 1;
+    const int64_t pool0 = pool, cells0 = cells;
+    for (;;) {
+      nwave = (int)(std::stable_partition(nodes.begin(), nodes.end(), is_wave) - nodes.begin());
+      std::stable_sort(nodes.begin(), nodes.begin() + nwave, [&](int u, int v) {
+        const int64_t bu = (len[right[u - n]] + kBand - 1) / kBand, bv = (len[right[v - n]] + kBand - 1) / kBand;
+        return bu != bv ? bu > bv : len[left[u - n]] > len[left[v - n]];
+      });
+      md.assign(nm, MergeDesc{});
+      batches.clear();
+      pool = pool0;
+      cells = cells0;
+      int64_t nib_total = 0, src_total = 0, scr_total = 0, score_cap = 0, score_used = 0, bnd_total = 0;
+      for (int q = 0; q < nm; ++q) {
+        const int v = nodes[q], a = left[v - n], b = right[v - n];
+        MergeDesc& d = md[q];
+        d.xoff = col[a];
+        d.yoff = col[b];
+        d.lx = (int)len[a];
+        d.ly = (int)len[b];
+        d.kx = kseq[a];
+        d.ky = kseq[b];
+        d.mac32 = (int64_t)d.kx * d.ky * smax < ((int64_t)1 << 31) ? 1 : 0;
+        d.bytes = d.kx > 255 ? 0 : d.ky * smax <= 127 ? 1 : d.ky * smax <= 32767 ? 2 : 0;
+        d.xmap = col[a];
+        d.ymap = col[b];
+        d.ooff = pool;
+        col[v] = pool;
+        pool += len[a] + len[b];   // capacity; the walk's length is read back below
+        d.nib = nib_total;
+        d.src = src_total;
+        src_total += d.lx + d.ly;
+        maxcols = std::max(maxcols, d.lx + d.ly);
+        cells += (int64_t)d.lx * d.ly;
+        if (q < nwave) {
+          const int64_t bands = (d.ly + kBand - 1) / kBand, nsup = pipe::supersteps_of(d.lx);
+          const int64_t words = padded(v);
+          if (batches.empty() || score_used + words > kScoreBatch) {
+            batches.push_back({q, 0, 0, 1});
+            score_used = 0;
+          }
+          Batch& bt = batches.back();
+          d.score = score_used;
+          score_used += words;
+          score_cap = std::max(score_cap, score_used);
+          d.tile0 = bt.tiles;
+          bt.tiles += (int)(bands * ((nsup * pipe::kStep + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps)));
+          bt.count += 1;
+          bt.warps = std::max(bt.warps, (int)std::min<int64_t>(bands, pipe::kWarps * pipe::kCluster));
+          d.bnd = bnd_total;
+          if (bands > pipe::kWarps * pipe::kCluster) bnd_total += d.lx;
+          nib_total += bands * nsup * 128 * kRows;
+        } else {
+          const int nstr = (d.ly + kMR - 1) / kMR;
+          nib_total += ((int64_t)nstr * (d.lx + kMR - 1) * kMR + 15) / 16 * 16;
+          d.scratch = scr_total;
+          scr_total += d.lx;
         }
-        Batch& bt = batches.back();
-        d.score = score_used;
-        score_used += words;
-        score_cap = std::max(score_cap, score_used);
-        d.tile0 = bt.tiles;
-        bt.tiles += (int)(bands * ((nsup * pipe::kStep + kScoreSteps * kScoreWarps - 1) / (kScoreSteps * kScoreWarps)));
-        bt.count += 1;
-        bt.warps = std::max(bt.warps, (int)std::min<int64_t>(bands, pipe::kWarps * pipe::kCluster));
-        d.bnd = bnd_total;
-        if (bands > pipe::kWarps * pipe::kCluster) bnd_total += d.lx;
-        nib_total += bands * nsup * 128 * kRows;
-      } else {
-        const int nstr = (d.ly + kMR - 1) / kMR;
-        nib_total += ((int64_t)nstr * (d.lx + kMR - 1) * kMR + 15) / 16 * 16;
-        d.scratch = scr_total;
-        scr_total += d.lx;
       }
+      rc = score_cap > score_room ? NWG_ERR_OOM : NWG_OK;
+      if (rc || (rc = M.nib.ensure((size_t)std::max<int64_t>(nib_total, 1))) ||
+          (rc = M.src.ensure(sizeof(int2) * (size_t)std::max<int64_t>(src_total, 1))) ||
+          (rc = M.scratch.ensure(sizeof(longlong2) * (size_t)std::max<int64_t>(scr_total, 1))) ||
+          (rc = M.bnd.ensure(sizeof(int2) * (size_t)std::max<int64_t>(bnd_total, 1))) ||
+          (rc = M.nops.ensure(sizeof(int32_t) * (2 * (size_t)nm + 1))) || (rc = M.md.ensure(sizeof(MergeDesc) * nm)) ||
+          (rc = M.score.ensure(sizeof(int) * (size_t)std::max<int64_t>(score_cap, 1)))) {
+        if (rc != NWG_ERR_OOM || score_max == 0) return fail(rc, "msa allocation");
+        M.score.release();
+        score_max = score_cap > kScoreBatch ? kScoreBatch : 0;
+        continue;
+      }
+      break;
     }
-    if ((rc = M.nib.ensure((size_t)std::max<int64_t>(nib_total, 1))) ||
-        (rc = M.src.ensure(sizeof(int2) * (size_t)std::max<int64_t>(src_total, 1))) ||
-        (rc = M.scratch.ensure(sizeof(longlong2) * (size_t)std::max<int64_t>(scr_total, 1))) ||
-        (rc = M.score.ensure(sizeof(int) * (size_t)std::max<int64_t>(score_cap, 1))) ||
-        (rc = M.bnd.ensure(sizeof(int2) * (size_t)std::max<int64_t>(bnd_total, 1))) ||
-        (rc = M.nops.ensure(sizeof(int32_t) * (2 * (size_t)nm + 1))) || (rc = M.md.ensure(sizeof(MergeDesc) * nm)))
-      return fail(rc, "msa allocation");
     if ((rc = cuda(cudaMemcpyAsync(M.md.p, md.data(), sizeof(MergeDesc) * nm, cudaMemcpyHostToDevice, s), "msa upload")))
       return rc;
     const MergeDesc* dmd = (const MergeDesc*)M.md.p;
@@ -817,6 +835,8 @@ int Ctx::msa(const int8_t* codes, const int64_t* offsets, int n, const int32_t* 
   ++launches;
   if (st) cudaEventRecord(ev1, s);
   if ((rc = cuda(cudaStreamSynchronize(s), "msa sync"))) return rc;
+  // scores beyond a batch's (one large merge) are not kept for the next call
+  if (M.score.cap > sizeof(int) * (size_t)kScoreBatch) M.score.release();
   M.n = n;
   M.L = L;
   *msa_len = L;
