@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -260,6 +261,11 @@ int Ctx::score_all_dev(const int8_t* d_codes, const int64_t* offsets, int n, flo
     st->kernel_ms += ms;
   }
   return NWG_OK;
+}
+
+int Ctx::injected_fork_error() {
+  const char* e = std::getenv("NWG_INJECT_FORK_ERROR");
+  return e && std::atoi(e) == 1 ? fail(NWG_ERR_CUDA, "injected error between fork and join") : NWG_OK;
 }
 
 cudaError_t allow_smem(const void* fn) {

@@ -252,6 +252,19 @@ struct Ctx {
           int64_t* msa_len, nwg_stats* st);
   int msa_rows(char* out, int64_t stride);
   int nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, nwg_nj_stats* st);
+  // Work forked from the stream to the branch streams: a call that returns before it
+  // has joined them waits for them here, since the next call reuses its buffers.
+  struct Fork {
+    Ctx& c;
+    bool joined = false;
+    ~Fork() {
+      if (!joined)
+        for (cudaStream_t b : c.branch) cudaStreamSynchronize(b);
+    }
+  };
+  // Failure injection for the tests (NWG_INJECT_FORK_ERROR=1): an error between the
+  // last launch on a branch stream and the join.
+  int injected_fork_error();
   int score_pairs(const int8_t* codes, const int64_t* offsets, int n, const int32_t* pi, const int32_t* pj,
                   int64_t npairs, int32_t* out, int64_t* pairs16);   // pairs.cu
   int trace_lanes_forced = 0;   // front width of the traceback kernel (0: chosen per call)

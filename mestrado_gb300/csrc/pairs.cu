@@ -521,6 +521,7 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
   a.sub = (const int8_t*)b_sub.p;
   // one launch's last jobs beside the next one's first
   const int sides = std::max(0, std::min(kinds_used - 1, (int)branch.size()));
+  Fork fork{*this, sides == 0};
   if (sides > 0 && (rc = cuda(cudaEventRecord(fork_ev, s), "pair-list streams"))) return rc;
   for (int k = 0; k < sides; ++k)
     if ((rc = cuda(cudaStreamWaitEvent(branch[k], fork_ev, 0), "pair-list streams"))) return rc;
@@ -542,10 +543,12 @@ int Ctx::score_pairs(const int8_t* codes, const int64_t* offsets, int n, const i
     if ((rc = cuda(cudaGetLastError(), "pair-list launch"))) return rc;
     ++launches;
   }
+  if (sides > 0 && (rc = injected_fork_error())) return rc;
   for (int k = 0; k < sides; ++k)
     if ((rc = cuda(cudaEventRecord(join_ev[k], branch[k]), "pair-list streams")) ||
         (rc = cuda(cudaStreamWaitEvent(s, join_ev[k], 0), "pair-list streams")))
       return rc;
+  fork.joined = true;
   if ((rc = cuda(cudaMemcpyAsync(out, b_out.p, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, s), "download")) ||
       (rc = cuda(cudaStreamSynchronize(s), "pair-list sync")))
     return rc;

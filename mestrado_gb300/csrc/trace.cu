@@ -489,6 +489,7 @@ static int launch_pipes(Ctx* c, const TraceArgs& a, const std::vector<int32_t>& 
     if (first[g + 1] - first[g] < c->sms) first[g] = first[g + 1];
   // the first non-empty group stays on the stream, the others fork from it
   if ((rc = c->cuda(cudaEventRecord(c->fork_ev, s), "fork"))) return rc;
+  Ctx::Fork fork{*c};
   int used = 0, b = -1;
   for (int g = 0; g < 3; ++g) {
     const int count = first[g + 1] - first[g];
@@ -505,8 +506,10 @@ static int launch_pipes(Ctx* c, const TraceArgs& a, const std::vector<int32_t>& 
     if (used++) ++c->launches;   // the caller counts the first
     ++b;
   }
+  if (b > 0 && (rc = c->injected_fork_error())) return rc;
   for (int k = 0; k < b; ++k)
     if ((rc = c->cuda(cudaStreamWaitEvent(s, c->join_ev[(size_t)k], 0), "join"))) return rc;
+  fork.joined = true;
   return NWG_OK;
 }
 
