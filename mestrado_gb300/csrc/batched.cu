@@ -196,21 +196,58 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   struct Group { int y, y2, nx, R, V, W, P, check; };
   std::vector<Group> groups;
   groups.reserve((size_t)Y.n / 2 + 1);
-  // A set that takes a fraction of the longest Y's chain runs on that Y's template
-  // throughout: one launch, and one kernel to load on its first use.
-  TuneChoice tc = c->choice_set(Y.len[0], X.maxlen, cells);
+  // A template per length pads least; a template per class makes fewer launches, each
+  // of which ends in a last wave that leaves SMs idle and loads its kernel on its
+  // first use in a process.  The estimate: the padded cells at the templates' rates
+  // and a fifth of the templates' longest chains.  700 sequences of median 300 and
+  // uneven lengths take 6.7 ms and 11.8 on the first call per class, 8.4 and 14.9 per
+  // length; 300 of median 500 2.8 and 7.6, 4.4 and 10.2; 1,500 in eight families of
+  // median 500 22.7 per class, 21.5 per length.
+  const auto plan_s = [&](bool fitted) {
+    struct Use {
+      TuneChoice t;
+      double chain;
+    };
+    std::vector<Use> uses;
+    double cols = 0.0, work = 0.0;
+    TuneChoice t{0, 0, 0};
+    for (int y = 0; y < Y.n; ++y) {
+      const int rows = Y.len[y];
+      if (triangle) cols += X.len[y];
+      if (y == 0 || rows != Y.len[y - 1]) {
+        t = c->choice_set(rows, X.maxlen, cells, fitted);
+        if (force32) t = int32_choice(t, c->plain7(longest));
+        const double chain = Ctx::chain_s(t, rows, X.maxlen);
+        auto u = std::find_if(uses.begin(), uses.end(),
+                              [&](const Use& v) { return v.t.R == t.R && v.t.V == t.V && v.t.W == t.W; });
+        if (u == uses.end()) uses.push_back({t, chain});
+        else u->chain = std::max(u->chain, chain);
+      }
+      work += (double)padded_rows(t, rows) * (triangle ? cols : xsum) / (force32 ? 4.5e12 : c->rate_of(t, rows));
+    }
+    for (const Use& u : uses) work += 0.2 * u.chain;
+    return work;
+  };
+  const bool fitted = cells > 1.0e12 || plan_s(true) <= plan_s(false);
+  TuneChoice tc = c->choice_set(Y.len[0], X.maxlen, cells, fitted);
   int tc_rows = Y.len[0];   // the rows of tc: groups of equal length share the choice
   double padded = 0.0, xcols = 0.0;
   for (int y = 0; y < Y.n; ++y) {
     if (triangle) xcols += X.len[y];
     padded += (double)padded_rows(tc, Y.len[y]) * (triangle ? xcols : xsum);
   }
-  const bool one = tc.V == 7 && padded / 7.0e12 < 0.25 * Ctx::chain_s(tc, Y.len[0], X.maxlen) &&
+  // A set whose padded rows at 7 TCUPS, the small templates' rate, take less than
+  // half the longest Y's chain runs on that Y's template throughout: one launch, and
+  // one kernel to load on its first use.  Uneven lengths, against several templates:
+  // 32 sequences of median 300 0.97 ms and 2.1 on the first call (1.17 and 5.3), 128
+  // 1.08 and 2.3 (1.47 and 5.7), 64 of median 700 2.9 and 4.5 (5.6 and 10.6), 8 of
+  // median 200 0.159 and 0.34 (0.148 and 1.65).
+  const bool one = tc.V == 7 && padded / 7.0e12 < 0.5 * Ctx::chain_s(tc, Y.len[0], X.maxlen) &&
                    !c->cands[tune_class(Y.len[0])].empty();
   for (int y = 0; y < Y.n;) {
     if (!one && Y.len[y] != tc_rows) {
       tc_rows = Y.len[y];
-      tc = c->choice_set(tc_rows, X.maxlen, cells);
+      tc = c->choice_set(tc_rows, X.maxlen, cells, fitted);
     }
     if (!force32 && rebase) {
       const int y2 = y + 1 < Y.n ? y + 1 : -1;

@@ -176,8 +176,15 @@ struct Ctx {
   static double chain_s(const TuneChoice& t, int rows, int cols) {   // seconds
     return padded_rows(t, rows) / (t.W * t.R) * (cols + t.W - 1) * (10.0 * t.R + 90.0) / 2.0e9;
   }
-  TuneChoice choice_set(int rows, int cols, double cells) const {
-    const TuneChoice t = choice(rows);
+  // fitted: the template that is the fastest for each length, else the class's first
+  // for all its Y.
+  double rate_of(const TuneChoice& t, int rows) const {   // cells/s over padded rows, about
+    for (const Cand& c : cands[tune_class(rows)])
+      if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) return c.rate;
+    return 9.0e12;
+  }
+  TuneChoice choice_set(int rows, int cols, double cells, bool fitted) const {
+    const TuneChoice t = fitted ? choice(rows) : allowed(tune[tune_class(rows)], rows);
     if (t.V != 7 || cands[tune_class(rows)].empty()) return t;
     constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // cells/s at 4, 8, 12, 16 rows
     const auto est = [&](const TuneChoice& c, double rate) {
@@ -185,9 +192,7 @@ struct Ctx {
       const double whole = cells * padded_rows(c, rows) / rows / rate;
       return std::max(chain, whole) + 0.25 * std::min(chain, whole);
     };
-    double rate = 9.0e12;
-    for (const Cand& c : cands[tune_class(rows)])
-      if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) rate = c.rate;
+    const double rate = rate_of(t, rows);
     // a set of many waves of jobs: the shortest chain would not show
     if (cells * padded_rows(t, rows) / rows / rate > 20.0 * chain_s(t, rows, cols)) return t;
     TuneChoice best = t;
