@@ -10,10 +10,11 @@
 //   F(r+1,c) = max(F, m - GD) - u(r,c-1),   E(r,c+1) = max(E, H - GD) - v(r-1,c)
 // -- the same comparisons as on the values themselves, so the same flags: 17
 // integer operations a cell, two of them on the way from a row's F to the next
-// row's (the F line uses GD >= 0: F - GD never beats F).  With GO >= GE, u and v
-// lie in [-GD, max S' + GD] (H >= F >= Hup - GD; a diagonal step gives
-// u = S' - v(r-1,c), an F step u <= 0, an E step no more than the cell where its
-// gap opened), and everything else within 2 max|S| + 4 GO.
+// row's (the F line uses GD >= 0: F - GD never beats F).  Difference recurrences
+// for affine gaps are published (Suzuki and Kasahara, BMC Bioinformatics 19:45,
+// 2018).  With GO >= GE, u and v lie in [-GD, max S' + GD] (H >= F >= Hup - GD; a
+// diagonal step gives u = S' - v(r-1,c), an F step u <= 0, an E step no more than
+// the cell where its gap opened), and everything else within 2 max|S| + 4 GO.
 //
 // A band is 32 R rows, R per lane of a warp, lane l one column behind lane
 // l - 1.  Consecutive bands run on consecutive warps, four to a CTA (one per
@@ -181,7 +182,7 @@ struct Rows {
 template <int R, class Score>
 __device__ void run_bands(Link& ln, const Wrap& wrap, Score& score, uint32_t* __restrict__ flags, int lx, int ly,
                           int GD, int gw, int nwarp) {
-  static_assert(R == 4 || R == 8, "rows per lane");
+  static_assert(R == 4, "a superstep's bits of one kind are one word");
   const int lane = threadIdx.x & 31;
   const int nb = (ly + 32 * R - 1) / (32 * R);
   const int nst = stages_of(lx), nsup = supersteps_of(lx);
@@ -249,8 +250,7 @@ __device__ void run_bands(Link& ln, const Wrap& wrap, Score& score, uint32_t* __
           if (j * kStep + i < lx) in[i] = __ldcg(wrap.row + j * kStep + i);
       }
       score.begin(j, ln);
-      constexpr int kAcc = R / 4;   // words per kind
-      uint32_t acc[4][kAcc] = {};
+      uint32_t acc[4] = {};   // a word per kind
       int op[kStep], of[kStep];
 #pragma unroll
       for (int i = 0; i < kStep; ++i) {
@@ -270,12 +270,11 @@ __device__ void run_bands(Link& ln, const Wrap& wrap, Score& score, uint32_t* __
           const int m = max(E, s[r]);
           const int h = max(F, m);
           const int hg = h - GD;
-          const int q = (i * R + r) >> 5;
           // sign bits: H != S', F < E, no continue up, no continue left
-          acc[0][q] = __funnelshift_l((uint32_t)(s[r] - h), acc[0][q], 1);
-          acc[1][q] = __funnelshift_l((uint32_t)(F - E), acc[1][q], 1);
-          acc[2][q] = __funnelshift_l((uint32_t)ncu, acc[2][q], 1);
-          acc[3][q] = __funnelshift_l((uint32_t)st.cl[r], acc[3][q], 1);
+          acc[0] = __funnelshift_l((uint32_t)(s[r] - h), acc[0], 1);
+          acc[1] = __funnelshift_l((uint32_t)(F - E), acc[1], 1);
+          acc[2] = __funnelshift_l((uint32_t)ncu, acc[2], 1);
+          acc[3] = __funnelshift_l((uint32_t)st.cl[r], acc[3], 1);
           ncu = F - hg;                                     // the row below
           st.cl[r] = E - hg;                                // the next column
           st.e[r] = max(E, hg) - vU;
@@ -288,12 +287,7 @@ __device__ void run_bands(Link& ln, const Wrap& wrap, Score& score, uint32_t* __
         score.column_done(t, st.n);
       }
       uint32_t* fw = flags + (((int64_t)g * nsup + j) * 32 + lane) * R;
-      if constexpr (R == 4) {
-        *reinterpret_cast<uint4*>(fw) = make_uint4(acc[0][0], acc[1][0], acc[2][0], acc[3][0]);
-      } else {
-        *reinterpret_cast<uint4*>(fw) = make_uint4(acc[0][0], acc[0][kAcc - 1], acc[1][0], acc[1][kAcc - 1]);
-        *reinterpret_cast<uint4*>(fw + 4) = make_uint4(acc[2][0], acc[2][kAcc - 1], acc[3][0], acc[3][kAcc - 1]);
-      }
+      *reinterpret_cast<uint4*>(fw) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
       score.end(j);
       if (got) give_back();
       if (to_next && j >= 3) {
