@@ -1,14 +1,15 @@
 // pairs.cu -- scores of an explicit pair list (nwg_score_pairs).
 //
-// pair_wave_kernel<R, P>: one warp per job, a job being P pairs in the halves
-// of every register (P = 2, int16x2 lanes: the pairs that provably stay inside
-// 16 bits) or one pair on int32 lanes (P = 1).  The warp is a wavefront: lane k
-// owns rows [kR, kR + R) of a band of 32R rows, one column behind lane k - 1,
-// in the register layout that carries T = H - go (layout 3 of wave_impl.cuh:
-// three DPX operations and two adds per word).  Unlike the all-pairs form, no
-// two pairs share a Y, so there is no profile to share: each warp builds its
+// One warp per job, a job being P pairs in the halves of every register (P = 2,
+// int16x2 lanes: the pairs that provably stay inside 16 bits) or one pair on
+// int32 lanes (P = 1).  The warp is a wavefront: lane k owns rows [kR, kR + R) of
+// a band of 32R rows, one column behind lane k - 1.  Unlike the all-pairs form,
+// no two pairs share a Y, so there is no profile to share: each warp builds its
 // own, one byte per (letter, row), with its scores made non-negative by a bias
-// so that one byte permute yields the word of both pairs.
+// so that one byte permute yields the word of both pairs.  pair7_kernel runs the
+// recurrence with the extension cost taken out (layout 7 of wave_impl.cuh);
+// pair_wave_kernel, on layout 3 (T = H - go, one add more per word), serves the
+// gap models and matrices that layout 7 does not hold.
 // Bound by integer issue and the latency of a step (two shuffles, the profile's
 // loads, two dependent maxima per row) at 10 to 16 warps per SM, which the
 // profiles' shared memory allows.  20,000 pairs of about 245 residues, the whole
