@@ -203,7 +203,11 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
   // uneven lengths take 6.7 ms and 11.8 on the first call per class, 8.4 and 14.9 per
   // length; 300 of median 500 2.8 and 7.6, 4.4 and 10.2; 1,500 in eight families of
   // median 500 22.7 per class, 21.5 per length.
-  const auto plan_s = [&](bool fitted) {
+  struct PlanCost {
+    double s;
+    int templates;
+  };
+  const auto plan_cost = [&](bool fitted) -> PlanCost {
     struct Use {
       TuneChoice t;
       double chain;
@@ -226,9 +230,15 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
       work += (double)padded_rows(t, rows) * (triangle ? cols : xsum) / (force32 ? 4.5e12 : c->rate_of(t, rows));
     }
     for (const Use& u : uses) work += 0.2 * u.chain;
-    return work;
+    return {work, (int)uses.size()};
   };
-  const bool fitted = cells > 1.0e12 || plan_s(true) <= plan_s(false);
+  PlanCost cost = plan_cost(true);
+  bool fitted = true;
+  if (cells <= 1.0e12) {
+    const PlanCost by_class = plan_cost(false);
+    fitted = cost.s <= 1.05 * by_class.s;   // alike: the one that pads least
+    if (!fitted) cost = by_class;
+  }
   TuneChoice tc = c->choice_set(Y.len[0], X.maxlen, cells, fitted);
   int tc_rows = Y.len[0];   // the rows of tc: groups of equal length share the choice
   double padded = 0.0, xcols = 0.0;
@@ -236,13 +246,14 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
     if (triangle) xcols += X.len[y];
     padded += (double)padded_rows(tc, Y.len[y]) * (triangle ? xcols : xsum);
   }
-  // A set whose padded rows at 7 TCUPS, the small templates' rate, take less than
-  // half the longest Y's chain runs on that Y's template throughout: one launch, and
-  // one kernel to load on its first use.  Uneven lengths, against several templates:
-  // 32 sequences of median 300 0.97 ms and 2.1 on the first call (1.17 and 5.3), 128
+  // A set whose padded rows at 7 TCUPS, the small templates' rate, take a fraction of
+  // the longest Y's chain runs on that Y's template throughout: one launch, and one
+  // kernel to load on its first use.  Uneven lengths, against several templates: 32
+  // sequences of median 300 0.97 ms and 2.1 on the first call (1.17 and 5.3), 128
   // 1.08 and 2.3 (1.47 and 5.7), 64 of median 700 2.9 and 4.5 (5.6 and 10.6), 8 of
-  // median 200 0.159 and 0.34 (0.148 and 1.65).
-  const bool one = tc.V == 7 && padded / 7.0e12 < 0.5 * Ctx::chain_s(tc, Y.len[0], X.maxlen) &&
+  // median 200 0.159 and 0.34 (0.148 and 1.65).  In place of two or three templates
+  // only below a quarter: 32 alike of 346 to 389 residues 0.124 ms, 0.113 on two.
+  const bool one = tc.V == 7 && padded / 7.0e12 < (cost.templates > 3 ? 0.5 : 0.25) * Ctx::chain_s(tc, Y.len[0], X.maxlen) &&
                    !c->cands[tune_class(Y.len[0])].empty();
   for (int y = 0; y < Y.n;) {
     if (!one && Y.len[y] != tc_rows) {

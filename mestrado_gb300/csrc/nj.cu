@@ -549,10 +549,11 @@ __device__ __forceinline__ void usum_warp(USum& x) {
 // are all the candidates.  Otherwise the CTAs scan their rows within the
 // threshold into the candidate list.
 // Threads per CTA, at most.  A thread per own row, so 512 do for 16 CTAs or more
-// and for 8 up to 4,096 taxa, with 128 registers.  Bounded at 1,024 the kernels
-// have 64 registers and spill in the candidate scan (400 taxa: 2.5 instead of 2.2
-// ms), but four CTAs of 256 threads fit an SM: for launches of more clusters than
-// the SMs hold one by one (100 jobs of 140 to 300 taxa: 14.8 instead of 24.7 ms).
+// and for 8 up to 4,096 taxa, with 128 registers: one CTA of 512 threads an SM, two
+// of 256.  Bounded at 1,024 the kernels have 64 registers and spill in the candidate
+// scan (400 taxa: 2.5 instead of 2.2 ms), but four CTAs of 256 threads fit an SM:
+// for launches of more clusters than that (100 jobs of 140 to 300 taxa: 14.8 instead
+// of 24.7 ms).
 constexpr int kLazyThreads = 512, kLazyThreadsMax = 1024;
 constexpr int kLazyMaxCtas = 160;         // team size, at most
 // From kCompactN slots on, the matrix is also compacted whenever one in
@@ -589,10 +590,12 @@ __host__ __device__ inline LazyLayout lazy_layout(int n0, int ld, int size) {
 // Threads per CTA, between 256 and 512 (more make every CTA barrier dearer than
 // their loads in flight save), at least one per own row and per CTA of the team, a
 // multiple of 32: one per four slots over the whole GPU, one per slot in a
-// cluster with its SMs to itself, whose CTAs have more rows to scan (500 taxa that tie within rounding:
-// 4.7 ms instead of 5.0, with distances of 1 to 999 2.73 instead of 2.82).
-inline int lazy_threads(int ld, int rows, int size, bool crowded) {
-  const int want = size <= 16 && !crowded ? ld : ld / 4;
+// cluster with the GPU to itself, whose CTAs have more rows to scan (500 taxa that tie within rounding:
+// 4.7 ms instead of 5.0, with distances of 1 to 999 2.73 instead of 2.82).  The
+// serving loop's batches share the GPU: 16 jobs of up to 512 taxa 12.2 ms, 12.8 with
+// the wide form where a batch is small.
+inline int lazy_threads(int ld, int rows, int size, bool alone) {
+  const int want = size <= 16 && alone ? ld : ld / 4;
   const int t = std::max(std::max(std::min(std::max(want, 256), 512), rows), size);
   return (t + 31) / 32 * 32;
 }
@@ -2173,7 +2176,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
     if ((rc = cuda(cudaMemcpyAsync(S.desc.p, &J, sizeof(J), cudaMemcpyHostToDevice, s), "nj upload"))) return rc;
     if (st) cudaEventRecord(ev0, s);
     if ((rc = cuda(n <= cta_nj_max_n() ? launch_nj_cta(S.desc.p, 1, n, s)
-                                       : launch_nj_cluster(S.desc.p, 1, n, nj_cluster_size(), sms, s),
+                                       : launch_nj_cluster(S.desc.p, 1, n, nj_cluster_size(), sms, true, s),
                    "nj launch")))
       return rc;
     ++launches;
@@ -2287,7 +2290,7 @@ int Ctx::nj(const float* D, int64_t ld, int n, bool device_D, nwg_join* joins, n
       g.stall = step == 0 && inject && std::atoi(inject) == 1 ? 1 : 0;
       {
         int a0 = step, a1 = seg_end, an = n, aw = watermark;
-        const int threads = lazy_threads(d.ld, (d.n0 + grid - 1) / grid, grid, false);
+        const int threads = lazy_threads(d.ld, (d.n0 + grid - 1) / grid, grid, true);
         void* args[] = {&d, &g, &a0, &a1, &an, &aw};
         if ((rc = cuda(cudaLaunchCooperativeKernel((const void*)nj_lazy_grid_kernel, dim3(grid), dim3(threads), args,
                                                    (size_t)smem, s),
@@ -2425,15 +2428,15 @@ void nj_job_setup(void* job_out, float* D, int n, int ld, char* base, nwg_join**
 
 size_t nj_job_desc_bytes() { return sizeof(NJJob); }
 
-// One job per cluster of C CTAs (C = 8 or 16); nmax: the largest job.
-cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, int sms, cudaStream_t s) {
+// One job per cluster of C CTAs (C = 8 or 16); nmax: the largest job; alone: no other
+// launch shares the SMs.
+cudaError_t launch_nj_cluster(const void* d_jobs, int njobs, int nmax, int C, int sms, bool alone, cudaStream_t s) {
   if (njobs <= 0) return cudaSuccess;
   const NJJob* jobs = reinterpret_cast<const NJJob*>(d_jobs);
   const int ld = nj_row_stride(nmax);
   const int bytes = (int)lazy_layout(nmax, ld, C).bytes;
-  const bool crowded = (int64_t)njobs * C > sms;
-  const int threads = lazy_threads(ld, (nmax + C - 1) / C, C, crowded);
-  const bool most = crowded || threads > kLazyThreads;
+  const int threads = lazy_threads(ld, (nmax + C - 1) / C, C, alone);
+  const bool most = (int64_t)njobs * C > 2 * (int64_t)sms || threads > kLazyThreads;
   const auto fn = C == 16 ? (most ? nj_cluster_kernel<16, kLazyThreadsMax> : nj_cluster_kernel<16, kLazyThreads>)
                           : (most ? nj_cluster_kernel<8, kLazyThreadsMax> : nj_cluster_kernel<8, kLazyThreads>);
   cudaError_t e;

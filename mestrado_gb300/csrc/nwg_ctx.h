@@ -181,12 +181,12 @@ struct Ctx {
   double rate_of(const TuneChoice& t, int rows) const {   // cells/s over padded rows, about
     for (const Cand& c : cands[tune_class(rows)])
       if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) return c.rate;
-    return 9.0e12;
+    constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // at 4, 8, 12, 16 rows, measured
+    return t.R < 20 ? kSlow[t.R / 4 - 1] : 9.0e12;
   }
   TuneChoice choice_set(int rows, int cols, double cells, bool fitted) const {
     const TuneChoice t = fitted ? choice(rows) : allowed(tune[tune_class(rows)], rows);
     if (t.V != 7 || cands[tune_class(rows)].empty()) return t;
-    constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // cells/s at 4, 8, 12, 16 rows
     const auto est = [&](const TuneChoice& c, double rate) {
       const double chain = chain_s(c, rows, cols);
       const double whole = cells * padded_rows(c, rows) / rows / rate;
@@ -200,7 +200,7 @@ struct Ctx {
     for (int W : {8, 32})   // few templates: the first use of each in a process loads it (0.5 to 1 ms)
       for (int R : {4, 8, 12, 16, 24, 32}) {
         const TuneChoice c{R, 7, W};
-        const double e = est(c, R < 20 ? kSlow[R / 4 - 1] : 9.0e12);
+        const double e = est(c, rate_of(c, rows));
         if (e < best_est) {
           best_est = e;
           best = c;

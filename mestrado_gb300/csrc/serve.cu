@@ -387,7 +387,8 @@ int Server::launch_batch(Slot& S) {
     return rc;
   if (cnt_g[1]) {
     const int csize = nmax_g[1] >= kNJWideN ? nj_cluster_size() : kNJClusterServe;
-    if ((rc = c.cuda(launch_nj_cluster((const char*)S.njdesc.p + desc * cnt_g[0], cnt_g[1], nmax_g[1], csize, c.sms, st),
+    if ((rc = c.cuda(launch_nj_cluster((const char*)S.njdesc.p + desc * cnt_g[0], cnt_g[1], nmax_g[1], csize, c.sms, false,
+                                       st),
                      "serve nj launch")))
       return rc;
   }
