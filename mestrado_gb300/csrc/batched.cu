@@ -213,21 +213,25 @@ static int get_plan(Ctx* c, const int64_t* xoff, int nx, const int64_t* yoff, in
       double chain;
     };
     std::vector<Use> uses;
-    double cols = 0.0, work = 0.0;
+    double cols = 0.0, work = 0.0, rate = 1.0;
     TuneChoice t{0, 0, 0};
     for (int y = 0; y < Y.n; ++y) {
       const int rows = Y.len[y];
       if (triangle) cols += X.len[y];
       if (y == 0 || rows != Y.len[y - 1]) {
         t = c->choice_set(rows, X.maxlen, cells, fitted);
-        if (force32) t = int32_choice(t, c->plain7(longest));
+        rate = c->rate_of(t, rows);
+        if (force32) {
+          t = int32_choice(t, c->plain7(longest));
+          rate = 4.5e12;
+        }
         const double chain = Ctx::chain_s(t, rows, X.maxlen);
         auto u = std::find_if(uses.begin(), uses.end(),
                               [&](const Use& v) { return v.t.R == t.R && v.t.V == t.V && v.t.W == t.W; });
         if (u == uses.end()) uses.push_back({t, chain});
         else u->chain = std::max(u->chain, chain);
       }
-      work += (double)padded_rows(t, rows) * (triangle ? cols : xsum) / (force32 ? 4.5e12 : c->rate_of(t, rows));
+      work += (double)padded_rows(t, rows) * (triangle ? cols : xsum) / rate;
     }
     for (const Use& u : uses) work += 0.2 * u.chain;
     return {work, (int)uses.size()};

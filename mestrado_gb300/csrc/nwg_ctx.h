@@ -181,8 +181,11 @@ struct Ctx {
   double rate_of(const TuneChoice& t, int rows) const {   // cells/s over padded rows, about
     for (const Cand& c : cands[tune_class(rows)])
       if (c.t.R == t.R && c.t.V == t.V && c.t.W == t.W) return c.rate;
-    constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // at 4, 8, 12, 16 rows, measured
-    return t.R < 20 ? kSlow[t.R / 4 - 1] : 9.0e12;
+    return small_rate(t.R);
+  }
+  static double small_rate(int R) {   // the wavefronts of few rows per lane, measured
+    constexpr double kSlow[] = {4.2e12, 6.5e12, 7.9e12, 8.4e12};   // at 4, 8, 12, 16 rows
+    return R < 20 ? kSlow[R / 4 - 1] : 9.0e12;
   }
   TuneChoice choice_set(int rows, int cols, double cells, bool fitted) const {
     const TuneChoice t = fitted ? choice(rows) : allowed(tune[tune_class(rows)], rows);
@@ -200,7 +203,7 @@ struct Ctx {
     for (int W : {8, 32})   // few templates: the first use of each in a process loads it (0.5 to 1 ms)
       for (int R : {4, 8, 12, 16, 24, 32}) {
         const TuneChoice c{R, 7, W};
-        const double e = est(c, rate_of(c, rows));
+        const double e = est(c, small_rate(R));
         if (e < best_est) {
           best_est = e;
           best = c;
